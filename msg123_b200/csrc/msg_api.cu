@@ -890,6 +890,7 @@ int msg_gpu_precond(msg_ctx_t *c, const double *r, double *z) {
   UPLOAD(c->tmpv, r, N * 8);
   if ((rc = apply_prec(c, c->tmpv, c->z))) return rc;
   MSG_CUDA(cudaStreamSynchronize(c->stream));
+  if ((rc = wave_check(c))) return rc;
   MSG_CUDA(cudaMemcpy(z, c->z, N * 8, cudaMemcpyDeviceToHost));
   return MSG_OK;
 }
@@ -1270,9 +1271,10 @@ static void free_ctx(msg_ctx *c) {
                 c->left_off, c->right_off, c->hydf_conn, c->abyd_conn, c->head_new, c->head_old, c->head_pre,
                 c->head_change, c->srat_new, c->srat_old, c->surf_head, c->surf_old, c->new_f, c->kr, c->kr_per,
                 c->alp, c->sto, c->stod, c->tmpv, c->dmat, c->lu, c->rhs, c->rhs_alt, c->head_old2, c->slope_rhs, c->dilu_d, c->r, c->rs,
-                c->p, c->v, c->t, c->z, c->part, c->plane_ptr, c->plane_cells, c->dmat_f, c->lu_f, c->dres};
+                c->p, c->v, c->t, c->z, c->part, c->wave_order, c->wave_ticket, c->wave_slots, c->dmat_f, c->lu_f, c->dres};
   for (auto q : dp) if (q) cudaFree(q);
   if (c->hpin) cudaFreeHost(c->hpin);
+  if (c->wave_err) cudaFreeHost(c->wave_err);
   for (int k = 0; k < 8; ++k) if (c->ev[k]) cudaEventDestroy(c->ev[k]);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;

@@ -64,9 +64,12 @@ struct msg_ctx {
   size_t npart;
   double *hpin;                                  // pinned host scalars
   double *dres;                                  // device reduction results [16]
-  // ---- wavefront ordering for DILU --------------------------------------------------------
-  int *plane_ptr, *plane_cells;
-  int nplanes;
+  // ---- DILU sweeps (msg_linear.cu): tile order, ticket counter, hand-over slots between tiles
+  int *wave_order;
+  unsigned *wave_ticket, wave_sweeps;            // ticket and error word; sweeps launched so far
+  void *wave_slots;
+  int wave_tiles;
+  int *wave_err;                                 // pinned: a wait between tiles ran out
   // ---- AMG ----------------------------------------------------------------------------------
   void *amg;                                     // msg::AmgState (msg_amg.cu)
   int amg_nlevel, amg_age, amg_force;
@@ -119,6 +122,7 @@ int flux_parts(const msg_ctx *c);   // F^2 partials the assembly pass writes (on
 
 // ---- msg_linear.cu ----------------------------------------------------------------------------
 int build_wavefront(msg_ctx *c);
+int wave_check(msg_ctx *c);   // after a host wait: whether a sweep gave up a wait between tiles
 int launch_precon_dilu(msg_ctx *c);
 int launch_solve_ilu(msg_ctx *c, const double *b, double *x);
 int launch_spmv(msg_ctx *c, const double *x, double *y);

@@ -1,4 +1,4 @@
-// msg_linear.cu -- stencil SpMV, DILU / ILU(0) by hyperplane wavefront, BiCGStab with
+// msg_linear.cu -- stencil SpMV, DILU / ILU(0) by pipelined tile sweeps, BiCGStab with
 // fused dot products, deterministic reductions and scans (B200, sm_100a).
 //
 // SpMV and the vector updates stream the DIA arrays (d, six off-diagonals) once per
@@ -6,11 +6,9 @@
 // partial per block and a fixed-order second stage (k_finish) sums them, so every
 // dot product repeats bit for bit from run to run.
 #include "msg_ctx.cuh"
-#include <cooperative_groups.h>
+#include <algorithm>
 #include <vector>
 #include <cmath>
-
-namespace cg = cooperative_groups;
 
 namespace msg {
 
@@ -287,7 +285,7 @@ __global__ void __launch_bounds__(256) k_lamlen(int n, const double *dh, const d
 static int fetch_partials(msg_ctx *c, int count) {
   MSG_CUDA(cudaMemcpyAsync(c->hpin, c->part, (size_t)count * 8, cudaMemcpyDeviceToHost, c->stream));
   MSG_CUDA(cudaStreamSynchronize(c->stream));
-  return MSG_OK;
+  return wave_check(c);
 }
 
 // Second reduction stage: block a sums part[a*nparts .. a*nparts + nparts) in a fixed
@@ -337,7 +335,7 @@ int fetch_res(msg_ctx *c, int count, double *out) {
   MSG_CUDA(cudaMemcpyAsync(c->hpin, c->dres, (size_t)count * 8, cudaMemcpyDeviceToHost, c->stream));
   MSG_CUDA(cudaStreamSynchronize(c->stream));
   for (int a = 0; a < count; ++a) out[a] = c->hpin[a];
-  return MSG_OK;
+  return wave_check(c);
 }
 
 int finish(msg_ctx *c, int nparts, int narr, double *out) {
@@ -453,129 +451,303 @@ int scale(msg_ctx *c, double *y, double a, int n) {
 }
 
 // ---------------------------------------------------------------------------------
-// DILU / ILU(0) by hyperplane wavefront.  In natural order on the 7-point stencil
-// the lower neighbours of cell (ix,iy,iz) are (ix-1,..), (..,iy-1,..), (..,iz-1), so
-// every cell of the plane ix+iy+iz = p depends only on plane p-1: processing planes
-// in order, cells of one plane in parallel, performs exactly the sequential
-// arithmetic of precon_dilu / solve_ilu (Linear_solution.f90:742-782, :803-855).
+// DILU / ILU(0) (precon_dilu / solve_ilu, Linear_solution.f90:742-782, :803-855).  In
+// natural order on the 7-point stencil cell (ix,iy,iz) depends on (ix-1,..), (..,iy-1,..)
+// and (..,iz-1) only, so cells in any order that respects this perform exactly the
+// sequential arithmetic.
+//
+// What bounds it is the chain of nx+ny+nz-2 dependent cells, so everything but that chain is
+// kept off the threads that walk it.  A block owns a kWX x kWY tile of columns, a thread one
+// column; at step s it takes its layer z = s - lx - ly.  The upper neighbour is the thread's
+// own last value (a register), the west and north ones come through shared memory, one
+// block barrier per step.  As many warps again copy the coefficients ahead (cp.async, eight
+// neighbouring cells of a row side by side) into a ring of layers, and one warp brings in
+// the columns of the tiles to the west and north.  Those cross through a slot per
+// value in global memory: an empty slot holds a signalling NaN, which no arithmetic result
+// is, so the value is its own flag and needs no fence; the reader empties it again for the
+// next sweep.  Blocks take their tiles from a counter in an order in which a tile follows
+// the two that it waits for, so they progress however many of them are resident; a wait
+// that lasts 1 s is given up and reported, and the sweep ends with wrong values.
+//
+// 96 x 81 x 40 cells: factor 1390 -> 134 us, solve 2000 -> 226 us against a grid-wide barrier
+// per plane of cells (4.6 to 6.5 us each); 20 x 20 x 50: 165 -> 40 and 195 -> 83 us against
+// one block for the grid, whose scattered loads took 1.1 to 1.9 us per plane.  A step is now
+// about 250 ns (the division 66 of them), a hop from tile to tile about 1 us; looking at a
+// slot more than one step ahead (kWAhead) only lengthens the lag between tiles (267 us per
+// solve at 4, 230 at 2, 214 at 1).
 // ---------------------------------------------------------------------------------
-int build_wavefront(msg_ctx *c) {
-  int nx = c->nx, ny = c->ny, nz = c->nz;
-  int np = nx + ny + nz - 2;
-  std::vector<int> ptr(np + 1, 0), cells(c->N);
-  for (int iz = 0; iz < nz; ++iz)
-    for (int iy = 0; iy < ny; ++iy)
-      for (int ix = 0; ix < nx; ++ix) ptr[ix + iy + iz + 1]++;
-  for (int p = 0; p < np; ++p) ptr[p + 1] += ptr[p];
-  std::vector<int> fill(ptr.begin(), ptr.end() - 1);
-  for (int iz = 0; iz < nz; ++iz)
-    for (int iy = 0; iy < ny; ++iy)
-      for (int ix = 0; ix < nx; ++ix) cells[fill[ix + iy + iz]++] = ix + nx * (iy + ny * iz);
-  c->nplanes = np;
-  MSG_CUDA(cudaMalloc(&c->plane_ptr, (size_t)(np + 1) * 4));
-  MSG_CUDA(cudaMalloc(&c->plane_cells, (size_t)c->N * 4));
-  MSG_CUDA(cudaMemcpy(c->plane_ptr, ptr.data(), (size_t)(np + 1) * 4, cudaMemcpyHostToDevice));
-  MSG_CUDA(cudaMemcpy(c->plane_cells, cells.data(), (size_t)c->N * 4, cudaMemcpyHostToDevice));
-  return MSG_OK;
-}
+constexpr int kWX = 16, kWY = 8, kWCols = kWX * kWY, kWThreads = 2 * kWCols + 32;
+// a layer is fetched kWFetch steps ahead of the first column of its 8 x 4 group and used up
+// to 7 + 3 steps after it
+constexpr int kWRing = 16, kWFetch = 6, kWAhead = 2, kWPitch = 24;
+constexpr unsigned long long kWEmpty = 0x7ff4a5a5a5a5a5a5ull;   // a signalling NaN
 
-struct WaveArgs {
+struct SweepArgs {
   Geo3 g;
-  const int *ptr, *cells;
-  int nplanes;
+  int tx;                        // tiles in x
+  const int *order;              // tile (x + tx * y) of each ticket
+  unsigned *ticket;
+  unsigned base;                 // ticket of this sweep's first tile
+  unsigned long long *west, *north;   // slots: west[(tile * nz + z) * kWY + ly], north[.. * kWX + lx]
+  int *err, *err_host;           // a wait was given up: device word, pinned word
   const double *dmat, *lu;
-  double *dd;            // DILU diagonal (out for factor, in for solve)
+  double *dd;                    // DILU diagonal (out for factor, in for solve)
   const double *b;
   double *x;
 };
 
-__device__ __forceinline__ void dilu_row(const WaveArgs &a, int i) {
-  int ix, iy, iz;
-  ijk(a.g, i, ix, iy, iz);
-  const size_t N = a.g.N;
-  double d = a.dmat[i];
-  if (iz > 0) { int j = i - a.g.nxy; double dinv = __ddiv_rn(1.0, a.dd[j]); d = __dsub_rn(d, __dmul_rn(__dmul_rn(a.lu[0 * N + i], dinv), a.lu[5 * N + j])); }
-  if (iy > 0) { int j = i - a.g.nx;  double dinv = __ddiv_rn(1.0, a.dd[j]); d = __dsub_rn(d, __dmul_rn(__dmul_rn(a.lu[1 * N + i], dinv), a.lu[4 * N + j])); }
-  if (ix > 0) { int j = i - 1;       double dinv = __ddiv_rn(1.0, a.dd[j]); d = __dsub_rn(d, __dmul_rn(__dmul_rn(a.lu[2 * N + i], dinv), a.lu[3 * N + j])); }
-  a.dd[i] = d;
+__device__ __forceinline__ unsigned long long ld_slot(const unsigned long long *p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_slot(unsigned long long *p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+// The value of a slot, waited for if it is still empty (v: what an earlier look found); the
+// slot is left empty.
+__device__ __forceinline__ double take_slot(const SweepArgs &a, unsigned long long *p, unsigned long long v, bool &dead) {
+  if (v == kWEmpty && !dead) {
+    unsigned long long t0 = 0, t1;
+    for (int it = 0; (v = ld_slot(p)) == kWEmpty; ++it) {
+      if ((it & 1023) == 1023) {
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
+        if (!t0) t0 = t1;
+        if (t1 - t0 > 1000000000ull || *(volatile int *)a.err) {
+          *(volatile int *)a.err = 1;
+          *(volatile int *)a.err_host = 1;
+          dead = true;
+          break;
+        }
+      }
+    }
+  }
+  st_slot(p, kWEmpty);
+  return __longlong_as_double((long long)v);
+}
+__device__ __forceinline__ void cp8(double *smem, const double *g) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(a), "l"(g) : "memory");
 }
 
-__device__ __forceinline__ void fwd_row(const WaveArgs &a, int i) {
-  int ix, iy, iz;
-  ijk(a.g, i, ix, iy, iz);
-  const size_t N = a.g.N;
-  double t = a.b[i];
-  if (iz > 0) t = __dsub_rn(t, __dmul_rn(a.lu[0 * N + i], a.x[i - a.g.nxy]));
-  if (iy > 0) t = __dsub_rn(t, __dmul_rn(a.lu[1 * N + i], a.x[i - a.g.nx]));
-  if (ix > 0) t = __dsub_rn(t, __dmul_rn(a.lu[2 * N + i], a.x[i - 1]));
-  a.x[i] = __ddiv_rn(t, a.dd[i]);
-}
+// values per cell in the ring, and its bytes
+template <int MODE>
+struct Sweep {
+  static constexpr int NV = MODE == 0 ? 7 : 5;
+  static constexpr int smem = kWRing * NV * kWCols * 8;
+};
 
-__device__ __forceinline__ void bwd_row(const WaveArgs &a, int i) {
-  int ix, iy, iz;
-  ijk(a.g, i, ix, iy, iz);
+// MODE 0: factor (dd; the values exchanged are 1/dd); MODE 1: forward solve (x from b);
+// MODE 2: backward solve (x in place), the same sweep with all three axes mirrored.
+template <int MODE>
+__global__ void __launch_bounds__(kWThreads) k_sweep(SweepArgs a) {
+  constexpr int NV = Sweep<MODE>::NV;
+  extern __shared__ double ring_mem[];
+  double(*ring)[NV][kWCols] = reinterpret_cast<double(*)[NV][kWCols]>(ring_mem);
+  __shared__ double ex[2][kWY + 1][kWPitch];     // step parity; row and column 0: the tiles before
+  __shared__ int s_tile;
+  const int t = threadIdx.x, wp = t >> 5, ln = t & 31;
+  if (t == 0) s_tile = a.order[atomicAdd(a.ticket, 1u) - a.base];
+  __syncthreads();
+  const int tile = s_tile, bx = tile % a.tx, by = tile / a.tx;
+  const int nx = a.g.nx, ny = a.g.ny, nz = a.g.nz, nxy = a.g.nxy;
   const size_t N = a.g.N;
-  double t = 0.0;
-  if (ix < a.g.nx - 1) t = __dadd_rn(t, __dmul_rn(a.lu[3 * N + i], a.x[i + 1]));
-  if (iy < a.g.ny - 1) t = __dadd_rn(t, __dmul_rn(a.lu[4 * N + i], a.x[i + a.g.nx]));
-  if (iz < a.g.nz - 1) t = __dadd_rn(t, __dmul_rn(a.lu[5 * N + i], a.x[i + a.g.nxy]));
-  a.x[i] = __dsub_rn(a.x[i], __ddiv_rn(t, a.dd[i]));
-}
-
-// MODE 0: factor; MODE 1: forward + backward solve.  COOP: grid-wide sync between
-// planes (cooperative launch); otherwise a single block with __syncthreads.
-template <int MODE, bool COOP>
-__global__ void __launch_bounds__(1024) k_wave(WaveArgs a) {
-  auto sync = [&]() {
-    if (COOP) cg::this_grid().sync();
-    else __syncthreads();
+  const int dz = MODE == 2 ? -nxy : nxy;
+  // first cell of the column (gx, gy), in mirrored coordinates in MODE 2
+  auto first = [&](int gx, int gy) {
+    return MODE == 2 ? (nx - 1 - gx) + nx * (ny - 1 - gy) + (nz - 1) * nxy : gx + nx * gy;
   };
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
-  for (int p = 0; p < a.nplanes; ++p) {
-    int b = a.ptr[p], e = a.ptr[p + 1];
-    for (int q = b + tid; q < e; q += nth) {
-      if (MODE == 0) dilu_row(a, a.cells[q]);
-      else fwd_row(a, a.cells[q]);
+  const int steps = min(kWX, nx - bx * kWX) + min(kWY, ny - by * kWY) + nz - 2;
+  if (wp < kWCols / 32) {
+    // ---- the chain: a warp owns 8 x 4 columns
+    const int lx = 8 * (wp % (kWX / 8)) + (ln & 7), ly = 4 * (wp / (kWX / 8)) + (ln >> 3);
+    const int gx = bx * kWX + lx, gy = by * kWY + ly;
+    const bool col = gx < nx && gy < ny, hx = gx > 0, hy = gy > 0;
+    const int layers = col ? nz : 0;
+    unsigned long long *wout = lx == kWX - 1 && gx + 1 < nx && col ? a.west + ((size_t)(tile + 1) * nz) * kWY + ly : nullptr;
+    unsigned long long *nout = ly == kWY - 1 && gy + 1 < ny && col ? a.north + ((size_t)(tile + a.tx) * nz) * kWX + lx : nullptr;
+    const bool edge = wout || nout;
+    size_t i = col ? first(gx, gy) : 0;
+    int z = -lx - ly;
+    double up = 0.0, q[NV];
+    auto load = [&]() {
+      const double *p = &ring[z & (kWRing - 1)][0][t];
+#pragma unroll
+      for (int k = 0; k < NV; ++k) q[k] = p[k * kWCols];
+    };
+    auto step = [&](const double(*in)[kWPitch], double(*out)[kWPitch]) {
+      const double xw = in[ly + 1][lx], xn = in[ly][lx + 1];
+      const bool on = (unsigned)z < (unsigned)layers, hz = z > 0;
+      double v;
+      if (MODE == 0) {
+        double d = q[0];
+        if (hz) d = __dsub_rn(d, __dmul_rn(__dmul_rn(q[1], up), q[4]));
+        if (hy) d = __dsub_rn(d, __dmul_rn(__dmul_rn(q[2], xn), q[5]));
+        if (hx) d = __dsub_rn(d, __dmul_rn(__dmul_rn(q[3], xw), q[6]));
+        v = __drcp_rn(d);
+        if (on) a.dd[i] = d;
+      } else if (MODE == 1) {
+        double r = q[0];
+        if (hz) r = __dsub_rn(r, __dmul_rn(q[2], up));
+        if (hy) r = __dsub_rn(r, __dmul_rn(q[3], xn));
+        if (hx) r = __dsub_rn(r, __dmul_rn(q[4], xw));
+        v = __ddiv_rn(r, q[1]);
+        if (on) a.x[i] = v;
+      } else {
+        double r = 0.0;
+        if (hx) r = __dadd_rn(r, __dmul_rn(q[4], xw));
+        if (hy) r = __dadd_rn(r, __dmul_rn(q[3], xn));
+        if (hz) r = __dadd_rn(r, __dmul_rn(q[2], up));
+        v = __dsub_rn(q[0], __ddiv_rn(r, q[1]));
+        if (on) a.x[i] = v;
+      }
+      out[ly + 1][lx + 1] = v;
+      if (on) {
+        up = v;
+        i += dz;
+        if (edge) {
+          if (wout) st_slot(wout + z * kWY, (unsigned long long)__double_as_longlong(v));
+          if (nout) st_slot(nout + z * kWX, (unsigned long long)__double_as_longlong(v));
+        }
+      }
+      ++z;
+      load();
+      __syncthreads();
+    };
+    __syncthreads();
+    load();
+    for (int s = 0; s < steps; s += 2) {
+      step(ex[1], ex[0]);
+      if (s + 1 < steps) step(ex[0], ex[1]);
     }
-    sync();
-  }
-  if (MODE == 1) {
-    for (int p = a.nplanes - 1; p >= 0; --p) {
-      int b = a.ptr[p], e = a.ptr[p + 1];
-      for (int q = b + tid; q < e; q += nth) bwd_row(a, a.cells[q]);
-      sync();
+  } else if (wp == kWCols / 32) {
+    // ---- the columns of the tiles before: lanes 0 .. kWY-1 west, the next kWX north
+    const bool w = ln < kWY, n = !w && ln < kWY + kWX;
+    const int k = w ? ln : ln - kWY, gx = bx * kWX + (w ? 0 : k), gy = by * kWY + (w ? k : 0);
+    const bool has = gx < nx && gy < ny && ((w && bx > 0) || (n && by > 0));
+    const int pitch = w ? kWY : kWX;
+    unsigned long long *slot = (w ? a.west : a.north) + (size_t)tile * nz * pitch + (has ? k : 0);
+    const int row = w ? k + 1 : 0, cl = w ? 0 : k + 1;
+    unsigned long long pre[kWAhead];
+    bool dead = false;
+#pragma unroll
+    for (int u = 0; u < kWAhead; ++u) {
+      const int z = u - k;
+      pre[u] = has && z >= 0 && z < nz ? ld_slot(slot + z * pitch) : kWEmpty;
     }
+    // before the barrier that step s follows: its values
+    for (int s0 = 0; s0 <= steps; s0 += kWAhead) {
+#pragma unroll
+      for (int u = 0; u < kWAhead; ++u) {
+        const int s = s0 + u, z = s - k;
+        if (s <= steps) {
+          if (has && z >= 0 && z < nz) ex[(s + 1) & 1][row][cl] = take_slot(a, slot + z * pitch, pre[u], dead);
+          const int za = z + kWAhead;
+          if (has && za >= 0 && za < nz) pre[u] = ld_slot(slot + za * pitch);
+          __syncthreads();
+        }
+      }
+    }
+  } else {
+    // ---- coefficients: a warp copies the 8 x 4 columns of one group (bands without a
+    // neighbour hold zeros; only those read at the neighbour need it to exist)
+    const int tt = t - kWCols - 32, gr = tt >> 5, wx = 8 * (gr % (kWX / 8)), wy = 4 * (gr / (kWX / 8));
+    const int gx = bx * kWX + wx + (ln & 7), gy = by * kWY + wy + (ln >> 3);
+    const bool hx = gx > 0, hy = gy > 0;
+    const int layers = gx < nx && gy < ny ? nz : 0;
+    int z = -wx - wy;
+    const double *p[NV];
+    const long long i0 = first(gx, gy) + (long long)z * dz;
+    if (MODE == 0) {
+      p[0] = a.dmat + i0;
+      p[1] = a.lu + i0; p[2] = a.lu + N + i0; p[3] = a.lu + 2 * N + i0;
+      p[4] = a.lu + 5 * N + i0 - nxy; p[5] = a.lu + 4 * N + i0 - nx; p[6] = a.lu + 3 * N + i0 - 1;
+    } else {
+      p[0] = (MODE == 1 ? a.b : a.x) + i0;
+      p[1] = a.dd + i0;
+      p[2] = a.lu + (MODE == 1 ? 0 : 5) * N + i0;
+      p[3] = a.lu + (MODE == 1 ? 1 : 4) * N + i0;
+      p[4] = a.lu + (MODE == 1 ? 2 : 3) * N + i0;
+    }
+    auto fetch = [&]() {
+      if ((unsigned)z < (unsigned)layers) {
+        double *q = &ring[z & (kWRing - 1)][0][tt];
+#pragma unroll
+        for (int k = 0; k < NV; ++k)
+          if (MODE != 0 || k < 4 || (k == 4 && z > 0) || (k == 5 && hy) || (k == 6 && hx)) cp8(q + k * kWCols, p[k]);
+      }
+#pragma unroll
+      for (int k = 0; k < NV; ++k) p[k] += dz;
+      ++z;
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // the barrier that step s follows: the layers of steps s and s + 1 have arrived
+    for (int s = 0; s < kWFetch; ++s) fetch();
+    for (int s = 0; s <= steps; ++s) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kWFetch - 2) : "memory");
+      __syncthreads();
+      fetch();
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
   }
 }
 
-static int launch_wave(msg_ctx *c, WaveArgs &a, int mode) {
-  const int kSmall = 1 << 18;
-  if (c->N <= kSmall) {
-    if (mode == 0) k_wave<0, false><<<1, 1024, 0, c->stream>>>(a);
-    else k_wave<1, false><<<1, 1024, 0, c->stream>>>(a);
-    MSG_CHECK_LAUNCH();
-    return MSG_OK;
-  }
-  int per_sm = 0;
-  void *fn = mode == 0 ? (void *)k_wave<0, true> : (void *)k_wave<1, true>;
-  MSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 1024, 0));
-  int sms = 0;
-  MSG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
-  int grid = sms * (per_sm > 0 ? per_sm : 1);
-  void *args[] = {&a};
-  MSG_CUDA(cudaLaunchCooperativeKernel(fn, grid, 1024, args, 0, c->stream));
-  __atomic_fetch_add(&g_launches, 1LL, __ATOMIC_RELAXED);
+// Tile order, slots (all empty), ticket counter and error words of the sweeps.
+int build_wavefront(msg_ctx *c) {
+  const int tx = (c->nx + kWX - 1) / kWX, ty = (c->ny + kWY - 1) / kWY, nt = tx * ty;
+  std::vector<int> order;
+  order.reserve(nt);
+  for (int d = 0; d < tx + ty - 1; ++d)
+    for (int y = std::max(0, d - tx + 1); y <= std::min(d, ty - 1); ++y) order.push_back((d - y) + tx * y);
+  const size_t nslot = (size_t)nt * c->nz * (kWX + kWY);
+  MSG_CUDA(cudaFuncSetAttribute(k_sweep<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sweep<0>::smem));
+  MSG_CUDA(cudaFuncSetAttribute(k_sweep<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sweep<1>::smem));
+  MSG_CUDA(cudaFuncSetAttribute(k_sweep<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sweep<2>::smem));
+  MSG_CUDA(cudaMalloc(&c->wave_order, (size_t)nt * 4));
+  MSG_CUDA(cudaMalloc(&c->wave_ticket, 8));      // ticket, error word
+  MSG_CUDA(cudaMalloc(&c->wave_slots, nslot * 8));
+  MSG_CUDA(cudaMallocHost((void **)&c->wave_err, 4));
+  *c->wave_err = 0;
+  c->wave_tiles = nt;
+  c->wave_sweeps = 0;
+  std::vector<unsigned long long> empty(nslot, kWEmpty);
+  MSG_CUDA(cudaMemcpyAsync(c->wave_slots, empty.data(), nslot * 8, cudaMemcpyHostToDevice, c->stream));
+  MSG_CUDA(cudaMemcpyAsync(c->wave_order, order.data(), (size_t)nt * 4, cudaMemcpyHostToDevice, c->stream));
+  MSG_CUDA(cudaMemsetAsync(c->wave_ticket, 0, 8, c->stream));
+  MSG_CUDA(cudaStreamSynchronize(c->stream));
   return MSG_OK;
 }
 
-int launch_precon_dilu(msg_ctx *c) {
-  WaveArgs a{geo3(c), c->plane_ptr, c->plane_cells, c->nplanes, c->dmat, c->lu, c->dilu_d, nullptr, nullptr};
-  return launch_wave(c, a, 0);
+// A sweep that gave up a wait has said so in wave_err (host memory); looked at after every
+// host wait on the stream.  The slots are then in an unknown state, so no sweep runs again.
+int wave_check(msg_ctx *c) {
+  if (c->wave_err && *(volatile int *)c->wave_err) {
+    set_error("DILU sweep: a wait between tiles ran out");
+    return MSG_ERR_CUDA;
+  }
+  return MSG_OK;
 }
 
+template <int MODE>
+static int launch_sweep(msg_ctx *c, const double *b, double *x) {
+  int rc = wave_check(c);
+  if (rc) return rc;
+  unsigned long long *slots = (unsigned long long *)c->wave_slots;
+  SweepArgs a{geo3(c), (c->nx + kWX - 1) / kWX, c->wave_order, c->wave_ticket,
+              c->wave_sweeps * (unsigned)c->wave_tiles, slots, slots + (size_t)c->wave_tiles * c->nz * kWY,
+              (int *)c->wave_ticket + 1, c->wave_err, c->dmat, c->lu, c->dilu_d, b, x};
+  k_sweep<MODE><<<c->wave_tiles, kWThreads, Sweep<MODE>::smem, c->stream>>>(a);
+  c->wave_sweeps++;
+  MSG_CHECK_LAUNCH();
+  return MSG_OK;
+}
+
+int launch_precon_dilu(msg_ctx *c) { return launch_sweep<0>(c, nullptr, nullptr); }
+
 int launch_solve_ilu(msg_ctx *c, const double *b, double *x) {
-  WaveArgs a{geo3(c), c->plane_ptr, c->plane_cells, c->nplanes, c->dmat, c->lu, c->dilu_d, b, x};
-  return launch_wave(c, a, 1);
+  int rc = launch_sweep<1>(c, b, x);
+  if (rc) return rc;
+  return launch_sweep<2>(c, nullptr, x);
 }
 
 int apply_prec(msg_ctx *c, const double *r, double *z) {
