@@ -329,7 +329,7 @@ constexpr int kHashSmall = 256, kSmallMaxCols = 120;   // fill-pass table for ro
 // the count pass: rows of at most kSmallMaxCols columns go through the kHashSmall variant
 // (a quarter of the shared memory, twice the resident warps), the others through kHash.
 template <int PASS, int HASH = kHash>
-__global__ void __launch_bounds__(32 * kSpgWarps) k_spgemm(int nrows, const int *ap, const int *ac, const double *av,
+__global__ void __launch_bounds__(32 * kSpgWarps) k_spgemm(const int *nrows, const int *ap, const int *ac, const double *av,
                                                            const double *adiag, const int *bp, const int *bc,
                                                            const double *bv, int split_diag, int *ocnt,
                                                            const int *cptr, int *ccol, double *cval, double *cdiag,
@@ -338,126 +338,130 @@ __global__ void __launch_bounds__(32 * kSpgWarps) k_spgemm(int nrows, const int 
   __shared__ int hk[kSpgWarps][HASH];
   __shared__ double hv[kSpgWarps][PASS == 1 ? HASH : 1];
   __shared__ int comp[kSpgWarps][kComp];
-  int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int rid = blockIdx.x * kSpgWarps + w;
-  if (rid >= nrows) return;
-  const int row = rows ? rows[rid] : rid;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int *K = hk[w];
   double *V = hv[w];
-  int a0 = ap[row], a1 = ap[row + 1];
-  int start = adiag ? a0 - 1 : a0;
-  int m = 0;
-  if (PASS == 1) {
-    // columns of this row (from the count pass; + 1 for a split-off diagonal)
-    m = cptr[row + 1] - cptr[row] + (split_diag ? 1 : 0);
-    if ((HASH == kHashSmall) != (m <= kSmallMaxCols)) return;   // the other variant's row
-  } else {
-    // products of this row -> table size (load factor <= 1/2 when it fits)
-    for (int k = start + lane; k < a1; k += 32) {
-      int j = (k < a0) ? row : ac[k];
-      m += bp[j + 1] - bp[j];
-    }
-    for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
-  }
-  int T = 32;
-  while (T < 2 * m && T < HASH) T <<= 1;
-  const unsigned mask = (unsigned)T - 1u;
-  for (int t = lane; t < T; t += 32) { K[t] = -1; if (PASS == 1) V[t] = 0.0; }
-  __syncwarp();
-  // PASS 0 only counts distinct columns: no values are loaded, multiplied or added
-  auto add = [&](int cc, double p) {
-    unsigned hsh = ((unsigned)cc * 2654435761u) & mask;
-    for (int probe = 0; probe < T; ++probe) {
-      int cur = atomicCAS(&K[hsh], -1, cc);
-      if (cur == -1 || cur == cc) {
-        if (PASS == 1) V[hsh] = __dadd_rn(V[hsh], p);
-        break;
+  const int nr = *nrows;
+  for (int rid = blockIdx.x * kSpgWarps + w; rid < nr; rid += gridDim.x * kSpgWarps) {
+    const int row = rows[rid];
+    int a0 = ap[row], a1 = ap[row + 1];
+    int start = adiag ? a0 - 1 : a0;
+    int m = 0;
+    if (PASS == 1) {
+      // columns of this row (from the count pass; + 1 for a split-off diagonal)
+      m = cptr[row + 1] - cptr[row] + (split_diag ? 1 : 0);
+      if ((HASH == kHashSmall) != (m <= kSmallMaxCols)) continue;   // the other variant's row
+    } else {
+      // products of this row -> table size (load factor <= 1/2 when it fits)
+      for (int k = start + lane; k < a1; k += 32) {
+        int j = (k < a0) ? row : ac[k];
+        m += bp[j + 1] - bp[j];
       }
-      hsh = (hsh + 1) & mask;
+      for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
     }
-  };
-  // kPf entries of A at a time: their B rows (up to 32 entries, one per lane) are loaded
-  // together, so the dependent loads of A's column -> B's row bounds -> B's entries overlap
-  // across entries; they are then added in entry order exactly as one at a time.
-  for (int kb = start; kb < a1; kb += kPf) {
-    int cols[kPf], lens[kPf];
-    double vals[kPf];
-#pragma unroll
-    for (int u = 0; u < kPf; ++u) {
-      const int k = kb + u;
-      lens[u] = 0; cols[u] = -1; vals[u] = 0.0;
-      if (k < a1) {
-        int j;
-        double coef = 0.0;
-        if (k < a0) { j = row; if (PASS == 1) coef = adiag[row]; }
-        else { j = ac[k]; if (PASS == 1) coef = av[k]; }
-        const int b0 = bp[j], len = bp[j + 1] - b0;
-        lens[u] = len;
-        if (lane < len) {
-          cols[u] = bc[b0 + lane];
-          if (PASS == 1) vals[u] = __dmul_rn(coef, bv[b0 + lane]);
+    int T = 32;
+    while (T < 2 * m && T < HASH) T <<= 1;
+    const unsigned mask = (unsigned)T - 1u;
+    for (int t = lane; t < T; t += 32) { K[t] = -1; if (PASS == 1) V[t] = 0.0; }
+    __syncwarp();
+    // PASS 0 only counts distinct columns: no values are loaded, multiplied or added
+    auto add = [&](int cc, double p) {
+      unsigned hsh = ((unsigned)cc * 2654435761u) & mask;
+      for (int probe = 0; probe < T; ++probe) {
+        int cur = atomicCAS(&K[hsh], -1, cc);
+        if (cur == -1 || cur == cc) {
+          if (PASS == 1) V[hsh] = __dadd_rn(V[hsh], p);
+          break;
         }
+        hsh = (hsh + 1) & mask;
       }
-    }
+    };
+    // kPf entries of A at a time: their B rows (up to 32 entries, one per lane) are loaded
+    // together, so the dependent loads of A's column -> B's row bounds -> B's entries overlap
+    // across entries; they are then added in entry order exactly as one at a time.
+    for (int kb = start; kb < a1; kb += kPf) {
+      int cols[kPf], lens[kPf];
+      double vals[kPf];
 #pragma unroll
-    for (int u = 0; u < kPf; ++u) {
-      const int k = kb + u;
-      if (k < a1) {
-        if (lens[u] <= 32) {
-          if (lane < lens[u]) add(cols[u], vals[u]);
-        } else {   // a B row longer than the warp: the whole row again, in chunks
+      for (int u = 0; u < kPf; ++u) {
+        const int k = kb + u;
+        lens[u] = 0; cols[u] = -1; vals[u] = 0.0;
+        if (k < a1) {
           int j;
           double coef = 0.0;
           if (k < a0) { j = row; if (PASS == 1) coef = adiag[row]; }
           else { j = ac[k]; if (PASS == 1) coef = av[k]; }
-          for (int q = bp[j] + lane; q < bp[j + 1]; q += 32) add(bc[q], PASS == 1 ? __dmul_rn(coef, bv[q]) : 0.0);
+          const int b0 = bp[j], len = bp[j + 1] - b0;
+          lens[u] = len;
+          if (lane < len) {
+            cols[u] = bc[b0 + lane];
+            if (PASS == 1) vals[u] = __dmul_rn(coef, bv[b0 + lane]);
+          }
         }
       }
+#pragma unroll
+      for (int u = 0; u < kPf; ++u) {
+        const int k = kb + u;
+        if (k < a1) {
+          if (lens[u] <= 32) {
+            if (lane < lens[u]) add(cols[u], vals[u]);
+          } else {   // a B row longer than the warp: the whole row again, in chunks
+            int j;
+            double coef = 0.0;
+            if (k < a0) { j = row; if (PASS == 1) coef = adiag[row]; }
+            else { j = ac[k]; if (PASS == 1) coef = av[k]; }
+            for (int q = bp[j] + lane; q < bp[j + 1]; q += 32) add(bc[q], PASS == 1 ? __dmul_rn(coef, bv[q]) : 0.0);
+          }
+        }
+        __syncwarp();
+      }
+    }
+    // compact occupied slots
+    int u = 0;
+    for (int base = 0; base < T; base += 32) {
+      int t = base + lane;
+      bool occ = K[t] >= 0;
+      unsigned bal = __ballot_sync(0xffffffffu, occ);
+      if (occ) {
+        int pos = u + __popc(bal & ((1u << lane) - 1));
+        if (pos < kComp) comp[w][pos] = t;
+      }
+      u += __popc(bal);
+    }
+    __syncwarp();
+    if (u > kHashMax) {
+      if (lane == 0) { atomicExch(overflow, 1); if (PASS == 0) ocnt[row] = 0; }
       __syncwarp();
+      continue;
     }
-  }
-  // compact occupied slots
-  int u = 0;
-  for (int base = 0; base < T; base += 32) {
-    int t = base + lane;
-    bool occ = K[t] >= 0;
-    unsigned bal = __ballot_sync(0xffffffffu, occ);
-    if (occ) {
-      int pos = u + __popc(bal & ((1u << lane) - 1));
-      if (pos < kComp) comp[w][pos] = t;
+    bool hasd = false;
+    if (split_diag) {
+      for (int t = lane; t < u; t += 32) if (K[comp[w][t]] == row) hasd = true;
+      hasd = __any_sync(0xffffffffu, hasd);
     }
-    u += __popc(bal);
-  }
-  __syncwarp();
-  if (u > kHashMax) {
-    if (lane == 0) { atomicExch(overflow, 1); if (PASS == 0) ocnt[row] = 0; }
-    return;
-  }
-  bool hasd = false;
-  if (split_diag) {
-    for (int t = lane; t < u; t += 32) if (K[comp[w][t]] == row) hasd = true;
-    hasd = __any_sync(0xffffffffu, hasd);
-  }
-  if (PASS == 0) {
-    if (lane == 0) ocnt[row] = u - (hasd ? 1 : 0);
-    return;
-  }
-  // rank sort by column
-  int out0 = cptr[row];
-  if (split_diag && lane == 0) cdiag[row] = 1.0;
-  __syncwarp();
-  for (int t = lane; t < u; t += 32) {
-    int slot = comp[w][t];
-    int key = K[slot];
-    if (split_diag && key == row) { cdiag[row] = V[slot]; continue; }
-    int rank = 0;
-    for (int v = 0; v < u; ++v) {
-      int k2 = K[comp[w][v]];
-      if (split_diag && k2 == row) continue;
-      rank += (k2 < key);
+    if (PASS == 0) {
+      if (lane == 0) ocnt[row] = u - (hasd ? 1 : 0);
+      __syncwarp();
+      continue;
     }
-    ccol[out0 + rank] = key;
-    cval[out0 + rank] = V[slot];
+    // rank sort by column
+    int out0 = cptr[row];
+    if (split_diag && lane == 0) cdiag[row] = 1.0;
+    __syncwarp();
+    for (int t = lane; t < u; t += 32) {
+      int slot = comp[w][t];
+      int key = K[slot];
+      if (split_diag && key == row) { cdiag[row] = V[slot]; continue; }
+      int rank = 0;
+      for (int v = 0; v < u; ++v) {
+        int k2 = K[comp[w][v]];
+        if (split_diag && k2 == row) continue;
+        rank += (k2 < key);
+      }
+      ccol[out0 + rank] = key;
+      cval[out0 + rank] = V[slot];
+    }
+    __syncwarp();
   }
 }
 
@@ -1115,7 +1119,7 @@ static int ensure_scratch(msg_ctx *c, AmgState *A, size_t n, size_t nnz) {
   if ((rc = dalloc(c, &A->has, cn))) return rc;
   if ((rc = dalloc(c, &A->st, cn))) return rc;
   if ((rc = dalloc(c, &A->flag, cn))) return rc;
-  if ((rc = dalloc(c, &A->aggid, cn))) return rc;
+  if ((rc = dalloc(c, &A->aggid, cn + 1))) return rc;
   if ((rc = dalloc(c, &A->agg2, cn))) return rc;
   if ((rc = dalloc(c, &A->tmpi, cn + 1))) return rc;
   if ((rc = dalloc(c, &A->t0m, cn))) return rc;
@@ -1142,7 +1146,7 @@ static int spgemm(msg_ctx *c, AmgState *A, int nrows, const int *ap, const int *
                   int **ccol, double **cval, double *cdiag, int *cnnz, int *ovf) {
   cudaStream_t s = c->stream;
   int rc;
-  int *cnt = nullptr, *longrows = nullptr, *nl = nullptr;
+  int *cnt = nullptr, *longrows = nullptr, *nl = nullptr;   // nl: long rows, overflow flag
   *ovf = 0;
   if ((rc = halloc(c, &cnt, nrows + 1))) return rc;
   if ((rc = halloc(c, &longrows, nrows + 1))) return rc;
@@ -1151,37 +1155,33 @@ static int spgemm(msg_ctx *c, AmgState *A, int nrows, const int *ap, const int *
   k_spgemm_t<0><<<(nrows + 127) / 128, 128, 0, s>>>(nrows, ap, ac, av, adiag, bp, bc, bv, split_diag, cnt, nullptr,
                                                    nullptr, nullptr, nullptr, longrows, nl);
   MSG_CHECK_LAUNCH();
-  int h[2];
-  MSG_CUDA(cudaMemcpyAsync(h, nl, 8, cudaMemcpyDeviceToHost, s));
-  MSG_CUDA(cudaStreamSynchronize(s));
-  const int nlong = h[0];
-  MSG_CUDA(cudaMemsetAsync(A->cnt, 0, 4, s));
-  if (nlong > 0) {
-    k_spgemm<0><<<(nlong + kSpgWarps - 1) / kSpgWarps, 32 * kSpgWarps, 0, s>>>(
-        nlong, ap, ac, av, adiag, bp, bc, bv, split_diag, cnt, nullptr, nullptr, nullptr, nullptr, A->cnt, longrows);
-    MSG_CHECK_LAUNCH();
-  }
+  // the count of the long rows stays on the device: a grid that fills the chip walks them
+  const int wb = std::min((nrows + kSpgWarps - 1) / kSpgWarps, 12 * kNumSM);
+  k_spgemm<0><<<wb, 32 * kSpgWarps, 0, s>>>(nl, ap, ac, av, adiag, bp, bc, bv, split_diag, cnt, nullptr, nullptr,
+                                            nullptr, nullptr, nl + 1, longrows);
+  MSG_CHECK_LAUNCH();
   if ((rc = halloc(c, cptr, nrows + 1))) return rc;
-  int tot = 0;
-  if ((rc = scan_exclusive(c, cnt, *cptr, nrows, &tot))) return rc;
-  if ((rc = read_counter(c, A, ovf))) return rc;
+  int got[3];
+  if ((rc = scan_exclusive(c, cnt, *cptr, nrows, got, nl, nl + 1))) return rc;
+  const int tot = got[0], nlong = got[1];
+  *ovf = got[2];
   if (*ovf) {
     hfree(S(c), cnt, s); hfree(S(c), longrows, s); hfree(S(c), nl, s); hfree(S(c), *cptr, s);
     *cptr = nullptr;
     return MSG_OK;
   }
-  MSG_CUDA(cudaMemcpyAsync(*cptr + nrows, &tot, 4, cudaMemcpyHostToDevice, s));
   if ((rc = halloc(c, ccol, tot))) return rc;
   if ((rc = halloc(c, cval, tot))) return rc;
   k_spgemm_t<1><<<(nrows + 127) / 128, 128, 0, s>>>(nrows, ap, ac, av, adiag, bp, bc, bv, split_diag, nullptr, *cptr,
                                                    *ccol, *cval, cdiag, nullptr, nullptr);
   MSG_CHECK_LAUNCH();
   if (nlong > 0) {
-    k_spgemm<1, kHashSmall><<<(nlong + kSpgWarps - 1) / kSpgWarps, 32 * kSpgWarps, 0, s>>>(
-        nlong, ap, ac, av, adiag, bp, bc, bv, split_diag, nullptr, *cptr, *ccol, *cval, cdiag, A->cnt, longrows);
+    const int wf = (nlong + kSpgWarps - 1) / kSpgWarps;
+    k_spgemm<1, kHashSmall><<<wf, 32 * kSpgWarps, 0, s>>>(nl, ap, ac, av, adiag, bp, bc, bv, split_diag, nullptr,
+                                                          *cptr, *ccol, *cval, cdiag, nl + 1, longrows);
     MSG_CHECK_LAUNCH();
-    k_spgemm<1, kHash><<<(nlong + kSpgWarps - 1) / kSpgWarps, 32 * kSpgWarps, 0, s>>>(
-        nlong, ap, ac, av, adiag, bp, bc, bv, split_diag, nullptr, *cptr, *ccol, *cval, cdiag, A->cnt, longrows);
+    k_spgemm<1, kHash><<<wf, 32 * kSpgWarps, 0, s>>>(nl, ap, ac, av, adiag, bp, bc, bv, split_diag, nullptr, *cptr,
+                                                     *ccol, *cval, cdiag, nl + 1, longrows);
     MSG_CHECK_LAUNCH();
   }
   hfree(S(c), cnt, s); hfree(S(c), longrows, s); hfree(S(c), nl, s);
@@ -1228,7 +1228,7 @@ static int coarsen(msg_ctx *c, AmgState *A, int lv, int *made) {
   }
   k_root_flag<<<nb(n), kThreads, 0, s>>>(n, A->st, A->flag);
   MSG_CHECK_LAUNCH();
-  int nc = 0;
+  int nc = 0, got[2];
   if ((rc = scan_exclusive(c, A->flag, A->aggid, n, &nc))) return rc;
   if (nc == 0 || nc >= n) return MSG_OK;
   AmgLevel C;
@@ -1242,15 +1242,10 @@ static int coarsen(msg_ctx *c, AmgState *A, int lv, int *made) {
   MSG_CUDA(cudaMemsetAsync(A->cnt, 0, 4, s));
   k_p_count<<<nb(n), kThreads, 0, s>>>(n, F.rowptr, F.col, A->sflag, C.agg, A->tmpi, A->cnt);
   MSG_CHECK_LAUNCH();
-  {
-    int ovp = 0;
-    if ((rc = read_counter(c, A, &ovp))) return rc;
-    if (ovp) { free_level(A, C, s); return MSG_OK; }
-  }
   if ((rc = halloc(c, &C.pptr, n + 1))) return rc;
-  int pnnz = 0;
-  if ((rc = scan_exclusive(c, A->tmpi, C.pptr, n, &pnnz))) return rc;
-  MSG_CUDA(cudaMemcpyAsync(C.pptr + n, &pnnz, 4, cudaMemcpyHostToDevice, s));
+  if ((rc = scan_exclusive(c, A->tmpi, C.pptr, n, got, A->cnt))) return rc;
+  if (got[1]) { free_level(A, C, s); return MSG_OK; }   // a row beyond kPRowMax
+  const int pnnz = got[0];
   C.pnnz = pnnz;
   if ((rc = halloc(c, &C.pcol, pnnz))) return rc;
   if ((rc = halloc(c, &C.pval, pnnz))) return rc;
@@ -1264,9 +1259,7 @@ static int coarsen(msg_ctx *c, AmgState *A, int lv, int *made) {
   k_r_count<<<nb(pnnz), kThreads, 0, s>>>(pnnz, C.pcol, rcnt);
   MSG_CHECK_LAUNCH();
   if ((rc = halloc(c, &C.rptr, nc + 1))) return rc;
-  int rn = 0;
-  if ((rc = scan_exclusive(c, rcnt, C.rptr, nc, &rn))) return rc;
-  MSG_CUDA(cudaMemcpyAsync(C.rptr + nc, &rn, 4, cudaMemcpyHostToDevice, s));
+  if ((rc = scan_exclusive(c, rcnt, C.rptr, nc, nullptr))) return rc;
   if ((rc = halloc(c, &C.rcol, pnnz))) return rc;
   if ((rc = halloc(c, &C.rval, pnnz))) return rc;
   MSG_CUDA(cudaMemsetAsync(rcnt, 0, (size_t)(nc + 1) * 4, s));

@@ -676,8 +676,9 @@ static int create_impl(msg_ctx *c, const msg_grid_t *g, const msg_params_t *p) {
   c->npart = npart;
   ALLOC(c->dres, 16 * 8);
   MSG_CUDA(cudaMallocHost((void **)&c->hpin, (size_t)kRedBlocks * 8 * 8));
-  int rc = build_connectivity(c, g);
+  int rc = scan_reserve(c, (int)N);
   if (rc) return rc;
+  if ((rc = build_connectivity(c, g))) return rc;
   if (p->precon_type == 0 || p->ref_quirks) {
     if ((rc = build_wavefront(c))) return rc;
   }
@@ -1271,10 +1272,11 @@ static void free_ctx(msg_ctx *c) {
                 c->left_off, c->right_off, c->hydf_conn, c->abyd_conn, c->head_new, c->head_old, c->head_pre,
                 c->head_change, c->srat_new, c->srat_old, c->surf_head, c->surf_old, c->new_f, c->kr, c->kr_per,
                 c->alp, c->sto, c->stod, c->tmpv, c->dmat, c->lu, c->rhs, c->rhs_alt, c->head_old2, c->slope_rhs, c->dilu_d, c->r, c->rs,
-                c->p, c->v, c->t, c->z, c->part, c->wave_order, c->wave_ticket, c->wave_slots, c->dmat_f, c->lu_f, c->dres};
+                c->p, c->v, c->t, c->z, c->part, c->scan_sums, c->wave_order, c->wave_ticket, c->wave_slots, c->dmat_f, c->lu_f, c->dres};
   for (auto q : dp) if (q) cudaFree(q);
   if (c->hpin) cudaFreeHost(c->hpin);
   if (c->wave_err) cudaFreeHost(c->wave_err);
+  if (c->box) cudaFreeHost(c->box);
   for (int k = 0; k < 8; ++k) if (c->ev[k]) cudaEventDestroy(c->ev[k]);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;

@@ -14,6 +14,12 @@ struct DevScalars {
   int conv, in_iter, done, pad;
 };
 
+// Words that a kernel hands to the host: pinned memory, complete when token is the awaited one.
+struct HostBox {
+  int v[4];
+  unsigned token;
+};
+
 }  // namespace msg
 
 struct msg_ctx {
@@ -64,6 +70,10 @@ struct msg_ctx {
   size_t npart;
   double *hpin;                                  // pinned host scalars
   double *dres;                                  // device reduction results [16]
+  // ---- scans (msg_linear.cu): chunk sums, and the box their totals reach the host in -------
+  int *scan_sums, scan_cap;
+  msg::HostBox *box;
+  unsigned box_token;
   // ---- DILU sweeps (msg_linear.cu): tile order, ticket counter, hand-over slots between tiles
   int *wave_order;
   unsigned *wave_ticket, wave_sweeps;            // ticket and error word; sweeps launched so far
@@ -164,6 +174,8 @@ void learned_free(msg_ctx *c);
 int apply_prec(msg_ctx *c, const double *r, double *z);
 
 // ---- scan (msg_linear.cu) ---------------------------------------------------------------------------
-int scan_exclusive(msg_ctx *c, const int *in, int *out, int n, int *total_host);
+int scan_reserve(msg_ctx *c, int n);
+int scan_exclusive(msg_ctx *c, const int *in, int *out, int n, int *got, const int *w1 = nullptr,
+                   const int *w2 = nullptr);
 
 }  // namespace msg

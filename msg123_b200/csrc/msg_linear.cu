@@ -7,8 +7,11 @@
 // dot product repeats bit for bit from run to run.
 #include "msg_ctx.cuh"
 #include <algorithm>
+#include <atomic>
 #include <vector>
 #include <cmath>
+#include <cstring>
+#include <thread>
 
 namespace msg {
 
@@ -26,68 +29,141 @@ __device__ __forceinline__ void ijk(const Geo3 &g, int i, int &ix, int &iy, int 
 }
 
 // ---------------------------------------------------------------------------------
-// Exclusive scan of int32 (three phases, 2048 elements per block).
+// Exclusive scan of int32 in two passes over chunks of kScanE elements: the chunks' sums,
+// then every block adds up the sums before its own chunk and scans the chunk (int sums are
+// the same in any order).  The last block writes the total behind the output and into the
+// context's box.  A serial pass over the chunk sums by one thread, and a third pass to add
+// them, took 7 us of the 22 us of a scan of 4.2M elements.
 // ---------------------------------------------------------------------------------
-constexpr int kScanT = 1024, kScanE = 2048;
+constexpr int kScanT = 256, kScanU = 16, kScanE = kScanT * kScanU;
 
-__global__ void k_scan_block(const int *in, int *out, int n, int *bsum) {
-  __shared__ int s[kScanE];
-  int base = blockIdx.x * kScanE;
-  for (int t = threadIdx.x; t < kScanE; t += kScanT) s[t] = (base + t < n) ? in[base + t] : 0;
+__device__ __forceinline__ int scan_block_sum(int v, int *sh) {   // valid in every thread
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
   __syncthreads();
-  // Blelloch up-sweep / down-sweep
-  int off = 1;
-  for (int d = kScanE >> 1; d > 0; d >>= 1) {
-    __syncthreads();
-    if ((int)threadIdx.x < d) {
-      int ai = off * (2 * threadIdx.x + 1) - 1, bi = off * (2 * threadIdx.x + 2) - 1;
-      s[bi] += s[ai];
-    }
-    off <<= 1;
+  int r = 0;
+#pragma unroll
+  for (int w = 0; w < kScanT / 32; ++w) r += sh[w];
+  __syncthreads();
+  return r;
+}
+
+__global__ void __launch_bounds__(kScanT) k_scan_sum(const int *__restrict__ in, int n, int *bsum) {
+  __shared__ int sh[kScanT / 32];
+  const int base = blockIdx.x * kScanE;
+  int v = 0;
+#pragma unroll
+  for (int u = 0; u < kScanU; ++u) {
+    const int i = base + u * kScanT + threadIdx.x;
+    if (i < n) v += in[i];
   }
-  if (threadIdx.x == 0) { bsum[blockIdx.x] = s[kScanE - 1]; s[kScanE - 1] = 0; }
-  for (int d = 1; d < kScanE; d <<= 1) {
-    off >>= 1;
-    __syncthreads();
-    if ((int)threadIdx.x < d) {
-      int ai = off * (2 * threadIdx.x + 1) - 1, bi = off * (2 * threadIdx.x + 2) - 1;
-      int t = s[ai]; s[ai] = s[bi]; s[bi] += t;
-    }
+  v = scan_block_sum(v, sh);
+  if (threadIdx.x == 0) bsum[blockIdx.x] = v;
+}
+
+__global__ void __launch_bounds__(kScanT) k_scan_apply(const int *__restrict__ in, int *out, int n,
+                                                       const int *__restrict__ bsum, const int *w1, const int *w2,
+                                                       HostBox *box, unsigned token) {
+  __shared__ int sh[kScanT / 32];
+  __shared__ int e[kScanE + kScanE / 32];                // one pad word per 32
+  const int t = threadIdx.x, base = blockIdx.x * kScanE;
+  int v = 0;
+  for (int k = t; k < (int)blockIdx.x; k += kScanT) v += bsum[k];
+  const int before = scan_block_sum(v, sh);
+#pragma unroll
+  for (int u = 0; u < kScanU; ++u) {
+    const int k = u * kScanT + t, i = base + k;
+    e[k + (k >> 5)] = i < n ? in[i] : 0;
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < kScanE; t += kScanT)
-    if (base + t < n) out[base + t] = s[t];
-}
-
-__global__ void k_scan_sums(int *bsum, int nb, int *total) {
-  // one thread: nb is at most a few tens of thousands
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    int acc = 0;
-    for (int b = 0; b < nb; ++b) { int v = bsum[b]; bsum[b] = acc; acc += v; }
-    *total = acc;
+  int x[kScanU], sum = 0;
+#pragma unroll
+  for (int u = 0; u < kScanU; ++u) {
+    const int k = t * kScanU + u;
+    x[u] = sum;
+    sum += e[k + (k >> 5)];
+  }
+  int inc = sum;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, inc, o);
+    if ((t & 31) >= o) inc += y;
+  }
+  if ((t & 31) == 31) sh[t >> 5] = inc;
+  __syncthreads();
+  int off = before + inc - sum;
+  for (int w = 0; w < (t >> 5); ++w) off += sh[w];
+#pragma unroll
+  for (int u = 0; u < kScanU; ++u) {
+    const int k = t * kScanU + u;
+    e[k + (k >> 5)] = off + x[u];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < kScanU; ++u) {
+    const int k = u * kScanT + t, i = base + k;
+    if (i < n) out[i] = e[k + (k >> 5)];
+  }
+  if (blockIdx.x == gridDim.x - 1 && t == kScanT - 1) {
+    const int total = off + sum;
+    out[n] = total;
+    if (box) {
+      box->v[0] = total;
+      box->v[1] = w1 ? *w1 : 0;
+      box->v[2] = w2 ? *w2 : 0;
+      __threadfence_system();
+      *(volatile unsigned *)&box->token = token;
+    }
   }
 }
 
-__global__ void k_scan_add(int *out, int n, const int *bsum) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] += bsum[i / kScanE];
+// Wait for the box's words of the scan launched last: the host looks at the pinned token
+// instead of waiting for the stream and copying the words (15 us a time; this takes 5).
+static int box_wait(msg_ctx *c) {
+  for (unsigned it = 1;; ++it) {
+    if (*(volatile unsigned *)&c->box->token == c->box_token) break;
+    if ((it & 0x3f) == 0) std::this_thread::yield();   // more worker threads than cores
+    if ((it & 0xfff) == 0) {   // a failed kernel never writes the token
+      const cudaError_t e = cudaStreamQuery(c->stream);
+      if (e == cudaSuccess && *(volatile unsigned *)&c->box->token == c->box_token) break;
+      if (e != cudaErrorNotReady) {
+        set_error("scan: %s", e == cudaSuccess ? "no result" : cudaGetErrorString(e));
+        return MSG_ERR_CUDA;
+      }
+    }
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  return MSG_OK;
 }
 
-int scan_exclusive(msg_ctx *c, const int *in, int *out, int n, int *total_host) {
-  int nb = (n + kScanE - 1) / kScanE;
-  int *bsum = nullptr;
-  MSG_CUDA(cudaMallocAsync(&bsum, (size_t)(nb + 1) * 4, c->stream));
-  k_scan_block<<<nb, kScanT, 0, c->stream>>>(in, out, n, bsum);
-  MSG_CHECK_LAUNCH();
-  k_scan_sums<<<1, 32, 0, c->stream>>>(bsum, nb, bsum + nb);
-  MSG_CHECK_LAUNCH();
-  k_scan_add<<<nblk(n), kThreads, 0, c->stream>>>(out, n, bsum);
-  MSG_CHECK_LAUNCH();
-  if (total_host) {
-    MSG_CUDA(cudaMemcpyAsync(total_host, bsum + nb, 4, cudaMemcpyDeviceToHost, c->stream));
-    MSG_CUDA(cudaStreamSynchronize(c->stream));
+// out[0 .. n]: exclusive scan of in[0 .. n) and, at n, the total.  got, when given, receives
+// the total and the device words w1, w2 (waits for them).
+int scan_exclusive(msg_ctx *c, const int *in, int *out, int n, int *got, const int *w1, const int *w2) {
+  const int nb = std::max(1, (n + kScanE - 1) / kScanE);
+  if (nb > c->scan_cap) { set_error("scan: %d elements", n); return MSG_ERR_STATE; }
+  if (nb > 1) {
+    k_scan_sum<<<nb, kScanT, 0, c->stream>>>(in, n, c->scan_sums);
+    MSG_CHECK_LAUNCH();
   }
-  MSG_CUDA(cudaFreeAsync(bsum, c->stream));
+  if (got) c->box_token++;
+  k_scan_apply<<<nb, kScanT, 0, c->stream>>>(in, out, n, c->scan_sums, w1, w2, got ? c->box : nullptr, c->box_token);
+  MSG_CHECK_LAUNCH();
+  if (got) {
+    int rc = box_wait(c);
+    if (rc) return rc;
+    got[0] = c->box->v[0];
+    if (w1) got[1] = c->box->v[1];
+    if (w2) got[2] = c->box->v[2];
+  }
+  return MSG_OK;
+}
+
+// Scratch of the scans of up to n elements, and the box.
+int scan_reserve(msg_ctx *c, int n) {
+  c->scan_cap = (n + kScanE - 1) / kScanE + 1;
+  MSG_CUDA(cudaMalloc(&c->scan_sums, (size_t)c->scan_cap * 4));
+  MSG_CUDA(cudaMallocHost((void **)&c->box, sizeof(HostBox)));
+  memset(c->box, 0, sizeof(HostBox));
+  c->box_token = 0;
   return MSG_OK;
 }
 

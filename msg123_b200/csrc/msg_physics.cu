@@ -660,16 +660,15 @@ int build_connectivity(msg_ctx *c, const msg_grid_t *g) {
   MSG_CUDA(cudaMalloc(&cnt, N * 4));
   MSG_CUDA(cudaMalloc(&lcnt, N * 4));
   MSG_CUDA(cudaMalloc(&rcnt, N * 4));
-  MSG_CUDA(cudaMalloc(&lscan, N * 4));
-  MSG_CUDA(cudaMalloc(&rscan, N * 4));
+  MSG_CUDA(cudaMalloc(&lscan, (N + 1) * 4));
+  MSG_CUDA(cudaMalloc(&rscan, (N + 1) * 4));
   k_csr_count<<<nblk(c->N), kThreads, 0, c->stream>>>(gg, cnt, lcnt, rcnt);
   MSG_CHECK_LAUNCH();
-  int total = 0, tl = 0, tr = 0;
+  int total = 0;
   int rc;
   if ((rc = scan_exclusive(c, cnt, c->offind, c->N, &total))) return rc;
-  if ((rc = scan_exclusive(c, lcnt, lscan, c->N, &tl))) return rc;
-  if ((rc = scan_exclusive(c, rcnt, rscan, c->N, &tr))) return rc;
-  MSG_CUDA(cudaMemcpyAsync(c->offind + c->N, &total, 4, cudaMemcpyHostToDevice, c->stream));
+  if ((rc = scan_exclusive(c, lcnt, lscan, c->N, nullptr))) return rc;
+  if ((rc = scan_exclusive(c, rcnt, rscan, c->N, nullptr))) return rc;
   c->nnz = total;
   MSG_CUDA(cudaMalloc(&c->offrow, (size_t)total * 4));
   MSG_CUDA(cudaMalloc(&c->conn_dir, (size_t)total * 4));
