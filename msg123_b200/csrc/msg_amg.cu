@@ -628,6 +628,134 @@ __global__ void __launch_bounds__(NT) k_gj(int n, double *M, int *piv_out) {
   }
 }
 
+// The same inverse for n <= 128 with the matrix in the registers of one block: thread
+// (tr, tc) of 32 x 32 holds the elements (tr + 32 i, tc + 32 j).  The identity half is never
+// stored: its column of the row that becomes pivot p is still a unit vector then, so it takes
+// the place of column p, which no later step reads (perm keeps which row's it is); every
+// element sees the operations of the augmented elimination in the same order.  Per pivot:
+// column p and the two rows to swap through shared memory, two barriers, and 2 n^2 FP64
+// operations on one SM (512 cycles at n = 128).  The augmented matrix in global memory took
+// 0.50 ms at 76 rows and 0.84 ms at 128, six barriers and a read and a write of 2 n^2 values
+// from L2 per pivot; here 0.083 ms at 60 rows against 0.279.
+constexpr int kGjReg = 128;
+template <int NB>
+__global__ void __launch_bounds__(1024) k_gj_reg(int n, const int *__restrict__ rowptr, const int *__restrict__ col,
+                                                 const double *__restrict__ val, const double *__restrict__ diag,
+                                                 const double *__restrict__ dense, double *inv) {
+  __shared__ double scol[2][kGjReg], srow[2][kGjReg], spiv[2][kGjReg];
+  __shared__ int perm[kGjReg];
+  const int tc = threadIdx.x & 31, tr = threadIdx.x >> 5;
+  double m[NB][NB];
+#pragma unroll
+  for (int i = 0; i < NB; ++i)
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+      const int r = tr + 32 * i, c = tc + 32 * j;
+      m[i][j] = dense && r < n && c < n ? dense[(size_t)r * n + c] : 0.0;
+    }
+  if (!dense) {   // CSR rows with the diagonal apart
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const int r = tr + 32 * i;
+      if (r < n) {
+        for (int k = rowptr[r]; k < rowptr[r + 1]; ++k) {
+          const int c = col[k];
+          const double v = val[k];
+#pragma unroll
+          for (int j = 0; j < NB; ++j)
+            if (tc + 32 * j == c) m[i][j] = v;
+        }
+#pragma unroll
+        for (int j = 0; j < NB; ++j)
+          if (tc + 32 * j == r) m[i][j] = diag[r];
+      }
+    }
+  }
+  if (threadIdx.x < kGjReg) perm[threadIdx.x] = threadIdx.x;
+#pragma unroll
+  for (int pb = 0; pb < NB; ++pb)   // unrolled, so that m is never indexed by a variable
+  for (int p = 32 * pb; p < min(n, 32 * pb + 32); ++p) {
+    double *sc = scol[p & 1], *sr = srow[p & 1], *sp = spiv[p & 1];
+    if (tc == (p & 31)) {
+#pragma unroll
+      for (int i = 0; i < NB; ++i) sc[tr + 32 * i] = m[i][pb];
+    }
+    __syncthreads();
+    // every warp finds the pivot: largest magnitude, ties to the lowest row
+    double best = -1.0;
+    int piv = n;
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const int r = tc + 32 * i;
+      if (r >= p && r < n) {
+        const double v = fabs(sc[r]);
+        if (v > best) { best = v; piv = r; }
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const double v = __shfl_xor_sync(0xffffffffu, best, o);
+      const int r = __shfl_xor_sync(0xffffffffu, piv, o);
+      if (v > best || (v == best && r < piv)) { best = v; piv = r; }
+    }
+    if (piv == n) piv = p;   // a column of NaN
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const int r = tr + 32 * i;
+      if (r == p || r == piv) {
+#pragma unroll
+        for (int j = 0; j < NB; ++j) {
+          if (r == p) sr[tc + 32 * j] = m[i][j];
+          if (r == piv) sp[tc + 32 * j] = m[i][j];
+        }
+      }
+    }
+    if (threadIdx.x == 0 && piv != p) {
+      const int q = perm[p];
+      perm[p] = perm[piv];
+      perm[piv] = q;
+    }
+    __syncthreads();
+    const double pinv = __ddiv_rn(1.0, sc[piv]);
+    double prow[NB];
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+      const int c = tc + 32 * j;
+      prow[j] = __dmul_rn(c == p ? 1.0 : sp[c], pinv);
+    }
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const int r = tr + 32 * i;
+      const double f = r == piv ? sc[p] : sc[r];
+#pragma unroll
+      for (int j = 0; j < NB; ++j) {
+        const int c = tc + 32 * j;
+        double base = r == piv ? sr[c] : m[i][j];
+        if (c == p) base = 0.0;
+        if (r == p) base = prow[j];
+        else if (f != 0.0) base = __dsub_rn(base, __dmul_rn(f, prow[j]));
+        m[i][j] = base;
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < NB; ++i)
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+      const int r = tr + 32 * i, c = tc + 32 * j;
+      if (r < n && c < n) inv[(size_t)r * n + perm[c]] = m[i][j];
+    }
+}
+static int launch_gj_reg(int n, const int *rowptr, const int *col, const double *val, const double *diag,
+                         const double *dense, double *inv, cudaStream_t s) {
+  if (n <= 32) k_gj_reg<1><<<1, 1024, 0, s>>>(n, rowptr, col, val, diag, dense, inv);
+  else if (n <= 64) k_gj_reg<2><<<1, 1024, 0, s>>>(n, rowptr, col, val, diag, dense, inv);
+  else if (n <= 96) k_gj_reg<3><<<1, 1024, 0, s>>>(n, rowptr, col, val, diag, dense, inv);
+  else k_gj_reg<4><<<1, 1024, 0, s>>>(n, rowptr, col, val, diag, dense, inv);
+  MSG_CHECK_LAUNCH();
+  return MSG_OK;
+}
+
 // [A | I] from a dense row-major matrix
 __global__ void k_dense_fill_rm(int n, const double *a, double *M) {
   int i = blockIdx.x;
@@ -1299,6 +1427,10 @@ static int dense_inverse(msg_ctx *c, AmgLevel &L) {
   cudaStream_t s = c->stream;
   double *M = nullptr;
   int *piv = nullptr;
+  if (n <= kGjReg) {
+    if ((rc = halloc(c, &L.cinv, (size_t)n * n))) return rc;
+    return launch_gj_reg(n, L.rowptr, L.col, L.val, L.diag, nullptr, L.cinv, s);
+  }
   if ((rc = halloc(c, &M, (size_t)n * 2 * n))) return rc;
   if ((rc = halloc(c, &piv, 1))) return rc;
   if ((rc = halloc(c, &L.cinv, (size_t)n * n))) return rc;
@@ -1665,6 +1797,14 @@ MSG_API int msg_gpu_dense_inverse(int32_t n, const double *a, double *inv) {
   int *piv = nullptr;
   const size_t nn = (size_t)n * n;
   MSG_CUDA(cudaMalloc(&da, nn * 8));
+  if (n <= kGjReg) {
+    MSG_CUDA(cudaMalloc(&dinv, nn * 8));
+    MSG_CUDA(cudaMemcpy(da, a, nn * 8, cudaMemcpyHostToDevice));
+    int rc = launch_gj_reg(n, nullptr, nullptr, nullptr, nullptr, da, dinv, 0);
+    if (!rc) MSG_CUDA(cudaMemcpy(inv, dinv, nn * 8, cudaMemcpyDeviceToHost));
+    cudaFree(da); cudaFree(dinv);
+    return rc;
+  }
   MSG_CUDA(cudaMalloc(&M, 2 * nn * 8));
   MSG_CUDA(cudaMalloc(&dinv, nn * 8));
   MSG_CUDA(cudaMalloc(&piv, 4));
