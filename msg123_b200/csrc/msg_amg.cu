@@ -18,6 +18,7 @@
 #include <cuda_bf16.h>
 #include <vector>
 #include <algorithm>
+#include <type_traits>
 
 namespace cg = cooperative_groups;
 
@@ -44,60 +45,102 @@ struct AmgLevel {
 
 struct AmgState {
   std::vector<AmgLevel> lv;
-  int *col0 = nullptr;           // level-1 CSR columns, 0-based
-  double *val0 = nullptr;        // level-1 CSR values (from the DIA Jacobian)
-  int *cnt = nullptr;            // device counter
-  int *hcnt = nullptr;           // pinned
-  size_t cap_n = 0;              // scratch capacity (rows)
-  size_t sflag_cap = 0;
+  int *col0 = nullptr;           // level-1 CSR columns, 0-based (export)
+  int mis_dia = 0, mis_csr = 0;  // largest grids of the cooperative MIS-2 kernels
   double *r0 = nullptr, *t0 = nullptr;   // level-1 V-cycle work vectors
   float *x0f = nullptr, *t0f = nullptr, *r0f = nullptr;   // level-1 FP32 work vectors (precision = 1)
   float *b0f = nullptr;                                   // FP32 rounding of the cycle's right-hand side
-  // setup scratch
-  unsigned char *sflag = nullptr;
-  int *has = nullptr, *st = nullptr, *flag = nullptr, *aggid = nullptr, *agg2 = nullptr, *tmpi = nullptr;
-  unsigned long long *t0m = nullptr, *t1 = nullptr, *t2 = nullptr;
-  double *tdm = nullptr;
-  // mixed precision level-1 images
-  float *d1f = nullptr, *lu1f = nullptr;
-  // Device arena for everything one hierarchy build allocates (levels, transfer operators,
-  // Galerkin temporaries): a bump pointer reset at each rebuild, so rebuilds never go to
-  // the allocator.  A build that outgrows it takes the rest from the stream-ordered pool
-  // and the arena is enlarged before the next build.
+  // Device arena for everything one hierarchy build allocates: the levels grow from the
+  // bottom, reset at each rebuild; what only the building of one level needs (strength
+  // flags, MIS-2 words, products) grows from the top, reset after the level.  Rebuilds never
+  // go to the allocator; a build that outgrows the arena takes the rest from the
+  // stream-ordered pool and the arena is enlarged before the next build.
   char *arena = nullptr;
-  size_t arena_cap = 0, arena_used = 0, arena_spill = 0;
+  size_t arena_cap = 0, arena_used = 0, arena_tmp = 0, arena_spill = 0;
 };
 
 static AmgState *S(msg_ctx *c) { return reinterpret_cast<AmgState *>(c->amg); }
 static int nb(int n) { return (n + kThreads - 1) / kThreads; }
 
 // ---------------------------------------------------------------------------------
+// Hierarchy build.  Level 1 is read in its DIA form: six bands, and the strong ones of a
+// cell as six bits of a byte, so a pass of the aggregation reads bytes of the stencil
+// neighbours instead of row bounds, columns, flags and 8-byte tuples.  The coarser levels
+// are CSR; `scol` is their column array with -1 at the weak entries.  They are small, so
+// their passes are laid out for latency: eight lanes per row where a row is reduced, a warp
+// per row where its entries are matched with each other.
+// ---------------------------------------------------------------------------------
+struct Bands {   // level 1
+  int nx, ny, nz, nxy, N;
+  const double *d, *lu;
+};
+__device__ __forceinline__ int band_off(const Bands &g, int d) {
+  return d == 0 ? -g.nxy : d == 1 ? -g.nx : d == 2 ? -1 : d == 3 ? 1 : d == 4 ? g.nx : g.nxy;
+}
+
+// ---------------------------------------------------------------------------------
 // Strength filter (make_grapfilt, Make_amg_matrix.f90:67-111):
 //   strong(i,k) <=> lu_k^2 > |d_i d_j theta^2| and d_i d_j lu_k > 0
 //   tdm_i = d_i + sum of the weak lu_k in CSR order
 // ---------------------------------------------------------------------------------
-__global__ void k_strength(int n, const int *rowptr, const int *col, const double *val, const double *diag,
-                           double th2, unsigned char *sflag, int *has, double *tdm) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ bool strong_entry(double di, double dj, double lu, double th2) {
+  const double ddmat = __dmul_rn(di, dj);
+  return __dmul_rn(lu, lu) > fabs(__dmul_rn(ddmat, th2)) && __dmul_rn(ddmat, lu) > 0.0;
+}
+// 3D grid of 32 x 8 tiles: mask byte and starting state of each cell.
+__global__ void k_strength_dia(Bands g, double th2, unsigned char *msk, unsigned char *st) {
+  const int ix = blockIdx.x * 32 + threadIdx.x, iy = blockIdx.y * 8 + threadIdx.y, iz = blockIdx.z;
+  if (ix >= g.nx || iy >= g.ny) return;
+  const size_t N = g.N;
+  const int i = ix + g.nx * (iy + g.ny * iz);
+  const bool has[6] = {iz > 0, iy > 0, ix > 0, ix < g.nx - 1, iy < g.ny - 1, iz < g.nz - 1};
+  const double di = g.d[i];
+  unsigned m = 0;
+#pragma unroll
+  for (int d = 0; d < 6; ++d)
+    if (has[d] && strong_entry(di, g.d[i + band_off(g, d)], g.lu[d * N + i], th2)) m |= 1u << d;
+  msk[i] = (unsigned char)m;
+  st[i] = m ? 1 : 0;
+}
+// A warp per row.
+__global__ void __launch_bounds__(128) k_strength_csr(int n, const int *__restrict__ rowptr, const int *__restrict__ col,
+                                                      const double *__restrict__ val, const double *__restrict__ diag,
+                                                      double th2, int *scol, unsigned char *st, double *tdm) {
+  const int i = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (i >= n) return;
-  double di = diag[i], t = di;
-  int h = 0;
-  for (int k = rowptr[i]; k < rowptr[i + 1]; ++k) {
-    int j = col[k];
-    double ddmat = __dmul_rn(di, diag[j]);
-    double lu = val[k];
-    bool s = (__dmul_rn(lu, lu) > fabs(__dmul_rn(ddmat, th2))) && (__dmul_rn(ddmat, lu) > 0.0);
-    sflag[k] = s;
-    if (s) h = 1;
-    else t = __dadd_rn(t, lu);
+  const int b = rowptr[i], e = rowptr[i + 1];
+  const double di = diag[i];
+  double t = di;
+  bool any = false;
+  for (int k0 = b; k0 < e; k0 += 32) {
+    const int k = k0 + lane;
+    double lu = 0.0;
+    bool s = false;
+    if (k < e) {
+      const int j = col[k];
+      lu = val[k];
+      s = strong_entry(di, diag[j], lu, th2);
+      scol[k] = s ? j : -1;
+    }
+    any |= s;
+    for (unsigned w = __ballot_sync(0xffffffffu, k < e && !s); w; w &= w - 1)
+      t = __dadd_rn(t, __shfl_sync(0xffffffffu, lu, __ffs(w) - 1));
   }
-  has[i] = h;
-  tdm[i] = t;
+  any = __any_sync(0xffffffffu, any);
+  if (lane == 0) { tdm[i] = t; st[i] = any ? 1 : 0; }
 }
 
 // ---------------------------------------------------------------------------------
 // MIS-2 in synchronous rounds.  Tuple = state(2 bits) | hash priority(30) | index(32);
-// state 0 = decided non-root or no strong link (never wins), 1 = undecided, 2 = root.
+// state 0 = decided non-root or no strong link (never wins), 1 = undecided, 2 = root.  A round
+// takes the largest tuple of each node's strong neighbourhood (itself included) and the
+// largest of those over the neighbourhood again; an undecided node that finds itself becomes
+// a root, one that finds a root drops out.
+//
+// All rounds run in one cooperative launch, a grid barrier between the two halves of a
+// round, and end with the first round that leaves nothing undecided.  The first half keeps
+// only whose tuple won (level 1: direction and state in a byte; CSR: index and state in a
+// word); the second makes the tuple again from the index, cheaper than 8-byte gathers.
 // ---------------------------------------------------------------------------------
 __device__ __forceinline__ unsigned mis_hash(unsigned x, unsigned lev) {
   x ^= 0x9e3779b9u * (lev + 1u);
@@ -109,93 +152,255 @@ __device__ __forceinline__ unsigned long long mis_tuple(int state, int i, int le
   return ((unsigned long long)state << 62) | ((unsigned long long)(mis_hash((unsigned)i, (unsigned)lev) & 0x3fffffffu) << 32) |
          (unsigned long long)(unsigned)i;
 }
+// few, large blocks: a barrier of the grid costs with the number of blocks; a level of at most
+// kMisSmall rows runs in one cluster, whose barrier is the hardware's
+constexpr int kMisSmall = 1 << 14, kMisCluster = 8;
+constexpr int kMisRounds = 64, kMisBlock = 512;
+constexpr unsigned kMisFinal = 1u << 29;   // CSR word: state in the two top bits, this, index (below 2^29)
 
-__global__ void k_mis_init(int n, const int *has, int *st) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) st[i] = has[i] ? 1 : 0;
+__device__ __forceinline__ void mis_decide(int i, unsigned long long t, unsigned char *st, bool &und) {
+  if ((unsigned)(t & 0xffffffffull) == (unsigned)i) st[i] = 2;
+  else if ((t >> 62) == 2ull) st[i] = 0;
+  else und = true;
+}
+// undecided nodes of the round, one atomic per warp
+__device__ __forceinline__ void mis_count(bool und, int *cnt) {
+  const unsigned b = __ballot_sync(0xffffffffu, und);
+  if ((threadIdx.x & 31) == 0 && b) atomicAdd(cnt, __popc(b));
 }
 
-// FROM_STATE: source tuples computed from st; else read from src.
-__global__ void k_mis_tuple(int n, const int *st, unsigned long long *t0, int lev) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) t0[i] = mis_tuple(st[i], i, lev);
-}
-
-__global__ void k_mis_max(int n, const int *rowptr, const int *col, const unsigned char *sflag,
-                          const unsigned long long *src, unsigned long long *dst) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  unsigned long long m = src[i];
-  for (int k = rowptr[i]; k < rowptr[i + 1]; ++k) {
-    if (!sflag[k]) continue;
-    unsigned long long v = src[col[k]];
-    if (v > m) m = v;
-  }
-  dst[i] = m;
-}
-
-// Decide the undecided nodes of this round and write the next round's tuples (t0); when
-// `undecided` is given, count the nodes still undecided (one atomic per warp).
-__global__ void k_mis_update(int n, int *st, const unsigned long long *t2, unsigned long long *t0, int lev,
-                             int *undecided) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  bool und = false;
-  if (i < n) {
-    int s = st[i];
-    if (s == 1) {
-      unsigned long long t = t2[i];
-      if ((unsigned)(t & 0xffffffffull) == (unsigned)i) s = 2;
-      else if ((t >> 62) == 2ull) s = 0;
-      else und = true;
-      st[i] = s;
+// Four neighbouring cells per thread (the byte arrays are padded to a multiple of four): one
+// load passes over four that are done.
+__global__ void __launch_bounds__(kMisBlock) k_mis_dia(Bands g, const unsigned char *__restrict__ msk, unsigned char *st,
+                                                       unsigned char *w1, int lev, int *cnt) {
+  const int nth = gridDim.x * blockDim.x, t0 = blockIdx.x * blockDim.x + threadIdx.x;
+  const int nq = (g.N + 3) / 4, nq32 = (nq + 31) & ~31;
+  for (int round = 0; round < kMisRounds; ++round) {
+    for (int t = t0; t < nq; t += nth) {
+      unsigned w = round > 0 ? reinterpret_cast<unsigned *>(w1)[t] : 0u;
+      if ((w & 0x80808080u) == 0x80808080u) continue;
+      const unsigned m4 = reinterpret_cast<const unsigned *>(msk)[t], s4 = reinterpret_cast<unsigned *>(st)[t];
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        const int i = 4 * t + v;
+        if (i < g.N && !(w >> (8 * v) & 128u)) {
+          const unsigned m = m4 >> (8 * v) & 255u;
+          const int s = s4 >> (8 * v) & 255u;
+          unsigned code = 6, ws = s;   // itself
+          bool fin = s != 1;
+          if (m) {
+            unsigned long long best = mis_tuple(s, i, lev);
+#pragma unroll
+            for (int d = 0; d < 6; ++d)
+              if (m >> d & 1) {
+                const int j = i + band_off(g, d), sj = st[j];
+                const unsigned long long u = mis_tuple(sj, j, lev);
+                if (u > best) { best = u; code = d; ws = sj; }
+                fin = fin && sj != 1;
+              }
+          }
+          w = (w & ~(255u << (8 * v))) | (code | ws << 3 | (fin ? 128u : 0u)) << (8 * v);
+        }
+      }
+      reinterpret_cast<unsigned *>(w1)[t] = w;
     }
-    t0[i] = mis_tuple(s, i, lev);
-  }
-  if (undecided) {
-    unsigned b = __ballot_sync(0xffffffffu, und);
-    if ((threadIdx.x & 31) == 0 && b) atomicAdd(undecided, __popc(b));
+    cg::this_grid().sync();
+    for (int t = t0; t < nq32; t += nth) {
+      int open = 0;
+      const unsigned s4 = t < nq ? reinterpret_cast<unsigned *>(st)[t] : 0u;
+      if (s4 & 0x01010101u) {   // state 1 is the only odd one
+        const unsigned m4 = reinterpret_cast<const unsigned *>(msk)[t];
+        auto tup = [&](int j) {
+          const unsigned w = w1[j], code = w & 7u;
+          return mis_tuple(w >> 3 & 3u, code == 6 ? j : j + band_off(g, code), lev);
+        };
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          const int i = 4 * t + v;
+          if (i < g.N && (s4 >> (8 * v) & 1u)) {
+            const unsigned m = m4 >> (8 * v) & 255u;
+            unsigned long long best = tup(i);
+#pragma unroll
+            for (int d = 0; d < 6; ++d)
+              if (m >> d & 1) {
+                const unsigned long long u = tup(i + band_off(g, d));
+                if (u > best) best = u;
+              }
+            bool und = false;
+            mis_decide(i, best, st, und);
+            open += und;
+          }
+        }
+      }
+      open = (int)__reduce_add_sync(0xffffffffu, (unsigned)open);
+      if ((threadIdx.x & 31) == 0 && open) atomicAdd(cnt + round, open);
+    }
+    cg::this_grid().sync();
+    if (*(volatile int *)(cnt + round) == 0) break;
   }
 }
 
-__global__ void k_root_flag(int n, const int *st, int *flag) {
+// eight lanes of a row: the largest of their values, in all of them
+__device__ __forceinline__ unsigned long long max8(unsigned long long v) {
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) {
+    const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
+    if (w > v) v = w;
+  }
+  return v;
+}
+__device__ __forceinline__ unsigned long long max4(unsigned long long v) {
+#pragma unroll
+  for (int o = 2; o > 0; o >>= 1) {
+    const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
+    if (w > v) v = w;
+  }
+  return v;
+}
+// Four lanes per row, each with four entries in flight: the passes wait for the chain row
+// bounds -> column -> word.
+template <bool CLUSTER>
+__global__ void __launch_bounds__(kMisBlock) k_mis_csr(int n, const int *__restrict__ rowptr, const int *__restrict__ scol,
+                                                       unsigned char *st, unsigned *w1, int lev, int *cnt) {
+  auto sync_all = [] {
+    if (CLUSTER) cg::this_cluster().sync();
+    else cg::this_grid().sync();
+  };
+  const int q = threadIdx.x & 3;
+  const int nrow = (gridDim.x * blockDim.x) >> 2, r0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
+  const int n8 = (n + 7) & ~7;   // all eight rows of a warp stay in the loop
+  // fn of the lane's strong neighbours in row i
+  auto each = [&](int i, auto word, auto fn) {
+    const int e = rowptr[i + 1];
+    for (int k = rowptr[i] + q; k < e; k += 16) {
+      int j[4];
+      unsigned w[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) j[u] = k + 4 * u < e ? scol[k + 4 * u] : -1;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) w[u] = j[u] >= 0 ? word(j[u]) : 0u;
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (j[u] >= 0) fn(j[u], w[u]);
+    }
+  };
+  for (int round = 0; round < kMisRounds; ++round) {
+    for (int i = r0; i < n8; i += nrow) {
+      unsigned long long best = 0ull;
+      const bool todo = i < n && (round == 0 || !(w1[i] & kMisFinal));
+      if (!__any_sync(0xffffffffu, todo)) continue;
+      bool open = false;   // something undecided in the neighbourhood
+      if (todo) {
+        if (q == 0) {
+          const int si = st[i];
+          best = mis_tuple(si, i, lev);
+          open = si == 1;
+        }
+        each(i, [&](int j) { return (unsigned)st[j]; },
+             [&](int j, unsigned sj) {
+               const unsigned long long v = mis_tuple((int)sj, j, lev);
+               if (v > best) best = v;
+               open = open || sj == 1;
+             });
+      }
+      best = max4(best);
+      const bool fin = !(__ballot_sync(0xffffffffu, open) >> (threadIdx.x & 28) & 0xfu);
+      if (todo && q == 0)
+        w1[i] = (unsigned)(best >> 62) << 30 | (fin ? kMisFinal : 0u) | (unsigned)(best & (kMisFinal - 1u));
+    }
+    sync_all();
+    for (int i = r0; i < n8; i += nrow) {
+      unsigned long long best = 0ull;
+      const bool open = i < n && st[i] == 1;
+      if (!__any_sync(0xffffffffu, open)) continue;
+      auto tup = [&](unsigned w) { return mis_tuple(w >> 30, (int)(w & (kMisFinal - 1u)), lev); };
+      if (open) {
+        if (q == 0) best = tup(w1[i]);
+        each(i, [&](int j) { return w1[j]; },
+             [&](int, unsigned w) {
+               const unsigned long long v = tup(w);
+               if (v > best) best = v;
+             });
+      }
+      best = max4(best);
+      bool und = false;
+      if (open && q == 0) mis_decide(i, best, st, und);
+      mis_count(und, cnt + round);
+    }
+    sync_all();
+    if (*(volatile int *)(cnt + round) == 0) break;
+  }
+}
+
+__global__ void k_root_flag(int n, const unsigned char *st, int *flag) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) flag[i] = (st[i] == 2);
 }
 
 // pass A: roots keep their id; others join the best root among strong neighbours
-__global__ void k_agg_a(int n, const int *rowptr, const int *col, const unsigned char *sflag, const int *st,
-                        const int *aggid, int *agg2, int lev) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+__global__ void k_agg_a_dia(Bands g, const unsigned char *__restrict__ msk, const unsigned char *__restrict__ st,
+                            const int *__restrict__ aggid, int *agg2, int lev) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= g.N) return;
   if (st[i] == 2) { agg2[i] = aggid[i]; return; }
-  unsigned long long best = 0; int bj = -1;
-  for (int k = rowptr[i]; k < rowptr[i + 1]; ++k) {
-    if (!sflag[k]) continue;
-    int j = col[k];
-    if (st[j] == 2) {
-      unsigned long long v = mis_tuple(1, j, lev);
-      if (v > best) { best = v; bj = j; }
+  const unsigned m = msk[i];
+  unsigned long long best = 0;
+  int bj = -1;
+#pragma unroll
+  for (int d = 0; d < 6; ++d)
+    if (m >> d & 1) {
+      const int j = i + band_off(g, d);
+      if (st[j] == 2) {
+        const unsigned long long v = mis_tuple(1, j, lev);
+        if (v > best) { best = v; bj = j; }
+      }
     }
-  }
   agg2[i] = bj >= 0 ? aggid[bj] : -1;
 }
-
 // pass B: unassigned rows join the best already-assigned strong neighbour
-__global__ void k_agg_b(int n, const int *rowptr, const int *col, const unsigned char *sflag, const int *agg2,
-                        int *agg, int lev) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  if (agg2[i] >= 0) { agg[i] = agg2[i]; return; }
-  unsigned long long best = 0; int bj = -1;
-  for (int k = rowptr[i]; k < rowptr[i + 1]; ++k) {
-    if (!sflag[k]) continue;
-    int j = col[k];
-    if (agg2[j] >= 0) {
-      unsigned long long v = mis_tuple(1, j, lev);
-      if (v > best) { best = v; bj = j; }
-    }
+__global__ void k_agg_b_dia(Bands g, const unsigned char *__restrict__ msk, const int *__restrict__ agg2, int *agg,
+                            int lev) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= g.N) return;
+  int a = agg2[i];
+  if (a < 0) {
+    const unsigned m = msk[i];
+    unsigned long long best = 0;
+    int bj = -1;
+#pragma unroll
+    for (int d = 0; d < 6; ++d)
+      if (m >> d & 1) {
+        const int j = i + band_off(g, d);
+        if (agg2[j] >= 0) {
+          const unsigned long long v = mis_tuple(1, j, lev);
+          if (v > best) { best = v; bj = j; }
+        }
+      }
+    a = bj >= 0 ? agg2[bj] : -1;
   }
-  agg[i] = bj >= 0 ? agg2[bj] : -1;
+  agg[i] = a;
+}
+// Passes A (ROOTS) and B of a CSR level, eight lanes per row.
+template <bool ROOTS>
+__global__ void __launch_bounds__(256) k_agg_csr(int n, const int *__restrict__ rowptr, const int *__restrict__ scol,
+                                                 const unsigned char *__restrict__ st, const int *__restrict__ in,
+                                                 int *out, int lev) {
+  const int q = threadIdx.x & 7, i = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+  unsigned long long best = 0;
+  bool own = true;
+  if (i < n) {
+    own = ROOTS ? st[i] == 2 : in[i] >= 0;
+    if (!own)
+      for (int k = rowptr[i] + q; k < rowptr[i + 1]; k += 8) {
+        const int j = scol[k];
+        if (j >= 0 && (ROOTS ? st[j] == 2 : in[j] >= 0)) {
+          const unsigned long long v = mis_tuple(1, j, lev);
+          if (v > best) best = v;
+        }
+      }
+  }
+  best = max8(best);
+  if (i < n && q == 0) out[i] = own ? in[i] : best ? in[(unsigned)(best & 0xffffffffull)] : -1;
 }
 
 // ---------------------------------------------------------------------------------
@@ -203,348 +408,436 @@ __global__ void k_agg_b(int n, const int *rowptr, const int *col, const unsigned
 //   columns in first-appearance order over the strong neighbours (CSR order), then
 //   the row's own aggregate; values v = -sum lu over strong j of that aggregate,
 //   v = v*omega/tdm, own += 1 - omega.
+// The fill pass also counts the entries of each column (the rows of R).
 // ---------------------------------------------------------------------------------
 constexpr int kPRowMax = 96;   // longer prolongation rows stop the coarsening (CPU oracle: same rule)
-__global__ void k_p_count(int n, const int *rowptr, const int *col, const unsigned char *sflag, const int *agg,
-                          int *cnt, int *overflow) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int list[kPRowMax];
-  int m = 0;
-  bool ovf = false;
-  for (int k = rowptr[i]; k < rowptr[i + 1]; ++k) {
-    if (!sflag[k]) continue;
-    int J = agg[col[k]];
-    if (J < 0) continue;
-    bool f = false;
-    for (int q = 0; q < m; ++q) if (list[q] == J) { f = true; break; }
-    if (!f) { if (m < kPRowMax) list[m++] = J; else ovf = true; }
+template <bool FILL>
+__global__ void k_p_dia(Bands g, const unsigned char *__restrict__ msk, const int *__restrict__ agg, double om,
+                        int *cnt, const int *__restrict__ pptr, int *pcol, double *pval, int *rcnt) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= g.N) return;
+  const size_t N = g.N;
+  const unsigned m = msk[i];
+  const int own = agg[i];
+  if (!m) {   // no strong neighbour: in no aggregate
+    if (!FILL) cnt[i] = 0;
+    return;
   }
-  int own = agg[i];
-  if (own >= 0) {
-    bool f = false;
-    for (int q = 0; q < m; ++q) if (list[q] == own) { f = true; break; }
-    if (!f) { if (m < kPRowMax) list[m++] = own; else ovf = true; }
+  int J[7];
+  unsigned first = 0;
+#pragma unroll
+  for (int d = 0; d < 7; ++d) {
+    J[d] = d < 6 ? (m >> d & 1 ? agg[i + band_off(g, d)] : -1) : own;
+    bool f = J[d] >= 0;
+#pragma unroll
+    for (int e = 0; e < d; ++e) f = f && J[e] != J[d];
+    first |= (unsigned)f << d;
   }
-  if (ovf) atomicExch(overflow, 1);
-  cnt[i] = m;
+  if (!FILL) { cnt[i] = __popc(first); return; }
+  double lu[6], t = g.d[i];
+  {
+    const int iz = i / g.nxy, rem = i - iz * g.nxy, iy = rem / g.nx, ix = rem - iy * g.nx;
+    const bool has[6] = {iz > 0, iy > 0, ix > 0, ix < g.nx - 1, iy < g.ny - 1, iz < g.nz - 1};
+#pragma unroll
+    for (int d = 0; d < 6; ++d) {
+      lu[d] = has[d] ? g.lu[d * N + i] : 0.0;
+      if (has[d] && !(m >> d & 1)) t = __dadd_rn(t, lu[d]);
+    }
+  }
+  int o = pptr[i];
+#pragma unroll
+  for (int d = 0; d < 7; ++d)
+    if (first >> d & 1) {
+      double v = 0.0;
+#pragma unroll
+      for (int e = 0; e < 6; ++e)
+        if (e >= d && J[e] == J[d]) v = __dsub_rn(v, lu[e]);
+      v = __ddiv_rn(__dmul_rn(v, om), t);
+      if (J[d] == own) v = __dsub_rn(__dadd_rn(v, 1.0), om);
+      pcol[o] = J[d];
+      pval[o] = v;
+      ++o;
+      atomicAdd(&rcnt[J[d]], 1);
+    }
 }
 
-__global__ void k_p_fill(int n, const int *rowptr, const int *col, const double *val, const unsigned char *sflag,
-                         const int *agg, const double *tdm, double om, const int *pptr, int *pcol, double *pval) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int b = pptr[i], e = pptr[i + 1];
-  int m = 0;
-  for (int k = rowptr[i]; k < rowptr[i + 1]; ++k) {
-    if (!sflag[k]) continue;
-    int J = agg[col[k]];
-    if (J < 0) continue;
-    int q;
-    for (q = 0; q < m; ++q) if (pcol[b + q] == J) break;
-    if (q == m && b + m < e) { pcol[b + m] = J; pval[b + m] = 0.0; m++; }
+// A warp per row of a CSR level: the aggregates of the strong neighbours in entry order (and
+// the own one last) as a list in shared memory; an entry whose aggregate stands nowhere
+// before it opens a column, and adds up the values of the entries that match it, in order.
+// Rows hold at most kHashMax off-diagonals (longer Galerkin rows stop the coarsening); a list
+// of that length would leave a quarter of the warps in flight, so rows beyond kPShort entries
+// are collected by the count pass and go through a launch of their own (LONG).
+constexpr int kHashMax = 700, kPShort = 64;
+template <bool FILL, bool LONG>
+__global__ void __launch_bounds__(128) k_p_csr(int n, const int *__restrict__ rowptr, const int *__restrict__ scol,
+                                               const double *__restrict__ val, const int *__restrict__ agg,
+                                               const double *__restrict__ tdm, double om, int *cnt, int *overflow,
+                                               int *longrows, int *nlong, const int *__restrict__ pptr, int *pcol,
+                                               double *pval, int *rcnt) {
+  constexpr int CAP = (LONG ? kHashMax : kPShort) + 4;
+  __shared__ int sj[4][CAP];
+  __shared__ double sv[4][FILL ? CAP : 1];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nr = LONG ? *nlong : n;
+  int *J = sj[w];
+  double *V = sv[w];
+  for (int rid = blockIdx.x * 4 + w; rid < nr; rid += gridDim.x * 4) {
+    const int i = LONG ? longrows[rid] : rid, b = rowptr[i], e = rowptr[i + 1], own = agg[i];
+    if (!LONG && e - b > kPShort) {
+      if (!FILL && lane == 0) longrows[atomicAdd(nlong, 1)] = i;
+      continue;
+    }
+    int m = 0;
+    for (int k0 = b; k0 < e; k0 += 32) {
+      const int k = k0 + lane, j = k < e ? scol[k] : -1, a = j >= 0 ? agg[j] : -1;
+      const unsigned bal = __ballot_sync(0xffffffffu, a >= 0);
+      if (a >= 0) {
+        const int pos = m + __popc(bal & ((1u << lane) - 1u));
+        J[pos] = a;
+        if (FILL) V[pos] = val[k];
+      }
+      m += __popc(bal);
+    }
+    const int len = m + (own >= 0 ? 1 : 0);
+    if (own >= 0 && lane == 0) J[m] = own;
+    __syncwarp();
+    int cols = 0;
+    for (int t0 = 0; t0 < len; t0 += 32) {
+      const int t = t0 + lane;
+      bool f = t < len;
+      const int a = f ? J[t] : -1;
+      for (int u = 0; u < t && f; ++u) f = J[u] != a;
+      const unsigned bal = __ballot_sync(0xffffffffu, f);
+      if (FILL && f) {
+        double v = 0.0;
+        for (int u = t; u < m; ++u)
+          if (J[u] == a) v = __dsub_rn(v, V[u]);
+        v = __ddiv_rn(__dmul_rn(v, om), tdm[i]);
+        if (a == own) v = __dsub_rn(__dadd_rn(v, 1.0), om);
+        const int o = pptr[i] + cols + __popc(bal & ((1u << lane) - 1u));
+        pcol[o] = a;
+        pval[o] = v;
+        atomicAdd(&rcnt[a], 1);
+      }
+      cols += __popc(bal);
+    }
+    if (!FILL && lane == 0) {
+      cnt[i] = min(cols, kPRowMax);
+      if (cols > kPRowMax) atomicExch(overflow, 1);
+    }
+    __syncwarp();
   }
-  int own = agg[i];
-  if (own >= 0) {
-    int q;
-    for (q = 0; q < m; ++q) if (pcol[b + q] == own) break;
-    if (q == m && b + m < e) { pcol[b + m] = own; pval[b + m] = 0.0; m++; }
-  }
-  if (m == 0) return;
-  for (int k = rowptr[i]; k < rowptr[i + 1]; ++k) {
-    if (!sflag[k]) continue;
-    int J = agg[col[k]];
-    if (J < 0) continue;
-    for (int q = 0; q < m; ++q)
-      if (pcol[b + q] == J) { pval[b + q] = __dsub_rn(pval[b + q], val[k]); break; }
-  }
-  double t = tdm[i];
-  for (int q = 0; q < m; ++q) pval[b + q] = __ddiv_rn(__dmul_rn(pval[b + q], om), t);
-  if (own >= 0)
-    for (int q = 0; q < m; ++q)
-      if (pcol[b + q] == own) { pval[b + q] = __dsub_rn(__dadd_rn(pval[b + q], 1.0), om); break; }
 }
 
-// R = P^T: counts, atomic fill, then sort every row by fine index (keys are unique).
-__global__ void k_r_count(int pnnz, const int *pcol, int *rcnt) {
-  int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < pnnz) atomicAdd(&rcnt[pcol[q]], 1);
-}
+// R = P^T: the entries fill their counted rows in any order, each with its row beside it; an
+// entry's place in the row is then the number of smaller fine indexes there (keys are
+// unique), a thread per entry reading a row of a few cached words.
 __global__ void k_r_fill(int nf, const int *pptr, const int *pcol, const double *pval, const int *rptr, int *fill,
-                         int *rcol, double *rval) {
+                         int *trow, int *tcol, double *tval) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nf) return;
   for (int q = pptr[i]; q < pptr[i + 1]; ++q) {
     int J = pcol[q];
     int pos = rptr[J] + atomicAdd(&fill[J], 1);
-    rcol[pos] = i;
-    rval[pos] = pval[q];
+    trow[pos] = J;
+    tcol[pos] = i;
+    tval[pos] = pval[q];
   }
 }
-// one warp per row; rank sort in shared memory (rows up to 1024 entries, longer rows
-// fall back to an in-place insertion sort by lane 0)
-constexpr int kRSortCap = 1024;
-__global__ void __launch_bounds__(128) k_r_sort(int nc, const int *rptr, int *rcol, double *rval) {
-  __shared__ int sc[4][kRSortCap];
-  __shared__ double sv[4][kRSortCap];
-  int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int row = blockIdx.x * 4 + w;
-  if (row >= nc) return;
-  int b = rptr[row], m = rptr[row + 1] - b;
-  if (m <= 1) return;
-  if (m > kRSortCap) {
-    if (lane == 0) {
-      for (int a = 1; a < m; ++a) {
-        int c0 = rcol[b + a]; double v0 = rval[b + a]; int q = a - 1;
-        while (q >= 0 && rcol[b + q] > c0) { rcol[b + q + 1] = rcol[b + q]; rval[b + q + 1] = rval[b + q]; --q; }
-        rcol[b + q + 1] = c0; rval[b + q + 1] = v0;
-      }
-    }
-    return;
-  }
-  for (int t = lane; t < m; t += 32) { sc[w][t] = rcol[b + t]; sv[w][t] = rval[b + t]; }
-  __syncwarp();
-  for (int t = lane; t < m; t += 32) {
-    int key = sc[w][t], rank = 0;
-    for (int u = 0; u < m; ++u) rank += (sc[w][u] < key);
-    rcol[b + rank] = key;
-    rval[b + rank] = sv[w][t];
-  }
+__global__ void k_r_rank(int nnz, const int *__restrict__ rptr, const int *__restrict__ trow,
+                         const int *__restrict__ tcol, const double *__restrict__ tval, int *rcol, double *rval,
+                         float *rval_f) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= nnz) return;
+  const int J = trow[e], b = rptr[J], end = rptr[J + 1], key = tcol[e];
+  int o = b;
+  for (int u = b; u < end; ++u) o += tcol[u] < key;
+  const double v = tval[e];
+  rcol[o] = key;
+  rval[o] = v;
+  if (rval_f) rval_f[o] = (float)v;
 }
 
 // ---------------------------------------------------------------------------------
 // Row-wise sparse product C = A*B with deterministic accumulation: A's entries of a
-// row are visited in order (its diagonal first when given), and for each of them the
-// lanes of a warp add coef*B(j,:) into a per-warp hash table.  B's rows hold unique
-// columns, so within one step every table slot receives at most one addition: each
-// column is summed in the order of A's entries, the order the CPU oracle uses.
-// Output columns ascending; with split_diag the diagonal goes to cdiag (1.0 if absent).
-// PASS 0 counts, PASS 1 writes.  Rows with more than kHashMax distinct columns set
-// *overflow, and the caller stops coarsening at that level.
+// row are visited in order (its diagonal first when given), and the products that fall on
+// one column are added in that order, the order the CPU oracle uses.
+//
+// A row's number of products is known from the row lengths alone, so its result goes to a
+// place of that size (`start`, a scan of the product counts) and its length beside it; no
+// pass counts distinct columns first.  A*P is read back through start and length as it
+// stands; the Galerkin operator, which stays, is then copied together, ascending columns,
+// diagonal apart (1.0 if absent).  More than kHashMax distinct columns set *overflow, and the
+// caller stops coarsening at that level.
 // ---------------------------------------------------------------------------------
-constexpr int kHash = 1024, kHashMax = 700, kSpgWarps = 3, kPf = 8;
-constexpr int kHashSmall = 256, kSmallMaxCols = 120;   // fill-pass table for rows of <= 120 columns
+constexpr int kShort = 64;   // products of a short row
 
-// HASH = table slots per warp.  The fill pass (PASS 1) knows each row's column count from
-// the count pass: rows of at most kSmallMaxCols columns go through the kHashSmall variant
-// (a quarter of the shared memory, twice the resident warps), the others through kHash.
-template <int PASS, int HASH = kHash>
-__global__ void __launch_bounds__(32 * kSpgWarps) k_spgemm(const int *nrows, const int *ap, const int *ac, const double *av,
-                                                           const double *adiag, const int *bp, const int *bc,
-                                                           const double *bv, int split_diag, int *ocnt,
-                                                           const int *cptr, int *ccol, double *cval, double *cdiag,
-                                                           int *overflow, const int *rows) {
-  constexpr int kComp = (HASH < kHashMax ? HASH : kHashMax) + 32;
-  __shared__ int hk[kSpgWarps][HASH];
-  __shared__ double hv[kSpgWarps][PASS == 1 ? HASH : 1];
-  __shared__ int comp[kSpgWarps][kComp];
+struct Spg {
+  const int *ap, *ac;            // A: rows, columns
+  const double *av, *adiag;      // values, diagonal (null: none)
+  const int *bs, *bl, *bc;       // B: row starts, lengths (null: bs[j + 1] - bs[j]), columns
+  const double *bv;
+  int split;                     // C's diagonal goes to cdiag and rows are sorted
+  const int *start;              // place of each row of C
+  int *len, *ccol;
+  double *cval, *cdiag;
+  __device__ __forceinline__ int blen(int j) const { return bl ? bl[j] : bs[j + 1] - bs[j]; }
+};
+
+// Products of each row, eight lanes per row.
+__global__ void __launch_bounds__(256) k_spg_bound(int n, Spg s, int *cnt) {
+  const int q = threadIdx.x & 7, i = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+  int m = 0;
+  if (i < n) {
+    if (s.adiag && q == 0) m = s.blen(i);
+    for (int k = s.ap[i] + q; k < s.ap[i + 1]; k += 8) m += s.blen(s.ac[k]);
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
+  if (i < n && q == 0) cnt[i] = m;
+}
+
+// A warp per row.  The lanes take an entry of A each (its B row's bounds), then a product each
+// (its entry by bisection of the entries' prefix sums), so a window of 32 products is loaded
+// together whatever the row lengths, the next one ahead of the current one's additions.
+// The window's columns are entered in a hash table together; its values are then added entry
+// by entry: B's rows hold unique columns, so within one entry a slot receives at most one
+// addition.
+// T: table slots.  T = kTabShort handles rows 0 .. *nrows of at most kShort products and
+// appends the others to `next`; the larger tables walk a list of rows and pass on to `next`
+// those whose columns fill more than three quarters of the table; the largest reports them.
+// (A list per row in which each product looks for its column took 1.5 times as long on rows
+// of 40 to 60 products and 6 times on rows of 500.)
+constexpr int kTabShort = 128, kTabMid = 256, kTabMax = 1024;
+template <int T>
+struct SpgShape {
+  static constexpr int warps = T == kTabMax ? 3 : 4;
+};
+template <int T>
+__global__ void __launch_bounds__(32 * SpgShape<T>::warps) k_spg_row(Spg s, int n, const int *__restrict__ nrows,
+                                                                     const int *__restrict__ rows, int *next,
+                                                                     int *nnext, int *overflow) {
+  constexpr int W = SpgShape<T>::warps, kCols = T == kTabMax ? kHashMax : T == kTabShort ? T : T * 3 / 4;
+  constexpr unsigned mask = T - 1;
+  __shared__ __align__(16) int hk[W][T + 4];
+  __shared__ double hv[W][T];
+  __shared__ unsigned short comp[W][T];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int *K = hk[w];
   double *V = hv[w];
-  const int nr = *nrows;
-  for (int rid = blockIdx.x * kSpgWarps + w; rid < nr; rid += gridDim.x * kSpgWarps) {
-    const int row = rows[rid];
-    int a0 = ap[row], a1 = ap[row + 1];
-    int start = adiag ? a0 - 1 : a0;
-    int m = 0;
-    if (PASS == 1) {
-      // columns of this row (from the count pass; + 1 for a split-off diagonal)
-      m = cptr[row + 1] - cptr[row] + (split_diag ? 1 : 0);
-      if ((HASH == kHashSmall) != (m <= kSmallMaxCols)) continue;   // the other variant's row
-    } else {
-      // products of this row -> table size (load factor <= 1/2 when it fits)
-      for (int k = start + lane; k < a1; k += 32) {
-        int j = (k < a0) ? row : ac[k];
-        m += bp[j + 1] - bp[j];
-      }
-      for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
+  const int nr = rows ? *nrows : n;
+  for (int rid = blockIdx.x * W + w; rid < nr; rid += gridDim.x * W) {
+    const int row = rows ? rows[rid] : rid, o = s.start[row];
+    if (T == kTabShort && s.start[row + 1] - o > kShort) {
+      if (lane == 0) next[atomicAdd(nnext, 1)] = row;
+      continue;
     }
-    int T = 32;
-    while (T < 2 * m && T < HASH) T <<= 1;
-    const unsigned mask = (unsigned)T - 1u;
-    for (int t = lane; t < T; t += 32) { K[t] = -1; if (PASS == 1) V[t] = 0.0; }
+#pragma unroll
+    for (int t = lane; t < T; t += 32) { K[t] = -1; V[t] = 0.0; }
     __syncwarp();
-    // PASS 0 only counts distinct columns: no values are loaded, multiplied or added
-    auto add = [&](int cc, double p) {
-      unsigned hsh = ((unsigned)cc * 2654435761u) & mask;
-      for (int probe = 0; probe < T; ++probe) {
-        int cur = atomicCAS(&K[hsh], -1, cc);
-        if (cur == -1 || cur == cc) {
-          if (PASS == 1) V[hsh] = __dadd_rn(V[hsh], p);
-          break;
-        }
-        hsh = (hsh + 1) & mask;
+    const int a0 = s.ap[row], a1 = s.ap[row + 1];
+    int fresh = 0;   // columns this lane opened
+    bool full = false;
+    for (int k0 = a0 - (s.adiag ? 1 : 0); k0 < a1 && !full; k0 += 32) {
+      const int k = k0 + lane;
+      int j = row, b0 = 0, len = 0;
+      double coef = 0.0;
+      if (k < a1) {
+        if (k >= a0) { j = s.ac[k]; coef = s.av[k]; }
+        else coef = s.adiag[row];
+        b0 = s.bs[j];
+        len = s.blen(j);
       }
-    };
-    // kPf entries of A at a time: their B rows (up to 32 entries, one per lane) are loaded
-    // together, so the dependent loads of A's column -> B's row bounds -> B's entries overlap
-    // across entries; they are then added in entry order exactly as one at a time.
-    for (int kb = start; kb < a1; kb += kPf) {
-      int cols[kPf], lens[kPf];
-      double vals[kPf];
+      int inc = len;
 #pragma unroll
-      for (int u = 0; u < kPf; ++u) {
-        const int k = kb + u;
-        lens[u] = 0; cols[u] = -1; vals[u] = 0.0;
-        if (k < a1) {
-          int j;
-          double coef = 0.0;
-          if (k < a0) { j = row; if (PASS == 1) coef = adiag[row]; }
-          else { j = ac[k]; if (PASS == 1) coef = av[k]; }
-          const int b0 = bp[j], len = bp[j + 1] - b0;
-          lens[u] = len;
-          if (lane < len) {
-            cols[u] = bc[b0 + lane];
-            if (PASS == 1) vals[u] = __dmul_rn(coef, bv[b0 + lane]);
+      for (int p = 1; p < 32; p <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, inc, p);
+        if (lane >= p) inc += y;
+      }
+      const int tot = __shfl_sync(0xffffffffu, inc, 31), rel = b0 - (inc - len);   // product t at rel + t
+      // window of product t0 + lane: entry, column, value
+      auto load = [&](int t0, int &e, int &c, double &v) {
+        const int t = t0 + lane;
+        e = 0;   // entries that end at or before product t
+#pragma unroll
+        for (int p = 16; p > 0; p >>= 1)
+          if (__shfl_sync(0xffffffffu, inc, e + p - 1) <= t) e += p;
+        const int at = __shfl_sync(0xffffffffu, rel, e) + t;
+        const double cf = __shfl_sync(0xffffffffu, coef, e);
+        c = -1;
+        v = 0.0;
+        if (t < tot) {
+          c = s.bc[at];
+          v = __dmul_rn(cf, s.bv[at]);
+        } else {
+          e = 32;
+        }
+      };
+      int e, c;
+      double v;
+      if (tot > 0) load(0, e, c, v);
+      for (int t0 = 0; t0 < tot; t0 += 32) {
+        int e1 = 32, c1 = -1;
+        double v1 = 0.0;
+        if (t0 + 32 < tot) load(t0 + 32, e1, c1, v1);
+        unsigned slot = 0;
+        if (c >= 0) {
+          slot = ((unsigned)c * 2654435761u) >> 20 & mask;
+          for (int probe = 0; probe < T; ++probe) {
+            const int cur = atomicCAS(&K[slot], -1, c);
+            if (cur == -1 || cur == c) { fresh += cur == -1; break; }
+            slot = (slot + 1) & mask;
           }
         }
-      }
-#pragma unroll
-      for (int u = 0; u < kPf; ++u) {
-        const int k = kb + u;
-        if (k < a1) {
-          if (lens[u] <= 32) {
-            if (lane < lens[u]) add(cols[u], vals[u]);
-          } else {   // a B row longer than the warp: the whole row again, in chunks
-            int j;
-            double coef = 0.0;
-            if (k < a0) { j = row; if (PASS == 1) coef = adiag[row]; }
-            else { j = ac[k]; if (PASS == 1) coef = av[k]; }
-            for (int q = bp[j] + lane; q < bp[j + 1]; q += 32) add(bc[q], PASS == 1 ? __dmul_rn(coef, bv[q]) : 0.0);
-          }
+        // entry by entry, in order
+        for (int q = __shfl_sync(0xffffffffu, e, 0);; ) {
+          if (e == q) V[slot] = __dadd_rn(V[slot], v);
+          __syncwarp();
+          const unsigned later = __ballot_sync(0xffffffffu, e > q && e < 32);
+          if (!later) break;
+          q = __shfl_sync(0xffffffffu, e, __ffs(later) - 1);
         }
-        __syncwarp();
+        e = e1; c = c1; v = v1;
+        if (T != kTabShort) {
+          full = __reduce_add_sync(0xffffffffu, fresh) > kCols;
+          if (full) break;
+        }
       }
     }
-    // compact occupied slots
+    if (T != kTabShort && full) {
+      if (lane == 0) {
+        s.len[row] = 0;
+        if (T == kTabMax) atomicExch(overflow, 1);
+        else next[atomicAdd(nnext, 1)] = row;
+      }
+      __syncwarp();
+      continue;
+    }
+    // compact: the u-th occupied slot's number to comp[u], its key to K[u] (u is at most the
+    // slot's own number, and a slot is read before a later one writes below it)
     int u = 0;
-    for (int base = 0; base < T; base += 32) {
-      int t = base + lane;
-      bool occ = K[t] >= 0;
-      unsigned bal = __ballot_sync(0xffffffffu, occ);
-      if (occ) {
-        int pos = u + __popc(bal & ((1u << lane) - 1));
-        if (pos < kComp) comp[w][pos] = t;
-      }
-      u += __popc(bal);
-    }
-    __syncwarp();
-    if (u > kHashMax) {
-      if (lane == 0) { atomicExch(overflow, 1); if (PASS == 0) ocnt[row] = 0; }
-      __syncwarp();
-      continue;
-    }
     bool hasd = false;
-    if (split_diag) {
-      for (int t = lane; t < u; t += 32) if (K[comp[w][t]] == row) hasd = true;
-      hasd = __any_sync(0xffffffffu, hasd);
-    }
-    if (PASS == 0) {
-      if (lane == 0) ocnt[row] = u - (hasd ? 1 : 0);
-      __syncwarp();
-      continue;
-    }
-    // rank sort by column
-    int out0 = cptr[row];
-    if (split_diag && lane == 0) cdiag[row] = 1.0;
-    __syncwarp();
-    for (int t = lane; t < u; t += 32) {
-      int slot = comp[w][t];
-      int key = K[slot];
-      if (split_diag && key == row) { cdiag[row] = V[slot]; continue; }
-      int rank = 0;
-      for (int v = 0; v < u; ++v) {
-        int k2 = K[comp[w][v]];
-        if (split_diag && k2 == row) continue;
-        rank += (k2 < key);
+    for (int base = 0; base < T; base += 32) {
+      const int t = base + lane, key = K[t];
+      const bool diag = s.split && key == row, occ = key >= 0 && !diag;
+      const unsigned bal = __ballot_sync(0xffffffffu, occ);
+      if (occ) {
+        const int pos = u + __popc(bal & ((1u << lane) - 1));
+        comp[w][pos] = (unsigned short)t;
+        K[pos] = key;
       }
-      ccol[out0 + rank] = key;
-      cval[out0 + rank] = V[slot];
+      if (diag) { s.cdiag[row] = V[t]; hasd = true; }
+      u += __popc(bal);
+      __syncwarp();
     }
+    hasd = __any_sync(0xffffffffu, hasd);
+    if (s.split && !hasd && lane == 0) s.cdiag[row] = 1.0;
+    if (lane < 4) K[u + lane] = 0x7fffffff;   // the rank loop reads four at a time
+    __syncwarp();
+    // rank sort by column
+    for (int t = lane; t < u; t += 32) {
+      const int key = K[t];
+      int rank = t;
+      if (s.split) {
+        rank = 0;
+        for (int q = 0; q < u; q += 4) {
+          const int4 k4 = *reinterpret_cast<const int4 *>(K + q);
+          rank += (k4.x < key) + (k4.y < key) + (k4.z < key) + (k4.w < key);
+        }
+      }
+      s.ccol[o + rank] = key;
+      s.cval[o + rank] = V[comp[w][t]];
+    }
+    if (lane == 0) s.len[row] = u;
     __syncwarp();
   }
 }
 
-
-// Thread-per-row variant for short rows (at most kTU distinct columns): the products
-// are summed one by one in generation order, exactly the CPU oracle's loop.  The column
-// set lives in registers (fully unrolled, predicated search, insert and sorting network:
-// no dynamically indexed local memory).  Rows that need more columns are appended to
-// `longrows` (PASS 0) or skipped (PASS 1) and go through the warp kernel above.
-constexpr int kTU = 16, kTM = 64;
-template <int PASS>
-__global__ void __launch_bounds__(128) k_spgemm_t(int nrows, const int *ap, const int *ac, const double *av,
-                                                  const double *adiag, const int *bp, const int *bc, const double *bv,
-                                                  int split_diag, int *ocnt, const int *cptr, int *ccol, double *cval,
-                                                  double *cdiag, int *longrows, int *nlong) {
-  int row = blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= nrows) return;
-  int uc[kTU];
-  double uv[kTU];
+// A*P on level 1: a thread per cell walks its bands (diagonal first) and the prolongation
+// rows behind them (0 to 3 entries, most one or none) and keeps the columns it has met in
+// shared memory (8 to 10 where there are any; as an unrolled search through registers this
+// took twice as long); the rare row of more than kTU columns works in its place in memory.
+constexpr int kTU = 12, kApT = 128;
+__global__ void k_ap_bound_dia(Bands g, const int *__restrict__ pptr, int *cnt) {
+  const int ix = blockIdx.x * 32 + threadIdx.x, iy = blockIdx.y * 8 + threadIdx.y, iz = blockIdx.z;
+  if (ix >= g.nx || iy >= g.ny) return;
+  const int i = ix + g.nx * (iy + g.ny * iz);
+  const bool has[6] = {iz > 0, iy > 0, ix > 0, ix < g.nx - 1, iy < g.ny - 1, iz < g.nz - 1};
+  int m = pptr[i + 1] - pptr[i];
 #pragma unroll
-  for (int t = 0; t < kTU; ++t) { uc[t] = 0x7fffffff; uv[t] = 0.0; }
+  for (int d = 0; d < 6; ++d)
+    if (has[d]) {
+      const int j = i + band_off(g, d);
+      m += pptr[j + 1] - pptr[j];
+    }
+  cnt[i] = m;
+}
+__global__ void __launch_bounds__(kApT) k_ap_dia(Bands g, const int *__restrict__ pptr, const int *__restrict__ pcol,
+                                                 const double *__restrict__ pval, const int *__restrict__ start,
+                                                 int *len, int *ccol, double *cval) {
+  __shared__ int uc[kTU][kApT];
+  __shared__ double uv[kTU][kApT];
+  const int ix = blockIdx.x * 32 + threadIdx.x, iy = blockIdx.y * (kApT / 32) + threadIdx.y, iz = blockIdx.z;
+  if (ix >= g.nx || iy >= g.ny) return;
+  const int tt = threadIdx.y * 32 + threadIdx.x;
+  const size_t N = g.N;
+  const int i = ix + g.nx * (iy + g.ny * iz);
+  const bool has[7] = {true, iz > 0, iy > 0, ix > 0, ix < g.nx - 1, iy < g.ny - 1, iz < g.nz - 1};
+  int q0[7], q1[7], fc[7], any = 0;
+  double fv[7];
+  // bounds and first entry of the seven prolongation rows, all loads in flight together
+#pragma unroll
+  for (int e = 0; e < 7; ++e) {
+    const int j = e == 0 ? i : i + band_off(g, e - 1);
+    q0[e] = has[e] ? pptr[j] : 0;
+    q1[e] = has[e] ? pptr[j + 1] : 0;
+    any |= q1[e] - q0[e];
+  }
+  if (!any) { len[i] = 0; return; }
+#pragma unroll
+  for (int e = 0; e < 7; ++e) {
+    fc[e] = q0[e] < q1[e] ? pcol[q0[e]] : -1;
+    fv[e] = q0[e] < q1[e] ? __dmul_rn(e == 0 ? g.d[i] : g.lu[(e - 1) * N + i], pval[q0[e]]) : 0.0;
+  }
+  const int o = start[i];
   int u = 0;
-  int a0 = ap[row], a1 = ap[row + 1];
-  int m = 0;
-  for (int k = adiag ? a0 - 1 : a0; k < a1; ++k) {
-    int j = (k < a0) ? row : ac[k];
-    m += bp[j + 1] - bp[j];
-  }
-  if (m > kTM) {   // long product list: the warp kernel is faster
-    if (PASS == 0) longrows[atomicAdd(nlong, 1)] = row;
-    return;
-  }
-  for (int k = adiag ? a0 - 1 : a0; k < a1; ++k) {
-    int j = (k < a0) ? row : ac[k];
-    double coef = (PASS == 0) ? 0.0 : ((k < a0) ? adiag[row] : av[k]);
-    for (int q = bp[j]; q < bp[j + 1]; ++q) {
-      int cc = bc[q];
-      double p = (PASS == 0) ? 0.0 : __dmul_rn(coef, bv[q]);   // PASS 0 counts columns only
-      bool found = false;
+  auto add = [&](int cc, double p) {
+    const int m = min(u, kTU);
+    for (int t = 0; t < m; ++t)
+      if (uc[t][tt] == cc) { uv[t][tt] = __dadd_rn(uv[t][tt], p); return; }
+    for (int t = kTU; t < u; ++t)
+      if (ccol[o + t] == cc) { cval[o + t] = __dadd_rn(cval[o + t], p); return; }
+    if (u < kTU) { uc[u][tt] = cc; uv[u][tt] = p; }
+    else { ccol[o + u] = cc; cval[o + u] = p; }
+    ++u;
+  };
 #pragma unroll
-      for (int t = 0; t < kTU; ++t)
-        if (uc[t] == cc) { if (PASS == 1) uv[t] = __dadd_rn(uv[t], p); found = true; }
-      if (!found) {
-        if (u == kTU) {   // too many columns for the register set
-          if (PASS == 0) { longrows[atomicAdd(nlong, 1)] = row; }
-          return;
-        }
-#pragma unroll
-        for (int t = 0; t < kTU; ++t)
-          if (t == u) { uc[t] = cc; uv[t] = p; }
-        ++u;
-      }
+  for (int e = 0; e < 7; ++e) {
+    if (fc[e] < 0) continue;
+    add(fc[e], fv[e]);
+    if (q0[e] + 1 < q1[e]) {
+      const double coef = e == 0 ? g.d[i] : g.lu[(e - 1) * N + i];
+      for (int q = q0[e] + 1; q < q1[e]; ++q) add(pcol[q], __dmul_rn(coef, pval[q]));
     }
   }
-  if (PASS == 0) {
-    int hasd = 0;
-    if (split_diag) {
-#pragma unroll
-      for (int t = 0; t < kTU; ++t) hasd |= (uc[t] == row);
-    }
-    ocnt[row] = u - hasd;
-    return;
+  len[i] = u;
+  for (int t = 0; t < min(u, kTU); ++t) { ccol[o + t] = uc[t][tt]; cval[o + t] = uv[t][tt]; }
+}
+
+// The Galerkin rows copied together, eight lanes per row, and their FP32 / BF16 images.
+__global__ void __launch_bounds__(256) k_spg_pack(int n, const int *__restrict__ start, const int *__restrict__ ptr,
+                                                  const int *__restrict__ tcol, const double *__restrict__ tval,
+                                                  const double *__restrict__ diag, int *col, double *val,
+                                                  __nv_bfloat16 *val_h, float *diag_f) {
+  const int q = threadIdx.x & 7, i = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+  if (i >= n) return;
+  const int s = start[i], o = ptr[i], m = ptr[i + 1] - o;
+  for (int k = q; k < m; k += 8) {
+    const double v = tval[s + k];
+    col[o + k] = tcol[s + k];
+    val[o + k] = v;
+    if (val_h) val_h[o + k] = __double2bfloat16(v);
   }
-  // odd-even transposition sort by column (empty slots hold INT_MAX and stay last)
-#pragma unroll
-  for (int r = 0; r < kTU; ++r) {
-#pragma unroll
-    for (int t = r & 1; t + 1 < kTU; t += 2) {
-      if (uc[t] > uc[t + 1]) {
-        int ci = uc[t]; uc[t] = uc[t + 1]; uc[t + 1] = ci;
-        double cv = uv[t]; uv[t] = uv[t + 1]; uv[t + 1] = cv;
-      }
-    }
-  }
-  int o = cptr[row];
-  if (split_diag) cdiag[row] = 1.0;
-#pragma unroll
-  for (int t = 0; t < kTU; ++t) {
-    if (t < u) {
-      if (split_diag && uc[t] == row) { cdiag[row] = uv[t]; continue; }
-      ccol[o] = uc[t]; cval[o] = uv[t]; ++o;
-    }
-  }
+  if (q == 0 && diag_f) diag_f[i] = (float)diag[i];
 }
 
 // ---------------------------------------------------------------------------------
@@ -629,34 +922,36 @@ __global__ void __launch_bounds__(NT) k_gj(int n, double *M, int *piv_out) {
 }
 
 // The same inverse for n <= 128 with the matrix in the registers of one block: thread
-// (tr, tc) of 32 x 32 holds the elements (tr + 32 i, tc + 32 j).  The identity half is never
+// (tr, tc) of 16 x 32 holds the elements (tr + 16 i, tc + 32 j).  The identity half is never
 // stored: its column of the row that becomes pivot p is still a unit vector then, so it takes
 // the place of column p, which no later step reads (perm keeps which row's it is); every
 // element sees the operations of the augmented elimination in the same order.  Per pivot:
-// column p and the two rows to swap through shared memory, two barriers, and 2 n^2 FP64
+// column p and the two rows to swap through shared memory, three barriers, and 2 n^2 FP64
 // operations on one SM (512 cycles at n = 128).  The augmented matrix in global memory took
 // 0.50 ms at 76 rows and 0.84 ms at 128, six barriers and a read and a write of 2 n^2 values
 // from L2 per pivot; here 0.083 ms at 60 rows against 0.279.
 constexpr int kGjReg = 128;
 template <int NB>
-__global__ void __launch_bounds__(1024) k_gj_reg(int n, const int *__restrict__ rowptr, const int *__restrict__ col,
+__global__ void __launch_bounds__(512) k_gj_reg(int n, const int *__restrict__ rowptr, const int *__restrict__ col,
                                                  const double *__restrict__ val, const double *__restrict__ diag,
                                                  const double *__restrict__ dense, double *inv) {
   __shared__ double scol[2][kGjReg], srow[2][kGjReg], spiv[2][kGjReg];
-  __shared__ int perm[kGjReg];
+  __shared__ int perm[kGjReg], s_piv;
+  __shared__ double s_pinv;
   const int tc = threadIdx.x & 31, tr = threadIdx.x >> 5;
-  double m[NB][NB];
+  constexpr int NR = 2 * NB;
+  double m[NR][NB];
 #pragma unroll
-  for (int i = 0; i < NB; ++i)
+  for (int i = 0; i < NR; ++i)
 #pragma unroll
     for (int j = 0; j < NB; ++j) {
-      const int r = tr + 32 * i, c = tc + 32 * j;
+      const int r = tr + 16 * i, c = tc + 32 * j;
       m[i][j] = dense && r < n && c < n ? dense[(size_t)r * n + c] : 0.0;
     }
   if (!dense) {   // CSR rows with the diagonal apart
 #pragma unroll
-    for (int i = 0; i < NB; ++i) {
-      const int r = tr + 32 * i;
+    for (int i = 0; i < NR; ++i) {
+      const int r = tr + 16 * i;
       if (r < n) {
         for (int k = rowptr[r]; k < rowptr[r + 1]; ++k) {
           const int c = col[k];
@@ -678,29 +973,40 @@ __global__ void __launch_bounds__(1024) k_gj_reg(int n, const int *__restrict__ 
     double *sc = scol[p & 1], *sr = srow[p & 1], *sp = spiv[p & 1];
     if (tc == (p & 31)) {
 #pragma unroll
-      for (int i = 0; i < NB; ++i) sc[tr + 32 * i] = m[i][pb];
+      for (int i = 0; i < NR; ++i) sc[tr + 16 * i] = m[i][pb];
     }
     __syncthreads();
-    // every warp finds the pivot: largest magnitude, ties to the lowest row
-    double best = -1.0;
-    int piv = n;
+    // one warp finds the pivot: largest magnitude (its bits, which order as the values do; a
+    // NaN does not count), ties to the lowest row
+    if (tr == 0) {
+      unsigned hi = 0, lo = 0;
+      int row = n;
 #pragma unroll
-    for (int i = 0; i < NB; ++i) {
-      const int r = tc + 32 * i;
-      if (r >= p && r < n) {
-        const double v = fabs(sc[r]);
-        if (v > best) { best = v; piv = r; }
+      for (int i = 0; i < NB; ++i) {
+        const int r = tc + 32 * i;
+        if (r >= p && r < n) {
+          const double v = fabs(sc[r]);
+          const unsigned h = (unsigned)__double2hiint(v) | 0x80000000u, l = (unsigned)__double2loint(v);
+          if (v == v && (h > hi || (h == hi && l > lo))) { hi = h; lo = l; row = r; }
+        }
+      }
+      const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+      const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+      row = (int)__reduce_min_sync(0xffffffffu, hi == mh && lo == ml ? (unsigned)row : (unsigned)n);
+      if (row == n) row = p;   // a column of NaN
+      if (tc == 0) {
+        s_piv = row;
+        s_pinv = __ddiv_rn(1.0, sc[row]);
+        const int q = perm[p];
+        perm[p] = perm[row];
+        perm[row] = q;
       }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      const double v = __shfl_xor_sync(0xffffffffu, best, o);
-      const int r = __shfl_xor_sync(0xffffffffu, piv, o);
-      if (v > best || (v == best && r < piv)) { best = v; piv = r; }
-    }
-    if (piv == n) piv = p;   // a column of NaN
+    __syncthreads();
+    const int piv = s_piv;
 #pragma unroll
-    for (int i = 0; i < NB; ++i) {
-      const int r = tr + 32 * i;
+    for (int i = 0; i < NR; ++i) {
+      const int r = tr + 16 * i;
       if (r == p || r == piv) {
 #pragma unroll
         for (int j = 0; j < NB; ++j) {
@@ -709,49 +1015,49 @@ __global__ void __launch_bounds__(1024) k_gj_reg(int n, const int *__restrict__ 
         }
       }
     }
-    if (threadIdx.x == 0 && piv != p) {
-      const int q = perm[p];
-      perm[p] = perm[piv];
-      perm[piv] = q;
-    }
     __syncthreads();
-    const double pinv = __ddiv_rn(1.0, sc[piv]);
+    const double pinv = s_pinv;
+    // only the block column pb holds column p, whose place the identity's column takes
+    const bool mine = tc == (p & 31);
     double prow[NB];
 #pragma unroll
-    for (int j = 0; j < NB; ++j) {
-      const int c = tc + 32 * j;
-      prow[j] = __dmul_rn(c == p ? 1.0 : sp[c], pinv);
-    }
+    for (int j = 0; j < NB; ++j) prow[j] = __dmul_rn(j == pb && mine ? 1.0 : sp[tc + 32 * j], pinv);
 #pragma unroll
-    for (int i = 0; i < NB; ++i) {
-      const int r = tr + 32 * i;
-      const double f = r == piv ? sc[p] : sc[r];
+    for (int i = 0; i < NR; ++i) {
+      const int r = tr + 16 * i;   // the same in all lanes of the warp
+      if (r == p) {
 #pragma unroll
-      for (int j = 0; j < NB; ++j) {
-        const int c = tc + 32 * j;
-        double base = r == piv ? sr[c] : m[i][j];
-        if (c == p) base = 0.0;
-        if (r == p) base = prow[j];
-        else if (f != 0.0) base = __dsub_rn(base, __dmul_rn(f, prow[j]));
-        m[i][j] = base;
+        for (int j = 0; j < NB; ++j) m[i][j] = prow[j];
+        continue;
+      }
+      double f = sc[r];
+      if (r == piv) {
+        f = sc[p];
+#pragma unroll
+        for (int j = 0; j < NB; ++j) m[i][j] = sr[tc + 32 * j];
+      }
+      if (mine) m[i][pb] = 0.0;
+      if (f != 0.0) {
+#pragma unroll
+        for (int j = 0; j < NB; ++j) m[i][j] = __dsub_rn(m[i][j], __dmul_rn(f, prow[j]));
       }
     }
   }
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < NB; ++i)
+  for (int i = 0; i < NR; ++i)
 #pragma unroll
     for (int j = 0; j < NB; ++j) {
-      const int r = tr + 32 * i, c = tc + 32 * j;
+      const int r = tr + 16 * i, c = tc + 32 * j;
       if (r < n && c < n) inv[(size_t)r * n + perm[c]] = m[i][j];
     }
 }
 static int launch_gj_reg(int n, const int *rowptr, const int *col, const double *val, const double *diag,
                          const double *dense, double *inv, cudaStream_t s) {
-  if (n <= 32) k_gj_reg<1><<<1, 1024, 0, s>>>(n, rowptr, col, val, diag, dense, inv);
-  else if (n <= 64) k_gj_reg<2><<<1, 1024, 0, s>>>(n, rowptr, col, val, diag, dense, inv);
-  else if (n <= 96) k_gj_reg<3><<<1, 1024, 0, s>>>(n, rowptr, col, val, diag, dense, inv);
-  else k_gj_reg<4><<<1, 1024, 0, s>>>(n, rowptr, col, val, diag, dense, inv);
+  if (n <= 32) k_gj_reg<1><<<1, 512, 0, s>>>(n, rowptr, col, val, diag, dense, inv);
+  else if (n <= 64) k_gj_reg<2><<<1, 512, 0, s>>>(n, rowptr, col, val, diag, dense, inv);
+  else if (n <= 96) k_gj_reg<3><<<1, 512, 0, s>>>(n, rowptr, col, val, diag, dense, inv);
+  else k_gj_reg<4><<<1, 512, 0, s>>>(n, rowptr, col, val, diag, dense, inv);
   MSG_CHECK_LAUNCH();
   return MSG_OK;
 }
@@ -1184,9 +1490,6 @@ __global__ void k_gemv_mixed(int n, const double *Ci, const float *b, float *x) 
 __global__ void k_d2f(int n, const double *a, float *b) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) b[i] = (float)a[i];
 }
-__global__ void k_d2h(int n, const double *a, __nv_bfloat16 *b) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) b[i] = __double2bfloat16(a[i]);
-}
 __global__ void k_f2d(int n, const float *a, double *b) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) b[i] = (double)a[i];
 }
@@ -1204,7 +1507,7 @@ template <typename T>
 static int halloc(msg_ctx *c, T **p, size_t n) {
   AmgState *A = S(c);
   const size_t bytes = ((n ? n : 1) * sizeof(T) + 255) & ~(size_t)255;
-  if (A->arena && A->arena_used + bytes <= A->arena_cap) {
+  if (A->arena && A->arena_used + A->arena_tmp + bytes <= A->arena_cap) {
     *p = reinterpret_cast<T *>(A->arena + A->arena_used);
     A->arena_used += bytes;
     return MSG_OK;
@@ -1213,6 +1516,32 @@ static int halloc(msg_ctx *c, T **p, size_t n) {
   MSG_CUDA(cudaMallocAsync((void **)p, bytes, c->stream));
   return MSG_OK;
 }
+
+// Temporaries of one level's building, given back together (stream order: the next level's
+// kernels may take the memory over).
+struct Temps {
+  msg_ctx *c;
+  std::vector<void *> pool;
+  explicit Temps(msg_ctx *ctx) : c(ctx) {}
+  ~Temps() {
+    S(c)->arena_tmp = 0;
+    for (void *q : pool) cudaFreeAsync(q, c->stream);
+  }
+  template <typename T>
+  int get(T **p, size_t n) {
+    AmgState *A = S(c);
+    const size_t bytes = ((n ? n : 1) * sizeof(T) + 255) & ~(size_t)255;
+    if (A->arena && A->arena_used + A->arena_tmp + bytes <= A->arena_cap) {
+      A->arena_tmp += bytes;
+      *p = reinterpret_cast<T *>(A->arena + A->arena_cap - A->arena_tmp);
+      return MSG_OK;
+    }
+    A->arena_spill += bytes;
+    MSG_CUDA(cudaMallocAsync((void **)p, bytes, c->stream));
+    pool.push_back(*p);
+    return MSG_OK;
+  }
+};
 
 // Release a pointer from halloc: arena memory is reclaimed at the next reset.
 static void hfree(AmgState *A, void *q, cudaStream_t s) {
@@ -1235,188 +1564,176 @@ static int dalloc(msg_ctx *c, T **p, size_t n) {
   return MSG_OK;
 }
 
-static int ensure_scratch(msg_ctx *c, AmgState *A, size_t n, size_t nnz) {
-  if (A->cap_n >= n && A->sflag) return MSG_OK;
+// C = A*B into rows of the places `start` (their scan, product counts by `bound`); long rows
+// through the hash kernels.  *ovf: device word set when a row has too many columns.
+static int spgemm_rows(msg_ctx *c, Temps &tmp, int n, Spg &g, int *cnt, int *ovf) {
   cudaStream_t s = c->stream;
-  void *p[] = {A->sflag, A->has, A->st, A->flag, A->aggid, A->agg2, A->tmpi, A->t0m, A->t1, A->t2, A->tdm};
-  for (void *q : p) if (q) cudaFreeAsync(q, s);
-  size_t cn = std::max(n, (size_t)1024);
-  int rc;
-  A->sflag_cap = std::max(nnz, cn * 7);
-  if ((rc = dalloc(c, &A->sflag, A->sflag_cap))) return rc;
-  if ((rc = dalloc(c, &A->has, cn))) return rc;
-  if ((rc = dalloc(c, &A->st, cn))) return rc;
-  if ((rc = dalloc(c, &A->flag, cn))) return rc;
-  if ((rc = dalloc(c, &A->aggid, cn + 1))) return rc;
-  if ((rc = dalloc(c, &A->agg2, cn))) return rc;
-  if ((rc = dalloc(c, &A->tmpi, cn + 1))) return rc;
-  if ((rc = dalloc(c, &A->t0m, cn))) return rc;
-  if ((rc = dalloc(c, &A->t1, cn))) return rc;
-  if ((rc = dalloc(c, &A->t2, cn))) return rc;
-  if ((rc = dalloc(c, &A->tdm, cn))) return rc;
-  A->cap_n = cn;
-  return MSG_OK;
-}
-
-static int read_counter(msg_ctx *c, AmgState *A, int *v) {
-  MSG_CUDA(cudaMemcpyAsync(A->hcnt, A->cnt, 4, cudaMemcpyDeviceToHost, c->stream));
-  MSG_CUDA(cudaStreamSynchronize(c->stream));
-  *v = *A->hcnt;
-  return MSG_OK;
-}
-
-
-// C = A*B (optionally with A's diagonal first, optionally splitting C's diagonal).
-// On return *cptr / *ccol / *cval (and cdiag) are allocated; *ovf set when a row
-// exceeds the warp kernel's table, in which case nothing is allocated.
-static int spgemm(msg_ctx *c, AmgState *A, int nrows, const int *ap, const int *ac, const double *av,
-                  const double *adiag, const int *bp, const int *bc, const double *bv, int split_diag, int **cptr,
-                  int **ccol, double **cval, double *cdiag, int *cnnz, int *ovf) {
-  cudaStream_t s = c->stream;
-  int rc;
-  int *cnt = nullptr, *longrows = nullptr, *nl = nullptr;   // nl: long rows, overflow flag
-  *ovf = 0;
-  if ((rc = halloc(c, &cnt, nrows + 1))) return rc;
-  if ((rc = halloc(c, &longrows, nrows + 1))) return rc;
-  if ((rc = halloc(c, &nl, 2))) return rc;
+  int rc, total = 0, *start = nullptr, *longrows = nullptr, *biggest = nullptr, *nl = nullptr;
+  k_spg_bound<<<(8 * (long long)n + 255) / 256, 256, 0, s>>>(n, g, cnt);
+  MSG_CHECK_LAUNCH();
+  if ((rc = tmp.get(&start, n + 1)) || (rc = tmp.get(&longrows, n)) || (rc = tmp.get(&biggest, n)) ||
+      (rc = tmp.get(&nl, 2)) || (rc = tmp.get(&g.len, n)))
+    return rc;
   MSG_CUDA(cudaMemsetAsync(nl, 0, 8, s));
-  k_spgemm_t<0><<<(nrows + 127) / 128, 128, 0, s>>>(nrows, ap, ac, av, adiag, bp, bc, bv, split_diag, cnt, nullptr,
-                                                   nullptr, nullptr, nullptr, longrows, nl);
+  if ((rc = scan_exclusive(c, cnt, start, n, &total))) return rc;
+  if ((rc = tmp.get(&g.ccol, total)) || (rc = tmp.get(&g.cval, total))) return rc;
+  g.start = start;
+  k_spg_row<kTabShort><<<(n + 3) / 4, 128, 0, s>>>(g, n, nullptr, nullptr, longrows, nl, nullptr);
   MSG_CHECK_LAUNCH();
-  // the count of the long rows stays on the device: a grid that fills the chip walks them
-  const int wb = std::min((nrows + kSpgWarps - 1) / kSpgWarps, 12 * kNumSM);
-  k_spgemm<0><<<wb, 32 * kSpgWarps, 0, s>>>(nl, ap, ac, av, adiag, bp, bc, bv, split_diag, cnt, nullptr, nullptr,
-                                            nullptr, nullptr, nl + 1, longrows);
+  // the counts of the long rows stay on the device: grids that fill the chip walk them
+  k_spg_row<kTabMid><<<std::min((n + 3) / 4, 12 * kNumSM), 128, 0, s>>>(g, n, nl, longrows, biggest, nl + 1, nullptr);
   MSG_CHECK_LAUNCH();
-  if ((rc = halloc(c, cptr, nrows + 1))) return rc;
-  int got[3];
-  if ((rc = scan_exclusive(c, cnt, *cptr, nrows, got, nl, nl + 1))) return rc;
-  const int tot = got[0], nlong = got[1];
-  *ovf = got[2];
-  if (*ovf) {
-    hfree(S(c), cnt, s); hfree(S(c), longrows, s); hfree(S(c), nl, s); hfree(S(c), *cptr, s);
-    *cptr = nullptr;
-    return MSG_OK;
-  }
-  if ((rc = halloc(c, ccol, tot))) return rc;
-  if ((rc = halloc(c, cval, tot))) return rc;
-  k_spgemm_t<1><<<(nrows + 127) / 128, 128, 0, s>>>(nrows, ap, ac, av, adiag, bp, bc, bv, split_diag, nullptr, *cptr,
-                                                   *ccol, *cval, cdiag, nullptr, nullptr);
+  k_spg_row<kTabMax><<<std::min((n + 2) / 3, 4 * kNumSM), 96, 0, s>>>(g, n, nl + 1, biggest, nullptr, nullptr, ovf);
   MSG_CHECK_LAUNCH();
-  if (nlong > 0) {
-    const int wf = (nlong + kSpgWarps - 1) / kSpgWarps;
-    k_spgemm<1, kHashSmall><<<wf, 32 * kSpgWarps, 0, s>>>(nl, ap, ac, av, adiag, bp, bc, bv, split_diag, nullptr,
-                                                          *cptr, *ccol, *cval, cdiag, nl + 1, longrows);
-    MSG_CHECK_LAUNCH();
-    k_spgemm<1, kHash><<<wf, 32 * kSpgWarps, 0, s>>>(nl, ap, ac, av, adiag, bp, bc, bv, split_diag, nullptr, *cptr,
-                                                     *ccol, *cval, cdiag, nl + 1, longrows);
-    MSG_CHECK_LAUNCH();
-  }
-  hfree(S(c), cnt, s); hfree(S(c), longrows, s); hfree(S(c), nl, s);
-  *cnnz = tot;
   return MSG_OK;
 }
 
 // Build level lv+1 from level lv; returns 1 when a coarser level was made, 0 otherwise.
 static int coarsen(msg_ctx *c, AmgState *A, int lv, int *made) {
   *made = 0;
-  AmgLevel &F = A->lv[lv];
-  const int n = F.n;
-  int rc;
-  if ((rc = ensure_scratch(c, A, n, F.nnz))) return rc;
-  if ((size_t)F.nnz > A->sflag_cap) {
-    cudaFreeAsync(A->sflag, c->stream);
-    if ((rc = dalloc(c, &A->sflag, F.nnz))) return rc;
-    A->sflag_cap = F.nnz;
-  }
+  const AmgLevel F = A->lv[lv];
+  const int n = F.n, n8 = (int)((8 * (long long)n + 255) / 256);
+  const bool dia = lv == 0;
+  int rc, got[2];
   cudaStream_t s = c->stream;
-  double th = (double)c->prm.amg_theta, th2 = th * th;
-  k_strength<<<nb(n), kThreads, 0, s>>>(n, F.rowptr, F.col, F.val, F.diag, th2, A->sflag, A->has, A->tdm);
-  MSG_CHECK_LAUNCH();
-  k_mis_init<<<nb(n), kThreads, 0, s>>>(n, A->has, A->st);
-  MSG_CHECK_LAUNCH();
-  // t0 = tuples of the current states; t1, t2 = the two max-propagation steps
-  unsigned long long *t0 = A->t0m;
-  k_mis_tuple<<<nb(n), kThreads, 0, s>>>(n, A->st, t0, lv);
-  MSG_CHECK_LAUNCH();
-  for (int round = 0; round < 64; ++round) {
-    k_mis_max<<<nb(n), kThreads, 0, s>>>(n, F.rowptr, F.col, A->sflag, t0, A->t1);
+  Temps tmp(c);
+  const Bands g{c->nx, c->ny, c->nz, c->nxy, c->N, c->dmat, c->lu};
+  const dim3 tb(32, 8), tg((c->nx + 31) / 32, (c->ny + 7) / 8, c->nz);   // level-1 stencil passes
+  const double th = (double)c->prm.amg_theta, th2 = th * th, om = (double)c->prm.jac_omega;
+  unsigned char *msk = nullptr, *st = nullptr, *w1b = nullptr;
+  int *scol = nullptr, *cnt = nullptr, *aggid = nullptr, *agg2 = nullptr, *words = nullptr;
+  unsigned *w1 = nullptr;
+  double *tdm = nullptr;
+  if ((rc = tmp.get(&st, n + 3)) || (rc = tmp.get(&cnt, n)) || (rc = tmp.get(&aggid, n + 1)) || (rc = tmp.get(&agg2, n)) ||
+      (rc = tmp.get(&words, kMisRounds + 3)))
+    return rc;
+  // too long: prolongation row, product row; rows beyond kPShort entries
+  int *ovf_p = words + kMisRounds, *ovf = ovf_p + 1, *npl = ovf + 1, *prow = nullptr;
+  MSG_CUDA(cudaMemsetAsync(words, 0, (kMisRounds + 3) * 4, s));
+  // strength and aggregates
+  if (dia) {
+    if ((rc = tmp.get(&msk, n + 3)) || (rc = tmp.get(&w1b, n + 3))) return rc;
+    k_strength_dia<<<tg, tb, 0, s>>>(g, th2, msk, st);
     MSG_CHECK_LAUNCH();
-    k_mis_max<<<nb(n), kThreads, 0, s>>>(n, F.rowptr, F.col, A->sflag, A->t1, A->t2);
+  } else {
+    if ((rc = tmp.get(&scol, F.nnz)) || (rc = tmp.get(&w1, n)) || (rc = tmp.get(&tdm, n)) || (rc = tmp.get(&prow, n)))
+      return rc;
+    k_strength_csr<<<(n + 3) / 4, 128, 0, s>>>(n, F.rowptr, F.col, F.val, F.diag, th2, scol, st, tdm);
     MSG_CHECK_LAUNCH();
-    const bool check = (round & 3) == 3 || round == 63;   // a round with nothing undecided is a no-op
-    if (check) MSG_CUDA(cudaMemsetAsync(A->cnt, 0, 4, s));
-    k_mis_update<<<nb(n), kThreads, 0, s>>>(n, A->st, A->t2, t0, lv, check ? A->cnt : nullptr);
-    MSG_CHECK_LAUNCH();
-    if (check) {
-      int und = 0;
-      if ((rc = read_counter(c, A, &und))) return rc;
-      if (und == 0) break;
-    }
   }
-  k_root_flag<<<nb(n), kThreads, 0, s>>>(n, A->st, A->flag);
+  {
+    int l = lv;
+    Bands gb = g;
+    if (dia) {
+      void *args[] = {&gb, &msk, &st, &w1b, &l, &words};
+      MSG_CUDA(cudaLaunchCooperativeKernel((void *)k_mis_dia, std::min((n + 4 * kMisBlock - 1) / (4 * kMisBlock), A->mis_dia), kMisBlock, args, 0, s));
+    } else {
+      int nn = n, *rp = F.rowptr;
+      void *args[] = {&nn, &rp, &scol, &st, &w1, &l, &words};
+      if (n <= kMisSmall) {
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = kMisCluster; at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cf = {};
+        cf.gridDim = dim3(kMisCluster); cf.blockDim = dim3(kMisBlock); cf.stream = s; cf.attrs = &at; cf.numAttrs = 1;
+        MSG_CUDA(cudaLaunchKernelExC(&cf, (const void *)k_mis_csr<true>, args));
+      } else
+      MSG_CUDA(cudaLaunchCooperativeKernel((void *)k_mis_csr<false>, (int)std::min((4 * (long long)n + kMisBlock - 1) / kMisBlock, (long long)A->mis_csr), kMisBlock, args, 0, s));
+    }
+    __atomic_fetch_add(&g_launches, 1LL, __ATOMIC_RELAXED);
+  }
+  k_root_flag<<<nb(n), kThreads, 0, s>>>(n, st, cnt);
   MSG_CHECK_LAUNCH();
-  int nc = 0, got[2];
-  if ((rc = scan_exclusive(c, A->flag, A->aggid, n, &nc))) return rc;
+  if ((rc = scan_exclusive(c, cnt, aggid, n, got))) return rc;
+  const int nc = got[0];
   if (nc == 0 || nc >= n) return MSG_OK;
   AmgLevel C;
   C.n = nc;
   if ((rc = halloc(c, &C.agg, n))) return rc;
-  k_agg_a<<<nb(n), kThreads, 0, s>>>(n, F.rowptr, F.col, A->sflag, A->st, A->aggid, A->agg2, lv);
-  MSG_CHECK_LAUNCH();
-  k_agg_b<<<nb(n), kThreads, 0, s>>>(n, F.rowptr, F.col, A->sflag, A->agg2, C.agg, lv);
+  if (dia) {
+    k_agg_a_dia<<<nb(n), kThreads, 0, s>>>(g, msk, st, aggid, agg2, lv);
+    MSG_CHECK_LAUNCH();
+    k_agg_b_dia<<<nb(n), kThreads, 0, s>>>(g, msk, agg2, C.agg, lv);
+  } else {
+    k_agg_csr<true><<<n8, 256, 0, s>>>(n, F.rowptr, scol, st, aggid, agg2, lv);
+    MSG_CHECK_LAUNCH();
+    k_agg_csr<false><<<n8, 256, 0, s>>>(n, F.rowptr, scol, st, agg2, C.agg, lv);
+  }
   MSG_CHECK_LAUNCH();
   // P
-  MSG_CUDA(cudaMemsetAsync(A->cnt, 0, 4, s));
-  k_p_count<<<nb(n), kThreads, 0, s>>>(n, F.rowptr, F.col, A->sflag, C.agg, A->tmpi, A->cnt);
+  auto p_rows = [&](auto fill, int *rcnt) -> int {
+    constexpr bool FILL = decltype(fill)::value;
+    k_p_csr<FILL, false><<<(n + 3) / 4, 128, 0, s>>>(n, F.rowptr, scol, F.val, C.agg, tdm, om, cnt, ovf_p, prow, npl,
+                                                    C.pptr, C.pcol, C.pval, rcnt);
+    MSG_CHECK_LAUNCH();
+    k_p_csr<FILL, true><<<std::min((n + 3) / 4, 2 * kNumSM), 128, 0, s>>>(n, F.rowptr, scol, F.val, C.agg, tdm, om, cnt,
+                                                                         ovf_p, prow, npl, C.pptr, C.pcol, C.pval, rcnt);
+    return MSG_OK;
+  };
+  if (dia) k_p_dia<false><<<nb(n), kThreads, 0, s>>>(g, msk, C.agg, om, cnt, nullptr, nullptr, nullptr, nullptr);
+  else if ((rc = p_rows(std::false_type(), nullptr))) return rc;
   MSG_CHECK_LAUNCH();
   if ((rc = halloc(c, &C.pptr, n + 1))) return rc;
-  if ((rc = scan_exclusive(c, A->tmpi, C.pptr, n, got, A->cnt))) return rc;
+  if ((rc = scan_exclusive(c, cnt, C.pptr, n, got, ovf_p))) return rc;
   if (got[1]) { free_level(A, C, s); return MSG_OK; }   // a row beyond kPRowMax
   const int pnnz = got[0];
   C.pnnz = pnnz;
-  if ((rc = halloc(c, &C.pcol, pnnz))) return rc;
-  if ((rc = halloc(c, &C.pval, pnnz))) return rc;
-  k_p_fill<<<nb(n), kThreads, 0, s>>>(n, F.rowptr, F.col, F.val, A->sflag, C.agg, A->tdm, (double)c->prm.jac_omega,
-                                      C.pptr, C.pcol, C.pval);
+  if ((rc = halloc(c, &C.pcol, pnnz)) || (rc = halloc(c, &C.pval, pnnz))) return rc;
+  int *rcnt = nullptr;
+  if ((rc = tmp.get(&rcnt, nc))) return rc;
+  MSG_CUDA(cudaMemsetAsync(rcnt, 0, (size_t)nc * 4, s));
+  if (dia) k_p_dia<true><<<nb(n), kThreads, 0, s>>>(g, msk, C.agg, om, nullptr, C.pptr, C.pcol, C.pval, rcnt);
+  else if ((rc = p_rows(std::true_type(), rcnt))) return rc;
   MSG_CHECK_LAUNCH();
   // R = P^T
-  int *rcnt = nullptr;
-  if ((rc = halloc(c, &rcnt, nc + 1))) return rc;
-  MSG_CUDA(cudaMemsetAsync(rcnt, 0, (size_t)(nc + 1) * 4, s));
-  k_r_count<<<nb(pnnz), kThreads, 0, s>>>(pnnz, C.pcol, rcnt);
-  MSG_CHECK_LAUNCH();
   if ((rc = halloc(c, &C.rptr, nc + 1))) return rc;
   if ((rc = scan_exclusive(c, rcnt, C.rptr, nc, nullptr))) return rc;
-  if ((rc = halloc(c, &C.rcol, pnnz))) return rc;
-  if ((rc = halloc(c, &C.rval, pnnz))) return rc;
-  MSG_CUDA(cudaMemsetAsync(rcnt, 0, (size_t)(nc + 1) * 4, s));
-  k_r_fill<<<nb(n), kThreads, 0, s>>>(n, C.pptr, C.pcol, C.pval, C.rptr, rcnt, C.rcol, C.rval);
+  if ((rc = halloc(c, &C.rcol, pnnz)) || (rc = halloc(c, &C.rval, pnnz))) return rc;
+  MSG_CUDA(cudaMemsetAsync(rcnt, 0, (size_t)nc * 4, s));
+  int *trow = nullptr, *tcol = nullptr;
+  double *tval = nullptr;
+  if ((rc = tmp.get(&trow, pnnz)) || (rc = tmp.get(&tcol, pnnz)) || (rc = tmp.get(&tval, pnnz))) return rc;
+  if (c->prm.precision == 1 && ((rc = halloc(c, &C.pval_f, pnnz)) || (rc = halloc(c, &C.rval_f, pnnz)))) return rc;
+  k_r_fill<<<nb(n), kThreads, 0, s>>>(n, C.pptr, C.pcol, C.pval, C.rptr, rcnt, trow, tcol, tval);
   MSG_CHECK_LAUNCH();
-  k_r_sort<<<(nc + 3) / 4, 128, 0, s>>>(nc, C.rptr, C.rcol, C.rval);
+  k_r_rank<<<nb(pnnz), kThreads, 0, s>>>(pnnz, C.rptr, trow, tcol, tval, C.rcol, C.rval, C.rval_f);
   MSG_CHECK_LAUNCH();
-  hfree(A, rcnt, s);
   // AP = A*P (diagonal first)
-  int *apptr = nullptr, *apcol = nullptr;
-  double *apval = nullptr;
-  int apn = 0, ovf = 0;
-  if ((rc = spgemm(c, A, n, F.rowptr, F.col, F.val, F.diag, C.pptr, C.pcol, C.pval, 0, &apptr, &apcol, &apval,
-                   nullptr, &apn, &ovf)))
+  Spg ap{F.rowptr, F.col, F.val, F.diag, C.pptr, nullptr, C.pcol, C.pval, 0, nullptr, nullptr, nullptr, nullptr, nullptr};
+  if (dia) {
+    int *start = nullptr;
+    k_ap_bound_dia<<<tg, tb, 0, s>>>(g, C.pptr, cnt);
+    MSG_CHECK_LAUNCH();
+    if ((rc = tmp.get(&start, n + 1)) || (rc = tmp.get(&ap.len, n))) return rc;
+    if ((rc = scan_exclusive(c, cnt, start, n, got))) return rc;
+    if ((rc = tmp.get(&ap.ccol, got[0])) || (rc = tmp.get(&ap.cval, got[0]))) return rc;
+    ap.start = start;
+    k_ap_dia<<<dim3(tg.x, (c->ny + kApT / 32 - 1) / (kApT / 32), tg.z), dim3(32, kApT / 32), 0, s>>>(g, C.pptr, C.pcol, C.pval, start, ap.len, ap.ccol, ap.cval);
+    MSG_CHECK_LAUNCH();
+  } else if ((rc = spgemm_rows(c, tmp, n, ap, cnt, ovf))) {
     return rc;
-  if (ovf) { free_level(A, C, s); return MSG_OK; }
+  }
   // A_c = R * AP, diagonal split off
-  if ((rc = halloc(c, &C.diag, nc))) return rc;
-  int cn = 0;
-  if ((rc = spgemm(c, A, nc, C.rptr, C.rcol, C.rval, nullptr, apptr, apcol, apval, 1, &C.rowptr, &C.col, &C.val,
-                   C.diag, &cn, &ovf)))
+  if ((rc = halloc(c, &C.diag, nc)) || (rc = halloc(c, &C.rowptr, nc + 1))) return rc;
+  Spg ra{C.rptr, C.rcol, C.rval, nullptr, ap.start, ap.len, ap.ccol, ap.cval, 1, nullptr, nullptr, nullptr, nullptr, C.diag};
+  if ((rc = spgemm_rows(c, tmp, nc, ra, cnt, ovf))) return rc;
+  if ((rc = scan_exclusive(c, ra.len, C.rowptr, nc, got, ovf))) return rc;
+  if (got[1]) { free_level(A, C, s); return MSG_OK; }   // a row beyond kHashMax
+  C.nnz = got[0];
+  if ((rc = halloc(c, &C.col, C.nnz)) || (rc = halloc(c, &C.val, C.nnz))) return rc;
+  if (c->prm.precision == 1) {
+    if ((rc = halloc(c, &C.val_h, C.nnz)) || (rc = halloc(c, &C.diag_f, nc)) || (rc = halloc(c, &C.xf, nc)) ||
+        (rc = halloc(c, &C.bf, nc)) || (rc = halloc(c, &C.rf, nc)) || (rc = halloc(c, &C.x2f, nc)))
+      return rc;
+    k_d2f<<<std::max(1, std::min(nb(pnnz), kRedBlocks * 4)), kThreads, 0, s>>>(pnnz, C.pval, C.pval_f);
+    MSG_CHECK_LAUNCH();
+  } else if ((rc = halloc(c, &C.x, nc)) || (rc = halloc(c, &C.b, nc)) || (rc = halloc(c, &C.r, nc)) ||
+             (rc = halloc(c, &C.x2, nc))) {
     return rc;
-  hfree(A, apptr, s); hfree(A, apcol, s); hfree(A, apval, s);
-  if (ovf) { free_level(A, C, s); return MSG_OK; }
-  C.nnz = cn;
-  if ((rc = halloc(c, &C.x, nc))) return rc;
-  if ((rc = halloc(c, &C.b, nc))) return rc;
-  if ((rc = halloc(c, &C.r, nc))) return rc;
-  if ((rc = halloc(c, &C.x2, nc))) return rc;
+  }
+  k_spg_pack<<<(8 * (long long)nc + 255) / 256, 256, 0, s>>>(nc, ra.start, C.rowptr, ra.ccol, ra.cval, C.diag, C.col,
+                                                            C.val, C.val_h, C.diag_f);
+  MSG_CHECK_LAUNCH();
   A->lv.push_back(C);
   *made = 1;
   return MSG_OK;
@@ -1462,20 +1779,18 @@ void amg_free(msg_ctx *c) {
   cudaStream_t s = c->stream;
   for (size_t l = 1; l < A->lv.size(); ++l) free_level(A, A->lv[l], s);
   A->lv.clear();
-  void *p[] = {A->col0, A->val0, A->cnt, A->r0, A->t0, A->x0f, A->t0f, A->r0f, A->b0f, A->sflag, A->has, A->st, A->flag, A->aggid, A->agg2, A->tmpi, A->t0m, A->t1,
-               A->t2, A->tdm, A->d1f, A->lu1f};
+  void *p[] = {A->col0, A->r0, A->t0, A->x0f, A->t0f, A->r0f, A->b0f};
   for (void *q : p) if (q) cudaFreeAsync(q, s);
   cudaStreamSynchronize(s);
-  if (A->hcnt) cudaFreeHost(A->hcnt);
   if (A->arena) cudaFree(A->arena);
   delete A;
   c->amg = nullptr;
 }
 
-// Per-cell bytes of the arena reserved when a context is made: one hierarchy build of the
-// block workloads (levels, transfer operators, Galerkin temporaries) takes about 150 B per
-// fine cell; a build that outgrows the reservation spills to the pool and the arena is
-// enlarged at the next build, as before.
+// Per-cell bytes of the arena reserved when a context is made: the levels and transfer
+// operators of the block workloads take about 100 B per fine cell, the temporaries of the
+// first coarsening about 80; a build that outgrows the reservation spills to the pool and
+// the arena is enlarged at the next build.
 constexpr size_t kArenaPerCell = 192;
 
 static int amg_state(msg_ctx *c);
@@ -1491,10 +1806,7 @@ int amg_reserve(msg_ctx *c) {
   const size_t cap = (kArenaPerCell * (size_t)c->N + ((size_t)1 << 20) - 1) & ~(((size_t)1 << 20) - 1);
   if (cudaMalloc((void **)&A->arena, cap) == cudaSuccess) A->arena_cap = cap;
   else { A->arena = nullptr; A->arena_cap = 0; cudaGetLastError(); }   // the builds use the pool
-  // and the setup scratch of the fine level (strength flags, MIS-2 state and tuples,
-  // temporaries: about 64 B per cell), which the first build would otherwise take from the
-  // pool: at 25.2M cells that first build then cost 20-45 ms more, varying from run to run
-  return ensure_scratch(c, A, (size_t)c->N, (size_t)c->nnz);
+  return MSG_OK;
 }
 
 static int amg_state(msg_ctx *c) {
@@ -1505,8 +1817,6 @@ static int amg_state(msg_ctx *c) {
     A = new AmgState();
     c->amg = A;
     if ((rc = dalloc(c, &A->col0, c->nnz))) return rc;
-    if ((rc = dalloc(c, &A->val0, c->nnz))) return rc;
-    if ((rc = dalloc(c, &A->cnt, 1))) return rc;
     if ((rc = dalloc(c, &A->r0, c->N))) return rc;
     if ((rc = dalloc(c, &A->t0, c->N))) return rc;
     if (c->prm.precision == 1) {
@@ -1515,7 +1825,12 @@ static int amg_state(msg_ctx *c) {
       if ((rc = dalloc(c, &A->r0f, c->N))) return rc;
       if ((rc = dalloc(c, &A->b0f, c->N))) return rc;
     }
-    MSG_CUDA(cudaMallocHost((void **)&A->hcnt, 4));
+    int sms = 0, per = 0;
+    MSG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+    MSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mis_dia, kMisBlock, 0));
+    A->mis_dia = sms * std::max(per, 1);
+    MSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mis_csr<false>, kMisBlock, 0));
+    A->mis_csr = sms * std::max(per, 1);
     k_col0<<<nb(c->nnz), kThreads, 0, s>>>(c->nnz, c->offrow, A->col0);
     MSG_CHECK_LAUNCH();
   }
@@ -1531,7 +1846,7 @@ int amg_setup(msg_ctx *c) {
   A->lv.clear();
   // reset the arena; enlarge it first when the previous build did not fit
   if (A->arena_spill) {
-    const size_t need = A->arena_used + A->arena_spill;
+    const size_t need = A->arena_used + A->arena_spill;   // (the temporaries of all levels: ample)
     if (A->arena) {
       MSG_CUDA(cudaStreamSynchronize(s));
       cudaFree(A->arena);
@@ -1542,11 +1857,10 @@ int amg_setup(msg_ctx *c) {
     if (cudaMalloc((void **)&A->arena, cap) == cudaSuccess) A->arena_cap = cap;
     else { A->arena = nullptr; cudaGetLastError(); }   // keep using the pool
   }
-  A->arena_used = 0;
+  A->arena_used = A->arena_tmp = 0;
   A->arena_spill = 0;
-  if ((rc = launch_dia_to_csr(c, A->val0))) return rc;
   AmgLevel L0;
-  L0.n = c->N; L0.nnz = c->nnz; L0.rowptr = c->offind; L0.col = A->col0; L0.diag = c->dmat; L0.val = A->val0;
+  L0.n = c->N; L0.nnz = c->nnz; L0.rowptr = c->offind; L0.col = A->col0; L0.diag = c->dmat;
   A->lv.push_back(L0);
   int maxlev = std::min(std::max(c->prm.amg_nlevel, 2), 16);
   while ((int)A->lv.size() < maxlev && A->lv.back().n > c->prm.amg_coarse_max) {
@@ -1556,29 +1870,6 @@ int amg_setup(msg_ctx *c) {
   }
   if (A->lv.size() > 1 && A->lv.back().n <= std::max(c->prm.amg_coarse_max, 1)) {
     if ((rc = dense_inverse(c, A->lv.back()))) return rc;
-  }
-  if (c->prm.precision == 1) {
-    for (size_t l = 1; l < A->lv.size(); ++l) {
-      AmgLevel &L = A->lv[l];
-      int nf = A->lv[l - 1].n;
-      if ((rc = halloc(c, &L.diag_f, L.n))) return rc;
-      if ((rc = halloc(c, &L.val_h, L.nnz))) return rc;
-      if ((rc = halloc(c, &L.pval_f, L.pnnz))) return rc;
-      if ((rc = halloc(c, &L.rval_f, L.pnnz))) return rc;
-      if ((rc = halloc(c, &L.xf, L.n))) return rc;
-      if ((rc = halloc(c, &L.bf, L.n))) return rc;
-      if ((rc = halloc(c, &L.rf, L.n))) return rc;
-      if ((rc = halloc(c, &L.x2f, L.n))) return rc;
-      int g = std::min(nb(std::max(L.nnz, L.pnnz)), kRedBlocks * 4);
-      k_d2f<<<std::min(nb(L.n), kRedBlocks * 4), kThreads, 0, s>>>(L.n, L.diag, L.diag_f);
-      MSG_CHECK_LAUNCH();
-      if (L.nnz) { k_d2h<<<g, kThreads, 0, s>>>(L.nnz, L.val, L.val_h); MSG_CHECK_LAUNCH(); }
-      k_d2f<<<g, kThreads, 0, s>>>(L.pnnz, L.pval, L.pval_f);
-      MSG_CHECK_LAUNCH();
-      k_d2f<<<g, kThreads, 0, s>>>(L.pnnz, L.rval, L.rval_f);
-      MSG_CHECK_LAUNCH();
-      (void)nf;
-    }
   }
   c->amg_nlevel = (int)A->lv.size();
   return MSG_OK;
@@ -1879,7 +2170,19 @@ MSG_API int msg_gpu_amg_level(msg_ctx_t *c, int32_t lv, int32_t *offind, int32_t
   if (offind) MSG_CUDA(cudaMemcpy(offind, L.rowptr, (size_t)(L.n + 1) * 4, cudaMemcpyDeviceToHost));
   if (offrow) MSG_CUDA(cudaMemcpy(offrow, L.col, (size_t)L.nnz * 4, cudaMemcpyDeviceToHost));
   if (dmat) MSG_CUDA(cudaMemcpy(dmat, L.diag, (size_t)L.n * 8, cudaMemcpyDeviceToHost));
-  if (lumat) MSG_CUDA(cudaMemcpy(lumat, L.val, (size_t)L.nnz * 8, cudaMemcpyDeviceToHost));
+  if (lumat && lv == 0) {   // the Jacobian's bands in CSR order
+    double *v = nullptr;
+    MSG_CUDA(cudaMalloc(&v, (size_t)L.nnz * 8));
+    int rc = launch_dia_to_csr(c, v);
+    if (!rc) {
+      MSG_CUDA(cudaStreamSynchronize(c->stream));
+      MSG_CUDA(cudaMemcpy(lumat, v, (size_t)L.nnz * 8, cudaMemcpyDeviceToHost));
+    }
+    cudaFree(v);
+    if (rc) return rc;
+  } else if (lumat) {
+    MSG_CUDA(cudaMemcpy(lumat, L.val, (size_t)L.nnz * 8, cudaMemcpyDeviceToHost));
+  }
   if (lv > 0) {
     int nf = S(c)->lv[lv - 1].n;
     if (pindex) MSG_CUDA(cudaMemcpy(pindex, L.pptr, (size_t)(nf + 1) * 4, cudaMemcpyDeviceToHost));

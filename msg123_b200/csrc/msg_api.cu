@@ -675,7 +675,7 @@ static int create_impl(msg_ctx *c, const msg_grid_t *g, const msg_params_t *p) {
   ALLOC(c->part, npart * 8);
   c->npart = npart;
   ALLOC(c->dres, 16 * 8);
-  MSG_CUDA(cudaMallocHost((void **)&c->hpin, (size_t)kRedBlocks * 8 * 8));
+  MSG_CUDA(cudaMallocHost((void **)&c->hpin, ((size_t)kRedBlocks * 8 + 16) * 8));   // and the box, wave_err
   int rc = scan_reserve(c, (int)N);
   if (rc) return rc;
   if ((rc = build_connectivity(c, g))) return rc;
@@ -1275,8 +1275,6 @@ static void free_ctx(msg_ctx *c) {
                 c->p, c->v, c->t, c->z, c->part, c->scan_sums, c->wave_order, c->wave_ticket, c->wave_slots, c->dmat_f, c->lu_f, c->dres};
   for (auto q : dp) if (q) cudaFree(q);
   if (c->hpin) cudaFreeHost(c->hpin);
-  if (c->wave_err) cudaFreeHost(c->wave_err);
-  if (c->box) cudaFreeHost(c->box);
   for (int k = 0; k < 8; ++k) if (c->ev[k]) cudaEventDestroy(c->ev[k]);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;

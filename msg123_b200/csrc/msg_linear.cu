@@ -161,7 +161,8 @@ int scan_exclusive(msg_ctx *c, const int *in, int *out, int n, int *got, const i
 int scan_reserve(msg_ctx *c, int n) {
   c->scan_cap = (n + kScanE - 1) / kScanE + 1;
   MSG_CUDA(cudaMalloc(&c->scan_sums, (size_t)c->scan_cap * 4));
-  MSG_CUDA(cudaMallocHost((void **)&c->box, sizeof(HostBox)));
+  // behind the reduction results in the context's pinned block
+  c->box = reinterpret_cast<HostBox *>(c->hpin + kRedBlocks * 8);
   memset(c->box, 0, sizeof(HostBox));
   c->box_token = 0;
   return MSG_OK;
@@ -782,7 +783,7 @@ int build_wavefront(msg_ctx *c) {
   MSG_CUDA(cudaMalloc(&c->wave_order, (size_t)nt * 4));
   MSG_CUDA(cudaMalloc(&c->wave_ticket, 8));      // ticket, error word
   MSG_CUDA(cudaMalloc(&c->wave_slots, nslot * 8));
-  MSG_CUDA(cudaMallocHost((void **)&c->wave_err, 4));
+  c->wave_err = reinterpret_cast<int *>(c->hpin + kRedBlocks * 8 + 8);
   *c->wave_err = 0;
   c->wave_tiles = nt;
   c->wave_sweeps = 0;
