@@ -11,8 +11,8 @@
 // Inference inside the time loop (learned_guess) runs the convolutions on the tcgen05
 // tensor cores with TMA-staged halo tiles and TMEM accumulators (msg_conv_tc.cu).
 // Training (forward with saved pre-activations, input and weight gradients) uses
-// implicit GEMMs with mma.sync m16n8k16 (BF16 x BF16 -> FP32): a warp owns 16
-// consecutive cells (the M dimension), the 16 output channels are two n8 tiles, and
+// implicit GEMMs with mma.sync m16n8k16 (BF16 x BF16 -> FP32) on tiles staged in shared memory:
+// 16 consecutive cells are the M dimension, the 16 output channels are two n8 tiles, and
 // each of the 27 taps is one k16 step over the 16 input channels.  The input-gradient
 // pass is the same kernel with the taps mirrored and the weights transposed; the weight
 // gradient reduces dz^T a over cells with the same instruction.
@@ -53,7 +53,6 @@ struct Net {
   std::recursive_mutex mu;
   float *m = nullptr, *v = nullptr, *grad = nullptr;
   float *part = nullptr;               // weight-gradient partials
-  int part_cap = 0;
   int step = 0;
   float dead = 0.1f;                   // deadband on the normalised correction
   // activations (sized for the largest grid seen)
@@ -94,18 +93,41 @@ __device__ __forceinline__ void mma_bf16(float d[4], unsigned a0, unsigned a1, u
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-__device__ __forceinline__ int nbr(const Grid3 &g, int cell, int tap) {
-  if (cell >= g.N) return -1;
-  int z = cell / g.nxy, rem = cell - z * g.nxy, y = rem / g.nx, x = rem - y * g.nx;
-  int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-  x += dx; y += dy; z += dz;
-  if (x < 0 || x >= g.nx || y < 0 || y >= g.ny || z < 0 || z >= g.nz) return -1;
-  return x + g.nx * (y + g.ny * z);
+// Training passes work on tiles of kTX x kTY x kTZ cells with a halo of one, staged in shared
+// memory as [cell][16 channels] of two 16-byte chunks; the chunks of a cell swap places with
+// bit 2 of its number, so that the eight rows of an ldmatrix, always eight cells in a row,
+// lie in different banks.  A 16-cell row of the tile is the M (convolutions) or K (weight
+// gradient) dimension of one mma.
+constexpr int kTX = 16, kTY = 8, kTZ = 4, kTCells = kTX * kTY * kTZ;
+constexpr int kHX = kTX + 2, kHY = kTY + 2, kHCells = kHX * kHY * (kTZ + 2);
+__device__ __forceinline__ unsigned tile_addr(unsigned base, int cell, int chunk) {
+  return base + cell * 32 + ((chunk ^ ((cell >> 2) & 1)) << 4);
 }
-
-__device__ __forceinline__ unsigned ld2(const __nv_bfloat16 *p, int cell, int ch) {
-  if (cell < 0) return 0u;
-  return *reinterpret_cast<const unsigned *>(p + (size_t)cell * kC + ch);
+__device__ __forceinline__ void cp16z(unsigned dst, const void *src, bool live) {   // 16 bytes, or zeros
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+template <bool TRANS>
+__device__ __forceinline__ void ldsm4(unsigned r[4], unsigned addr) {
+  if (TRANS)
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+  else
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+// The tile at (x0, y0, z0) with its halo (HALO) or without, zeros outside the grid.
+template <bool HALO>
+__device__ __forceinline__ void load_tile(const Grid3 &g, const __nv_bfloat16 *__restrict__ p, int x0, int y0, int z0,
+                                          unsigned dst) {
+  constexpr int NX = HALO ? kHX : kTX, NY = HALO ? kHY : kTY, NC = HALO ? kHCells : kTCells, H = HALO ? 1 : 0;
+  for (int e = threadIdx.x; e < 2 * NC; e += blockDim.x) {
+    const int c = e >> 1, q = e & 1;
+    const int hz = c / (NX * NY), r = c - hz * (NX * NY), hy = r / NX, hx = r - hy * NX;
+    const int x = x0 + hx - H, y = y0 + hy - H, z = z0 + hz - H;
+    const bool live = x >= 0 && x < g.nx && y >= 0 && y < g.ny && z >= 0 && z < g.nz;
+    const size_t cell = live ? x + (size_t)g.nx * (y + (size_t)g.ny * z) : 0;
+    cp16z(tile_addr(dst, c, q), p + cell * kC + 8 * q, live);
+  }
 }
 
 __device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
@@ -116,126 +138,176 @@ __device__ __forceinline__ float gelu_d(float x) {
 // Convolution over all 27 taps.  MODE 0: forward hidden layer (z, GELU -> a_out);
 // MODE 1: forward output layer (channel 0 -> out); MODE 2: input gradient
 // (acc * gelu'(zprev) -> dz_out).  W is [tap][co][ci] (already mirrored/transposed for MODE 2).
+// A block per tile; a warp takes the tile's four rows of one y, so a tap's weights are read
+// once for four products.  A thread's own scattered loads of every tap (a division per cell
+// and tap, 27 reads of each activation from L2) took 0.64 ms on 1.57M cells; this takes 0.11,
+// about three times its 200 MB at the copy rate.
+constexpr int kConvSmem = kHCells * 32 + kWl * 2;
 template <int MODE>
-__global__ void __launch_bounds__(256) k_conv(Grid3 g, const __nv_bfloat16 *__restrict__ in,
-                                              const __nv_bfloat16 *__restrict__ W, const float *__restrict__ bias,
-                                              float *z_out, __nv_bfloat16 *a_out, float *out,
-                                              const float *__restrict__ zprev, __nv_bfloat16 *dz_out) {
-  __shared__ __align__(16) __nv_bfloat16 sw[kWl];
-  for (int k = threadIdx.x; k < kWl / 8; k += blockDim.x)
-    reinterpret_cast<uint4 *>(sw)[k] = reinterpret_cast<const uint4 *>(W)[k];
+__global__ void __launch_bounds__(32 * kTY) k_conv(Grid3 g, const __nv_bfloat16 *__restrict__ in,
+                                                   const __nv_bfloat16 *__restrict__ W, const float *__restrict__ bias,
+                                                   float *z_out, __nv_bfloat16 *a_out, float *out,
+                                                   const float *__restrict__ zprev, __nv_bfloat16 *dz_out) {
+  extern __shared__ __align__(128) unsigned char smem_tile[];
+  const unsigned act = (unsigned)__cvta_generic_to_shared(smem_tile), wts = act + kHCells * 32;
+  const int x0 = blockIdx.x * kTX, y0 = blockIdx.y * kTY, z0 = blockIdx.z * kTZ;
+  load_tile<true>(g, in, x0, y0, z0, act);
+  for (int e = threadIdx.x; e < kWl / 8; e += blockDim.x) cp16z(tile_addr(wts, e >> 1, e & 1), W + 8 * e, true);
+  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
   __syncthreads();
-  const int lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int c0 = warp * 16;
-  if (c0 >= g.N) return;
-  const int ca = c0 + gq, cb = c0 + gq + 8;
-  float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, gq = lane >> 2, tq = lane & 3;
+  const int mi = lane >> 3, arow = (lane & 7) + 8 * (mi & 1), ach = mi >> 1;    // A: cells, channels
+  const int brow = (lane & 7) + 8 * (mi >> 1), bch = mi & 1;                    // B: output channel, input channels
+  float d[kTZ][8];
+#pragma unroll
+  for (int m = 0; m < kTZ; ++m)
+#pragma unroll
+    for (int q = 0; q < 8; ++q) d[m][q] = 0.f;
 #pragma unroll 3
   for (int tap = 0; tap < kTaps; ++tap) {
-    int na = nbr(g, ca, tap), nb2 = nbr(g, cb, tap);
-    unsigned a0 = ld2(in, na, 2 * tq), a1 = ld2(in, nb2, 2 * tq);
-    unsigned a2 = ld2(in, na, 2 * tq + 8), a3 = ld2(in, nb2, 2 * tq + 8);
-    const __nv_bfloat16 *wt = sw + tap * kC * kC;
-    unsigned b00 = *reinterpret_cast<const unsigned *>(wt + gq * kC + 2 * tq);
-    unsigned b01 = *reinterpret_cast<const unsigned *>(wt + gq * kC + 2 * tq + 8);
-    unsigned b10 = *reinterpret_cast<const unsigned *>(wt + (gq + 8) * kC + 2 * tq);
-    unsigned b11 = *reinterpret_cast<const unsigned *>(wt + (gq + 8) * kC + 2 * tq + 8);
-    mma_bf16(d0, a0, a1, a2, a3, b00, b01);
-    mma_bf16(d1, a0, a1, a2, a3, b10, b11);
+    const int tz = tap / 9, ty = (tap / 3) % 3, tx = tap % 3;
+    unsigned b[4];
+    ldsm4<false>(b, tile_addr(wts, tap * kC + brow, bch));
+#pragma unroll
+    for (int m = 0; m < kTZ; ++m) {
+      unsigned a[4];
+      ldsm4<false>(a, tile_addr(act, ((m + tz) * kHY + w + ty) * kHX + tx + arow, ach));
+      mma_bf16(d[m], a[0], a[1], a[2], a[3], b[0], b[1]);
+      mma_bf16(d[m] + 4, a[0], a[1], a[2], a[3], b[2], b[3]);
+    }
   }
-  // epilogue: d0 -> channels 2t,2t+1 ; d1 -> 8+2t, 8+2t+1 ; [0,1] cell a, [2,3] cell b
-  const int cells[2] = {ca, cb};
+  // d[0..3] -> channels 2t, 2t+1 of cells gq, gq + 8; d[4..7] -> 8 + 2t, 9 + 2t
+  const int y = y0 + w;
+  if (y >= g.ny) return;
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    int cell = cells[h];
-    if (cell >= g.N) continue;
-    float v[4] = {d0[2 * h], d0[2 * h + 1], d1[2 * h], d1[2 * h + 1]};
-    int ch[4] = {2 * tq, 2 * tq + 1, 8 + 2 * tq, 9 + 2 * tq};
-    if (MODE == 0) {
+  for (int m = 0; m < kTZ; ++m) {
+    const int z = z0 + m;
+    if (z >= g.nz) break;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        float zz = v[q] + bias[ch[q]];
-        z_out[(size_t)cell * kC + ch[q]] = zz;
-        a_out[(size_t)cell * kC + ch[q]] = __float2bfloat16(gelu(zz));
+    for (int h = 0; h < 2; ++h) {
+      const int x = x0 + gq + 8 * h;
+      if (x >= g.nx) continue;
+      const size_t cell = x + (size_t)g.nx * (y + (size_t)g.ny * z);
+      if (MODE == 1) {
+        if (tq == 0) out[cell] = d[m][2 * h] + bias[0];
+        continue;
       }
-    } else if (MODE == 1) {
-      if (tq == 0) out[cell] = v[0] + bias[0];
-    } else {
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
-        dz_out[(size_t)cell * kC + ch[q]] = __float2bfloat16(v[q] * gelu_d(zprev[(size_t)cell * kC + ch[q]]));
+      for (int k = 0; k < 2; ++k) {   // channels 8 k + 2 tq and the next
+        const float v0 = d[m][4 * k + 2 * h], v1 = d[m][4 * k + 2 * h + 1];
+        const size_t o = cell * kC + 8 * k + 2 * tq;
+        if (MODE == 0) {
+          const float za = v0 + bias[8 * k + 2 * tq], zb = v1 + bias[8 * k + 2 * tq + 1];
+          *reinterpret_cast<float2 *>(z_out + o) = make_float2(za, zb);
+          *reinterpret_cast<__nv_bfloat162 *>(a_out + o) = __halves2bfloat162(__float2bfloat16(gelu(za)), __float2bfloat16(gelu(zb)));
+        } else {
+          const float2 zp = *reinterpret_cast<const float2 *>(zprev + o);
+          *reinterpret_cast<__nv_bfloat162 *>(dz_out + o) =
+              __halves2bfloat162(__float2bfloat16(v0 * gelu_d(zp.x)), __float2bfloat16(v1 * gelu_d(zp.y)));
+        }
+      }
     }
   }
 }
 
-// Weight gradient: part[blk][tap][co][ci] = sum over this block's cells of
-// dz[cell][co] * in[nbr(cell,tap)][ci]; bias gradient from tap 13 blocks (dz sums).
-// grid = (chunks, 27); each warp walks 16-cell steps of the chunk.
-constexpr int kWgChunk = 4096;
-__global__ void __launch_bounds__(128) k_wgrad(Grid3 g, const __nv_bfloat16 *__restrict__ dz,
-                                               const __nv_bfloat16 *__restrict__ in, float *part) {
-  __shared__ float red[4][kC * kC];
+// Weight gradient: sum over cells of dz[cell][co] * in[nbr(cell,tap)][ci], and bias gradient
+// (the sum of dz).  Each block walks tiles (its number, then every gridDim.x-th); a warp
+// takes the nine taps of one dz plane and half of the tile's rows, so a row's dz serves nine
+// products.  Sums leave the tensor cores every kWgFlush tiles (64 products of 16 cells) and
+// are added in FP32 to the warp's part[2 * block + half][tap][co][ci]; the parts are added
+// up in order by k_reduce_parts.  One launch row per tap and 2-byte gathers took 1.34 ms on
+// 1.57M cells; this takes 0.11.
+constexpr int kWgBlocks = 2 * kNumSM, kWgThreads = 192, kWgFlush = 4, kWgSmem = (kHCells + kTCells) * 32;
+__global__ void __launch_bounds__(kWgThreads) k_wgrad(Grid3 g, int tx, int ty, int ntiles,
+                                                      const __nv_bfloat16 *__restrict__ dz,
+                                                      const __nv_bfloat16 *__restrict__ in, float *part, float *bpart) {
+  extern __shared__ __align__(128) unsigned char smem_tile[];
+  const unsigned act = (unsigned)__cvta_generic_to_shared(smem_tile), grd = act + kHCells * 32;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, gq = lane >> 2, tq = lane & 3;
-  const int tap = blockIdx.y;
-  const int start = blockIdx.x * kWgChunk;
-  float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int c0 = start + w * 16; c0 < min(start + kWgChunk, g.N); c0 += 64) {
-    // A = dz^T (M = co, K = 16 cells): rows gq / gq+8, k = 2t,2t+1 / 2t+8,2t+9
-    auto pk = [&](const __nv_bfloat16 *p, int cellA, int cellB, int ch) -> unsigned {
-      unsigned lo = 0, hi = 0;
-      if (cellA >= 0 && cellA < g.N) lo = __bfloat16_as_ushort(p[(size_t)cellA * kC + ch]);
-      if (cellB >= 0 && cellB < g.N) hi = __bfloat16_as_ushort(p[(size_t)cellB * kC + ch]);
-      return lo | (hi << 16);
-    };
-    int k0 = c0 + 2 * tq, k1 = c0 + 2 * tq + 1, k8 = c0 + 2 * tq + 8, k9 = c0 + 2 * tq + 9;
-    unsigned a0 = pk(dz, k0, k1, gq), a1 = pk(dz, k0, k1, gq + 8);
-    unsigned a2 = pk(dz, k8, k9, gq), a3 = pk(dz, k8, k9, gq + 8);
-    // B = shifted input (K = cells, N = ci): n = gq (tile 0) / gq + 8 (tile 1)
-    int n0 = (k0 < g.N) ? nbr(g, k0, tap) : -1, n1 = (k1 < g.N) ? nbr(g, k1, tap) : -1;
-    int n8 = (k8 < g.N) ? nbr(g, k8, tap) : -1, n9 = (k9 < g.N) ? nbr(g, k9, tap) : -1;
-    unsigned b00 = pk(in, n0, n1, gq), b01 = pk(in, n8, n9, gq);
-    unsigned b10 = pk(in, n0, n1, gq + 8), b11 = pk(in, n8, n9, gq + 8);
-    mma_bf16(d0, a0, a1, a2, a3, b00, b01);
-    mma_bf16(d1, a0, a1, a2, a3, b10, b11);
+  const int plane = w % 3, half = w / 3;
+  const int mi = lane >> 3;
+  const int arow = (lane & 7) + 8 * (mi >> 1), ach = mi & 1;    // A = dz^T: cells, output channels
+  const int brow = (lane & 7) + 8 * (mi & 1), bch = mi >> 1;    // B: cells, input channels
+  float *mine = part + ((size_t)(2 * blockIdx.x + half) * kTaps + plane * 9) * kC * kC;
+  float d[9][8], bs = 0.f;
+  auto clear = [&]() {
+#pragma unroll
+    for (int t = 0; t < 9; ++t)
+#pragma unroll
+      for (int q = 0; q < 8; ++q) d[t][q] = 0.f;
+  };
+  bool first = true;
+  auto flush = [&]() {
+#pragma unroll
+    for (int t = 0; t < 9; ++t)
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int co = gq + (q & 2 ? 8 : 0), ci = 2 * tq + (q & 1) + (q & 4 ? 8 : 0);
+        float *o = mine + (t * kC + co) * kC + ci;
+        *o = first ? d[t][q] : *o + d[t][q];
+      }
+    first = false;
+  };
+  clear();
+  int since = 0;
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const int bz = tile / (tx * ty), r = tile - bz * tx * ty, by = r / tx, bx = r - by * tx;
+    __syncthreads();   // the last tile has been read
+    load_tile<true>(g, in, bx * kTX, by * kTY, bz * kTZ, act);
+    load_tile<false>(g, dz, bx * kTX, by * kTY, bz * kTZ, grd);
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    for (int k = 0; k < kTY * kTZ / 2; ++k) {
+      const int row = half * (kTY * kTZ / 2) + k, z = row / kTY, y = row % kTY;
+      unsigned a[4];
+      ldsm4<true>(a, tile_addr(grd, row * kTX + arow, ach));
+#pragma unroll
+      for (int t = 0; t < 9; ++t) {
+        unsigned b[4];
+        ldsm4<true>(b, tile_addr(act, ((z + plane) * kHY + y + t / 3) * kHX + t % 3 + brow, bch));
+        mma_bf16(d[t], a[0], a[1], a[2], a[3], b[0], b[1]);
+        mma_bf16(d[t] + 4, a[0], a[1], a[2], a[3], b[2], b[3]);
+      }
+    }
+    if (threadIdx.x < 128) {   // bias: channel t & 15, the cells of residue t >> 4 mod 8
+      const int ch = threadIdx.x & 15;
+      for (int c = threadIdx.x >> 4; c < kTCells; c += 8)
+        bs += __bfloat162float(*reinterpret_cast<const __nv_bfloat16 *>(
+            smem_tile + (tile_addr(grd, c, ch >> 3) - act) + 2 * (ch & 7)));
+    }
+    if (++since == kWgFlush) {
+      flush();
+      clear();
+      since = 0;
+    }
   }
-  // D[co][ci]: d0 -> (co gq / gq+8, ci 2t,2t+1), d1 -> ci + 8
-  float *r = red[w];
-  r[gq * kC + 2 * tq] = d0[0];       r[gq * kC + 2 * tq + 1] = d0[1];
-  r[(gq + 8) * kC + 2 * tq] = d0[2]; r[(gq + 8) * kC + 2 * tq + 1] = d0[3];
-  r[gq * kC + 8 + 2 * tq] = d1[0];       r[gq * kC + 9 + 2 * tq] = d1[1];
-  r[(gq + 8) * kC + 8 + 2 * tq] = d1[2]; r[(gq + 8) * kC + 9 + 2 * tq] = d1[3];
+  if (since || first) flush();
+  __shared__ float sh[128];
   __syncthreads();
-  for (int e = threadIdx.x; e < kC * kC; e += blockDim.x) {
-    float s = red[0][e] + red[1][e] + red[2][e] + red[3][e];
-    part[((size_t)blockIdx.x * kTaps + tap) * kC * kC + e] = s;
-  }
-}
-
-// bias gradient partials: sum of dz over cells per channel
-__global__ void __launch_bounds__(256) k_bgrad(Grid3 g, const __nv_bfloat16 *dz, float *part) {
-  __shared__ float sh[256];
-  int ch = threadIdx.x & 15;
-  float s = 0.f;
-  int start = blockIdx.x * kWgChunk;
-  for (int c = start + (threadIdx.x >> 4); c < min(start + kWgChunk, g.N); c += 16)
-    s += __bfloat162float(dz[(size_t)c * kC + ch]);
-  sh[threadIdx.x] = s;
+  if (threadIdx.x < 128) sh[threadIdx.x] = bs;
   __syncthreads();
-  if (threadIdx.x < 16) {
+  if (threadIdx.x < kC) {
     float t = 0.f;
-    for (int k = 0; k < 16; ++k) t += sh[k * 16 + threadIdx.x];
-    part[(size_t)blockIdx.x * kC + threadIdx.x] = t;
+    for (int k = 0; k < 8; ++k) t += sh[k * kC + threadIdx.x];
+    bpart[blockIdx.x * kC + threadIdx.x] = t;
   }
 }
 
-// sum weight partials in chunk order into grad (deterministic)
-__global__ void k_reduce_parts(int nchunks, const float *part, int len, float *grad) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= len) return;
+// sum the parts in order into grad (deterministic): eight runs of parts per value, then the
+// runs
+__global__ void __launch_bounds__(256) k_reduce_parts(int nparts, const float *__restrict__ part, int len, float *grad) {
+  __shared__ float sh[8][32];
+  const int e = blockIdx.x * 32 + (threadIdx.x & 31), q = threadIdx.x >> 5;
+  const int per = (nparts + 7) / 8, k1 = min(nparts, (q + 1) * per);
   float s = 0.f;
-  for (int k = 0; k < nchunks; ++k) s += part[(size_t)k * len + e];
-  grad[e] = s;
+  if (e < len)
+    for (int k = q * per; k < k1; ++k) s += part[(size_t)k * len + e];
+  sh[q][threadIdx.x & 31] = s;
+  __syncthreads();
+  if (q == 0 && e < len) {
+    for (int k = 1; k < 8; ++k) s += sh[k][threadIdx.x];
+    grad[e] = s;
+  }
 }
 
 // loss: dL/dout = 2 (out - y) / N, written as channel 0 of dz; partial sums of the squared error
@@ -245,10 +317,10 @@ __global__ void __launch_bounds__(256) k_loss(int n, const float *out, const flo
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     float e = out[i] - y[i];
     s += (double)e * e;
-    __nv_bfloat16 *q = dz + (size_t)i * kC;
-    q[0] = __float2bfloat16(2.0f * e / (float)n);
-#pragma unroll
-    for (int c = 1; c < kC; ++c) q[c] = __float2bfloat16(0.f);
+    uint4 q = make_uint4(0u, 0u, 0u, 0u), *d = reinterpret_cast<uint4 *>(dz + (size_t)i * kC);
+    d[1] = q;
+    q.x = __bfloat16_as_ushort(__float2bfloat16(2.0f * e / (float)n));
+    d[0] = q;
   }
   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
@@ -376,25 +448,32 @@ static int cnn_reserve(Net &n, int N) {
   if (n.dz2) cudaFree(n.dz2);
   MSG_CUDA(cudaMalloc(&n.dz, (size_t)N * kC * 2));
   MSG_CUDA(cudaMalloc(&n.dz2, (size_t)N * kC * 2));
-  int chunks = (N + kWgChunk - 1) / kWgChunk;
-  if (n.part) cudaFree(n.part);
-  n.part_cap = chunks;
-  MSG_CUDA(cudaMalloc(&n.part, (size_t)chunks * kTaps * kC * kC * 4));
+  if (!n.part) {
+    MSG_CUDA(cudaMalloc(&n.part, ((size_t)2 * kWgBlocks * kWl + kWgBlocks * kC) * 4));
+    MSG_CUDA(cudaFuncSetAttribute(k_conv<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSmem));
+    MSG_CUDA(cudaFuncSetAttribute(k_conv<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSmem));
+    MSG_CUDA(cudaFuncSetAttribute(k_conv<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSmem));
+    MSG_CUDA(cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem));
+  }
   n.cap = N;
   return MSG_OK;
 }
 
+static dim3 tiles(const Grid3 &g) {
+  return dim3((g.nx + kTX - 1) / kTX, (g.ny + kTY - 1) / kTY, (g.nz + kTZ - 1) / kTZ);
+}
+
 static int cnn_forward(Net &n, const Grid3 &g, const __nv_bfloat16 *x) {
   cudaStream_t s = n.stream;
-  int blocks = (g.N + 127) / 128;   // 8 warps x 16 cells
+  const dim3 blocks = tiles(g);
   const __nv_bfloat16 *in = x;
   for (int l = 0; l < kLayers - 1; ++l) {
-    k_conv<0><<<blocks, 256, 0, s>>>(g, in, n.w16 + (size_t)l * kWl, n.w32 + (size_t)l * kPl + kWl, n.z[l],
+    k_conv<0><<<blocks, 32 * kTY, kConvSmem, s>>>(g, in, n.w16 + (size_t)l * kWl, n.w32 + (size_t)l * kPl + kWl, n.z[l],
                                      n.a[l + 1], nullptr, nullptr, nullptr);
     MSG_CHECK_LAUNCH();
     in = n.a[l + 1];
   }
-  k_conv<1><<<blocks, 256, 0, s>>>(g, in, n.w16 + (size_t)3 * kWl, n.w32 + (size_t)3 * kPl + kWl, nullptr, nullptr,
+  k_conv<1><<<blocks, 32 * kTY, kConvSmem, s>>>(g, in, n.w16 + (size_t)3 * kWl, n.w32 + (size_t)3 * kPl + kWl, nullptr, nullptr,
                                    n.z[3], nullptr, nullptr);
   MSG_CHECK_LAUNCH();
   return MSG_OK;
@@ -403,21 +482,20 @@ static int cnn_forward(Net &n, const Grid3 &g, const __nv_bfloat16 *x) {
 // backward from dz (channel 0 = dL/dout) at the output; grad filled
 static int cnn_backward(Net &n, const Grid3 &g, const __nv_bfloat16 *x) {
   cudaStream_t s = n.stream;
-  int blocks = (g.N + 127) / 128;
-  int chunks = (g.N + kWgChunk - 1) / kWgChunk;
+  const dim3 blocks = tiles(g);
+  const int ntiles = (int)(blocks.x * blocks.y * blocks.z), wb = std::min(ntiles, kWgBlocks);
   __nv_bfloat16 *dz = n.dz, *dzn = n.dz2;
+  float *bpart = n.part + (size_t)2 * kWgBlocks * kWl;
   for (int l = kLayers - 1; l >= 0; --l) {
     const __nv_bfloat16 *in = (l == 0) ? x : n.a[l];
-    k_wgrad<<<dim3(chunks, kTaps), 128, 0, s>>>(g, dz, in, n.part);
+    k_wgrad<<<wb, kWgThreads, kWgSmem, s>>>(g, blocks.x, blocks.y, ntiles, dz, in, n.part, bpart);
     MSG_CHECK_LAUNCH();
-    k_reduce_parts<<<(kWl + 255) / 256, 256, 0, s>>>(chunks, n.part, kWl, n.grad + (size_t)l * kPl);
+    k_reduce_parts<<<(kWl + 31) / 32, 256, 0, s>>>(2 * wb, n.part, kWl, n.grad + (size_t)l * kPl);
     MSG_CHECK_LAUNCH();
-    k_bgrad<<<chunks, 256, 0, s>>>(g, dz, n.part);
-    MSG_CHECK_LAUNCH();
-    k_reduce_parts<<<1, 32, 0, s>>>(chunks, n.part, kC, n.grad + (size_t)l * kPl + kWl);
+    k_reduce_parts<<<1, 256, 0, s>>>(wb, bpart, kC, n.grad + (size_t)l * kPl + kWl);
     MSG_CHECK_LAUNCH();
     if (l > 0) {
-      k_conv<2><<<blocks, 256, 0, s>>>(g, dz, n.wt16 + (size_t)l * kWl, nullptr, nullptr, nullptr, nullptr,
+      k_conv<2><<<blocks, 32 * kTY, kConvSmem, s>>>(g, dz, n.wt16 + (size_t)l * kWl, nullptr, nullptr, nullptr, nullptr,
                                        n.z[l - 1], dzn);
       MSG_CHECK_LAUNCH();
       std::swap(dz, dzn);
