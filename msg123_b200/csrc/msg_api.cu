@@ -127,10 +127,11 @@ static int make_matvec(msg_ctx *c, double *l2_rhs, bool reuse, bool assembled = 
   return MSG_OK;
 }
 
-static int solve_linalg(msg_ctx *c, double init_norm, double *x, double *last_norm, bool x_zero = false) {
+static int solve_linalg(msg_ctx *c, double init_norm, double *x, double *last_norm, bool x_zero = false,
+                        ErrAhead *ahead = nullptr) {
   if (c->timing) cudaEventRecord(c->ev[3], c->stream);
   c->bnorm = init_norm;
-  int rc = solve_bicgs(c, x, x_zero);
+  int rc = solve_bicgs(c, x, x_zero, ahead);
   if (rc) return rc;
   *last_norm = c->rnorm;
   if (c->timing) {
@@ -377,7 +378,7 @@ static int convlog_push(msg_ctx *c, int maxnun) {
 // calc_numsol (Nonlinear_solution.f90:33-294)
 static int calc_numsol(msg_ctx *c, msg_stats_t *stx) {
   const int n = c->N;
-  int rc, maxnun = 0, status = MSG_NEWTON_MAXIT, nan = 0;
+  int rc, maxnun = 0, status = MSG_NEWTON_MAXIT;
   double maxunk, check_val;
   msg_stats_t st;
   memset(&st, 0, sizeof(st));
@@ -415,12 +416,12 @@ static int calc_numsol(msg_ctx *c, msg_stats_t *stx) {
     if (c->prm.maxinn_iter < 1) MSG_CUDA(cudaMemsetAsync(c->head_change, 0, (size_t)n * 8, c->stream));
     c->conv_flag = 0;
     c->errtol = c->prm.lin_tol > 0 ? c->prm.lin_tol : c->eta;
-    if ((rc = solve_linalg(c, c->l2_pre, c->head_change, &c->l2_jnorm, true))) return rc;   // from dh = 0
+    ErrAhead full{c->head_new, c->head_pre, false, {}};
+    if ((rc = solve_linalg(c, c->l2_pre, c->head_change, &c->l2_jnorm, true, &full))) return rc;   // from dh = 0
     st.inner_total += c->in_iter; st.in_iter_last = c->in_iter;
     // head_new = head_pre + dh, formed inside check_abserrmax's pass
-    if ((rc = abserrmax(c, c->head_new, c->head_pre, &c->maxvar, &maxunk, &maxnun, &nan, c->head_change))) return rc;
-    const double maxvar_full = c->maxvar, maxunk_full = maxunk;   // of the full step, for the line search below
-    const int maxnun_full = maxnun, nan_full = nan;
+    if (!full.done && (rc = abserrmax(c, c->head_new, c->head_pre, full.e, c->head_change))) return rc;
+    c->maxvar = full.e.change; maxunk = full.e.value; maxnun = full.e.cell;
     check_val = std::fabs(c->maxvar) * c->len_scal;
     maxunk = std::fabs(maxunk) * c->len_scal;
     double crit = c->prm.criteria_rel ? c->prm.criteria * maxunk : c->prm.criteria;
@@ -437,11 +438,8 @@ static int calc_numsol(msg_ctx *c, msg_stats_t *stx) {
       if ((rc = run_backtr(c))) return rc;
       evaluated = true;
       // check_abserrmax again: the same values as above unless the line search moved head_new
-      if (c->head_moved) {
-        if ((rc = abserrmax(c, c->head_new, c->head_pre, &c->maxvar, &maxunk, &maxnun, &nan))) return rc;
-      } else {
-        c->maxvar = maxvar_full; maxunk = maxunk_full; maxnun = maxnun_full; nan = nan_full;
-      }
+      if (c->head_moved && (rc = abserrmax(c, c->head_new, c->head_pre, full.e))) return rc;
+      c->maxvar = full.e.change; maxunk = full.e.value; maxnun = full.e.cell;
       check_val = std::fabs(c->maxvar) * c->len_scal;
       maxunk = std::fabs(maxunk) * c->len_scal;
       crit = c->prm.criteria_rel ? c->prm.criteria * maxunk : c->prm.criteria;
@@ -674,7 +672,7 @@ static int create_impl(msg_ctx *c, const msg_grid_t *g, const msg_params_t *p) {
   npart = std::max(npart, (size_t)((g->nx + 31) / 32) * ((g->ny + 7) / 8) * g->nz + 64);
   ALLOC(c->part, npart * 8);
   c->npart = npart;
-  ALLOC(c->dres, 16 * 8);
+  ALLOC(c->dres, 24 * 8);
   MSG_CUDA(cudaMallocHost((void **)&c->hpin, ((size_t)kRedBlocks * 8 + 16) * 8));   // and the box, wave_err
   int rc = scan_reserve(c, (int)N);
   if (rc) return rc;
@@ -1272,7 +1270,7 @@ static void free_ctx(msg_ctx *c) {
                 c->left_off, c->right_off, c->hydf_conn, c->abyd_conn, c->head_new, c->head_old, c->head_pre,
                 c->head_change, c->srat_new, c->srat_old, c->surf_head, c->surf_old, c->new_f, c->kr, c->kr_per,
                 c->alp, c->sto, c->stod, c->tmpv, c->dmat, c->lu, c->rhs, c->rhs_alt, c->head_old2, c->slope_rhs, c->dilu_d, c->r, c->rs,
-                c->p, c->v, c->t, c->z, c->part, c->scan_sums, c->wave_order, c->wave_ticket, c->wave_slots, c->dmat_f, c->lu_f, c->dres};
+                c->p, c->v, c->t, c->z, c->part, c->scan_sums, c->fin_scratch, c->fin_cnt, c->wave_order, c->wave_ticket, c->wave_slots, c->dmat_f, c->lu_f, c->dres};
   for (auto q : dp) if (q) cudaFree(q);
   if (c->hpin) cudaFreeHost(c->hpin);
   for (int k = 0; k < 8; ++k) if (c->ev[k]) cudaEventDestroy(c->ev[k]);

@@ -69,7 +69,11 @@ struct msg_ctx {
   double *part;                                  // reduction partials [npart]
   size_t npart;
   double *hpin;                                  // pinned host scalars
-  double *dres;                                  // device reduction results [16]
+  double *dres;                                  // device reduction results [24]
+  double *fin_scratch;                           // second reduction stage of long arrays
+  int *fin_cnt;
+  unsigned *res_word, res_token;                 // pinned word behind published results, and its value
+  int one_half;                                  // the last solve from x = 0 ended at its first residual norm
   // ---- scans (msg_linear.cu): chunk sums, and the box their totals reach the host in -------
   int *scan_sums, scan_cap;
   msg::HostBox *box;
@@ -137,16 +141,27 @@ int launch_precon_dilu(msg_ctx *c);
 int launch_solve_ilu(msg_ctx *c, const double *b, double *x);
 int launch_spmv(msg_ctx *c, const double *x, double *y);
 // x in/out (device), uses c->rhs, c->bnorm, c->errtol; x_zero: x holds zeros on entry
-int solve_bicgs(msg_ctx *c, double *x, bool x_zero = false);
-// reductions (results land in c->hpin after a sync)
+// largest change and largest value of an update, the cell (1-based) of the change, any NaN
+struct ErrMax {
+  double change, value;
+  int cell, nan;
+};
+struct ErrAhead {          // abserrmax of xn = xp + x, taken inside the solve when done
+  double *xn;
+  const double *xp;
+  bool done;
+  ErrMax e;
+};
+int solve_bicgs(msg_ctx *c, double *x, bool x_zero = false, ErrAhead *ahead = nullptr);
+// reductions (results land in c->hpin with the token that fetch_res waits for)
 int dot(msg_ctx *c, const double *a, const double *b, int n, double *out);   // sync + host value
 // sum narr partial arrays (nparts each, consecutive in c->part) on the device; sync; host values
 int finish(msg_ctx *c, int nparts, int narr, double *out);
-int finish_to(msg_ctx *c, int nparts, int narr, int slot);   // into dres[slot..], no wait
-int fetch_res(msg_ctx *c, int count, double *out);           // dres[0..count) to the host (waits)
+int finish_to(msg_ctx *c, int nparts, int narr, int slot, int count = 0);   // into dres[slot..]; count > 0:
+                                                                             // dres[0..count) to the host
+int fetch_res(msg_ctx *c, int count, double *out);                          // waits for them
 int norm1(msg_ctx *c, const double *a, int n, double *out);
-int abserrmax(msg_ctx *c, double *xn, const double *xp, double *chmax, double *xmax, int *nun, int *nan,
-              const double *dh = nullptr);   // dh: form xn = xp + dh first
+int abserrmax(msg_ctx *c, double *xn, const double *xp, ErrMax &e, const double *dh = nullptr);   // dh: form xn = xp + dh first
 int lam_length(msg_ctx *c, const double *dh, const double *hn, double *out);
 // ||dh||^2, ||f||^2, (s, jv) (jv null: (s, b - r)) and lam_length(dh, hn) in one pass
 int backtr_stats(msg_ctx *c, const double *dh, const double *hn, const double *f, const double *s, const double *jv,

@@ -15,6 +15,8 @@
 
 namespace msg {
 
+constexpr int kFinArr = 4;   // arrays of one second reduction stage; counters: theirs, the stage's, abserrmax's
+
 struct Geo3 {
   int nx, ny, nz, nxy, N;
 };
@@ -116,17 +118,18 @@ __global__ void __launch_bounds__(kScanT) k_scan_apply(const int *__restrict__ i
   }
 }
 
-// Wait for the box's words of the scan launched last: the host looks at the pinned token
-// instead of waiting for the stream and copying the words (15 us a time; this takes 5).
-static int box_wait(msg_ctx *c) {
+// Wait until a kernel has written `token` behind its results in pinned memory: the host looks
+// at the word instead of copying the results and waiting for the stream (15 us a time; this
+// takes 5).
+static int token_wait(msg_ctx *c, const unsigned *at, unsigned token) {
   for (unsigned it = 1;; ++it) {
-    if (*(volatile unsigned *)&c->box->token == c->box_token) break;
+    if (*(const volatile unsigned *)at == token) break;
     if ((it & 0x3f) == 0) std::this_thread::yield();   // more worker threads than cores
     if ((it & 0xfff) == 0) {   // a failed kernel never writes the token
       const cudaError_t e = cudaStreamQuery(c->stream);
-      if (e == cudaSuccess && *(volatile unsigned *)&c->box->token == c->box_token) break;
+      if (e == cudaSuccess && *(const volatile unsigned *)at == token) break;
       if (e != cudaErrorNotReady) {
-        set_error("scan: %s", e == cudaSuccess ? "no result" : cudaGetErrorString(e));
+        set_error("wait for a result: %s", e == cudaSuccess ? "none" : cudaGetErrorString(e));
         return MSG_ERR_CUDA;
       }
     }
@@ -148,7 +151,7 @@ int scan_exclusive(msg_ctx *c, const int *in, int *out, int n, int *got, const i
   k_scan_apply<<<nb, kScanT, 0, c->stream>>>(in, out, n, c->scan_sums, w1, w2, got ? c->box : nullptr, c->box_token);
   MSG_CHECK_LAUNCH();
   if (got) {
-    int rc = box_wait(c);
+    int rc = token_wait(c, &c->box->token, c->box_token);
     if (rc) return rc;
     got[0] = c->box->v[0];
     if (w1) got[1] = c->box->v[1];
@@ -157,7 +160,8 @@ int scan_exclusive(msg_ctx *c, const int *in, int *out, int n, int *got, const i
   return MSG_OK;
 }
 
-// Scratch of the scans of up to n elements, and the box.
+// Scratch of the scans of up to n elements and of the second reduction stage, and the pinned
+// words results reach the host in.
 int scan_reserve(msg_ctx *c, int n) {
   c->scan_cap = (n + kScanE - 1) / kScanE + 1;
   MSG_CUDA(cudaMalloc(&c->scan_sums, (size_t)c->scan_cap * 4));
@@ -165,6 +169,12 @@ int scan_reserve(msg_ctx *c, int n) {
   c->box = reinterpret_cast<HostBox *>(c->hpin + kRedBlocks * 8);
   memset(c->box, 0, sizeof(HostBox));
   c->box_token = 0;
+  c->res_word = reinterpret_cast<unsigned *>(c->hpin + kRedBlocks * 8 + 9);
+  *c->res_word = 0;
+  c->res_token = 0;
+  MSG_CUDA(cudaMalloc(&c->fin_scratch, (size_t)4 * 8 * 1024 * 8));
+  MSG_CUDA(cudaMalloc(&c->fin_cnt, (kFinArr + 2) * 4));
+  MSG_CUDA(cudaMemsetAsync(c->fin_cnt, 0, (kFinArr + 2) * 4, c->stream));
   return MSG_OK;
 }
 
@@ -229,48 +239,100 @@ __global__ void k_bicg_p(int n, const double *pin, double *p, const double *r, c
     p[i] = __dadd_rn(r[i], __dmul_rn(beta, __dsub_rn(pin[i], __dmul_rn(omega, v[i]))));
 }
 
+// Sums of NV values over groups of 256 consecutive elements, one partial per group (the order
+// of block_sum): a block takes kGr groups, so a thread has that many loads in flight and one
+// barrier serves them all.  One group per block, with two barriers per value, left k_dot2 at
+// a third of the copy rate.
+constexpr int kGr = 4;
+static int ngroups(int n) { return (n + 255) / 256; }
+static int gblk(int n) { return (ngroups(n) + kGr - 1) / kGr; }
+template <int NV>
+__device__ __forceinline__ void group_sums(double (&v)[NV][kGr], int ng, double *part) {
+  __shared__ double sh[NV][kGr][8];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int a = 0; a < NV; ++a)
+#pragma unroll
+      for (int k = 0; k < kGr; ++k) v[a][k] = __dadd_rn(v[a][k], __shfl_down_sync(0xffffffffu, v[a][k], o));
+  if (lane == 0) {
+#pragma unroll
+    for (int a = 0; a < NV; ++a)
+#pragma unroll
+      for (int k = 0; k < kGr; ++k) sh[a][k][w] = v[a][k];
+  }
+  __syncthreads();
+  const int t = threadIdx.x;
+  if (t < NV * kGr) {
+    const int a = t / kGr, k = t % kGr, g = blockIdx.x * kGr + k;
+    double r = 0.0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) r = __dadd_rn(r, sh[a][k][i]);
+    if (g < ng) part[(size_t)a * ng + g] = r;
+  }
+}
+
+// A quotient of two scalars, each on the device or (null pointer) from the host: the step
+// lengths of BiCGStab without a host round trip to form them.
+struct Quot {
+  const double *num, *den;
+  double hnum;
+  __device__ __forceinline__ double get() const { return __ddiv_rn(num ? *num : hnum, *den); }
+};
+
 // x = xin + a*z; r = rin - a*w; partials ||r||^2 and (r, rs).  xin null: x starts at zero
 // (0 + a*z, the value the zeroed x gave, without reading it); rin: the residual before the
 // update (the right-hand side itself on the first update from x = 0).
-__global__ void __launch_bounds__(256) k_bicg_xr(int n, const double *xin, double *x, const double *rin, double *r,
-                                                 const double *z, const double *w, const double *rs, double a,
+__global__ void __launch_bounds__(256) k_bicg_xr(int n, int ng, const double *xin, double *x, const double *rin, double *r,
+                                                 const double *z, const double *w, const double *rs, Quot quot,
                                                  double *part) {
-  __shared__ double sh[8];
-  double s0 = 0.0, s1 = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    x[i] = __dadd_rn(xin ? xin[i] : 0.0, __dmul_rn(a, z[i]));
-    double ri = __dsub_rn(rin[i], __dmul_rn(a, w[i]));
-    r[i] = ri;
-    s0 = __dadd_rn(s0, __dmul_rn(ri, ri));
-    s1 = __dadd_rn(s1, __dmul_rn(ri, rs[i]));
+  const double a = quot.get();
+  double v[2][kGr], zi[kGr], wi[kGr], ri[kGr], si[kGr], xi[kGr];
+  const int i0 = blockIdx.x * (256 * kGr) + threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < kGr; ++k) {
+    const int i = i0 + 256 * k;
+    const bool in = i < n;
+    zi[k] = in ? z[i] : 0.0; wi[k] = in ? w[i] : 0.0; ri[k] = in ? rin[i] : 0.0; si[k] = in ? rs[i] : 0.0;
+    xi[k] = in && xin ? xin[i] : 0.0;
   }
-  double t = block_sum<256>(s0, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = t;
-  t = block_sum<256>(s1, sh);
-  if (threadIdx.x == 0) part[gridDim.x + blockIdx.x] = t;
+#pragma unroll
+  for (int k = 0; k < kGr; ++k) {
+    const int i = i0 + 256 * k;
+    v[0][k] = v[1][k] = 0.0;
+    if (i < n) {
+      x[i] = __dadd_rn(xi[k], __dmul_rn(a, zi[k]));
+      const double t = __dsub_rn(ri[k], __dmul_rn(a, wi[k]));
+      r[i] = t;
+      v[0][k] = __dmul_rn(t, t);
+      v[1][k] = __dmul_rn(t, si[k]);
+    }
+  }
+  group_sums<2>(v, ng, part);
 }
 
-__global__ void __launch_bounds__(256) k_dot2(int n, const double *a, const double *b, const double *cc, double *part) {
-  __shared__ double sh[8];
-  double s0 = 0.0, s1 = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    s0 = __dadd_rn(s0, __dmul_rn(a[i], b[i]));
-    if (cc) s1 = __dadd_rn(s1, __dmul_rn(a[i], cc[i]));
+// partials of (a, b)
+__global__ void __launch_bounds__(256) k_dot(int n, int ng, const double *a, const double *b, double *part) {
+  double v[1][kGr];
+  const int i0 = blockIdx.x * (256 * kGr) + threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < kGr; ++k) {
+    const int i = i0 + 256 * k;
+    v[0][k] = i < n ? __dmul_rn(a[i], b[i]) : 0.0;
   }
-  double t = block_sum<256>(s0, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = t;
-  if (cc) {
-    t = block_sum<256>(s1, sh);
-    if (threadIdx.x == 0) part[gridDim.x + blockIdx.x] = t;
-  }
+  group_sums<1>(v, ng, part);
 }
 
-__global__ void __launch_bounds__(256) k_norm1(int n, const double *a, double *part) {
-  __shared__ double sh[8];
-  double s0 = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) s0 = __dadd_rn(s0, fabs(a[i]));
-  double t = block_sum<256>(s0, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = t;
+__global__ void __launch_bounds__(256) k_norm1(int n, int ng, const double *a, double *part) {
+  double v[1][kGr];
+  const int i0 = blockIdx.x * (256 * kGr) + threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < kGr; ++k) {
+    const int i = i0 + 256 * k;
+    v[0][k] = i < n ? fabs(a[i]) : 0.0;
+  }
+  group_sums<1>(v, ng, part);
 }
 
 __global__ void k_axpby(int n, double *y, const double *x, double a, const double *w) {
@@ -292,42 +354,102 @@ __device__ __forceinline__ ArgMax amax(ArgMax p, ArgMax q) {
   return p;
 }
 
+// What a finishing kernel hands to the host: `count` results from res into pinned words, then
+// the token (null word: nothing).
+struct Publish {
+  const double *res;
+  double *host;
+  int count;
+  unsigned *word, token;
+  __device__ __forceinline__ void operator()() const {   // one thread, all results written
+    if (!word) return;
+    __threadfence();
+    for (int k = 0; k < count; ++k) host[k] = __ldcg(res + k);
+    __threadfence_system();
+    *(volatile unsigned *)word = token;
+  }
+};
+// True in the block that arrives last of `total` (all its threads); the counter is left at 0.
+__device__ __forceinline__ bool last_block(int *cnt, int total) {
+  __shared__ int s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_last = atomicAdd(cnt, 1) == total - 1;
+    if (s_last) *cnt = 0;
+  }
+  __syncthreads();
+  if (s_last) __threadfence();
+  return s_last;
+}
+
 // dh non-null: first forms xn = xp + 1*dh (the Newton update, the axpby it replaces, same
-// rounding) and writes it, so xn is not read back.
+// rounding) and writes it, so xn is not read back.  The last block to finish reduces the
+// blocks' results to res[0 .. 6]: |change|, change, cell, |value|, value, cell, any NaN.
 __global__ void __launch_bounds__(256) k_abserrmax(int n, double *xn, const double *xp, const double *dh,
-                                                   double *part) {
+                                                   double *part, double *res, int *cnt, Publish pub) {
   __shared__ ArgMax s1[256], s2[256];
   __shared__ int snan[256];
   ArgMax c = {0.0, 0.0, -1}, x = {0.0, 0.0, -1};
   int nan = 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    double v;
-    if (dh) {
-      v = __dadd_rn(xp[i], __dmul_rn(1.0, dh[i]));
-      xn[i] = v;
-    } else {
-      v = xn[i];
+  const int st = gridDim.x * blockDim.x;
+  for (int i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += 4 * st) {
+    double p[4], v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = i0 + u * st;
+      p[u] = i < n ? xp[i] : 0.0;
+      v[u] = i < n ? (dh ? dh[i] : xn[i]) : 0.0;
     }
-    if (v != v) nan = 1;
-    double dv = __dsub_rn(v, xp[i]);
-    c = amax(c, ArgMax{fabs(dv), dv, i});
-    x = amax(x, ArgMax{fabs(v), v, i});
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = i0 + u * st;
+      if (i < n) {
+        double t = v[u];
+        if (dh) {
+          t = __dadd_rn(p[u], __dmul_rn(1.0, t));
+          xn[i] = t;
+        }
+        if (t != t) nan = 1;
+        const double dv = __dsub_rn(t, p[u]);
+        c = amax(c, ArgMax{fabs(dv), dv, i});
+        x = amax(x, ArgMax{fabs(t), t, i});
+      }
+    }
   }
-  s1[threadIdx.x] = c; s2[threadIdx.x] = x; snan[threadIdx.x] = nan;
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) {
-      s1[threadIdx.x] = amax(s1[threadIdx.x], s1[threadIdx.x + o]);
-      s2[threadIdx.x] = amax(s2[threadIdx.x], s2[threadIdx.x + o]);
-      snan[threadIdx.x] |= snan[threadIdx.x + o];
-    }
+  auto reduce = [&]() {
+    s1[threadIdx.x] = c; s2[threadIdx.x] = x; snan[threadIdx.x] = nan;
     __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    double *q = part + (size_t)blockIdx.x * 8;
+    for (int o = 128; o > 0; o >>= 1) {
+      if ((int)threadIdx.x < o) {
+        s1[threadIdx.x] = amax(s1[threadIdx.x], s1[threadIdx.x + o]);
+        s2[threadIdx.x] = amax(s2[threadIdx.x], s2[threadIdx.x + o]);
+        snan[threadIdx.x] |= snan[threadIdx.x + o];
+      }
+      __syncthreads();
+    }
+  };
+  auto put = [&](double *q) {
     q[0] = s1[0].a; q[1] = s1[0].v; q[2] = (double)s1[0].idx;
     q[3] = s2[0].a; q[4] = s2[0].v; q[5] = (double)s2[0].idx;
     q[6] = (double)snan[0];
+  };
+  reduce();
+  if (threadIdx.x == 0) put(part + (size_t)blockIdx.x * 8);
+  if (!last_block(cnt, gridDim.x)) return;
+  c = x = ArgMax{0.0, 0.0, -1};
+  nan = 0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += 256) {
+    const double *q = part + (size_t)b * 8;
+    const ArgMax cb = {__ldcg(q), __ldcg(q + 1), (int)__ldcg(q + 2)}, xb = {__ldcg(q + 3), __ldcg(q + 4), (int)__ldcg(q + 5)};
+    if (cb.idx >= 0) c = amax(c, cb);
+    if (xb.idx >= 0) x = amax(x, xb);
+    nan |= (int)__ldcg(q + 6);
+  }
+  reduce();
+  if (threadIdx.x == 0) {
+    put(res);
+    pub();
   }
 }
 
@@ -365,141 +487,193 @@ static int fetch_partials(msg_ctx *c, int count) {
   return wave_check(c);
 }
 
-// Second reduction stage: block a sums part[a*nparts .. a*nparts + nparts) in a fixed
-// order, so every result repeats bit for bit: each thread keeps eight running sums over
-// the strided elements (eight loads in flight instead of one dependent chain), combines
-// them in a fixed tree, then the block reduces in a fixed tree.
-// MAXB: bit a set -> block a takes the maximum of its array instead of the sum.
-template <int MAXB = 0>
-__global__ void __launch_bounds__(1024) k_finish(const double *part, int nparts, double *out) {
+// Second reduction stage: array a is part[a*nparts .. a*nparts + nparts), summed in a fixed
+// order, so every result repeats bit for bit: thread t keeps eight running sums over the
+// elements t + 1024 u + 8192 k, u = 0 .. 7, combines them in a fixed tree, then the block
+// reduces in a fixed tree.  Long arrays give each u a block of its own (split = 8) and the
+// last block to finish combines them, the same sums: one block needed 42 us for 98 304
+// partials, of which it had too few loads in flight.  When count > 0 the block that finishes
+// the last array hands results to the host.
+// MAXB: bit a set -> array a takes the maximum instead of the sum.
+constexpr int kFinSplit = 8;
+template <int MAXB>
+__global__ void __launch_bounds__(1024) k_finish(const double *part, int nparts, int narr, int split, double *out,
+                                                 double *scratch, int *cnt, Publish pub) {
   __shared__ double sh[1024];
-  const double *p = part + (size_t)blockIdx.x * nparts;
-  const bool mx = (MAXB >> blockIdx.x) & 1;
+  const int arr = blockIdx.x / split, t = threadIdx.x;
+  const double *p = part + (size_t)arr * nparts;
+  const bool mx = (MAXB >> arr) & 1;
+  auto comb = [&](double x, double y) { return mx ? fmax(x, y) : __dadd_rn(x, y); };
   constexpr int U = 8;
   double a[U];
 #pragma unroll
   for (int u = 0; u < U; ++u) a[u] = 0.0;
-  for (int base = threadIdx.x; base < nparts; base += U * blockDim.x) {
+  if (split == 1) {
+    for (int base = t; base < nparts; base += U * 1024) {
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int i = base + u * blockDim.x;
-      if (i < nparts) a[u] = mx ? fmax(a[u], p[i]) : __dadd_rn(a[u], p[i]);
+      for (int u = 0; u < U; ++u) {
+        const int i = base + u * 1024;
+        if (i < nparts) a[u] = comb(a[u], p[i]);
+      }
     }
+  } else {
+    const int u = blockIdx.x % split;
+    double s = 0.0;
+    for (int base = t + u * 1024; base < nparts; base += 8 * U * 1024) {
+      double x[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) x[k] = base + k * U * 1024 < nparts ? p[base + k * U * 1024] : 0.0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (base + k * U * 1024 < nparts) s = comb(s, x[k]);
+    }
+    scratch[(arr * U + u) * 1024 + t] = s;
+    if (!last_block(cnt + arr, split)) return;
+#pragma unroll
+    for (int k = 0; k < U; ++k) a[k] = __ldcg(scratch + (arr * U + k) * 1024 + t);
   }
-  double s;
-  if (mx) s = fmax(fmax(fmax(a[0], a[1]), fmax(a[2], a[3])), fmax(fmax(a[4], a[5]), fmax(a[6], a[7])));
-  else s = __dadd_rn(__dadd_rn(__dadd_rn(a[0], a[1]), __dadd_rn(a[2], a[3])),
-                     __dadd_rn(__dadd_rn(a[4], a[5]), __dadd_rn(a[6], a[7])));
-  sh[threadIdx.x] = s;
+  sh[t] = comb(comb(comb(a[0], a[1]), comb(a[2], a[3])), comb(comb(a[4], a[5]), comb(a[6], a[7])));
   __syncthreads();
   for (int o = 512; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o)
-      sh[threadIdx.x] = mx ? fmax(sh[threadIdx.x], sh[threadIdx.x + o]) : __dadd_rn(sh[threadIdx.x], sh[threadIdx.x + o]);
+    if (t < o) sh[t] = comb(sh[t], sh[t + o]);
     __syncthreads();
   }
-  if (threadIdx.x == 0) out[blockIdx.x] = sh[0];
+  if (t == 0) {
+    out[arr] = sh[0];
+    if (pub.word) {
+      __threadfence();
+      const bool last = narr == 1 || atomicAdd(cnt + kFinArr, 1) == narr - 1;
+      if (last) {
+        if (narr > 1) cnt[kFinArr] = 0;
+        pub();
+      }
+    }
+  }
 }
 
-// Second stage into dres[slot .. slot + narr) without waiting: results of several
-// reductions come back with one fetch_res (one host round trip).
-int finish_to(msg_ctx *c, int nparts, int narr, int slot) {
-  k_finish<<<narr, 1024, 0, c->stream>>>(c->part, nparts, c->dres + slot);
+// The reduction results come to the host with the kernel that finishes the last of them:
+// publish(c, count) in its launch, then fetch_res.
+static Publish publish(msg_ctx *c, int count) {
+  if (!count) return Publish{nullptr, nullptr, 0, nullptr, 0};
+  return Publish{c->dres, c->hpin, count, c->res_word, ++c->res_token};
+}
+
+template <int MAXB = 0>
+static int launch_finish(msg_ctx *c, int nparts, int narr, int slot, int count) {
+  const int split = nparts > kFinSplit * 1024 ? kFinSplit : 1;
+  k_finish<MAXB><<<narr * split, 1024, 0, c->stream>>>(c->part, nparts, narr, split, c->dres + slot, c->fin_scratch,
+                                                       c->fin_cnt, publish(c, count));
   MSG_CHECK_LAUNCH();
   return MSG_OK;
 }
 
+// Second stage into dres[slot .. slot + narr) without waiting: results of several reductions
+// come back with one fetch_res, of which the last finish_to names the count.
+int finish_to(msg_ctx *c, int nparts, int narr, int slot, int count) {
+  return launch_finish(c, nparts, narr, slot, count);
+}
+
 int fetch_res(msg_ctx *c, int count, double *out) {
-  MSG_CUDA(cudaMemcpyAsync(c->hpin, c->dres, (size_t)count * 8, cudaMemcpyDeviceToHost, c->stream));
-  MSG_CUDA(cudaStreamSynchronize(c->stream));
+  int rc = token_wait(c, c->res_word, c->res_token);
+  if (rc) return rc;
   for (int a = 0; a < count; ++a) out[a] = c->hpin[a];
   return wave_check(c);
 }
 
 int finish(msg_ctx *c, int nparts, int narr, double *out) {
-  int rc = finish_to(c, nparts, narr, 0);
+  int rc = finish_to(c, nparts, narr, 0, narr);
   if (rc) return rc;
   return fetch_res(c, narr, out);
 }
 
 int dot(msg_ctx *c, const double *a, const double *b, int n, double *out) {
-  k_dot2<<<nblk(n), 256, 0, c->stream>>>(n, a, b, nullptr, c->part);
+  k_dot<<<gblk(n), 256, 0, c->stream>>>(n, ngroups(n), a, b, c->part);
   MSG_CHECK_LAUNCH();
-  return finish(c, nblk(n), 1, out);
+  return finish(c, ngroups(n), 1, out);
 }
 
 int norm1(msg_ctx *c, const double *a, int n, double *out) {
-  k_norm1<<<nblk(n), 256, 0, c->stream>>>(n, a, c->part);
+  k_norm1<<<gblk(n), 256, 0, c->stream>>>(n, ngroups(n), a, c->part);
   MSG_CHECK_LAUNCH();
-  return finish(c, nblk(n), 1, out);
+  return finish(c, ngroups(n), 1, out);
 }
 
-int abserrmax(msg_ctx *c, double *xn, const double *xp, double *chmax, double *xmax, int *nun, int *nan,
-              const double *dh) {
-  k_abserrmax<<<kRedBlocks, 256, 0, c->stream>>>(c->N, xn, xp, dh, c->part);
+constexpr int kResErr = 5;   // abserrmax's seven results in dres (behind the line search's five)
+static int launch_abserrmax(msg_ctx *c, double *xn, const double *xp, const double *dh) {
+  k_abserrmax<<<kRedBlocks, 256, 0, c->stream>>>(c->N, xn, xp, dh, c->part, c->dres + kResErr, c->fin_cnt + kFinArr + 1,
+                                                 publish(c, kResErr + 7));
   MSG_CHECK_LAUNCH();
-  int rc = fetch_partials(c, kRedBlocks * 8);
-  if (rc) return rc;
-  double ca = 0.0, cv = 0.0, xa = 0.0, xv = 0.0;
-  long ci = -1, xi = -1;
-  int nn = 0;
-  for (int b = 0; b < kRedBlocks; ++b) {
-    const double *q = c->hpin + (size_t)b * 8;
-    long i1 = (long)q[2], i2 = (long)q[5];
-    if (i1 >= 0 && (q[0] > ca || (q[0] == ca && i1 > ci))) { ca = q[0]; cv = q[1]; ci = i1; }
-    if (i2 >= 0 && (q[3] > xa || (q[3] == xa && i2 > xi))) { xa = q[3]; xv = q[4]; xi = i2; }
-    nn |= (int)q[6];
-  }
-  *nan = nn;
-  if (!nn) { *chmax = cv; *xmax = xv; *nun = (int)ci + 1; }
-  else { *chmax = 0.0; *xmax = NAN; *nun = 0; }
+  return MSG_OK;
+}
+static void errmax_result(const double *q, ErrMax &e) {
+  e.nan = (int)q[6];
+  if (!e.nan) { e.change = q[1]; e.value = q[4]; e.cell = (int)q[2] + 1; }
+  else { e.change = 0.0; e.value = NAN; e.cell = 0; }
+}
+
+int abserrmax(msg_ctx *c, double *xn, const double *xp, ErrMax &e, const double *dh) {
+  int rc = launch_abserrmax(c, xn, xp, dh);
+  double got[kResErr + 7];
+  if (rc || (rc = fetch_res(c, kResErr + 7, got))) return rc;
+  errmax_result(got + kResErr, e);
   return MSG_OK;
 }
 
 // The line search's four reductions over the full step in one pass (run_backtr,
 // Nonlinear_solution.f90:441-512): ||dh||^2, ||F(h + dh)||^2, the slope (s, J dh) and
-// lam_length's largest ratio |dh| / |h|.  The sums use the grid and order of k_dot2, so each
+// lam_length's largest ratio |dh| / |h|.  The sums use the groups and order of k_dot, so each
 // has the bits of its own dot product; J dh is jv, or b - r (BiCGStab's residual from dh = 0)
-// formed with the rounding of the axpby it replaces.  The maximum is exact whatever the grid.
-__global__ void __launch_bounds__(256) k_backtr_stats(int n, const double *dh, const double *hn, const double *f,
+// formed with the rounding of the axpby it replaces.  The maximum is exact whatever the
+// grouping: one per block, in the place of its first group.
+__global__ void __launch_bounds__(256) k_backtr_stats(int n, int ng, const double *dh, const double *hn, const double *f,
                                                       const double *s, const double *jv, const double *b,
                                                       const double *r, double *part) {
-  __shared__ double sh[8];
-  __shared__ double sm[256];
-  double s0 = 0.0, s1 = 0.0, s2 = 0.0, num = 1.0, den = 1.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const double d = dh[i], fi = f[i];
-    s0 = __dadd_rn(s0, __dmul_rn(d, d));
-    s1 = __dadd_rn(s1, __dmul_rn(fi, fi));
-    const double j = jv ? jv[i] : __dadd_rn(b[i], __dmul_rn(-1.0, r[i]));
-    s2 = __dadd_rn(s2, __dmul_rn(s[i], j));
-    const double h = fabs(hn[i]), a = fabs(d);
-    if (h != 0.0 && ratio_greater(a, h, num, den)) { num = a; den = h; }
+  __shared__ double sm[8];
+  double v[3][kGr], num = 1.0, den = 1.0;
+  double di[kGr], hi[kGr], fi[kGr], si[kGr], ji[kGr], bi[kGr];
+  const int i0 = blockIdx.x * (256 * kGr) + threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < kGr; ++k) {
+    const int i = i0 + 256 * k;
+    const bool in = i < n;
+    di[k] = in ? dh[i] : 0.0; hi[k] = in ? hn[i] : 0.0; fi[k] = in ? f[i] : 0.0; si[k] = in ? s[i] : 0.0;
+    ji[k] = in ? (jv ? jv[i] : r[i]) : 0.0;
+    bi[k] = !in || jv ? 0.0 : b == s ? si[k] : b[i];
   }
-  double t = block_sum<256>(s0, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = t;
-  t = block_sum<256>(s1, sh);
-  if (threadIdx.x == 0) part[gridDim.x + blockIdx.x] = t;
-  t = block_sum<256>(s2, sh);
-  if (threadIdx.x == 0) part[2 * gridDim.x + blockIdx.x] = t;
-  sm[threadIdx.x] = __ddiv_rn(num, den);
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) sm[threadIdx.x] = fmax(sm[threadIdx.x], sm[threadIdx.x + o]);
-    __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kGr; ++k) {
+    v[0][k] = v[1][k] = v[2][k] = 0.0;
+    if (i0 + 256 * k < n) {
+      v[0][k] = __dmul_rn(di[k], di[k]);
+      v[1][k] = __dmul_rn(fi[k], fi[k]);
+      const double j = jv ? ji[k] : __dadd_rn(bi[k], __dmul_rn(-1.0, ji[k]));
+      v[2][k] = __dmul_rn(si[k], j);
+      const double h = fabs(hi[k]), a = fabs(di[k]);
+      if (h != 0.0 && ratio_greater(a, h, num, den)) { num = a; den = h; }
+    }
   }
-  if (threadIdx.x == 0) part[3 * gridDim.x + blockIdx.x] = sm[0];
+  double m = __ddiv_rn(num, den);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = m;
+  group_sums<3>(v, ng, part);   // its barrier covers sm
+  if (threadIdx.x < kGr) {
+    const int g = blockIdx.x * kGr + threadIdx.x;
+    m = 0.0;
+    if (threadIdx.x == 0)
+      for (int w = 0; w < 8; ++w) m = fmax(m, sm[w]);
+    if (g < ng) part[(size_t)3 * ng + g] = m;
+  }
 }
 
 int backtr_stats(msg_ctx *c, const double *dh, const double *hn, const double *f, const double *s, const double *jv,
                  const double *b, const double *r, double out[5], bool slot4) {
-  const int nb = nblk(c->N);
-  if ((size_t)4 * nb > c->npart) { set_error("backtr_stats: partials buffer too small"); return MSG_ERR_STATE; }
-  k_backtr_stats<<<nb, 256, 0, c->stream>>>(c->N, dh, hn, f, s, jv, b, r, c->part);
+  const int ng = ngroups(c->N);
+  if ((size_t)4 * ng > c->npart) { set_error("backtr_stats: partials buffer too small"); return MSG_ERR_STATE; }
+  k_backtr_stats<<<gblk(c->N), 256, 0, c->stream>>>(c->N, ng, dh, hn, f, s, jv, b, r, c->part);
   MSG_CHECK_LAUNCH();
-  k_finish<8><<<4, 1024, 0, c->stream>>>(c->part, nb, c->dres);
-  MSG_CHECK_LAUNCH();
-  int rc = fetch_res(c, slot4 ? 5 : 4, out);
-  if (rc) return rc;
+  int rc = launch_finish<8>(c, ng, 4, 0, slot4 ? 5 : 4);
+  if (rc || (rc = fetch_res(c, slot4 ? 5 : 4, out))) return rc;
   out[3] = std::fmax(1.0, out[3]);
   return MSG_OK;
 }
@@ -842,25 +1016,33 @@ int apply_prec(msg_ctx *c, const double *r, double *z) {
 
 // ---------------------------------------------------------------------------------
 // solve_bicgs (Linear_solution.f90:234-493): right-preconditioned BiCGStab, x0 = x.
+//
+// The step lengths are formed on the device by the kernels that use them, so the host waits
+// only for the residual norms it decides on.  With `ahead`, the Newton update's change
+// (abserrmax over ahead->xn = ahead->xp + x) is taken together with the first residual norm
+// when the last solve ended there, which a solve with one AMG V-cycle usually does: one wait
+// fewer; a wrong guess costs the pass.
 // ---------------------------------------------------------------------------------
-int solve_bicgs(msg_ctx *c, double *x, bool x_zero) {
+int solve_bicgs(msg_ctx *c, double *x, bool x_zero, ErrAhead *ahead) {
   const int n = c->N;
   const Geo3 g = geo3(c);
   int rc;
-  const int nb = nblk(n);
-  double red[2];
-  double sk = 0.0, sk0 = 1.0e20, sk2, alpha = 0.0, beta, omega = 1.0, ts, tt;
+  const int nb = nblk(n), ng = ngroups(n), gb = gblk(n);
+  double sk = 0.0, sk0 = 1.0e20, alpha = 0.0, beta, omega = 1.0;
   bool need_dilu = (c->prm.precon_type == 0) || c->prm.ref_quirks;
   // r* (fixed during the solve), the first search direction and the residual before the
   // first update.  From x = 0 all three are b itself: nothing is copied, and x is first
   // written (not read) by the first update.
   const double *rs, *p1, *r1;
+  // reduction results: (v, r*), ||r||^2 after the first update, <b, b>; behind abserrmax's
+  // those of the second half
+  enum { kSk2 = 0, kR1 = 1, kBB = 2, kTs = kResErr + 7, kR2 = kTs + 2 };
   if (x_zero) {
     if (need_dilu && (rc = launch_precon_dilu(c))) return rc;
-    // sk = <b, b>, collected with the first (v, r*) in one host round trip
-    k_dot2<<<nb, 256, 0, c->stream>>>(n, c->rhs, c->rhs, nullptr, c->part);
+    // sk = <b, b>, collected with the first residual norm
+    k_dot<<<gb, 256, 0, c->stream>>>(n, ng, c->rhs, c->rhs, c->part);
     MSG_CHECK_LAUNCH();
-    if ((rc = finish_to(c, nb, 1, 2))) return rc;
+    if ((rc = finish_to(c, ng, 1, kBB, 0))) return rc;
     rs = p1 = r1 = c->rhs;
   } else {
     // r = b - A x
@@ -873,9 +1055,11 @@ int solve_bicgs(msg_ctx *c, double *x, bool x_zero) {
     r1 = c->r;
   }
   c->conv_flag = 0;
+  double got[kR2 + 2];
   for (c->in_iter = 1; c->in_iter <= c->prm.maxinn_iter; ++c->in_iter) {
+    const bool first = (c->in_iter == 1);
     const double *p = c->p;
-    if (c->in_iter == 1) {
+    if (first) {
       p = p1;
     } else {
       beta = (sk / sk0) * (alpha / omega);
@@ -885,40 +1069,39 @@ int solve_bicgs(msg_ctx *c, double *x, bool x_zero) {
     if ((rc = apply_prec(c, p, c->z))) return rc;
     k_spmv<1, false><<<nb, 256, 0, c->stream>>>(g, c->dmat, c->lu, c->z, nullptr, c->v, rs, c->part);
     MSG_CHECK_LAUNCH();
-    if (x_zero && c->in_iter == 1) {
-      double got[3];
-      if ((rc = finish_to(c, nb, 1, 0)) || (rc = fetch_res(c, 3, got))) return rc;
-      red[0] = got[0];
-      sk = got[2];
-    } else if ((rc = finish(c, nb, 1, red))) {
-      return rc;
-    }
-    sk2 = red[0];
-    alpha = sk / sk2;
-    const bool first = (c->in_iter == 1);
-    k_bicg_xr<<<nb, 256, 0, c->stream>>>(n, first && x_zero ? nullptr : x, x, first ? r1 : c->r, c->r, c->z, c->v,
-                                        rs, alpha, c->part);
+    if ((rc = finish_to(c, nb, 1, kSk2, 0))) return rc;
+    const bool from_bb = x_zero && first;   // sk = <b, b> is still on the device
+    k_bicg_xr<<<gb, 256, 0, c->stream>>>(n, ng, first && x_zero ? nullptr : x, x, first ? r1 : c->r, c->r, c->z, c->v, rs,
+                                        Quot{from_bb ? c->dres + kBB : nullptr, c->dres + kSk2, sk}, c->part);
     MSG_CHECK_LAUNCH();
-    if ((rc = finish(c, nb, 1, red))) return rc;
-    c->rnorm = red[0];
+    const bool spec = ahead && from_bb && c->one_half;
+    if ((rc = finish_to(c, ng, 1, kR1, spec ? 0 : 3))) return rc;
+    if (spec && (rc = launch_abserrmax(c, ahead->xn, ahead->xp, x))) return rc;
+    if ((rc = fetch_res(c, spec ? kResErr + 7 : 3, got))) return rc;
+    if (from_bb) sk = got[kBB];
+    alpha = sk / got[kSk2];
+    c->rnorm = got[kR1];
     c->conv_flag = (std::sqrt(c->rnorm / c->bnorm) <= c->errtol) ? 1 : 0;
+    if (first) c->one_half = c->conv_flag;
+    if (spec && c->conv_flag == 1) {
+      ahead->done = true;
+      errmax_result(got + kResErr, ahead->e);
+    }
     if (c->conv_flag == 1) break;
     if ((rc = apply_prec(c, c->r, c->z))) return rc;
     k_spmv<2, false><<<nb, 256, 0, c->stream>>>(g, c->dmat, c->lu, c->z, nullptr, c->t, c->r, c->part);
     MSG_CHECK_LAUNCH();
-    if ((rc = finish(c, nb, 2, red))) return rc;
-    ts = red[0];
-    tt = red[1];
-    omega = ts / tt;
-    k_bicg_xr<<<nb, 256, 0, c->stream>>>(n, x, x, c->r, c->r, c->z, c->t, rs, omega, c->part);
+    if ((rc = finish_to(c, nb, 2, kTs, 0))) return rc;
+    k_bicg_xr<<<gb, 256, 0, c->stream>>>(n, ng, x, x, c->r, c->r, c->z, c->t, rs, Quot{c->dres + kTs, c->dres + kTs + 1, 0.0},
+                                        c->part);
     MSG_CHECK_LAUNCH();
-    if ((rc = finish(c, nb, 2, red))) return rc;
-    c->rnorm = red[0];
-    double sk_next = red[1];
+    if ((rc = finish_to(c, ng, 2, kR2, kR2 + 2)) || (rc = fetch_res(c, kR2 + 2, got))) return rc;
+    omega = got[kTs] / got[kTs + 1];
+    c->rnorm = got[kR2];
     c->conv_flag = (std::sqrt(c->rnorm / c->bnorm) <= c->errtol) ? 1 : 0;
     if (c->conv_flag == 1 || c->in_iter == c->prm.maxinn_iter) break;
     sk0 = sk;
-    sk = sk_next;
+    sk = got[kR2 + 1];
   }
   if (c->in_iter > c->prm.maxinn_iter) c->in_iter = c->prm.maxinn_iter;
   return MSG_OK;
