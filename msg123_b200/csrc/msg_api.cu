@@ -596,6 +596,11 @@ extern "C" {
 const char *msg_gpu_last_error(void) { return get_error(); }
 
 #define ALLOC(ptr, bytes) MSG_CUDA(cudaMalloc((void **)&(ptr), (bytes)))
+#define COPY_OUT(dst, src, bytes)                          \
+  do {                                                     \
+    int rc_ = copy_out((dst), (src), (bytes));             \
+    if (rc_) return rc_;                                   \
+  } while (0)
 #define UPLOAD(dst, src, bytes) MSG_CUDA(cudaMemcpyAsync((dst), (src), (bytes), cudaMemcpyHostToDevice, c->stream))
 
 static int create_impl(msg_ctx *c, const msg_grid_t *g, const msg_params_t *p) {
@@ -665,8 +670,8 @@ static int create_impl(msg_ctx *c, const msg_grid_t *g, const msg_params_t *p) {
     ALLOC(c->dmat_f, N * 4);
     ALLOC(c->lu_f, 6 * N * 4);
   }
-  // up to four arrays of one partial per block of 256 cells (the line search's k_backtr_stats)
-  size_t npart = std::max((size_t)kRedBlocks * 8, 4 * (size_t)nblk((int)N) + 64);
+  // up to nine arrays of one partial per block of 256 cells (the mass volumes)
+  size_t npart = std::max((size_t)kRedBlocks * 8, 9 * (size_t)nblk((int)N) + 64);
   // the flux passes' 3D grid can have more blocks than nblk(N) when nx or ny is not a
   // multiple of the tile (32 x 8)
   npart = std::max(npart, (size_t)((g->nx + 31) / 32) * ((g->ny + 7) / 8) * g->nz + 64);
@@ -703,6 +708,7 @@ int msg_gpu_create(const msg_grid_t *grid, const msg_params_t *params, msg_ctx_t
   msg_ctx *c = new (std::nothrow) msg_ctx();
   if (!c) { set_error("out of host memory"); return MSG_ERR_ARG; }
   memset(c, 0, sizeof(*c));
+  stage_ref();
   int rc = create_impl(c, grid, params);
   if (rc) { free_ctx(c); return rc; }
   *out = c;
@@ -717,13 +723,13 @@ int msg_gpu_get_connect(msg_ctx_t *c, int32_t *offind, int32_t *offrow, int32_t 
                         int32_t *right_off, double *hydf_conn, double *abyd_conn, int32_t *nnz) {
   if (!c) return MSG_ERR_ARG;
   size_t M = c->nnz;
-  if (offind) MSG_CUDA(cudaMemcpy(offind, c->offind, (c->N + 1) * 4, cudaMemcpyDeviceToHost));
-  if (offrow) MSG_CUDA(cudaMemcpy(offrow, c->offrow, M * 4, cudaMemcpyDeviceToHost));
-  if (conn_dir) MSG_CUDA(cudaMemcpy(conn_dir, c->conn_dir, M * 4, cudaMemcpyDeviceToHost));
-  if (left_off) MSG_CUDA(cudaMemcpy(left_off, c->left_off, M * 4, cudaMemcpyDeviceToHost));
-  if (right_off) MSG_CUDA(cudaMemcpy(right_off, c->right_off, M * 4, cudaMemcpyDeviceToHost));
-  if (hydf_conn) MSG_CUDA(cudaMemcpy(hydf_conn, c->hydf_conn, M * 8, cudaMemcpyDeviceToHost));
-  if (abyd_conn) MSG_CUDA(cudaMemcpy(abyd_conn, c->abyd_conn, M * 8, cudaMemcpyDeviceToHost));
+  if (offind) COPY_OUT(offind, c->offind, (c->N + 1) * 4);
+  if (offrow) COPY_OUT(offrow, c->offrow, M * 4);
+  if (conn_dir) COPY_OUT(conn_dir, c->conn_dir, M * 4);
+  if (left_off) COPY_OUT(left_off, c->left_off, M * 4);
+  if (right_off) COPY_OUT(right_off, c->right_off, M * 4);
+  if (hydf_conn) COPY_OUT(hydf_conn, c->hydf_conn, M * 8);
+  if (abyd_conn) COPY_OUT(abyd_conn, c->abyd_conn, M * 8);
   if (nnz) *nnz = c->nnz;
   return MSG_OK;
 }
@@ -791,12 +797,9 @@ int msg_gpu_get_state(msg_ctx_t *c, double *head_new, double *head_old, double *
   if (!c) return MSG_ERR_ARG;
   size_t N = c->N, S = c->S;
   MSG_CUDA(cudaStreamSynchronize(c->stream));
-  if (head_new) MSG_CUDA(cudaMemcpy(head_new, c->head_new, N * 8, cudaMemcpyDeviceToHost));
-  if (head_old) MSG_CUDA(cudaMemcpy(head_old, c->head_old, N * 8, cudaMemcpyDeviceToHost));
-  if (srat_new) MSG_CUDA(cudaMemcpy(srat_new, c->srat_new, N * 8, cudaMemcpyDeviceToHost));
-  if (srat_old) MSG_CUDA(cudaMemcpy(srat_old, c->srat_old, N * 8, cudaMemcpyDeviceToHost));
-  if (surf_head) MSG_CUDA(cudaMemcpy(surf_head, c->surf_head, S * 8, cudaMemcpyDeviceToHost));
-  return MSG_OK;
+  const CopyOut jobs[5] = {{head_new, c->head_new, N * 8}, {head_old, c->head_old, N * 8}, {srat_new, c->srat_new, N * 8},
+                           {srat_old, c->srat_old, N * 8}, {surf_head, c->surf_head, S * 8}};
+  return copy_out(jobs, 5);
 }
 
 int msg_gpu_set_recharge(msg_ctx_t *c, const double *calc_rech) {
@@ -814,9 +817,9 @@ int msg_gpu_srat_rperm(msg_ctx_t *c, const double *pres, double pertur, double *
   int rc = launch_srat_rperm(c, c->tmpv, pertur, c->v, c->t, c->z);
   if (rc) return rc;
   MSG_CUDA(cudaStreamSynchronize(c->stream));
-  if (srat) MSG_CUDA(cudaMemcpy(srat, c->v, N * 8, cudaMemcpyDeviceToHost));
-  if (rperm) MSG_CUDA(cudaMemcpy(rperm, c->t, N * 8, cudaMemcpyDeviceToHost));
-  if (sstor) MSG_CUDA(cudaMemcpy(sstor, c->z, N * 8, cudaMemcpyDeviceToHost));
+  if (srat) COPY_OUT(srat, c->v, N * 8);
+  if (rperm) COPY_OUT(rperm, c->t, N * 8);
+  if (sstor) COPY_OUT(sstor, c->z, N * 8);
   return MSG_OK;
 }
 
@@ -827,7 +830,7 @@ int msg_gpu_calc_func(msg_ctx_t *c, const double *infx, double *funcv) {
   int rc = launch_calc_func(c, c->tmpv, c->new_f, false);
   if (rc) return rc;
   MSG_CUDA(cudaStreamSynchronize(c->stream));
-  MSG_CUDA(cudaMemcpy(funcv, c->new_f, N * 8, cudaMemcpyDeviceToHost));
+  COPY_OUT(funcv, c->new_f, N * 8);
   return MSG_OK;
 }
 
@@ -841,14 +844,14 @@ int msg_gpu_make_matvec(msg_ctx_t *c, double *dmat, double *lumat, double *rhs) 
   if (lumat) {
     double *tmp = nullptr;
     ALLOC(tmp, (size_t)c->nnz * 8);
-    if ((rc = launch_dia_to_csr(c, tmp))) return rc;
-    MSG_CUDA(cudaStreamSynchronize(c->stream));
-    MSG_CUDA(cudaMemcpy(lumat, tmp, (size_t)c->nnz * 8, cudaMemcpyDeviceToHost));
+    rc = launch_dia_to_csr(c, tmp);
+    if (!rc && cudaStreamSynchronize(c->stream) == cudaSuccess) rc = copy_out(lumat, tmp, (size_t)c->nnz * 8);
     cudaFree(tmp);
+    if (rc) return rc;
   }
   MSG_CUDA(cudaStreamSynchronize(c->stream));
-  if (dmat) MSG_CUDA(cudaMemcpy(dmat, c->dmat, N * 8, cudaMemcpyDeviceToHost));
-  if (rhs) MSG_CUDA(cudaMemcpy(rhs, c->rhs, N * 8, cudaMemcpyDeviceToHost));
+  if (dmat) COPY_OUT(dmat, c->dmat, N * 8);
+  if (rhs) COPY_OUT(rhs, c->rhs, N * 8);
   return MSG_OK;
 }
 
@@ -890,7 +893,7 @@ int msg_gpu_precond(msg_ctx_t *c, const double *r, double *z) {
   if ((rc = apply_prec(c, c->tmpv, c->z))) return rc;
   MSG_CUDA(cudaStreamSynchronize(c->stream));
   if ((rc = wave_check(c))) return rc;
-  MSG_CUDA(cudaMemcpy(z, c->z, N * 8, cudaMemcpyDeviceToHost));
+  COPY_OUT(z, c->z, N * 8);
   return MSG_OK;
 }
 
@@ -904,7 +907,7 @@ int msg_gpu_solve_linalg(msg_ctx_t *c, double init_norm, double errtol, double *
   int rc = solve_linalg(c, init_norm, c->head_change, &ln);
   if (rc) return rc;
   MSG_CUDA(cudaStreamSynchronize(c->stream));
-  MSG_CUDA(cudaMemcpy(inx, c->head_change, N * 8, cudaMemcpyDeviceToHost));
+  COPY_OUT(inx, c->head_change, N * 8);
   if (last_norm) *last_norm = ln;
   if (in_iter) *in_iter = c->in_iter;
   if (conv_flag) *conv_flag = c->conv_flag;
@@ -919,7 +922,7 @@ int msg_gpu_vecjacf(msg_ctx_t *c, const double *x, const double *v, double *out)
   int rc = vecjacf(c, c->head_pre, c->head_change, c->tmpv);
   if (rc) return rc;
   MSG_CUDA(cudaStreamSynchronize(c->stream));
-  MSG_CUDA(cudaMemcpy(out, c->tmpv, N * 8, cudaMemcpyDeviceToHost));
+  COPY_OUT(out, c->tmpv, N * 8);
   return MSG_OK;
 }
 
@@ -996,13 +999,7 @@ int msg_gpu_read_restart(const char *path, int32_t ncalc, double len_scal, doubl
 
 int msg_gpu_calc_mass(msg_ctx_t *c, double *out9) {
   if (!c || !out9) return MSG_ERR_ARG;
-  double *d = nullptr;
-  ALLOC(d, 9 * 8);
-  int rc = launch_mass(c, d);
-  if (rc) return rc;
-  MSG_CUDA(cudaMemcpy(out9, d, 9 * 8, cudaMemcpyDeviceToHost));
-  cudaFree(d);
-  return MSG_OK;
+  return launch_mass(c, out9);
 }
 
 int msg_gpu_cell_mass(msg_ctx_t *c, double *sto, double *con, double *sea, double *wel, double *rec, double *sur,
@@ -1017,29 +1014,25 @@ int msg_gpu_cell_mass(msg_ctx_t *c, double *sto, double *con, double *sea, doubl
   int rc = launch_cell_mass(c, c->r, c->rs, c->v, c->p, ts, ts + S, ts + 2 * S, ts + 3 * S, ts + 4 * S);
   if (rc) { if (ts != c->t) cudaFree(ts); return rc; }
   MSG_CUDA(cudaStreamSynchronize(c->stream));
-  if (sto) MSG_CUDA(cudaMemcpy(sto, c->r, N * 8, cudaMemcpyDeviceToHost));
-  if (con) MSG_CUDA(cudaMemcpy(con, c->rs, N * 8, cudaMemcpyDeviceToHost));
-  if (sea) MSG_CUDA(cudaMemcpy(sea, c->v, N * 8, cudaMemcpyDeviceToHost));
-  if (wel) MSG_CUDA(cudaMemcpy(wel, c->p, N * 8, cudaMemcpyDeviceToHost));
-  double *hs[5] = {rec, sur, riv, lak, drn};
-  for (int q = 0; q < 5; ++q)
-    if (hs[q]) MSG_CUDA(cudaMemcpy(hs[q], ts + q * S, S * 8, cudaMemcpyDeviceToHost));
+  const CopyOut jobs[9] = {{sto, c->r, N * 8}, {con, c->rs, N * 8}, {sea, c->v, N * 8}, {wel, c->p, N * 8}, {rec, ts, S * 8},
+                           {sur, ts + S, S * 8}, {riv, ts + 2 * S, S * 8}, {lak, ts + 3 * S, S * 8}, {drn, ts + 4 * S, S * 8}};
+  rc = copy_out(jobs, 9);
   if (ts != c->t) cudaFree(ts);
-  return MSG_OK;
+  return rc;
 }
 
 int msg_gpu_velocity(msg_ctx_t *c, double *facev, double *pointv) {
   if (!c) return MSG_ERR_ARG;
   const size_t N = c->N;
-  double *dv = nullptr;
-  ALLOC(dv, 9 * N * 8);
-  int rc = launch_velocity(c, dv, dv + 6 * N);
-  if (rc) { cudaFree(dv); return rc; }
+  // Krylov and line-search vectors, free between solves, hold the device copies
+  double *const dv[9] = {c->r, c->rs, c->p, c->v, c->t, c->z, c->tmpv, c->new_f, c->rhs_alt};
+  int rc = launch_velocity(c, dv);
+  if (rc) return rc;
   MSG_CUDA(cudaStreamSynchronize(c->stream));
-  if (facev) MSG_CUDA(cudaMemcpy(facev, dv, 6 * N * 8, cudaMemcpyDeviceToHost));
-  if (pointv) MSG_CUDA(cudaMemcpy(pointv, dv + 6 * N, 3 * N * 8, cudaMemcpyDeviceToHost));
-  cudaFree(dv);
-  return MSG_OK;
+  CopyOut jobs[9];
+  for (int k = 0; k < 9; ++k)
+    jobs[k] = CopyOut{k < 6 ? (facev ? facev + k * N : nullptr) : (pointv ? pointv + (k - 6) * N : nullptr), dv[k], N * 8};
+  return copy_out(jobs, 9);
 }
 
 int msg_gpu_set_wells(msg_ctx_t *c, int32_t nwell, const int32_t *well_index, const int32_t *well_conn,
@@ -1275,6 +1268,7 @@ static void free_ctx(msg_ctx *c) {
   if (c->hpin) cudaFreeHost(c->hpin);
   for (int k = 0; k < 8; ++k) if (c->ev[k]) cudaEventDestroy(c->ev[k]);
   if (c->stream) cudaStreamDestroy(c->stream);
+  stage_unref();
   delete c;
 }
 }  // namespace msg

@@ -127,8 +127,8 @@ int launch_calc_func(msg_ctx *c, const double *h, double *F, bool norm);
 int launch_make_matvec(msg_ctx *c, bool reuse = false, double *rhs_out = nullptr);   // rhs_out null: c->rhs
 // Export the DIA Jacobian into the reference CSR order.
 int launch_dia_to_csr(msg_ctx *c, double *lumat_dev);
-int launch_mass(msg_ctx *c, double *out9_dev);
-int launch_velocity(msg_ctx *c, double *facev, double *pointv);
+int launch_mass(msg_ctx *c, double out9[9]);
+int launch_velocity(msg_ctx *c, double *const out[9]);   // six faces, then x, y, z
 int launch_cell_mass(msg_ctx *c, double *sto, double *con, double *sea, double *wel, double *rec, double *sur,
                      double *riv, double *lak, double *drn);
 int launch_wells(msg_ctx *c);
@@ -160,6 +160,7 @@ int finish(msg_ctx *c, int nparts, int narr, double *out);
 int finish_to(msg_ctx *c, int nparts, int narr, int slot, int count = 0);   // into dres[slot..]; count > 0:
                                                                              // dres[0..count) to the host
 int fetch_res(msg_ctx *c, int count, double *out);                          // waits for them
+int finish9(msg_ctx *c, int nparts, double out[9]);   // nine arrays, nparts each
 int norm1(msg_ctx *c, const double *a, int n, double *out);
 int abserrmax(msg_ctx *c, double *xn, const double *xp, ErrMax &e, const double *dh = nullptr);   // dh: form xn = xp + dh first
 int lam_length(msg_ctx *c, const double *dh, const double *hn, double *out);
@@ -168,6 +169,17 @@ int backtr_stats(msg_ctx *c, const double *dh, const double *hn, const double *f
                  const double *b, const double *r, double out[5], bool slot4);   // slot4: also dres[4] (pending)
 int axpby(msg_ctx *c, double *y, const double *x, double a, const double *w, int n);   // y = x + a*w
 int scale(msg_ctx *c, double *y, double a, int n);
+
+// ---- msg_copy.cu ------------------------------------------------------------------------------
+struct CopyOut {
+  void *dst;
+  const void *src;
+  size_t bytes;
+};
+int copy_out(const CopyOut *jobs, int n);                  // device -> host, src complete; null dst: none
+int copy_out(void *dst, const void *src, size_t bytes);
+void stage_ref();      // one per context or network that may call it
+void stage_unref();
 
 // ---- msg_amg.cu ---------------------------------------------------------------------------------
 int amg_setup(msg_ctx *c);

@@ -619,6 +619,7 @@ MSG_API int msg_gpu_cnn_create(int32_t seed, msg_cnn_t **out) {
   if (!out) return MSG_ERR_ARG;
   msg_cnn *h = new msg_cnn();
   Net &n = h->net;
+  stage_ref();
   MSG_CUDA(cudaStreamCreateWithFlags(&n.stream, cudaStreamNonBlocking));
   MSG_CUDA(cudaMalloc(&n.w32, kNParam * 4));
   MSG_CUDA(cudaMalloc(&n.m, kNParam * 4));
@@ -667,6 +668,7 @@ MSG_API void msg_gpu_cnn_destroy(msg_cnn_t *h) {
   for (int l = 0; l < kLayers; ++l) { if (n.a[l]) cudaFree(n.a[l]); if (n.z[l]) cudaFree(n.z[l]); }
   for (auto &smp : n.data) { cudaFree(smp.x); cudaFree(smp.y); }
   cudaStreamDestroy(n.stream);
+  stage_unref();
   delete h;
 }
 
@@ -789,7 +791,7 @@ MSG_API int msg_gpu_cnn_loss_grad(msg_cnn_t *h, int32_t sample, double *loss, fl
   }
   if (out) {
     MSG_CUDA(cudaStreamSynchronize(n.stream));
-    MSG_CUDA(cudaMemcpy(out, n.z[3], (size_t)smp.g.N * 4, cudaMemcpyDeviceToHost));
+    if ((rc = copy_out(out, n.z[3], (size_t)smp.g.N * 4))) return rc;
   }
   return MSG_OK;
 }
@@ -806,8 +808,7 @@ static int cnn_infer(msg_cnn_t *h, int32_t sample, float *out, int withhold) {
   const float *o = nullptr;
   if ((rc = cnn_forward_tc(n, n.stream, &o, withhold))) return rc;
   if ((rc = conv_check(n.plan, n.stream))) return rc;
-  MSG_CUDA(cudaMemcpy(out, o, (size_t)smp.g.N * 4, cudaMemcpyDeviceToHost));
-  return MSG_OK;
+  return copy_out(out, o, (size_t)smp.g.N * 4);
 }
 
 MSG_API int msg_gpu_cnn_infer(msg_cnn_t *h, int32_t sample, float *out) { return cnn_infer(h, sample, out, -1); }

@@ -544,15 +544,18 @@ __global__ void __launch_bounds__(256) k_cell_mass(FluxArgs a, const double *h_o
 }
 
 // calc_outvelc (Calc_output.f90:168-241) for cell i: the Darcy velocity through each face
-// (face-major facev[d*N + i], d = up, north, west, east, south, down): regular faces
+// (one array per face: up, north, west, east, south, down): regular faces
 // hydf * relat * delhead * (1/dis12) in the reference's product order; the top face the
 // sea term (sea layer above) or else the surface term, both with 1/dis2face(up); the bottom
 // face of the lowest layer the unit-gradient velocity -Ksz kr under free drainage (an
-// extension); faces with no connection 0.  Then the cell-centred components pointv[c*N + i]
-// (c = x, y, z) from the opposite face pairs: half the difference where the two velocities
+// extension); faces with no connection 0.  Then the cell-centred components
+// (arrays 6, 7, 8: x, y, z) from the opposite face pairs: half the difference where the two velocities
 // have opposite signs, the whole difference otherwise, z negated (upward positive).
+struct Out9 {
+  double *v[9];
+};
 __global__ void __launch_bounds__(256) k_velocity(FluxArgs a, const double *invd, const double *top_invd,
-                                                  const float *ksz, double *facev, double *pointv) {
+                                                  const float *ksz, Out9 out) {
   const Geo g = a.g;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= g.N) return;
@@ -585,14 +588,14 @@ __global__ void __launch_bounds__(256) k_velocity(FluxArgs a, const double *invd
   }
   if (a.free_drainage && iz == g.nz - 1) fv[5] = -__dmul_rn((double)ksz[i], kri);
 #pragma unroll
-  for (int d = 0; d < 6; ++d) facev[(size_t)d * N + i] = fv[d];
+  for (int d = 0; d < 6; ++d) out.v[d][i] = fv[d];
 #pragma unroll
   for (int d = 1; d <= 3; ++d) {
     double x = fv[d - 1], y = fv[6 - d], v;
     if ((x > 0.0 && y < 0.0) || (x < 0.0 && y > 0.0)) v = __dmul_rn(__dsub_rn(x, y), 0.5);
     else v = __dsub_rn(x, y);
     if (d == 1) v = -v;
-    pointv[(size_t)(3 - d) * N + i] = v;
+    out.v[6 + 3 - d][i] = v;
   }
 }
 
@@ -779,7 +782,7 @@ int launch_dia_to_csr(msg_ctx *c, double *lumat_dev) {
   return MSG_OK;
 }
 
-int launch_mass(msg_ctx *c, double *out9_dev) {
+int launch_mass(msg_ctx *c, double out9[9]) {
   // old-level vG (alp_old) into tmpv / kr_per scratch, then new-level into srat_new / kr / alp
   double *alp_old = c->tmpv, *s_tmp = c->sto, *kr_tmp = c->kr_per;
   int rc;
@@ -788,24 +791,13 @@ int launch_mass(msg_ctx *c, double *out9_dev) {
   FluxArgs a = flux_args(c, c->head_new);
   a.surf_head = c->surf_old;
   int nb = nblk(c->N);
-  double *part9 = nullptr;
-  MSG_CUDA(cudaMalloc(&part9, (size_t)9 * nb * 8));
   k_mass<<<nb, 256, 0, c->stream>>>(a, c->head_old, c->srat_old, c->srat_new, c->alp, alp_old, c->poro, c->cell_vol,
-                                     c->delt_inv, c->delt, part9);
+                                     c->delt_inv, c->delt, c->part);
   MSG_CHECK_LAUNCH();
-  std::vector<double> hp((size_t)9 * nb);
-  MSG_CUDA(cudaMemcpyAsync(hp.data(), part9, hp.size() * 8, cudaMemcpyDeviceToHost, c->stream));
-  MSG_CUDA(cudaStreamSynchronize(c->stream));
-  cudaFree(part9);
-  double out[9] = {0};
+  double got[9];
+  if ((rc = finish9(c, nb, got))) return rc;
   const int map[9] = {0, 1, 2, 4, 7, 8, 3, 5, 6};
-  for (int q = 0; q < 9; ++q) {
-    double s = 0.0;
-    for (int b = 0; b < nb; ++b) s += hp[(size_t)q * nb + b];
-    out[map[q]] = s;
-  }
-  MSG_CUDA(cudaMemcpyAsync(out9_dev, out, sizeof(out), cudaMemcpyHostToDevice, c->stream));
-  MSG_CUDA(cudaStreamSynchronize(c->stream));
+  for (int q = 0; q < 9; ++q) out9[map[q]] = got[q];
   return MSG_OK;
 }
 
@@ -826,12 +818,14 @@ int launch_cell_mass(msg_ctx *c, double *sto, double *con, double *sea, double *
   return MSG_OK;
 }
 
-int launch_velocity(msg_ctx *c, double *facev, double *pointv) {
+int launch_velocity(msg_ctx *c, double *const out[9]) {
   // rel_perm at head_new, as calc_outvelc reads it after the step
   int rc;
   if ((rc = launch_srat_rperm(c, c->head_new, 0.0, c->srat_new, c->kr, c->alp))) return rc;
   FluxArgs a = flux_args(c, c->head_new);
-  k_velocity<<<nblk(c->N), 256, 0, c->stream>>>(a, c->invd, c->top_invd, c->ksz, facev, pointv);
+  Out9 o;
+  for (int k = 0; k < 9; ++k) o.v[k] = out[k];
+  k_velocity<<<nblk(c->N), 256, 0, c->stream>>>(a, c->invd, c->top_invd, c->ksz, o);
   MSG_CHECK_LAUNCH();
   return MSG_OK;
 }

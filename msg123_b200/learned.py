@@ -101,14 +101,14 @@ class Cnn:
     def loss_grad(self, sample=0, want_grad=True, want_out=False, n=None):
         loss = C.c_double()
         g = np.zeros(self.nparam, np.float32) if want_grad else None
-        o = np.zeros(n, np.float32) if want_out else None
+        o = np.empty(n, np.float32) if want_out else None
         _check(_lib().msg_gpu_cnn_loss_grad(self.h, int(sample), C.byref(loss), abi.fptr(g), abi.fptr(o)),
                "cnn_loss_grad")
         return loss.value, g, o
 
     def infer(self, sample, n):
         """Output of the tensor-core (tcgen05) inference path on stored sample `sample`."""
-        o = np.zeros(n, np.float32)
+        o = np.empty(n, np.float32)
         _check(_lib().msg_gpu_cnn_infer(self.h, int(sample), abi.fptr(o)), "cnn_infer")
         return o
 

@@ -149,9 +149,9 @@ class GpuSolver:
     # -- topology ---------------------------------------------------------------------
     def connect(self):
         N, M = self.n, self.nnz
-        out = dict(offind=np.zeros(N + 1, np.int32), offrow=np.zeros(M, np.int32), conn_dir=np.zeros(M, np.int32),
-                   left_off=np.zeros(M, np.int32), right_off=np.zeros(M, np.int32),
-                   hydf=np.zeros(M), abyd=np.zeros(M))
+        out = dict(offind=np.empty(N + 1, np.int32), offrow=np.empty(M, np.int32), conn_dir=np.empty(M, np.int32),
+                   left_off=np.empty(M, np.int32), right_off=np.empty(M, np.int32),
+                   hydf=np.empty(M), abyd=np.empty(M))
         _check(load_library().msg_gpu_get_connect(self.h, iptr(out["offind"]), iptr(out["offrow"]),
                                                   iptr(out["conn_dir"]), iptr(out["left_off"]),
                                                   iptr(out["right_off"]), dptr(out["hydf"]), dptr(out["abyd"]),
@@ -175,7 +175,7 @@ class GpuSolver:
         N, S = self.n, self.ncals
         sizes = (("head_new", N), ("head_old", N), ("srat_new", N), ("srat_old", N), ("surf_head", S))
         if out is None:
-            out = {k: np.zeros(n) for k, n in sizes}
+            out = {k: np.empty(n) for k, n in sizes}
         for k, n in sizes:
             a = out.get(k)
             if a is not None and (a.dtype != np.float64 or not a.flags.c_contiguous or a.size != n):
@@ -194,7 +194,7 @@ class GpuSolver:
         nondimensional like head_new."""
         L = load_library()
         L.msg_gpu_water_table.argtypes = [C.c_void_p, abi.PD]
-        out = np.zeros(self.ncals)
+        out = np.empty(self.ncals)
         _check(L.msg_gpu_water_table(self.h, dptr(out)), "water_table")
         return out
 
@@ -265,18 +265,18 @@ class GpuSolver:
     # -- reference routines -----------------------------------------------------------------
     def srat_rperm(self, pres, pertur=0.0):
         N = self.n
-        s, k, ss = np.zeros(N), np.zeros(N), np.zeros(N)
+        s, k, ss = np.empty(N), np.empty(N), np.empty(N)
         _check(load_library().msg_gpu_srat_rperm(self.h, dptr(_f64(pres)), C.c_double(pertur), dptr(s), dptr(k),
                                                  dptr(ss)), "srat_rperm")
         return s, k, ss
 
     def calc_func(self, x):
-        f = np.zeros(self.n)
+        f = np.empty(self.n)
         _check(load_library().msg_gpu_calc_func(self.h, dptr(_f64(x)), dptr(f)), "calc_func")
         return f
 
     def make_matvec(self):
-        d, lu, r = np.zeros(self.n), np.zeros(self.nnz), np.zeros(self.n)
+        d, lu, r = np.empty(self.n), np.empty(self.nnz), np.empty(self.n)
         _check(load_library().msg_gpu_make_matvec(self.h, dptr(d), dptr(lu), dptr(r)), "make_matvec")
         return d, lu, r
 
@@ -285,12 +285,12 @@ class GpuSolver:
                "set_system")
 
     def precond(self, r):
-        z = np.zeros(self.n)
+        z = np.empty(self.n)
         _check(load_library().msg_gpu_precond(self.h, dptr(_f64(r)), dptr(z)), "precond")
         return z
 
     def vecjacf(self, x, v):
-        out = np.zeros(self.n)
+        out = np.empty(self.n)
         _check(load_library().msg_gpu_vecjacf(self.h, dptr(_f64(x)), dptr(_f64(v)), dptr(out)), "vecjacf")
         return out
 
@@ -330,7 +330,7 @@ class GpuSolver:
         N, S = self.n, self.ncals
         keys = (("sto", N), ("con", N), ("sea", N), ("wel", N), ("rec", S), ("sur", S), ("riv", S), ("lak", S),
                 ("drn", S))
-        out = {k: np.zeros(n) for k, n in keys}
+        out = {k: np.empty(n) for k, n in keys}
         _check(L.msg_gpu_cell_mass(self.h, *(dptr(out[k]) for k, _ in keys)), "cell_mass")
         return out
 
@@ -339,7 +339,7 @@ class GpuSolver:
         pointv [3, ncalc] x, y, z)."""
         L = load_library()
         L.msg_gpu_velocity.argtypes = [C.c_void_p, abi.PD, abi.PD]
-        fv, pv = np.zeros(6 * self.n), np.zeros(3 * self.n)
+        fv, pv = np.empty(6 * self.n), np.empty(3 * self.n)
         _check(L.msg_gpu_velocity(self.h, dptr(fv), dptr(pv)), "velocity")
         return fv.reshape(6, self.n), pv.reshape(3, self.n)
 
