@@ -1494,6 +1494,189 @@ __global__ void k_f2d(int n, const float *a, double *b) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) b[i] = (double)a[i];
 }
 
+// ---------------------------------------------------------------------------------
+// The small levels of a V-cycle in one launch: one cluster of blocks walks down from the
+// first level of at most kTailRows rows and back up, its barrier (a fraction of a
+// microsecond) between the passes that are launches of 4 us each otherwise.  Every row is
+// computed as by the kernels of the larger levels, in the same order.  (A persistent grid
+// over the whole chip, whose barrier costs as much as a launch, had not paid.)
+// ---------------------------------------------------------------------------------
+// A dense coarsest level beyond kTailDense rows wants the whole chip's bandwidth.
+constexpr int kTailRows = 8192, kTailDense = 512, kTailBlocks = 8, kTailThreads = 1024, kTailMax = 16;
+template <typename T, typename TV>
+struct TailLevel {
+  int n;
+  const int *rowptr, *col;
+  const TV *val;
+  const T *diag;
+  const int *rptr, *rcol, *pptr, *pcol;   // to this level from the one before, and back
+  const T *rval, *pval;
+  T *x, *b, *r, *x2;
+};
+template <typename T, typename TV>
+struct TailArgs {
+  int nl, sweeps;
+  T w;
+  const double *cinv;                     // dense inverse of the last level, or null
+  TailLevel<T, TV> lv[kTailMax];
+};
+
+// FP64 rows: eight lanes share a row's loads and products and add the products in entry order
+// (every lane the same sum).  Ends together in all lanes of the warp.
+template <typename F>
+__device__ __forceinline__ double ordered_sum8(double t, int beg, int end, F product) {
+  const int q = threadIdx.x & 7;
+  while (__any_sync(0xffffffffu, beg < end)) {
+    const double p = beg + q < end ? product(beg + q) : 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const double v = __shfl_sync(0xffffffffu, p, u, 8);
+      if (beg + u < end) t = __dadd_rn(t, v);
+    }
+    beg += 8;
+  }
+  return t;
+}
+
+template <typename T, typename TV>
+__global__ void __launch_bounds__(kTailThreads) k_cycle_tail(TailArgs<T, TV> a) {
+  constexpr bool F64 = sizeof(T) == 8;
+  const int nt = kTailBlocks * kTailThreads, t = blockIdx.x * kTailThreads + threadIdx.x;
+  auto sync_all = [] { cg::this_cluster().sync(); };
+  auto first = [&](const TailLevel<T, TV> &L, T *x) {   // from x = 0
+    for (int i = t; i < L.n; i += nt) {
+      if constexpr (F64) x[i] = __ddiv_rn(__dmul_rn(a.w, L.b[i]), L.diag[i]);
+      else x[i] = (a.w * L.b[i]) / L.diag[i];
+    }
+    sync_all();
+  };
+  // y = x + w (b - A x) / d, or (RES) y = b - A x
+  auto pass = [&](const TailLevel<T, TV> &L, const T *x, T *y, bool res) {
+    if constexpr (F64) {
+      for (int i0 = 0; i0 < L.n; i0 += nt / 8) {
+        const int i = i0 + (t >> 3);
+        const bool live = i < L.n;
+        const double di = live ? L.diag[i] : 1.0, xi = live ? x[i] : 0.0;
+        const double s = ordered_sum8(__dmul_rn(di, xi), live ? L.rowptr[i] : 0, live ? L.rowptr[i + 1] : 0,
+                                      [&](int k) { return __dmul_rn(L.val[k], x[L.col[k]]); });
+        if (live && (t & 7) == 0) {
+          const double r = __dsub_rn(L.b[i], s);
+          y[i] = res ? r : __dadd_rn(xi, __ddiv_rn(__dmul_rn(a.w, r), di));
+        }
+      }
+    } else {
+      for (int g0 = 0; g0 < L.n; g0 += nt / 2) {
+        const int i0 = g0 + (t >> 2) * 2, q = t & 3, i = i0 + (q & 1);
+        const bool own = q < 2 && i < L.n;
+        float bi = 0.f, di = 1.f, xi = 0.f, o0, o1;
+        if (own) { bi = L.b[i]; di = L.diag[i]; xi = x[i]; }
+        csr_off_h4x2(i0, q, L.n, L.rowptr, L.col, L.val, x, o0, o1);
+        if (own) {
+          const float r = bi - (di * xi + (q ? o1 : o0));
+          y[i] = res ? r : xi + (a.w * r) / di;
+        }
+      }
+    }
+    sync_all();
+  };
+  auto restrict_to = [&](const TailLevel<T, TV> &C, const T *r) {
+    if constexpr (F64) {
+      for (int i0 = 0; i0 < C.n; i0 += nt / 8) {
+        const int i = i0 + (t >> 3);
+        const bool live = i < C.n;
+        const double s = ordered_sum8(0.0, live ? C.rptr[i] : 0, live ? C.rptr[i + 1] : 0,
+                                      [&](int k) { return __dmul_rn(C.rval[k], r[C.rcol[k]]); });
+        if (live && (t & 7) == 0) C.b[i] = s;
+      }
+    } else {
+      for (int g0 = 0; g0 < C.n; g0 += nt / 2) {
+        const int i0 = g0 + (t >> 2) * 2, q = t & 3, i = i0 + (q & 1);
+        float t0, t1;
+        csr_off_h4x2(i0, q, C.n, C.rptr, C.rcol, C.rval, r, t0, t1);
+        if (q < 2 && i < C.n) C.b[i] = q ? t1 : t0;
+      }
+    }
+    sync_all();
+  };
+  auto prolong = [&](const TailLevel<T, TV> &C, int nf, T *x) {
+    for (int i = t; i < nf; i += nt) {
+      const int b = C.pptr[i], e = C.pptr[i + 1];
+      if constexpr (F64) {
+        double s = 0.0;
+        for (int k = b; k < e; ++k) s = __dadd_rn(s, __dmul_rn(C.pval[k], C.x[C.pcol[k]]));
+        x[i] = __dadd_rn(x[i], s);
+      } else {
+        x[i] = x[i] + csr_row_from(0.f, b, e, C.pcol, C.pval, C.x);
+      }
+    }
+    sync_all();
+  };
+  const int sw = a.sweeps;
+  // where the iterate lies: sweeps alternate between two buffers and end in x
+  auto start = [&](const TailLevel<T, TV> &L, T *&cur, T *&oth) {
+    cur = sw > 0 && sw % 2 == 0 ? L.x2 : L.x;
+    oth = cur == L.x ? L.x2 : L.x;
+  };
+  auto smooth = [&](const TailLevel<T, TV> &L, T *&cur, T *&oth, int k) {
+    for (; k > 0; --k) {
+      pass(L, cur, oth, false);
+      T *q = cur;
+      cur = oth;
+      oth = q;
+    }
+  };
+  auto pre = [&](const TailLevel<T, TV> &L, T *&cur, T *&oth) {
+    start(L, cur, oth);
+    if (sw == 0) {
+      for (int i = t; i < L.n; i += nt) cur[i] = T(0);
+      sync_all();
+    } else {
+      first(L, cur);
+      smooth(L, cur, oth, sw - 1);
+    }
+  };
+  T *cur, *oth;
+  for (int l = 0; l + 1 < a.nl; ++l) {
+    const TailLevel<T, TV> &L = a.lv[l];
+    pre(L, cur, oth);
+    pass(L, cur, L.r, true);
+    restrict_to(a.lv[l + 1], L.r);
+  }
+  {
+    const TailLevel<T, TV> &L = a.lv[a.nl - 1];
+    if (a.cinv) {
+      const double *Ci = a.cinv;
+      if constexpr (F64) {
+        for (int i0 = 0; i0 < L.n; i0 += nt / 8) {
+          const int i = i0 + (t >> 3);
+          const bool live = i < L.n;
+          const double s = ordered_sum8(0.0, 0, live ? L.n : 0, [&](int j) { return __dmul_rn(Ci[(size_t)i * L.n + j], L.b[j]); });
+          if (live && (t & 7) == 0) L.x[i] = s;
+        }
+      } else {
+        for (int row = t >> 5; row < L.n; row += nt / 32) {
+          double s = 0.0;
+          for (int j = t & 31; j < L.n; j += 32) s += Ci[(size_t)row * L.n + j] * (double)L.b[j];
+#pragma unroll
+          for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+          if ((t & 31) == 0) L.x[row] = (float)s;
+        }
+      }
+      sync_all();
+    } else {
+      pre(L, cur, oth);
+      smooth(L, cur, oth, sw);
+    }
+  }
+  for (int l = a.nl - 2; l >= 0; --l) {
+    const TailLevel<T, TV> &L = a.lv[l];
+    start(L, cur, oth);
+    if (sw > 1 && sw % 2 == 0) { T *q = cur; cur = oth; oth = q; }   // after sw - 1 sweeps
+    prolong(a.lv[l + 1], L.n, cur);
+    smooth(L, cur, oth, sw);
+  }
+}
+
 __global__ void k_col0(int nnz, const int *offrow1, int *col0) {
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < nnz) col0[k] = offrow1[k] - 1;
@@ -1875,6 +2058,46 @@ int amg_setup(msg_ctx *c) {
   return MSG_OK;
 }
 
+// Levels l .. of a V-cycle from their right-hand side to their correction, when they are
+// small; *done is left 0 when they are not.
+template <typename T>
+static int cycle_tail(msg_ctx *c, int l, int *done) {
+  constexpr bool F64 = sizeof(T) == 8;
+  using TV = typename std::conditional<F64, double, __nv_bfloat16>::type;
+  AmgState *A = S(c);
+  const int nl = (int)A->lv.size() - l;
+  *done = 0;
+  if (A->lv[l].n > kTailRows || nl > kTailMax || A->lv.back().n > kTailDense) return MSG_OK;
+  TailArgs<T, TV> a;
+  a.nl = nl;
+  a.sweeps = std::max(c->prm.amg_sweeps, 0);
+  a.w = (T)c->prm.smooth_omega;
+  a.cinv = A->lv.back().cinv;
+  for (int k = 0; k < nl; ++k) {
+    const AmgLevel &L = A->lv[l + k];
+    TailLevel<T, TV> &q = a.lv[k];
+    q.n = L.n;
+    q.rowptr = L.rowptr; q.col = L.col;
+    q.rptr = L.rptr; q.rcol = L.rcol; q.pptr = L.pptr; q.pcol = L.pcol;
+    if constexpr (F64) {
+      q.val = L.val; q.diag = L.diag; q.rval = L.rval; q.pval = L.pval;
+      q.x = L.x; q.b = L.b; q.r = L.r; q.x2 = L.x2;
+    } else {
+      q.val = L.val_h; q.diag = L.diag_f; q.rval = L.rval_f; q.pval = L.pval_f;
+      q.x = L.xf; q.b = L.bf; q.r = L.rf; q.x2 = L.x2f;
+    }
+  }
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = kTailBlocks; at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cf = {};
+  cf.gridDim = dim3(kTailBlocks); cf.blockDim = dim3(kTailThreads); cf.stream = c->stream; cf.attrs = &at; cf.numAttrs = 1;
+  MSG_CUDA(cudaLaunchKernelEx(&cf, k_cycle_tail<T, TV>, a));
+  __atomic_fetch_add(&g_launches, 1LL, __ATOMIC_RELAXED);
+  *done = 1;
+  return MSG_OK;
+}
+
 // One V-cycle z = M^-1 r (x = 0 start, amg_sweeps Jacobi sweeps before and after).
 static int vcycle(msg_ctx *c, int l, const double *b, double *x) {
   AmgState *A = S(c);
@@ -1884,6 +2107,10 @@ static int vcycle(msg_ctx *c, int l, const double *b, double *x) {
   const double w = (double)c->prm.smooth_omega;
   const int g = nb(n);
   const bool last = (l == (int)A->lv.size() - 1);
+  if (l > 0) {
+    int done = 0, rc = cycle_tail<double>(c, l, &done);
+    if (rc || done) return rc;
+  }
   if (last && L.cinv) {
     k_gemv<<<nb(n), kThreads, 0, s>>>(n, L.cinv, b, x);
     MSG_CHECK_LAUNCH();
@@ -1944,6 +2171,10 @@ static int vcycle_f(msg_ctx *c, int l, const float *b, float *x) {
   const float w = c->prm.smooth_omega;
   const int g = nb(n);
   const bool last = (l == (int)A->lv.size() - 1);
+  {
+    int done = 0, rc = cycle_tail<float>(c, l, &done);
+    if (rc || done) return rc;
+  }
   if (last && L.cinv) {
     k_gemv_mixed<<<(int)(((long long)n * 32 + kThreads - 1) / kThreads), kThreads, 0, s>>>(n, L.cinv, b, x);
     MSG_CHECK_LAUNCH();
