@@ -608,7 +608,8 @@ int norm1(msg_ctx *c, const double *a, int n, double *out) {
 
 constexpr int kResErr = 5;   // abserrmax's seven results in dres (behind the line search's five)
 static int launch_abserrmax(msg_ctx *c, double *xn, const double *xp, const double *dh) {
-  k_abserrmax<<<kRedBlocks, 256, 0, c->stream>>>(c->N, xn, xp, dh, c->part, c->dres + kResErr, c->fin_cnt + kFinArr + 1,
+  const int g = std::min(kRedBlocks, gblk(c->N));   // a maximum: the same whatever the grid
+  k_abserrmax<<<g, 256, 0, c->stream>>>(c->N, xn, xp, dh, c->part, c->dres + kResErr, c->fin_cnt + kFinArr + 1,
                                                  publish(c, kResErr + 7));
   MSG_CHECK_LAUNCH();
   return MSG_OK;
@@ -738,7 +739,7 @@ int scale(msg_ctx *c, double *y, double a, int n) {
 constexpr int kWX = 16, kWY = 8, kWCols = kWX * kWY, kWThreads = 2 * kWCols + 32;
 // a layer is fetched kWFetch steps ahead of the first column of its 8 x 4 group and used up
 // to 7 + 3 steps after it
-constexpr int kWRing = 16, kWFetch = 6, kWAhead = 2, kWPitch = 24;
+constexpr int kWRing = 16, kWFetch = 6, kWAhead = 1, kWPitch = 24;
 constexpr unsigned long long kWEmpty = 0x7ff4a5a5a5a5a5a5ull;   // a signalling NaN
 
 struct SweepArgs {
