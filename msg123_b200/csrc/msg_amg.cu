@@ -1970,11 +1970,11 @@ void amg_free(msg_ctx *c) {
   c->amg = nullptr;
 }
 
-// Per-cell bytes of the arena reserved when a context is made: the levels and transfer
-// operators of the block workloads take about 100 B per fine cell, the temporaries of the
-// first coarsening about 80; a build that outgrows the reservation spills to the pool and
-// the arena is enlarged at the next build.
-constexpr size_t kArenaPerCell = 192;
+// Per-cell bytes of the arena reserved when a context is made: a build of the block and
+// ensemble workloads takes 150 to 200 B per fine cell at its peak, the first coarsening
+// (levels and transfer operators end at 55 to 80); a build that outgrows the reservation
+// spills to the pool and the arena is enlarged at the next build.
+constexpr size_t kArenaPerCell = 288;
 
 static int amg_state(msg_ctx *c);
 
@@ -2029,7 +2029,7 @@ int amg_setup(msg_ctx *c) {
   A->lv.clear();
   // reset the arena; enlarge it first when the previous build did not fit
   if (A->arena_spill) {
-    const size_t need = A->arena_used + A->arena_spill;   // (the temporaries of all levels: ample)
+    const size_t need = A->arena_cap + A->arena_spill;   // what did not fit beside a full arena
     if (A->arena) {
       MSG_CUDA(cudaStreamSynchronize(s));
       cudaFree(A->arena);

@@ -51,7 +51,8 @@ __global__ void k_extrap(int n, double *h, const double *h_old, const double *h_
 }
 // out = -(f2 - f1) / eps; with NEG the caller passes g = -f1, and f2 - f1 = f2 + g exactly.
 template <bool NEG>
-__global__ void k_vecjac_out(int n, double *out, const double *f2, const double *f1, double eps_inv) {
+__global__ void k_vecjac_out(int n, double *out, const double *f2, const double *f1, Step eps) {
+  const double eps_inv = __ddiv_rn(1.0, eps.get());
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     out[i] = __dmul_rn(-(NEG ? __dadd_rn(f2[i], f1[i]) : __dsub_rn(f2[i], f1[i])), eps_inv);
 }
@@ -69,18 +70,11 @@ __global__ void k_csr_to_dia(int nx, int ny, int nz, const int *offind, const do
   for (int d = 0; d < 6; ++d) lu[(size_t)d * N + i] = has[d] ? lumat[k++] : 0.0;
 }
 
-static double sum_part(msg_ctx *c, int count, int *rc) {
-  double v = 0.0;
-  *rc = finish(c, count, 1, &v);
-  return v;
-}
-
-// calc_func + its squared norm
-static int func_norm(msg_ctx *c, const double *h, double *F, double *l2) {
+// calc_func's squared norm (at h, or at the trial point formed into h)
+static int func_norm(msg_ctx *c, double *h, double *F, double *l2, const Trial *trial = nullptr) {
   if (c->timing) cudaEventRecord(c->ev[7], c->stream);
-  int rc = launch_calc_func(c, h, F, true);
-  if (rc) return rc;
-  *l2 = sum_part(c, flux_parts(c), &rc);   // synchronises the stream
+  int rc = launch_calc_func(c, h, F, true, 0, 1, trial);
+  if (rc || (rc = fetch_res(c, 1, l2))) return rc;
   c->l2_last = *l2;
   if (c->timing) {
     cudaEventRecord(c->ev[0], c->stream);
@@ -99,12 +93,10 @@ static int func_norm(msg_ctx *c, const double *h, double *F, double *l2) {
 static int make_matvec(msg_ctx *c, double *l2_rhs, bool reuse, bool assembled = false) {
   cudaEvent_t *ev = c->ev;
   if (c->timing) cudaEventRecord(ev[0], c->stream);
-  int rc = assembled ? MSG_OK : launch_make_matvec(c, reuse);
+  // ||F||^2: a host round trip, which calc_numsol needs at its first iteration only
+  int rc = assembled ? MSG_OK : launch_make_matvec(c, reuse, nullptr, 0, l2_rhs ? 1 : 0);
   if (rc) return rc;
-  if (l2_rhs) {   // ||F||^2 (a host round trip; calc_numsol needs it at its first iteration only)
-    *l2_rhs = sum_part(c, flux_parts(c), &rc);
-    if (rc) return rc;
-  }
+  if (l2_rhs && (rc = fetch_res(c, 1, l2_rhs))) return rc;
   if (c->timing) cudaEventRecord(ev[1], c->stream);
   if (c->prm.precon_type == 1 && !c->prm.ref_quirks) {
     // amg_lag = k >= 1: the hierarchy built at a time step's first Newton iteration is
@@ -148,7 +140,9 @@ static int solve_linalg(msg_ctx *c, double init_norm, double *x, double *last_no
 // the make_matvec right-hand side of the iterate x it was assembled at, whose arithmetic is
 // that of calc_func term for term, so the finite difference is the same bit for bit and
 // one residual evaluation is saved.
-static int vecjacf(msg_ctx *c, const double *x, const double *v, double *out, const double *neg_f1 = nullptr) {
+// The sums behind eps stay on the device, where the perturbed head and the quotient need them:
+// no host round trip.
+static int vecjacf(msg_ctx *c, double *x, const double *v, double *out, const double *neg_f1 = nullptr) {
   const int n = c->N;
   const double *f1 = neg_f1;
   double *f2 = c->t, *jc = c->z;
@@ -158,27 +152,22 @@ static int vecjacf(msg_ctx *c, const double *x, const double *v, double *out, co
     if ((rc = func_norm(c, x, c->v, &dummy))) return rc;
     f1 = c->v;
   }
-  double l2_v, l2_x, l1_v;
-  if ((rc = dot(c, v, v, n, &l2_v))) return rc;
-  if ((rc = dot(c, x, v, n, &l2_x))) return rc;
-  if ((rc = norm1(c, v, n, &l1_v))) return rc;
-  double sign = (l2_x < 0.0) ? -1.0 : 1.0;
-  double eps = sign * std::sqrt(MACHI_EPS) * std::fmax(std::fabs(l2_x), l1_v) / l2_v;
-  double eps_inv = 1.0 / eps;
-  if ((rc = axpby(c, jc, x, eps, v, n))) return rc;
-  if ((rc = func_norm(c, jc, f2, &dummy))) return rc;
-  if (neg_f1) k_vecjac_out<true><<<nblk(n), 256, 0, c->stream>>>(n, out, f2, f1, eps_inv);
-  else k_vecjac_out<false><<<nblk(n), 256, 0, c->stream>>>(n, out, f2, f1, eps_inv);
+  if ((rc = launch_eps_sums(c, x, v))) return rc;
+  const Step eps{0.0, c->dres + kResEps, std::sqrt(MACHI_EPS)};
+  const Trial at{x, v, eps};
+  if ((rc = c->timing ? func_norm(c, jc, f2, &dummy, &at) : launch_calc_func(c, jc, f2, false, 0, 0, &at))) return rc;
+  if (neg_f1) k_vecjac_out<true><<<nblk(n), 256, 0, c->stream>>>(n, out, f2, f1, eps);
+  else k_vecjac_out<false><<<nblk(n), 256, 0, c->stream>>>(n, out, f2, f1, eps);
   MSG_CHECK_LAUNCH();
   return MSG_OK;
 }
 
+// the residual's norm at head_pre + in_lam * dh, formed into head_new
 static int calc_funcl2norm(msg_ctx *c, double in_lam) {
   c->asm_ahead = 0;   // head_new moves off the point the system was assembled at
   c->head_moved = 1;
-  int rc = axpby(c, c->head_new, c->head_pre, in_lam, c->head_change, c->N);
-  if (rc) return rc;
-  return func_norm(c, c->head_new, c->new_f, &c->l2_new);
+  const Trial at{c->head_pre, c->head_change, Step{in_lam, nullptr, 0.0}};
+  return func_norm(c, c->head_new, nullptr, &c->l2_new, &at);
 }
 
 // run_backtr (Nonlinear_solution.f90:441-631)
@@ -220,13 +209,11 @@ static int run_backtr(msg_ctx *c) {
     double dummy;
     if ((rc = func_norm(c, c->head_new, c->new_f, &dummy))) return rc;
   } else if (ahead) {
-    if ((rc = launch_make_matvec(c, false, c->rhs_alt))) return rc;
-    if ((rc = finish_to(c, flux_parts(c), 1, 4))) return rc;
+    if ((rc = launch_make_matvec(c, false, c->rhs_alt, 4))) return rc;
     fnew = c->rhs_alt;   // -F: the same squares
     c->asm_ahead = 1;
   } else {
-    if ((rc = launch_calc_func(c, c->head_new, c->new_f, true))) return rc;
-    if ((rc = finish_to(c, flux_parts(c), 1, 4))) return rc;
+    if ((rc = launch_calc_func(c, c->head_new, c->new_f, true, 4))) return rc;
   }
   // ||dh||^2, ||F(head_new)||^2, the slope and lam_length in one pass; lam_length is taken
   // again if dh is shortened (the slope, from J dh of the unshortened step, is scaled below)
@@ -448,7 +435,7 @@ static int calc_numsol(msg_ctx *c, msg_stats_t *stx) {
       if (c->conv_flag != 1 && c->back_flag != 1) set_eater(c);
     }
     if (evaluated) c->l2_new = c->l2_last;
-    else if ((rc = func_norm(c, c->head_new, c->new_f, &c->l2_new))) return rc;
+    else if ((rc = func_norm(c, c->head_new, nullptr, &c->l2_new))) return rc;
     st.back_total += c->back_iter; st.back_iter_last = c->back_iter;
     double conv_var = c->maxvar * c->len_scal;
     if (c->clog_on && (rc = convlog_push(c, maxnun))) return rc;
@@ -531,10 +518,10 @@ static int advance(msg_ctx *c, int nsteps, double rech_until, double rech_after,
       if (c->prm.guess_select) {
         // keep the learned guess only if its residual is below the extrapolation's
         double fl = 0.0, fe = 0.0;
-        if ((rc = func_norm(c, c->head_new, c->new_f, &fl))) return rc;
+        if ((rc = func_norm(c, c->head_new, nullptr, &fl))) return rc;
         k_extrap<<<nblk(n), 256, 0, c->stream>>>(n, c->head_pre, c->head_old, c->head_old2, c->delt / c->delt_old1);
         MSG_CHECK_LAUNCH();
-        if ((rc = func_norm(c, c->head_pre, c->new_f, &fe))) return rc;
+        if ((rc = func_norm(c, c->head_pre, nullptr, &fe))) return rc;
         if (!(fl < fe)) {
           // the extrapolation was evaluated last: its S, kr and storage serve the first assembly
           if ((rc = copy_d2d(c, c->head_new, c->head_pre, n))) return rc;

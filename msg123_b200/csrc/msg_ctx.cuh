@@ -2,6 +2,7 @@
 // between the translation units of libmsg123gpu.so.
 #pragma once
 #include "msg_common.cuh"
+#include "msg_reduce.cuh"
 #include "../../include/msg123_gpu.h"
 
 namespace msg {
@@ -121,10 +122,17 @@ int build_connectivity(msg_ctx *c, const msg_grid_t *g);
 int launch_srat_rperm(msg_ctx *c, const double *h, double pertur, double *srat, double *kr, double *alp);
 int launch_water_table(msg_ctx *c, double *wt);
 // F = calc_func(h); also writes srat_new and kr (rel_perm).  partial sums of F^2 in c->part[0..].
-int launch_calc_func(msg_ctx *c, const double *h, double *F, bool norm);
+// norm: ||F||^2 into dres[slot] (count > 0: and dres[0..count) to the host).  F null: not
+// stored.  trial: h is formed in the pass as trial->x + step * trial->dh.
+struct Trial {
+  const double *x, *dh;
+  Step step;
+};
+int launch_calc_func(msg_ctx *c, double *h, double *F, bool norm, int slot = 0, int count = 0, const Trial *trial = nullptr);
 // make_matvec at c->head_new: dmat, lu (DIA), rhs = -F.  reuse: srat_new, kr and sto
 // already hold the values at head_new (the last calc_func was evaluated there).
-int launch_make_matvec(msg_ctx *c, bool reuse = false, double *rhs_out = nullptr);   // rhs_out null: c->rhs
+// ||F||^2 into dres[slot], as above; rhs_out null: c->rhs
+int launch_make_matvec(msg_ctx *c, bool reuse = false, double *rhs_out = nullptr, int slot = 0, int count = 0);
 // Export the DIA Jacobian into the reference CSR order.
 int launch_dia_to_csr(msg_ctx *c, double *lumat_dev);
 int launch_mass(msg_ctx *c, double out9[9]);
@@ -157,17 +165,20 @@ int solve_bicgs(msg_ctx *c, double *x, bool x_zero = false, ErrAhead *ahead = nu
 int dot(msg_ctx *c, const double *a, const double *b, int n, double *out);   // sync + host value
 // sum narr partial arrays (nparts each, consecutive in c->part) on the device; sync; host values
 int finish(msg_ctx *c, int nparts, int narr, double *out);
-int finish_to(msg_ctx *c, int nparts, int narr, int slot, int count = 0);   // into dres[slot..]; count > 0:
-                                                                             // dres[0..count) to the host
-int fetch_res(msg_ctx *c, int count, double *out);                          // waits for them
+int fetch_res(msg_ctx *c, int count, double *out);   // waits for the results published last
 int finish9(msg_ctx *c, int nparts, double out[9]);   // nine arrays, nparts each
-int norm1(msg_ctx *c, const double *a, int n, double *out);
+// the second stage of a kernel's narr arrays of c->part: make_fin for its launch, then end_fin
+Fin make_fin(msg_ctx *c, int nparts, int narr, int slot, int count);
+template <int MAXB = 0>
+int end_fin(msg_ctx *c, const Fin &f, int count);
+// (v, v), (x, v), |v|_1 into dres[kResEps ..]
+constexpr int kResEps = 16;
+int launch_eps_sums(msg_ctx *c, const double *x, const double *v);
 int abserrmax(msg_ctx *c, double *xn, const double *xp, ErrMax &e, const double *dh = nullptr);   // dh: form xn = xp + dh first
 int lam_length(msg_ctx *c, const double *dh, const double *hn, double *out);
 // ||dh||^2, ||f||^2, (s, jv) (jv null: (s, b - r)) and lam_length(dh, hn) in one pass
 int backtr_stats(msg_ctx *c, const double *dh, const double *hn, const double *f, const double *s, const double *jv,
                  const double *b, const double *r, double out[5], bool slot4);   // slot4: also dres[4] (pending)
-int axpby(msg_ctx *c, double *y, const double *x, double a, const double *w, int n);   // y = x + a*w
 int scale(msg_ctx *c, double *y, double a, int n);
 
 // ---- msg_copy.cu ------------------------------------------------------------------------------

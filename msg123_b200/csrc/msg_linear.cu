@@ -15,7 +15,7 @@
 
 namespace msg {
 
-constexpr int kFinArr = 4;   // arrays of one second reduction stage; counters: theirs, the stage's, abserrmax's
+constexpr int kFinArr = 4;   // arrays of one second reduction stage; counters: theirs, the stage's, abserrmax's, fin_block's
 
 struct Geo3 {
   int nx, ny, nz, nxy, N;
@@ -173,8 +173,8 @@ int scan_reserve(msg_ctx *c, int n) {
   *c->res_word = 0;
   c->res_token = 0;
   MSG_CUDA(cudaMalloc(&c->fin_scratch, (size_t)4 * 8 * 1024 * 8));
-  MSG_CUDA(cudaMalloc(&c->fin_cnt, (kFinArr + 2) * 4));
-  MSG_CUDA(cudaMemsetAsync(c->fin_cnt, 0, (kFinArr + 2) * 4, c->stream));
+  MSG_CUDA(cudaMalloc(&c->fin_cnt, (kFinArr + 3) * 4));
+  MSG_CUDA(cudaMemsetAsync(c->fin_cnt, 0, (kFinArr + 3) * 4, c->stream));
   return MSG_OK;
 }
 
@@ -199,11 +199,11 @@ __device__ __forceinline__ double stencil_row(const Geo3 &g, int i, const double
   return t;
 }
 
-template <int MODE, bool RESID>
+template <int MODE, bool RESID, bool FUSE>
 __global__ void __launch_bounds__(256) k_spmv(Geo3 g, const double *__restrict__ d, const double *__restrict__ lu,
                                               const double *__restrict__ x, const double *__restrict__ b,
                                               double *__restrict__ y, const double *__restrict__ w1,
-                                              double *part) {
+                                              double *part, Fin fin) {
   __shared__ double sh[8];
   double a0 = 0.0, a1 = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < g.N; i += gridDim.x * blockDim.x) {
@@ -221,10 +221,11 @@ __global__ void __launch_bounds__(256) k_spmv(Geo3 g, const double *__restrict__
     double s = block_sum<256>(a1, sh);
     if (threadIdx.x == 0) part[gridDim.x + blockIdx.x] = s;
   }
+  if (FUSE) fin_block(fin, gridDim.x);
 }
 
 int launch_spmv(msg_ctx *c, const double *x, double *y) {
-  k_spmv<0, false><<<nblk(c->N), 256, 0, c->stream>>>(geo3(c), c->dmat, c->lu, x, nullptr, y, nullptr, nullptr);
+  k_spmv<0, false, false><<<nblk(c->N), 256, 0, c->stream>>>(geo3(c), c->dmat, c->lu, x, nullptr, y, nullptr, nullptr, Fin{});
   MSG_CHECK_LAUNCH();
   return MSG_OK;
 }
@@ -284,9 +285,10 @@ struct Quot {
 // x = xin + a*z; r = rin - a*w; partials ||r||^2 and (r, rs).  xin null: x starts at zero
 // (0 + a*z, the value the zeroed x gave, without reading it); rin: the residual before the
 // update (the right-hand side itself on the first update from x = 0).
+template <bool FUSE>
 __global__ void __launch_bounds__(256) k_bicg_xr(int n, int ng, const double *xin, double *x, const double *rin, double *r,
                                                  const double *z, const double *w, const double *rs, Quot quot,
-                                                 double *part) {
+                                                 double *part, Fin fin) {
   const double a = quot.get();
   double v[2][kGr], zi[kGr], wi[kGr], ri[kGr], si[kGr], xi[kGr];
   const int i0 = blockIdx.x * (256 * kGr) + threadIdx.x;
@@ -310,10 +312,12 @@ __global__ void __launch_bounds__(256) k_bicg_xr(int n, int ng, const double *xi
     }
   }
   group_sums<2>(v, ng, part);
+  if (FUSE) fin_block(fin, gridDim.x);
 }
 
 // partials of (a, b)
-__global__ void __launch_bounds__(256) k_dot(int n, int ng, const double *a, const double *b, double *part) {
+template <bool FUSE>
+__global__ void __launch_bounds__(256) k_dot(int n, int ng, const double *a, const double *b, double *part, Fin fin) {
   double v[1][kGr];
   const int i0 = blockIdx.x * (256 * kGr) + threadIdx.x;
 #pragma unroll
@@ -322,22 +326,24 @@ __global__ void __launch_bounds__(256) k_dot(int n, int ng, const double *a, con
     v[0][k] = i < n ? __dmul_rn(a[i], b[i]) : 0.0;
   }
   group_sums<1>(v, ng, part);
+  if (FUSE) fin_block(fin, gridDim.x);
 }
 
-__global__ void __launch_bounds__(256) k_norm1(int n, int ng, const double *a, double *part) {
-  double v[1][kGr];
+// partials of (v, v), (x, v) and |v|_1
+template <bool FUSE>
+__global__ void __launch_bounds__(256) k_eps_sums(int n, int ng, const double *x, const double *y, double *part, Fin fin) {
+  double v[3][kGr];
   const int i0 = blockIdx.x * (256 * kGr) + threadIdx.x;
 #pragma unroll
   for (int k = 0; k < kGr; ++k) {
     const int i = i0 + 256 * k;
-    v[0][k] = i < n ? fabs(a[i]) : 0.0;
+    const double yi = i < n ? y[i] : 0.0, xi = i < n ? x[i] : 0.0;
+    v[0][k] = __dmul_rn(yi, yi);
+    v[1][k] = __dmul_rn(xi, yi);
+    v[2][k] = fabs(yi);
   }
-  group_sums<1>(v, ng, part);
-}
-
-__global__ void k_axpby(int n, double *y, const double *x, double a, const double *w) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    y[i] = __dadd_rn(x[i], __dmul_rn(a, w[i]));
+  group_sums<3>(v, ng, part);
+  if (FUSE) fin_block(fin, gridDim.x);
 }
 
 __global__ void k_scale(int n, double *y, double a) {
@@ -352,35 +358,6 @@ struct ArgMax {
 __device__ __forceinline__ ArgMax amax(ArgMax p, ArgMax q) {
   if (q.a > p.a || (q.a == p.a && q.idx > p.idx)) return q;
   return p;
-}
-
-// What a finishing kernel hands to the host: `count` results from res into pinned words, then
-// the token (null word: nothing).
-struct Publish {
-  const double *res;
-  double *host;
-  int count;
-  unsigned *word, token;
-  __device__ __forceinline__ void operator()() const {   // one thread, all results written
-    if (!word) return;
-    __threadfence();
-    for (int k = 0; k < count; ++k) host[k] = __ldcg(res + k);
-    __threadfence_system();
-    *(volatile unsigned *)word = token;
-  }
-};
-// True in the block that arrives last of `total` (all its threads); the counter is left at 0.
-__device__ __forceinline__ bool last_block(int *cnt, int total) {
-  __shared__ int s_last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    s_last = atomicAdd(cnt, 1) == total - 1;
-    if (s_last) *cnt = 0;
-  }
-  __syncthreads();
-  if (s_last) __threadfence();
-  return s_last;
 }
 
 // dh non-null: first forms xn = xp + 1*dh (the Newton update, the axpby it replaces, same
@@ -567,11 +544,19 @@ static int launch_finish(msg_ctx *c, int nparts, int narr, int slot, int count, 
   return MSG_OK;
 }
 
-// Second stage into dres[slot .. slot + narr) without waiting: results of several reductions
-// come back with one fetch_res, of which the last finish_to names the count.
-int finish_to(msg_ctx *c, int nparts, int narr, int slot, int count) {
-  return launch_finish(c, nparts, narr, slot, count);
+// Second stage of narr arrays into dres[slot ..]: by the writing kernel's last block, or, for
+// long arrays, a launch after it.  Results of several stages come back with one fetch_res,
+// of which the last names the count.
+Fin make_fin(msg_ctx *c, int nparts, int narr, int slot, int count) {
+  const bool fuse = nparts <= kFuseParts;
+  return Fin{fuse, c->part, nparts, narr, c->dres + slot, c->fin_cnt + kFinArr + 2, publish(c, fuse ? count : 0)};
 }
+template <int MAXB>
+int end_fin(msg_ctx *c, const Fin &f, int count) {
+  if (f.fuse) return MSG_OK;
+  return launch_finish<MAXB>(c, f.nparts, f.narr, (int)(f.out - c->dres), count);
+}
+template int end_fin<0>(msg_ctx *, const Fin &, int);
 
 int fetch_res(msg_ctx *c, int count, double *out) {
   int rc = token_wait(c, c->res_word, c->res_token);
@@ -581,7 +566,7 @@ int fetch_res(msg_ctx *c, int count, double *out) {
 }
 
 int finish(msg_ctx *c, int nparts, int narr, double *out) {
-  int rc = finish_to(c, nparts, narr, 0, narr);
+  int rc = launch_finish(c, nparts, narr, 0, narr);
   if (rc) return rc;
   return fetch_res(c, narr, out);
 }
@@ -594,16 +579,25 @@ int finish9(msg_ctx *c, int nparts, double out[9]) {
   return fetch_res(c, 9, out);
 }
 
-int dot(msg_ctx *c, const double *a, const double *b, int n, double *out) {
-  k_dot<<<gblk(n), 256, 0, c->stream>>>(n, ngroups(n), a, b, c->part);
+static int launch_dot(msg_ctx *c, const double *a, const double *b, int n, int slot, int count) {
+  const Fin f = make_fin(c, ngroups(n), 1, slot, count);
+  (f.fuse ? k_dot<true> : k_dot<false>)<<<gblk(n), 256, 0, c->stream>>>(n, ngroups(n), a, b, c->part, f);
   MSG_CHECK_LAUNCH();
-  return finish(c, ngroups(n), 1, out);
+  return end_fin(c, f, count);
 }
 
-int norm1(msg_ctx *c, const double *a, int n, double *out) {
-  k_norm1<<<gblk(n), 256, 0, c->stream>>>(n, ngroups(n), a, c->part);
+int dot(msg_ctx *c, const double *a, const double *b, int n, double *out) {
+  int rc = launch_dot(c, a, b, n, 0, 1);
+  if (rc) return rc;
+  return fetch_res(c, 1, out);
+}
+
+int launch_eps_sums(msg_ctx *c, const double *x, const double *v) {
+  const int n = c->N;
+  const Fin f = make_fin(c, ngroups(n), 3, kResEps, 0);
+  (f.fuse ? k_eps_sums<true> : k_eps_sums<false>)<<<gblk(n), 256, 0, c->stream>>>(n, ngroups(n), x, v, c->part, f);
   MSG_CHECK_LAUNCH();
-  return finish(c, ngroups(n), 1, out);
+  return end_fin(c, f, 0);
 }
 
 constexpr int kResErr = 5;   // abserrmax's seven results in dres (behind the line search's five)
@@ -634,9 +628,10 @@ int abserrmax(msg_ctx *c, double *xn, const double *xp, ErrMax &e, const double 
 // has the bits of its own dot product; J dh is jv, or b - r (BiCGStab's residual from dh = 0)
 // formed with the rounding of the axpby it replaces.  The maximum is exact whatever the
 // grouping: one per block, in the place of its first group.
+template <bool FUSE>
 __global__ void __launch_bounds__(256) k_backtr_stats(int n, int ng, const double *dh, const double *hn, const double *f,
                                                       const double *s, const double *jv, const double *b,
-                                                      const double *r, double *part) {
+                                                      const double *r, double *part, Fin fin) {
   __shared__ double sm[8];
   double v[3][kGr], num = 1.0, den = 1.0;
   double di[kGr], hi[kGr], fi[kGr], si[kGr], ji[kGr], bi[kGr];
@@ -673,15 +668,17 @@ __global__ void __launch_bounds__(256) k_backtr_stats(int n, int ng, const doubl
       for (int w = 0; w < 8; ++w) m = fmax(m, sm[w]);
     if (g < ng) part[(size_t)3 * ng + g] = m;
   }
+  if (FUSE) fin_block<8>(fin, gridDim.x);
 }
 
 int backtr_stats(msg_ctx *c, const double *dh, const double *hn, const double *f, const double *s, const double *jv,
                  const double *b, const double *r, double out[5], bool slot4) {
   const int ng = ngroups(c->N);
   if ((size_t)4 * ng > c->npart) { set_error("backtr_stats: partials buffer too small"); return MSG_ERR_STATE; }
-  k_backtr_stats<<<gblk(c->N), 256, 0, c->stream>>>(c->N, ng, dh, hn, f, s, jv, b, r, c->part);
+  const Fin fin = make_fin(c, ng, 4, 0, slot4 ? 5 : 4);
+  (fin.fuse ? k_backtr_stats<true> : k_backtr_stats<false>)<<<gblk(c->N), 256, 0, c->stream>>>(c->N, ng, dh, hn, f, s, jv, b, r, c->part, fin);
   MSG_CHECK_LAUNCH();
-  int rc = launch_finish<8>(c, ng, 4, 0, slot4 ? 5 : 4);
+  int rc = end_fin<8>(c, fin, slot4 ? 5 : 4);
   if (rc || (rc = fetch_res(c, slot4 ? 5 : 4, out))) return rc;
   out[3] = std::fmax(1.0, out[3]);
   return MSG_OK;
@@ -695,12 +692,6 @@ int lam_length(msg_ctx *c, const double *dh, const double *hn, double *out) {
   double m = 1.0;
   for (int b = 0; b < kRedBlocks; ++b) m = std::fmax(m, c->hpin[b]);
   *out = m;
-  return MSG_OK;
-}
-
-int axpby(msg_ctx *c, double *y, const double *x, double a, const double *w, int n) {
-  k_axpby<<<nblk(n), 256, 0, c->stream>>>(n, y, x, a, w);
-  MSG_CHECK_LAUNCH();
   return MSG_OK;
 }
 
@@ -1049,13 +1040,11 @@ int solve_bicgs(msg_ctx *c, double *x, bool x_zero, ErrAhead *ahead) {
   if (x_zero) {
     if (need_dilu && (rc = launch_precon_dilu(c))) return rc;
     // sk = <b, b>, collected with the first residual norm
-    k_dot<<<gb, 256, 0, c->stream>>>(n, ng, c->rhs, c->rhs, c->part);
-    MSG_CHECK_LAUNCH();
-    if ((rc = finish_to(c, ng, 1, kBB, 0))) return rc;
+    if ((rc = launch_dot(c, c->rhs, c->rhs, n, kBB, 0))) return rc;
     rs = p1 = r1 = c->rhs;
   } else {
     // r = b - A x
-    k_spmv<0, true><<<nb, 256, 0, c->stream>>>(g, c->dmat, c->lu, x, c->rhs, c->r, nullptr, nullptr);
+    k_spmv<0, true, false><<<nb, 256, 0, c->stream>>>(g, c->dmat, c->lu, x, c->rhs, c->r, nullptr, nullptr, Fin{});
     MSG_CHECK_LAUNCH();
     if (need_dilu && (rc = launch_precon_dilu(c))) return rc;
     MSG_CUDA(cudaMemcpyAsync(c->rs, c->r, (size_t)n * 8, cudaMemcpyDeviceToDevice, c->stream));
@@ -1076,15 +1065,17 @@ int solve_bicgs(msg_ctx *c, double *x, bool x_zero, ErrAhead *ahead) {
       MSG_CHECK_LAUNCH();
     }
     if ((rc = apply_prec(c, p, c->z))) return rc;
-    k_spmv<1, false><<<nb, 256, 0, c->stream>>>(g, c->dmat, c->lu, c->z, nullptr, c->v, rs, c->part);
+    Fin f = make_fin(c, nb, 1, kSk2, 0);
+    (f.fuse ? k_spmv<1, false, true> : k_spmv<1, false, false>)<<<nb, 256, 0, c->stream>>>(g, c->dmat, c->lu, c->z, nullptr, c->v, rs, c->part, f);
     MSG_CHECK_LAUNCH();
-    if ((rc = finish_to(c, nb, 1, kSk2, 0))) return rc;
+    if ((rc = end_fin(c, f, 0))) return rc;
     const bool from_bb = x_zero && first;   // sk = <b, b> is still on the device
-    k_bicg_xr<<<gb, 256, 0, c->stream>>>(n, ng, first && x_zero ? nullptr : x, x, first ? r1 : c->r, c->r, c->z, c->v, rs,
-                                        Quot{from_bb ? c->dres + kBB : nullptr, c->dres + kSk2, sk}, c->part);
-    MSG_CHECK_LAUNCH();
     const bool spec = ahead && from_bb && c->one_half;
-    if ((rc = finish_to(c, ng, 1, kR1, spec ? 0 : 3))) return rc;
+    f = make_fin(c, ng, 1, kR1, spec ? 0 : 3);
+    (f.fuse ? k_bicg_xr<true> : k_bicg_xr<false>)<<<gb, 256, 0, c->stream>>>(n, ng, first && x_zero ? nullptr : x, x, first ? r1 : c->r, c->r, c->z, c->v, rs,
+                                        Quot{from_bb ? c->dres + kBB : nullptr, c->dres + kSk2, sk}, c->part, f);
+    MSG_CHECK_LAUNCH();
+    if ((rc = end_fin(c, f, spec ? 0 : 3))) return rc;
     if (spec && (rc = launch_abserrmax(c, ahead->xn, ahead->xp, x))) return rc;
     if ((rc = fetch_res(c, spec ? kResErr + 7 : 3, got))) return rc;
     if (from_bb) sk = got[kBB];
@@ -1098,13 +1089,15 @@ int solve_bicgs(msg_ctx *c, double *x, bool x_zero, ErrAhead *ahead) {
     }
     if (c->conv_flag == 1) break;
     if ((rc = apply_prec(c, c->r, c->z))) return rc;
-    k_spmv<2, false><<<nb, 256, 0, c->stream>>>(g, c->dmat, c->lu, c->z, nullptr, c->t, c->r, c->part);
+    f = make_fin(c, nb, 2, kTs, 0);
+    (f.fuse ? k_spmv<2, false, true> : k_spmv<2, false, false>)<<<nb, 256, 0, c->stream>>>(g, c->dmat, c->lu, c->z, nullptr, c->t, c->r, c->part, f);
     MSG_CHECK_LAUNCH();
-    if ((rc = finish_to(c, nb, 2, kTs, 0))) return rc;
-    k_bicg_xr<<<gb, 256, 0, c->stream>>>(n, ng, x, x, c->r, c->r, c->z, c->t, rs, Quot{c->dres + kTs, c->dres + kTs + 1, 0.0},
-                                        c->part);
+    if ((rc = end_fin(c, f, 0))) return rc;
+    f = make_fin(c, ng, 2, kR2, kR2 + 2);
+    (f.fuse ? k_bicg_xr<true> : k_bicg_xr<false>)<<<gb, 256, 0, c->stream>>>(n, ng, x, x, c->r, c->r, c->z, c->t, rs, Quot{c->dres + kTs, c->dres + kTs + 1, 0.0},
+                                        c->part, f);
     MSG_CHECK_LAUNCH();
-    if ((rc = finish_to(c, ng, 2, kR2, kR2 + 2)) || (rc = fetch_res(c, kR2 + 2, got))) return rc;
+    if ((rc = end_fin(c, f, kR2 + 2)) || (rc = fetch_res(c, kR2 + 2, got))) return rc;
     omega = got[kTs] / got[kTs + 1];
     c->rnorm = got[kR2];
     c->conv_flag = (std::sqrt(c->rnorm / c->bnorm) <= c->errtol) ? 1 : 0;

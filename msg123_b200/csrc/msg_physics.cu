@@ -212,17 +212,29 @@ struct CellArgs {
   const float *reta, *retn, *resi, *poro, *ss;
   double delt_inv, newper, newper_inv;
   double *srat, *kr, *kr_per, *sto, *stod;
+  // TRIAL: h is formed here, h_out = x + step * dh
+  const double *x, *dh;
+  double *h_out;
+  Step step;
 };
 
 // ASM = false: calc_func's pass; ASM = true: make_matvec's pass.  REUSE (with ASM): S, kr
 // and the storage term at h are already in srat / kr / sto from a residual evaluation at
 // the same h (the previous Newton iteration ends with one), so only the perturbed
 // evaluation at h + newper is made -- the same values bit for bit, half the pow calls.
-template <bool ASM, bool REUSE = false, int FORM = 0>
+// TRIAL: the head is the line search's trial point (or the perturbed head of J v), formed and
+// stored by this pass.
+template <bool ASM, bool REUSE = false, int FORM = 0, bool TRIAL = false>
 __global__ void k_cell(int N, CellArgs a) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  double hi = a.h[i], top = a.top[i];
+  double hi, top = a.top[i];
+  if (TRIAL) {
+    hi = __dadd_rn(a.x[i], __dmul_rn(a.step.get(), a.dh[i]));
+    a.h_out[i] = hi;
+  } else {
+    hi = a.h[i];
+  }
   float reta = a.reta[i], retn = a.retn[i], resi = a.resi[i], poro = a.poro[i], ss = a.ss[i];
   if (REUSE) {
     VG v;
@@ -272,6 +284,7 @@ struct FluxArgs {
   double *dmat, *lu;  // assembly outputs
   float *dmat_f, *lu_f;   // FP32 images for the mixed-precision V-cycle (nullable)
   double *part;       // partial sums of F^2 (nullable)
+  Fin fin;            // and their second stage
 };
 
 // func_surfterm for one top cell; returns the term and the Jacobian delh/over pair.
@@ -331,7 +344,7 @@ __device__ __forceinline__ double stage_term(const double *st, int S, int s, dou
 // The flux passes run on a 3D grid of 256-thread blocks, each a 32 (x) by 8 (y) tile of one
 // layer (blockIdx.z), so a cell's grid coordinates come from its block and lane with no
 // integer division; flux_parts(c) is the number of blocks (one F^2 partial each).
-template <bool ASM>
+template <bool ASM, bool FUSE>
 __device__ __forceinline__ void flux_body(const FluxArgs &a, double *sh) {
   const Geo g = a.g;
   const int ix = blockIdx.x * 32 + (threadIdx.x & 31), iy = blockIdx.y * 8 + (threadIdx.x >> 5), iz = blockIdx.z;
@@ -423,27 +436,30 @@ __device__ __forceinline__ void flux_body(const FluxArgs &a, double *sh) {
       a.dmat[i] = dd;
       if (a.dmat_f) a.dmat_f[i] = (float)dd;
     } else {
-      a.F[i] = f;
+      if (a.F) a.F[i] = f;
     }
     f2 = __dmul_rn(f, f);
   }
   if (a.part) {
     double s = block_sum<256>(f2, sh);
     if (threadIdx.x == 0) a.part[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)] = s;
+    if (FUSE) fin_block(a.fin, gridDim.x * gridDim.y * gridDim.z);
   }
 }
 
 // Residual pass: at most 48 registers so that five 256-thread blocks stay resident per SM
 // (the pass is bound by the latency of its 27 loads per cell, not by bandwidth).
+template <bool FUSE>
 __global__ void __launch_bounds__(256, 5) k_flux_res(FluxArgs a) {
   __shared__ double sh[8];
-  flux_body<false>(a, sh);
+  flux_body<false, FUSE>(a, sh);
 }
 
 // Assembly pass (residual + Jacobian rows).
+template <bool FUSE>
 __global__ void __launch_bounds__(256) k_flux_asm(FluxArgs a) {
   __shared__ double sh[8];
-  flux_body<true>(a, sh);
+  flux_body<true, FUSE>(a, sh);
 }
 
 // DIA -> reference CSR order export of lumat.
@@ -733,6 +749,7 @@ static FluxArgs flux_args(msg_ctx *c, const double *h) {
   a.newper = c->newper; a.newper_inv = c->newper_inv;
   a.F = nullptr; a.dmat = nullptr; a.lu = nullptr; a.part = nullptr;
   a.dmat_f = nullptr; a.lu_f = nullptr;
+  a.fin = Fin{};
   return a;
 }
 
@@ -742,23 +759,32 @@ static CellArgs cell_args(msg_ctx *c, const double *h) {
   a.reta = c->reta; a.retn = c->retn; a.resi = c->resi; a.poro = c->poro; a.ss = c->ss;
   a.delt_inv = c->delt_inv; a.newper = c->newper; a.newper_inv = c->newper_inv;
   a.srat = c->srat_new; a.kr = c->kr; a.kr_per = c->kr_per; a.sto = c->sto; a.stod = c->stod;
+  a.x = a.dh = nullptr; a.h_out = nullptr; a.step = Step{};
   return a;
 }
 
-int launch_calc_func(msg_ctx *c, const double *h, double *F, bool norm) {
+int launch_calc_func(msg_ctx *c, double *h, double *F, bool norm, int slot, int count, const Trial *trial) {
   const int bc = c->blk_cell > 0 ? c->blk_cell : kThreads;
+  CellArgs ca = cell_args(c, h);
   auto k = c->prm.vg_form ? k_cell<false, false, 1> : k_cell<false, false, 0>;
-  k<<<(c->N + bc - 1) / bc, bc, 0, c->stream>>>(c->N, cell_args(c, h));
+  if (trial) {
+    ca.x = trial->x; ca.dh = trial->dh; ca.h_out = h; ca.step = trial->step;
+    k = c->prm.vg_form ? k_cell<false, false, 1, true> : k_cell<false, false, 0, true>;
+  }
+  k<<<(c->N + bc - 1) / bc, bc, 0, c->stream>>>(c->N, ca);
   MSG_CHECK_LAUNCH();
   FluxArgs a = flux_args(c, h);
   a.F = F;
-  a.part = norm ? c->part : nullptr;
-  k_flux_res<<<flux_grid(c), 256, 0, c->stream>>>(a);
+  if (norm) {
+    a.part = c->part;
+    a.fin = make_fin(c, flux_parts(c), 1, slot, count);
+  }
+  (a.fin.fuse ? k_flux_res<true> : k_flux_res<false>)<<<flux_grid(c), 256, 0, c->stream>>>(a);
   MSG_CHECK_LAUNCH();
-  return MSG_OK;
+  return norm ? end_fin(c, a.fin, count) : MSG_OK;
 }
 
-int launch_make_matvec(msg_ctx *c, bool reuse, double *rhs_out) {
+int launch_make_matvec(msg_ctx *c, bool reuse, double *rhs_out, int slot, int count) {
   const int bc = c->blk_cell > 0 ? c->blk_cell : kThreads;
   auto k = c->prm.vg_form ? (reuse ? k_cell<true, true, 1> : k_cell<true, false, 1>)
                            : (reuse ? k_cell<true, true, 0> : k_cell<true, false, 0>);
@@ -771,9 +797,10 @@ int launch_make_matvec(msg_ctx *c, bool reuse, double *rhs_out) {
   a.dmat_f = c->dmat_f;
   a.lu_f = c->lu_f;
   a.part = c->part;
-  k_flux_asm<<<flux_grid(c), 256, 0, c->stream>>>(a);
+  a.fin = make_fin(c, flux_parts(c), 1, slot, count);
+  (a.fin.fuse ? k_flux_asm<true> : k_flux_asm<false>)<<<flux_grid(c), 256, 0, c->stream>>>(a);
   MSG_CHECK_LAUNCH();
-  return MSG_OK;
+  return end_fin(c, a.fin, count);
 }
 
 int launch_dia_to_csr(msg_ctx *c, double *lumat_dev) {
