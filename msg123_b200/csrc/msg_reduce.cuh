@@ -36,12 +36,14 @@ __device__ __forceinline__ bool last_block(int *cnt, int total) {
 }
 
 // Second stage by the last block of the kernel that wrote the partials (fuse), for arrays of
-// at most kFuseParts: the sums of k_finish, whose thread t adds the elements t + 1024 u,
-// u = 0 .. 7, in a tree before the tree over t; here a thread stands for four of its threads.
-// Longer arrays keep the separate launch, which has more than one block to load them, and a
-// kernel of their own (FUSE = false): the registers of this stage would halve the resident
-// blocks of the passes that stream memory.
-constexpr int kFuseParts = 8192;
+// at most kFuseParts: the sums of k_finish, whose thread t starts with element t; here a
+// thread stands for four of its threads.
+// It saves a launch (the 20 000-cell box 5.15 -> 4.3 ms) but holds every block until its
+// ticket has gone round; with more blocks than the chip takes at once that costs more than
+// the launch (364k cells, 1444 blocks: 9.1 against 8.6 ms).  Longer arrays therefore keep the
+// separate launch, and a kernel of their own (FUSE = false): the registers of this stage
+// would also halve the resident blocks of the passes that stream memory.
+constexpr int kFuseParts = 512;
 struct Fin {
   bool fuse;
   const double *part;
@@ -64,13 +66,9 @@ __device__ __forceinline__ void fin_block(const Fin &f, int nblocks) {
     double s[4];
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
-      double x[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int i = t + 256 * v + 1024 * u;
-        x[u] = i < f.nparts ? comb(0.0, __ldcg(p + i)) : 0.0;
-      }
-      s[v] = comb(comb(comb(x[0], x[1]), comb(x[2], x[3])), comb(comb(x[4], x[5]), comb(x[6], x[7])));
+      // u = 0 only: the others lie beyond kFuseParts, and their zeros add nothing
+      const int i = t + 256 * v;
+      s[v] = i < f.nparts ? comb(0.0, __ldcg(p + i)) : 0.0;
     }
     sh[t] = comb(comb(s[0], s[2]), comb(s[1], s[3]));
     __syncthreads();
