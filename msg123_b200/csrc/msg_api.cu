@@ -821,6 +821,12 @@ int msg_gpu_calc_func(msg_ctx_t *c, const double *infx, double *funcv) {
   return MSG_OK;
 }
 
+// Device scratch for off-diagonals in CSR order, made by the first call that passes them.
+static int csr_scratch(msg_ctx *c) {
+  if (!c->csr_tmp) ALLOC(c->csr_tmp, (size_t)std::max(c->nnz, 1) * 8);
+  return MSG_OK;
+}
+
 int msg_gpu_make_matvec(msg_ctx_t *c, double *dmat, double *lumat, double *rhs) {
   if (!c) return MSG_ERR_ARG;
   c->amg_force = 1;   // a direct call always rebuilds the hierarchy
@@ -829,17 +835,11 @@ int msg_gpu_make_matvec(msg_ctx_t *c, double *dmat, double *lumat, double *rhs) 
   if (rc) return rc;
   size_t N = c->N;
   if (lumat) {
-    double *tmp = nullptr;
-    ALLOC(tmp, (size_t)c->nnz * 8);
-    rc = launch_dia_to_csr(c, tmp);
-    if (!rc && cudaStreamSynchronize(c->stream) == cudaSuccess) rc = copy_out(lumat, tmp, (size_t)c->nnz * 8);
-    cudaFree(tmp);
-    if (rc) return rc;
+    if ((rc = csr_scratch(c)) || (rc = launch_dia_to_csr(c, c->csr_tmp))) return rc;
   }
   MSG_CUDA(cudaStreamSynchronize(c->stream));
-  if (dmat) COPY_OUT(dmat, c->dmat, N * 8);
-  if (rhs) COPY_OUT(rhs, c->rhs, N * 8);
-  return MSG_OK;
+  const CopyOut jobs[3] = {{lumat, c->csr_tmp, (size_t)c->nnz * 8}, {dmat, c->dmat, N * 8}, {rhs, c->rhs, N * 8}};
+  return copy_out(jobs, 3);
 }
 
 int msg_gpu_set_system(msg_ctx_t *c, const double *dmat, const double *lumat, const double *rhs) {
@@ -847,10 +847,10 @@ int msg_gpu_set_system(msg_ctx_t *c, const double *dmat, const double *lumat, co
   size_t N = c->N;
   UPLOAD(c->dmat, dmat, N * 8);
   UPLOAD(c->rhs, rhs, N * 8);
-  double *tmp = nullptr;
-  ALLOC(tmp, (size_t)c->nnz * 8);
-  UPLOAD(tmp, lumat, (size_t)c->nnz * 8);
-  k_csr_to_dia<<<nblk(c->N), kThreads, 0, c->stream>>>(c->nx, c->ny, c->nz, c->offind, tmp, c->lu);
+  int rc = csr_scratch(c);
+  if (rc) return rc;
+  UPLOAD(c->csr_tmp, lumat, (size_t)c->nnz * 8);
+  k_csr_to_dia<<<nblk(c->N), kThreads, 0, c->stream>>>(c->nx, c->ny, c->nz, c->offind, c->csr_tmp, c->lu);
   MSG_CHECK_LAUNCH();
   if (c->dmat_f) {
     k_to_f32<<<kRedBlocks, kThreads, 0, c->stream>>>(N, c->dmat, c->dmat_f);
@@ -858,13 +858,8 @@ int msg_gpu_set_system(msg_ctx_t *c, const double *dmat, const double *lumat, co
     k_to_f32<<<kRedBlocks, kThreads, 0, c->stream>>>(6 * N, c->lu, c->lu_f);
     MSG_CHECK_LAUNCH();
   }
-  MSG_CUDA(cudaStreamSynchronize(c->stream));
-  cudaFree(tmp);
   MSG_CUDA(cudaMemcpyAsync(c->slope_rhs, c->rhs, N * 8, cudaMemcpyDeviceToDevice, c->stream));
-  if (c->prm.precon_type == 1 && !c->prm.ref_quirks) {
-    int rc = amg_setup(c);
-    if (rc) return rc;
-  }
+  if (c->prm.precon_type == 1 && !c->prm.ref_quirks && (rc = amg_setup(c))) return rc;
   MSG_CUDA(cudaStreamSynchronize(c->stream));
   return MSG_OK;
 }
@@ -1250,7 +1245,7 @@ static void free_ctx(msg_ctx *c) {
                 c->left_off, c->right_off, c->hydf_conn, c->abyd_conn, c->head_new, c->head_old, c->head_pre,
                 c->head_change, c->srat_new, c->srat_old, c->surf_head, c->surf_old, c->new_f, c->kr, c->kr_per,
                 c->alp, c->sto, c->stod, c->tmpv, c->dmat, c->lu, c->rhs, c->rhs_alt, c->head_old2, c->slope_rhs, c->dilu_d, c->r, c->rs,
-                c->p, c->v, c->t, c->z, c->part, c->scan_sums, c->fin_scratch, c->fin_cnt, c->wave_order, c->wave_ticket, c->wave_slots, c->dmat_f, c->lu_f, c->dres};
+                c->p, c->v, c->t, c->z, c->part, c->scan_sums, c->csr_tmp, c->fin_scratch, c->fin_cnt, c->wave_order, c->wave_ticket, c->wave_slots, c->dmat_f, c->lu_f, c->dres};
   for (auto q : dp) if (q) cudaFree(q);
   if (c->hpin) cudaFreeHost(c->hpin);
   for (int k = 0; k < 8; ++k) if (c->ev[k]) cudaEventDestroy(c->ev[k]);

@@ -54,6 +54,7 @@ struct msg_ctx {
   // ---- reference CSR built on the GPU (export / tests) -------------------------------
   int *offind, *offrow, *conn_dir, *left_off, *right_off;
   double *hydf_conn, *abyd_conn;
+  double *csr_tmp;                               // [nnz] off-diagonals on their way in or out (lazily)
   // ---- state -------------------------------------------------------------------------
   double *head_new, *head_old, *head_pre, *head_change, *srat_new, *srat_old, *head_old2;
   double *surf_head, *surf_old, *new_f;
