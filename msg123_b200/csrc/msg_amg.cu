@@ -41,6 +41,39 @@ struct AmgLevel {
   float *diag_f = nullptr, *val_f = nullptr, *pval_f = nullptr, *rval_f = nullptr;
   __nv_bfloat16 *val_h = nullptr;
   float *xf = nullptr, *bf = nullptr, *rf = nullptr, *x2f = nullptr;
+  void *pack = nullptr;                   // rows of this and the following levels for k_cycle_tail_f
+};
+
+// The mixed cycle's small levels (k_cycle_tail_f): what one launch works on, laid out by a build.
+constexpr int kTailBlocks = 8, kTailMax = 16;
+constexpr int kTailSlices = 192;          // of a block, over all levels
+struct TailMatF {                         // byte offsets of a block's rows in shared memory; cap: room for entries
+  int rp, cl, v, cap;
+};
+struct TailLevelF {
+  int n, per;                             // per: rows of a block, a multiple of 4
+  int v[2], b, d;                         // two whole iterates; the block's right-hand side and diagonal
+  TailMatF R, P;
+  const int *rowptr, *col;                // null at a dense last level
+  const __nv_bfloat16 *val;
+  const float *diag;
+  const int *rptr, *rcol, *pptr, *pcol;   // R: to this level from the one before; P: to this level from the one after
+  const float *rval, *pval;
+};
+struct TailHead {                         // of a block: its slices' first words (-1: no room) and widths, over all levels
+  int words, sl0[kTailMax], off[kTailSlices], wid[kTailSlices];
+  int base[2 * kTailMax], in[2 * kTailMax];   // R, P: first entry copied (a multiple of 8); whether the rows fit
+};
+struct TailArgsF {
+  int nl, sweeps, pool, words;            // slices: offset in shared memory, room (words of a block)
+  float w;
+  TailHead *head;                         // by block, as are the slices behind them
+  uint32_t *slices;
+  const double *cinv;                     // dense inverse of the last level, or null
+  const float *b;                         // of the first level, as is x
+  float *x;
+  int shared;                             // bytes in all
+  TailLevelF lv[kTailMax];
 };
 
 struct AmgState {
@@ -57,6 +90,9 @@ struct AmgState {
   // stream-ordered pool and the arena is enlarged before the next build.
   char *arena = nullptr;
   size_t arena_cap = 0, arena_used = 0, arena_tmp = 0, arena_spill = 0;
+  bool tail_set = false;                  // shared-memory limit of k_cycle_tail_f raised
+  int tail_level = -1;                    // its first level, -1 none
+  TailArgsF tail;
 };
 
 static AmgState *S(msg_ctx *c) { return reinterpret_cast<AmgState *>(c->amg); }
@@ -1251,14 +1287,14 @@ __device__ __forceinline__ float ldf(const __nv_bfloat16 *p) { return __bfloat16
 // grid2r(n): four threads per two rows.
 template <typename TV>
 __device__ __forceinline__ void csr_off_h4x2(int i0, int q, int n, const int *rp, const int *cl, const TV *v,
-                                             const float *x, float &t0, float &t1) {
+                                             const float *x, float &t0, float &t1, int k0 = 0) {
   float s[2] = {0.f, 0.f};
   int k[2], e[2];
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     const bool live = i0 + r < n;
-    k[r] = live ? rp[i0 + r] + q : 0;
-    e[r] = live ? rp[i0 + r + 1] : 0;
+    k[r] = live ? rp[i0 + r] - k0 + q : 0;
+    e[r] = live ? rp[i0 + r + 1] - k0 : 0;
   }
   while (k[0] < e[0] || k[1] < e[1]) {
     int c[2][4];
@@ -1502,23 +1538,20 @@ __global__ void k_f2d(int n, const float *a, double *b) {
 // over the whole chip, whose barrier costs as much as a launch, had not paid.)
 // ---------------------------------------------------------------------------------
 // A dense coarsest level beyond kTailDense rows wants the whole chip's bandwidth.
-constexpr int kTailRows = 8192, kTailDense = 512, kTailBlocks = 8, kTailThreads = 1024, kTailMax = 16;
-template <typename T, typename TV>
+constexpr int kTailRows = 8192, kTailDense = 512, kTailThreads = 1024, kTailThreadsF = 512;
 struct TailLevel {
   int n;
   const int *rowptr, *col;
-  const TV *val;
-  const T *diag;
+  const double *val, *diag;
   const int *rptr, *rcol, *pptr, *pcol;   // to this level from the one before, and back
-  const T *rval, *pval;
-  T *x, *b, *r, *x2;
+  const double *rval, *pval;
+  double *x, *b, *r, *x2;
 };
-template <typename T, typename TV>
 struct TailArgs {
   int nl, sweeps;
-  T w;
+  double w;
   const double *cinv;                     // dense inverse of the last level, or null
-  TailLevel<T, TV> lv[kTailMax];
+  TailLevel lv[kTailMax];
 };
 
 // FP64 rows: eight lanes share a row's loads and products and add the products in entry order
@@ -1538,129 +1571,85 @@ __device__ __forceinline__ double ordered_sum8(double t, int beg, int end, F pro
   return t;
 }
 
-template <typename T, typename TV>
-__global__ void __launch_bounds__(kTailThreads) k_cycle_tail(TailArgs<T, TV> a) {
-  constexpr bool F64 = sizeof(T) == 8;
+__global__ void __launch_bounds__(kTailThreads) k_cycle_tail(TailArgs a) {
   const int nt = kTailBlocks * kTailThreads, t = blockIdx.x * kTailThreads + threadIdx.x;
   auto sync_all = [] { cg::this_cluster().sync(); };
-  auto first = [&](const TailLevel<T, TV> &L, T *x) {   // from x = 0
-    for (int i = t; i < L.n; i += nt) {
-      if constexpr (F64) x[i] = __ddiv_rn(__dmul_rn(a.w, L.b[i]), L.diag[i]);
-      else x[i] = (a.w * L.b[i]) / L.diag[i];
-    }
+  auto first = [&](const TailLevel &L, double *x) {   // from x = 0
+    for (int i = t; i < L.n; i += nt) x[i] = __ddiv_rn(__dmul_rn(a.w, L.b[i]), L.diag[i]);
     sync_all();
   };
   // y = x + w (b - A x) / d, or (RES) y = b - A x
-  auto pass = [&](const TailLevel<T, TV> &L, const T *x, T *y, bool res) {
-    if constexpr (F64) {
-      for (int i0 = 0; i0 < L.n; i0 += nt / 8) {
-        const int i = i0 + (t >> 3);
-        const bool live = i < L.n;
-        const double di = live ? L.diag[i] : 1.0, xi = live ? x[i] : 0.0;
-        const double s = ordered_sum8(__dmul_rn(di, xi), live ? L.rowptr[i] : 0, live ? L.rowptr[i + 1] : 0,
-                                      [&](int k) { return __dmul_rn(L.val[k], x[L.col[k]]); });
-        if (live && (t & 7) == 0) {
-          const double r = __dsub_rn(L.b[i], s);
-          y[i] = res ? r : __dadd_rn(xi, __ddiv_rn(__dmul_rn(a.w, r), di));
-        }
-      }
-    } else {
-      for (int g0 = 0; g0 < L.n; g0 += nt / 2) {
-        const int i0 = g0 + (t >> 2) * 2, q = t & 3, i = i0 + (q & 1);
-        const bool own = q < 2 && i < L.n;
-        float bi = 0.f, di = 1.f, xi = 0.f, o0, o1;
-        if (own) { bi = L.b[i]; di = L.diag[i]; xi = x[i]; }
-        csr_off_h4x2(i0, q, L.n, L.rowptr, L.col, L.val, x, o0, o1);
-        if (own) {
-          const float r = bi - (di * xi + (q ? o1 : o0));
-          y[i] = res ? r : xi + (a.w * r) / di;
-        }
+  auto pass = [&](const TailLevel &L, const double *x, double *y, bool res) {
+    for (int i0 = 0; i0 < L.n; i0 += nt / 8) {
+      const int i = i0 + (t >> 3);
+      const bool live = i < L.n;
+      const double di = live ? L.diag[i] : 1.0, xi = live ? x[i] : 0.0;
+      const double s = ordered_sum8(__dmul_rn(di, xi), live ? L.rowptr[i] : 0, live ? L.rowptr[i + 1] : 0,
+                                    [&](int k) { return __dmul_rn(L.val[k], x[L.col[k]]); });
+      if (live && (t & 7) == 0) {
+        const double r = __dsub_rn(L.b[i], s);
+        y[i] = res ? r : __dadd_rn(xi, __ddiv_rn(__dmul_rn(a.w, r), di));
       }
     }
     sync_all();
   };
-  auto restrict_to = [&](const TailLevel<T, TV> &C, const T *r) {
-    if constexpr (F64) {
-      for (int i0 = 0; i0 < C.n; i0 += nt / 8) {
-        const int i = i0 + (t >> 3);
-        const bool live = i < C.n;
-        const double s = ordered_sum8(0.0, live ? C.rptr[i] : 0, live ? C.rptr[i + 1] : 0,
-                                      [&](int k) { return __dmul_rn(C.rval[k], r[C.rcol[k]]); });
-        if (live && (t & 7) == 0) C.b[i] = s;
-      }
-    } else {
-      for (int g0 = 0; g0 < C.n; g0 += nt / 2) {
-        const int i0 = g0 + (t >> 2) * 2, q = t & 3, i = i0 + (q & 1);
-        float t0, t1;
-        csr_off_h4x2(i0, q, C.n, C.rptr, C.rcol, C.rval, r, t0, t1);
-        if (q < 2 && i < C.n) C.b[i] = q ? t1 : t0;
-      }
+  auto restrict_to = [&](const TailLevel &C, const double *r) {
+    for (int i0 = 0; i0 < C.n; i0 += nt / 8) {
+      const int i = i0 + (t >> 3);
+      const bool live = i < C.n;
+      const double s = ordered_sum8(0.0, live ? C.rptr[i] : 0, live ? C.rptr[i + 1] : 0,
+                                    [&](int k) { return __dmul_rn(C.rval[k], r[C.rcol[k]]); });
+      if (live && (t & 7) == 0) C.b[i] = s;
     }
     sync_all();
   };
-  auto prolong = [&](const TailLevel<T, TV> &C, int nf, T *x) {
+  auto prolong = [&](const TailLevel &C, int nf, double *x) {
     for (int i = t; i < nf; i += nt) {
-      const int b = C.pptr[i], e = C.pptr[i + 1];
-      if constexpr (F64) {
-        double s = 0.0;
-        for (int k = b; k < e; ++k) s = __dadd_rn(s, __dmul_rn(C.pval[k], C.x[C.pcol[k]]));
-        x[i] = __dadd_rn(x[i], s);
-      } else {
-        x[i] = x[i] + csr_row_from(0.f, b, e, C.pcol, C.pval, C.x);
-      }
+      double s = 0.0;
+      for (int k = C.pptr[i], e = C.pptr[i + 1]; k < e; ++k) s = __dadd_rn(s, __dmul_rn(C.pval[k], C.x[C.pcol[k]]));
+      x[i] = __dadd_rn(x[i], s);
     }
     sync_all();
   };
   const int sw = a.sweeps;
   // where the iterate lies: sweeps alternate between two buffers and end in x
-  auto start = [&](const TailLevel<T, TV> &L, T *&cur, T *&oth) {
-    cur = sw > 0 && sw % 2 == 0 ? L.x2 : L.x;
+  auto start = [&](const TailLevel &L, double *&cur, double *&oth) {
+    cur = sw > 0 ? L.x2 : L.x;            // 2 sw - 1 sweeps
     oth = cur == L.x ? L.x2 : L.x;
   };
-  auto smooth = [&](const TailLevel<T, TV> &L, T *&cur, T *&oth, int k) {
+  auto smooth = [&](const TailLevel &L, double *&cur, double *&oth, int k) {
     for (; k > 0; --k) {
       pass(L, cur, oth, false);
-      T *q = cur;
+      double *q = cur;
       cur = oth;
       oth = q;
     }
   };
-  auto pre = [&](const TailLevel<T, TV> &L, T *&cur, T *&oth) {
+  auto pre = [&](const TailLevel &L, double *&cur, double *&oth) {
     start(L, cur, oth);
     if (sw == 0) {
-      for (int i = t; i < L.n; i += nt) cur[i] = T(0);
+      for (int i = t; i < L.n; i += nt) cur[i] = 0.0;
       sync_all();
     } else {
       first(L, cur);
       smooth(L, cur, oth, sw - 1);
     }
   };
-  T *cur, *oth;
+  double *cur, *oth;
   for (int l = 0; l + 1 < a.nl; ++l) {
-    const TailLevel<T, TV> &L = a.lv[l];
+    const TailLevel &L = a.lv[l];
     pre(L, cur, oth);
     pass(L, cur, L.r, true);
     restrict_to(a.lv[l + 1], L.r);
   }
   {
-    const TailLevel<T, TV> &L = a.lv[a.nl - 1];
+    const TailLevel &L = a.lv[a.nl - 1];
     if (a.cinv) {
-      const double *Ci = a.cinv;
-      if constexpr (F64) {
-        for (int i0 = 0; i0 < L.n; i0 += nt / 8) {
-          const int i = i0 + (t >> 3);
-          const bool live = i < L.n;
-          const double s = ordered_sum8(0.0, 0, live ? L.n : 0, [&](int j) { return __dmul_rn(Ci[(size_t)i * L.n + j], L.b[j]); });
-          if (live && (t & 7) == 0) L.x[i] = s;
-        }
-      } else {
-        for (int row = t >> 5; row < L.n; row += nt / 32) {
-          double s = 0.0;
-          for (int j = t & 31; j < L.n; j += 32) s += Ci[(size_t)row * L.n + j] * (double)L.b[j];
-#pragma unroll
-          for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-          if ((t & 31) == 0) L.x[row] = (float)s;
-        }
+      for (int i0 = 0; i0 < L.n; i0 += nt / 8) {
+        const int i = i0 + (t >> 3);
+        const bool live = i < L.n;
+        const double s = ordered_sum8(0.0, 0, live ? L.n : 0, [&](int j) { return __dmul_rn(a.cinv[(size_t)i * L.n + j], L.b[j]); });
+        if (live && (t & 7) == 0) L.x[i] = s;
       }
       sync_all();
     } else {
@@ -1669,11 +1658,298 @@ __global__ void __launch_bounds__(kTailThreads) k_cycle_tail(TailArgs<T, TV> a) 
     }
   }
   for (int l = a.nl - 2; l >= 0; --l) {
-    const TailLevel<T, TV> &L = a.lv[l];
+    const TailLevel &L = a.lv[l];
     start(L, cur, oth);
-    if (sw > 1 && sw % 2 == 0) { T *q = cur; cur = oth; oth = q; }   // after sw - 1 sweeps
+    if (sw > 0 && sw % 2 == 0) { double *q = cur; cur = oth; oth = q; }   // after sw - 1 sweeps
     prolong(a.lv[l + 1], L.n, cur);
     smooth(L, cur, oth, sw);
+  }
+}
+
+// The same of the mixed cycle, out of shared memory: every block keeps the iterates whole, the
+// lanes that finish a row storing it into all blocks' copies, and the operator rows that it
+// computes.  A pass is bounded by the shared memory's loads, so an off-diagonal is one word
+// (column and BF16 value), laid out by slices of sixteen rows, a warp's, in the order in which
+// the lanes take them (without bank conflicts): a load of it and one of x per entry.  Rows of
+// the transfers, used once, are copied as they are; what does not fit is read from memory.
+// The build lays the slices out, so that a launch copies them as they are (laid out by each
+// launch: 8 us more at 3507 rows).  A whole cycle against the passes out of L2: 113 -> 92 us on
+// 64 x 57 x 33 cells (1270 rows at the first small level), 141 -> 114 on 113 x 87 x 37 (3507),
+// 422 -> 379 on 256 x 256 x 64 (3880).  What is left is latency: 1.2 us a pass of a small
+// level, most of it the barrier, the rows' store and the control that every warp walks; so 512
+// threads (1024 take 2 us more a cycle, 256 6 us more).
+constexpr int kTailShared = 222 * 1024;   // of a block's 227 KB
+// bytes from src (16-byte aligned, in an allocation of a multiple of 256 bytes), by NT threads
+template <int NT>
+__device__ __forceinline__ void tail_fetch(char *dst, const void *src, int bytes, int i) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  for (int o = i * 16; o < bytes; o += NT * 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + o), "l"((const char *)src + o) : "memory");
+}
+
+__device__ __forceinline__ int tail_row(const TailLevelF &L, int rank) { return min(L.n, rank * L.per); }
+
+// What k_cycle_tail_f's block of the same number will copy: extents of its rows of the
+// transfers, slices of its operators' rows (as wide as the longest row wants, in steps of
+// two; the first that find no room and all behind them are left to memory).
+__global__ void __launch_bounds__(kTailThreads) k_tail_pack(const __grid_constant__ TailArgsF a) {
+  __shared__ TailLevelF lv[kTailMax];     // a copy: constants under a variable index answer slowly
+  __shared__ TailHead h;
+  const int t = threadIdx.x, rank = blockIdx.x, lane = t & 31, warp = t >> 5, q = t & 3, nl = a.nl;
+#pragma unroll
+  for (int l = 0; l < kTailMax; ++l)
+    if (t == 16 * l && l < nl) lv[l] = a.lv[l];
+  __syncthreads();
+  int nsl = 0;
+  for (int l = 0; l < nl; ++l) {
+    const TailLevelF &L = lv[l];
+    if (t == 0) h.sl0[l] = nsl;
+    if (!L.rowptr) continue;
+    const int r0 = tail_row(L, rank), nr = tail_row(L, rank + 1) - r0, ns = (nr + 15) / 16;
+    for (int s = warp; s < ns; s += kTailThreads / 32) {
+      const int j = s * 16 + (lane & 15);
+      const int len = j < nr ? L.rowptr[r0 + j + 1] - L.rowptr[r0 + j] : 0;
+      const int w = (__reduce_max_sync(0xffffffffu, (len + 3) / 4) + 1) & ~1;
+      if (lane == 0) h.wid[nsl + s] = w;
+    }
+    nsl += ns;
+  }
+  if (warp == kTailThreads / 32 - 1 && lane < 2 * nl) {
+    const TailLevelF &L = lv[lane >> 1];
+    const TailMatF &m = lane & 1 ? L.P : L.R;
+    const int *rp = lane & 1 ? L.pptr : L.rptr;
+    const int r0 = tail_row(L, rank), nr = tail_row(L, rank + 1) - r0;
+    bool fits = m.cap > 0 && nr > 0;      // r0 is a multiple of 4 where there are rows
+    int b = 0;
+    if (fits) {
+      b = rp[r0] & ~7;
+      fits = rp[r0 + nr] - b <= m.cap;
+    }
+    h.base[lane] = b;
+    h.in[lane] = fits;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    int run = 0, words = 0;
+    for (int s0 = 0; s0 < nsl; s0 += 32) {
+      const int w = s0 + lane < nsl ? h.wid[s0 + lane] * 64 : 0;
+      int e = w;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, e, o);
+        if (lane >= o) e += v;
+      }
+      const bool fits = run + e <= a.words;
+      if (s0 + lane < nsl) h.off[s0 + lane] = fits ? run + e - w : -1;
+      words = max(words, (int)__reduce_max_sync(0xffffffffu, fits ? run + e : 0));
+      run += __shfl_sync(0xffffffffu, e, 31);
+    }
+    if (lane == 0) h.words = words;
+  }
+  __syncthreads();
+  for (int i = t; i < (int)(sizeof(TailHead) / 4); i += kTailThreads)
+    reinterpret_cast<int *>(a.head + rank)[i] = reinterpret_cast<const int *>(&h)[i];
+  uint32_t *out = a.slices + (size_t)rank * a.words;
+  for (int l = 0; l < nl; ++l) {
+    const TailLevelF &L = lv[l];
+    if (!L.rowptr) continue;
+    const int r0 = tail_row(L, rank), nr = tail_row(L, rank + 1) - r0;
+    const uint32_t pad = (uint32_t)((L.n + 1) & ~1) << 16;
+    for (int s = warp; s * 16 < nr; s += kTailThreads / 32) {
+      const int o = h.off[h.sl0[l] + s], w = h.wid[h.sl0[l] + s], j = s * 16 + (lane >> 2) * 2;
+      if (o < 0) continue;
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        int k = 0, e = 0;
+        if (j + r < nr) { k = L.rowptr[r0 + j + r] + q; e = L.rowptr[r0 + j + r + 1]; }
+        for (int u = 0; u < w; ++u) {
+          const int kk = k + 4 * u;
+          out[o + (2 * u + r) * 32 + lane] = kk < e ? (uint32_t)L.col[kk] << 16 | __bfloat16_as_ushort(L.val[kk]) : pad;
+        }
+      }
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kTailThreadsF) k_cycle_tail_f(const __grid_constant__ TailArgsF a) {
+  extern __shared__ __align__(16) char sm[];
+  __shared__ TailLevelF lv[kTailMax];     // a copy: constants under a variable index answer slowly
+  __shared__ TailHead h;
+  auto cl = cg::this_cluster();
+  const int t = threadIdx.x, rank = (int)cl.block_rank(), lane = t & 31, warp = t >> 5, q = t & 3, nl = a.nl, sw = a.sweeps;
+  auto vec = [&](int o) { return reinterpret_cast<float *>(sm + o); };
+  auto first_row = [&](const TailLevelF &L) { return tail_row(L, rank); };
+  auto own_rows = [&](const TailLevelF &L) { return tail_row(L, rank + 1) - tail_row(L, rank); };
+  for (int i = t; i < (int)(sizeof(TailHead) / 4); i += kTailThreadsF)
+    reinterpret_cast<int *>(&h)[i] = reinterpret_cast<const int *>(a.head + rank)[i];
+#pragma unroll
+  for (int l = 0; l < kTailMax; ++l)
+    if (t == 16 * l && l < nl) lv[l] = a.lv[l];
+  __syncthreads();
+  const int *off = h.off, *wid = h.wid, *sl0 = h.sl0, *base = h.base, *in = h.in;
+  // ---- everything on its way: slices, transfers and diagonals, the first sweep
+  uint32_t *pool = reinterpret_cast<uint32_t *>(sm + a.pool);
+  tail_fetch<kTailThreadsF>(sm + a.pool, a.slices + (size_t)rank * a.words, h.words * 4, t);
+  for (int k = warp; k < 3 * nl; k += kTailThreadsF / 32) {
+    const int l = k / 3, m = k % 3;
+    const TailLevelF &L = lv[l];
+    const int r0 = first_row(L), nr = own_rows(L);
+    if (m == 2) {
+      if (L.diag) tail_fetch<32>(sm + L.d, L.diag + r0, nr * 4, lane);
+    } else if (in[2 * l + m]) {
+      const TailMatF &M = m ? L.P : L.R;
+      const int *rp = m ? L.pptr : L.rptr, b = base[2 * l + m], n = rp[r0 + nr] - b;
+      tail_fetch<32>(sm + M.rp, rp + r0, (nr + 1) * 4, lane);
+      tail_fetch<32>(sm + M.cl, (m ? L.pcol : L.rcol) + b, n * 4, lane);
+      tail_fetch<32>(sm + M.v, (m ? L.pval : L.rval) + b, n * 4, lane);
+    }
+  }
+  if (t < 2 * nl) vec(lv[t >> 1].v[t & 1])[(lv[t >> 1].n + 1) & ~1] = 0.f;   // what the padding multiplies
+  const bool dense0 = a.cinv && nl == 1;
+  {                                       // the first level's right-hand side and first sweep, whole in every block
+    const TailLevelF &L = lv[0];
+    const int r0 = first_row(L), nr = own_rows(L);
+    const int n = L.n;
+    const float *d = L.diag;
+    float *lb = vec(L.b), *x = vec(L.v[0]);
+    for (int i0 = t; i0 < n; i0 += 4 * kTailThreadsF) {
+      float b[4], di[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = i0 + u * kTailThreadsF;
+        b[u] = i < n ? a.b[i] : 0.f;
+        di[u] = i < n && !dense0 ? d[i] : 1.f;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = i0 + u * kTailThreadsF;
+        if (i >= r0 && i < r0 + nr) lb[i - r0] = b[u];
+        if (i < n) x[i] = dense0 ? b[u] : sw > 0 ? (a.w * b[u]) / di[u] : 0.f;
+      }
+    }
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  cl.sync();                              // also: every block's shared memory exists
+  // ---- passes, one at a time: smoothing from v[k & 1] to the other, k = 0 .. sw - 2 on the
+  // way down and .. 2 sw - 2 on the way up, r in the iterate that is free
+  enum { kSmooth, kResidual, kRestrict, kProlong, kDense };
+  bool up = false, out = false;
+  for (int l = 0, k = 0, res = 0; l >= 0;) {
+    const TailLevelF &L = lv[l];
+    const bool last = l == nl - 1;
+    int kind, lw = l;                     // lw: the level whose rows are computed
+    if (!up && last && a.cinv) kind = kDense;
+    else if (up && res) kind = kProlong;
+    else if (k < (up || last ? 2 * sw - 1 : sw - 1)) kind = kSmooth;
+    else if (up || last) {                // level finished: prolong to the one before
+      up = true;
+      res = 1;
+      k = max(sw - 1, 0);
+      --l;
+      continue;
+    } else kind = res ? kRestrict : kResidual;
+    if (kind == kRestrict) lw = l + 1;
+    const TailLevelF &W = lv[lw];
+    const int r0 = first_row(W), nr = own_rows(W), cur = L.v[k & 1], oth = L.v[~k & 1];
+    out = kind == kSmooth && l == 0 && (up || last) && k == 2 * sw - 2;   // the cycle's last pass
+    // rows j and j + 1 (r0, j even; copies end on a pair) to every block, two blocks a lane
+    auto put = [&](int o, int j, float y) {
+      const float2 y2 = make_float2(__shfl_sync(0xffffffffu, y, 0, 4), __shfl_sync(0xffffffffu, y, 1, 4));
+      if (j >= nr) return;
+      float2 *dst = reinterpret_cast<float2 *>(vec(o) + r0 + j);
+      *cl.map_shared_rank(dst, 2 * q) = y2;
+      *cl.map_shared_rank(dst, 2 * q + 1) = y2;
+    };
+    if (kind <= kResidual) {              // y = x + w (b - A x) / d, or b - A x
+      const float *x = vec(cur), *xr = x + r0, *b = vec(W.b), *d = vec(W.d);
+      for (int s = warp; s * 16 < nr; s += kTailThreadsF / 32) {
+        const int j = s * 16 + (lane >> 2) * 2, i = j + (q & 1), o = off[sl0[l] + s], w = wid[sl0[l] + s];
+        float bi = 0.f, di = 1.f, xi = 0.f, s0 = 0.f, s1 = 0.f;
+        if (i < nr) { bi = b[i]; di = d[i]; xi = xr[i]; }
+        if (o >= 0) {
+          const uint32_t *p = pool + o + lane;
+#pragma unroll 2
+          for (int u = 0; u < w; u += 2, p += 128) {
+            const uint32_t e0 = p[0], f0 = p[32], e1 = p[64], f1 = p[96];
+            const float xe0 = x[e0 >> 16], xf0 = x[f0 >> 16], xe1 = x[e1 >> 16], xf1 = x[f1 >> 16];
+            s0 += __uint_as_float(e0 << 16) * xe0;
+            s1 += __uint_as_float(f0 << 16) * xf0;
+            s0 += __uint_as_float(e1 << 16) * xe1;
+            s1 += __uint_as_float(f1 << 16) * xf1;
+          }
+          s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
+          s1 += __shfl_xor_sync(0xffffffffu, s1, 1);
+          s0 += __shfl_xor_sync(0xffffffffu, s0, 2);
+          s1 += __shfl_xor_sync(0xffffffffu, s1, 2);
+        } else {
+          csr_off_h4x2(j, q, nr, W.rowptr + r0, W.col, W.val, x, s0, s1);
+        }
+        const float r = bi - (di * xi + ((q & 1) ? s1 : s0));
+        const float y = i >= nr ? 0.f : kind == kResidual ? r : xi + (a.w * r) / di;
+        if (!out) put(oth, j, y);
+        else if (q < 2 && i < nr) a.x[r0 + i] = y;
+      }
+      if (kind == kSmooth) ++k;
+      else res = 1;
+    } else if (kind == kRestrict) {       // b = R r and the first sweep from it; a dense level: b itself
+      const float *x = vec(oth), *d = vec(W.d);
+      float *b = vec(W.b);
+      const bool dense = a.cinv && lw == nl - 1;
+      for (int s = warp; s * 16 < nr; s += kTailThreadsF / 32) {
+        const int j = s * 16 + (lane >> 2) * 2, i = j + (q & 1);
+        float s0, s1;
+        if (in[2 * lw])
+          csr_off_h4x2(j, q, nr, reinterpret_cast<const int *>(sm + W.R.rp), reinterpret_cast<const int *>(sm + W.R.cl),
+                       vec(W.R.v), x, s0, s1, base[2 * lw]);
+        else csr_off_h4x2(j, q, nr, W.rptr + r0, W.rcol, W.rval, x, s0, s1);
+        float y = (q & 1) ? s1 : s0;
+        if (i >= nr) y = 0.f;
+        else {
+          if (q < 2) b[i] = y;
+          if (!dense) y = sw > 0 ? (a.w * y) / d[i] : 0.f;
+        }
+        put(W.v[0], j, y);
+      }
+      l = lw;
+      k = res = 0;
+    } else if (kind == kProlong) {        // x += P x of the level after
+      const float *xc = vec(lv[l + 1].v[(a.cinv && l == nl - 2) || sw > 0]);   // 2 sw - 1 sweeps change buffers
+      const int mk = 2 * l + 1, b0 = base[mk];
+      const int *srp = reinterpret_cast<const int *>(sm + L.P.rp), *sc = reinterpret_cast<const int *>(sm + L.P.cl);
+      float *x = vec(cur) + r0;
+      for (int j = t; j < nr; j += kTailThreadsF) {
+        const float s = in[mk] ? csr_row_from(0.f, srp[j] - b0, srp[j + 1] - b0, sc, vec(L.P.v), xc)
+                               : csr_row_from(0.f, L.pptr[r0 + j], L.pptr[r0 + j + 1], L.pcol, L.pval, xc);
+        const float y = x[j] + s;
+#pragma unroll
+        for (int w = 0; w < kTailBlocks; ++w) *cl.map_shared_rank(x + j, w) = y;
+      }
+      res = 0;
+    } else {                              // dense: b whole in v[0], x to v[1]
+      const int n = L.n, per = (n + kTailBlocks - 1) / kTailBlocks;
+      const int d0 = min(n, rank * per), d1 = min(n, d0 + per);
+      const float *b = vec(L.v[0]);
+      for (int i = d0 + warp; i < d1; i += kTailThreadsF / 32) {
+        const double *Ci = a.cinv + (size_t)i * n;
+        double s = 0.0;
+#pragma unroll 4
+        for (int j = lane; j < n; j += 32) s += Ci[j] * (double)b[j];
+#pragma unroll
+        for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane < kTailBlocks) *cl.map_shared_rank(vec(L.v[1]) + i, lane) = (float)s;
+      }
+      up = true;
+      res = 1;
+      k = max(sw - 1, 0);
+      --l;
+    }
+    if (out) break;
+    cl.sync();
+  }
+  if (!out) {                             // no sweeps, or the dense level alone
+    const TailLevelF &L = lv[0];
+    const float *x = vec(L.v[dense0 || sw > 0]) + first_row(L);
+    for (int j = t; j < own_rows(L); j += kTailThreadsF) a.x[first_row(L) + j] = x[j];
   }
 }
 
@@ -1736,7 +2012,7 @@ static void hfree(AmgState *A, void *q, cudaStream_t s) {
 
 static void free_level(AmgState *A, AmgLevel &L, cudaStream_t s) {
   void *p[] = {L.rowptr, L.col, L.diag, L.val, L.pptr, L.pcol, L.pval, L.rptr, L.rcol, L.rval, L.agg, L.cinv,
-               L.x, L.b, L.r, L.x2, L.diag_f, L.val_f, L.pval_f, L.rval_f, L.val_h, L.xf, L.bf, L.rf, L.x2f};
+               L.x, L.b, L.r, L.x2, L.diag_f, L.val_f, L.pval_f, L.rval_f, L.val_h, L.xf, L.bf, L.rf, L.x2f, L.pack};
   for (void *q : p) hfree(A, q, s);
   L = AmgLevel();
 }
@@ -2020,6 +2296,91 @@ static int amg_state(msg_ctx *c) {
   return MSG_OK;
 }
 
+template <typename K, typename Args>
+static int tail_launch(msg_ctx *c, K kernel, const Args &a, int threads, int shared) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = kTailBlocks; at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cf = {};
+  cf.gridDim = dim3(kTailBlocks); cf.blockDim = dim3(threads); cf.dynamicSmemBytes = shared;
+  cf.stream = c->stream; cf.attrs = &at; cf.numAttrs = 1;
+  MSG_CUDA(cudaLaunchKernelEx(&cf, kernel, a));
+  __atomic_fetch_add(&g_launches, 1LL, __ATOMIC_RELAXED);
+  return MSG_OK;
+}
+// Levels l .. of a V-cycle from their right-hand side to their correction, when they are
+// small; *done is left 0 when they are not.
+static bool tail_takes(const AmgState *A, int l) {
+  return A->lv[l].n <= kTailRows && (int)A->lv.size() - l <= kTailMax && A->lv.back().n <= kTailDense;
+}
+// Lays the small levels out for k_cycle_tail_f at the end of a build.
+static int tail_setup(msg_ctx *c) {
+  AmgState *A = S(c);
+  int l = 1, rc;
+  A->tail_level = -1;
+  while (l < (int)A->lv.size() && !tail_takes(A, l)) ++l;
+  if (c->prm.precision != 1 || l >= (int)A->lv.size()) return MSG_OK;
+  TailArgsF &a = A->tail;
+  const int nl = a.nl = (int)A->lv.size() - l;
+  a.cinv = A->lv.back().cinv;
+  a.b = A->lv[l].bf;
+  a.x = A->lv[l].xf;
+  int used = 0, slices = 0;
+  auto place = [&](size_t bytes) {
+    const int o = used;
+    used += (int)((bytes + 15) & ~(size_t)15);
+    return o;
+  };
+  size_t words = 0;
+  for (int k = 0; k < nl; ++k) {
+    const AmgLevel &L = A->lv[l + k], *N = k + 1 < nl ? &A->lv[l + k + 1] : nullptr;
+    const bool dense = a.cinv && !N;
+    TailLevelF &q = a.lv[k];
+    q.n = L.n;
+    q.per = ((L.n + kTailBlocks - 1) / kTailBlocks + 3) & ~3;
+    q.rowptr = dense ? nullptr : L.rowptr; q.col = L.col; q.val = L.val_h; q.diag = L.diag_f;
+    q.rptr = L.rptr; q.rcol = L.rcol; q.rval = L.rval_f;
+    q.pptr = N ? N->pptr : nullptr; q.pcol = N ? N->pcol : nullptr; q.pval = N ? N->pval_f : nullptr;
+    for (int v = 0; v < 2; ++v) q.v[v] = place(((size_t)L.n + 2) * 4);
+    q.b = place((size_t)q.per * 4);
+    q.d = place((size_t)q.per * 4);
+    slices += (q.per + 15) / 16;
+    // a slice's rows are padded to its longest and blocks differ: 2.2 words per entry
+    if (!dense) words += (size_t)L.nnz / kTailBlocks * 11 / 5 + 512;
+  }
+  if (used > kTailShared || slices > kTailSlices) return MSG_OK;
+  a.words = (int)std::min(words, (size_t)(kTailShared - used) / 4) & ~3;
+  a.pool = place((size_t)a.words * 4);
+  // transfers while there is room: an even share of the entries and half as many
+  auto hold = [&](TailMatF &m, int per, int nnz) {
+    const int cap = (nnz / kTailBlocks / 2 * 3 + 64 + 7) & ~7, before = used;
+    m.rp = place((size_t)(per + 1) * 4);
+    m.cl = place((size_t)cap * 4);
+    m.v = place((size_t)cap * 4);
+    m.cap = used <= kTailShared ? cap : 0;
+    if (!m.cap) used = before;
+  };
+  for (int k = 0; k < nl; ++k) {
+    a.lv[k].R.cap = a.lv[k].P.cap = 0;
+    if (k > 0) hold(a.lv[k].R, a.lv[k].per, A->lv[l + k].pnnz);
+    if (k + 1 < nl) hold(a.lv[k].P, a.lv[k].per, A->lv[l + k + 1].pnnz);
+  }
+  a.shared = used;
+  char *pack = nullptr;
+  if ((rc = halloc(c, &pack, kTailBlocks * (sizeof(TailHead) + (size_t)a.words * 4)))) return rc;
+  A->lv[l].pack = pack;
+  a.head = reinterpret_cast<TailHead *>(pack);
+  a.slices = reinterpret_cast<uint32_t *>(pack + kTailBlocks * sizeof(TailHead));
+  if (!A->tail_set) {
+    MSG_CUDA(cudaFuncSetAttribute(k_cycle_tail_f, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailShared));
+    A->tail_set = true;
+  }
+  k_tail_pack<<<kTailBlocks, kTailThreads, 0, c->stream>>>(a);
+  MSG_CHECK_LAUNCH();
+  A->tail_level = l;
+  return MSG_OK;
+}
+
 int amg_setup(msg_ctx *c) {
   int rc;
   if ((rc = amg_state(c))) return rc;
@@ -2054,48 +2415,34 @@ int amg_setup(msg_ctx *c) {
   if (A->lv.size() > 1 && A->lv.back().n <= std::max(c->prm.amg_coarse_max, 1)) {
     if ((rc = dense_inverse(c, A->lv.back()))) return rc;
   }
+  if ((rc = tail_setup(c))) return rc;
   c->amg_nlevel = (int)A->lv.size();
   return MSG_OK;
 }
 
-// Levels l .. of a V-cycle from their right-hand side to their correction, when they are
-// small; *done is left 0 when they are not.
-template <typename T>
 static int cycle_tail(msg_ctx *c, int l, int *done) {
-  constexpr bool F64 = sizeof(T) == 8;
-  using TV = typename std::conditional<F64, double, __nv_bfloat16>::type;
   AmgState *A = S(c);
-  const int nl = (int)A->lv.size() - l;
   *done = 0;
-  if (A->lv[l].n > kTailRows || nl > kTailMax || A->lv.back().n > kTailDense) return MSG_OK;
-  TailArgs<T, TV> a;
-  a.nl = nl;
+  if (!tail_takes(A, l)) return MSG_OK;
+  TailArgs a;
+  a.nl = (int)A->lv.size() - l;
   a.sweeps = std::max(c->prm.amg_sweeps, 0);
-  a.w = (T)c->prm.smooth_omega;
+  a.w = (double)c->prm.smooth_omega;
   a.cinv = A->lv.back().cinv;
-  for (int k = 0; k < nl; ++k) {
+  for (int k = 0; k < a.nl; ++k) {
     const AmgLevel &L = A->lv[l + k];
-    TailLevel<T, TV> &q = a.lv[k];
-    q.n = L.n;
-    q.rowptr = L.rowptr; q.col = L.col;
-    q.rptr = L.rptr; q.rcol = L.rcol; q.pptr = L.pptr; q.pcol = L.pcol;
-    if constexpr (F64) {
-      q.val = L.val; q.diag = L.diag; q.rval = L.rval; q.pval = L.pval;
-      q.x = L.x; q.b = L.b; q.r = L.r; q.x2 = L.x2;
-    } else {
-      q.val = L.val_h; q.diag = L.diag_f; q.rval = L.rval_f; q.pval = L.pval_f;
-      q.x = L.xf; q.b = L.bf; q.r = L.rf; q.x2 = L.x2f;
-    }
+    a.lv[k] = {L.n, L.rowptr, L.col, L.val, L.diag, L.rptr, L.rcol, L.pptr, L.pcol, L.rval, L.pval, L.x, L.b, L.r, L.x2};
   }
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = kTailBlocks; at.val.clusterDim.y = at.val.clusterDim.z = 1;
-  cudaLaunchConfig_t cf = {};
-  cf.gridDim = dim3(kTailBlocks); cf.blockDim = dim3(kTailThreads); cf.stream = c->stream; cf.attrs = &at; cf.numAttrs = 1;
-  MSG_CUDA(cudaLaunchKernelEx(&cf, k_cycle_tail<T, TV>, a));
-  __atomic_fetch_add(&g_launches, 1LL, __ATOMIC_RELAXED);
   *done = 1;
-  return MSG_OK;
+  return tail_launch(c, k_cycle_tail, a, kTailThreads, 0);
+}
+static int cycle_tail_f(msg_ctx *c, int l, int *done) {
+  AmgState *A = S(c);
+  *done = l == A->tail_level;
+  if (!*done) return MSG_OK;
+  A->tail.sweeps = std::max(c->prm.amg_sweeps, 0);
+  A->tail.w = c->prm.smooth_omega;
+  return tail_launch(c, k_cycle_tail_f, A->tail, kTailThreadsF, A->tail.shared);
 }
 
 // One V-cycle z = M^-1 r (x = 0 start, amg_sweeps Jacobi sweeps before and after).
@@ -2108,7 +2455,7 @@ static int vcycle(msg_ctx *c, int l, const double *b, double *x) {
   const int g = nb(n);
   const bool last = (l == (int)A->lv.size() - 1);
   if (l > 0) {
-    int done = 0, rc = cycle_tail<double>(c, l, &done);
+    int done = 0, rc = cycle_tail(c, l, &done);
     if (rc || done) return rc;
   }
   if (last && L.cinv) {
@@ -2172,7 +2519,7 @@ static int vcycle_f(msg_ctx *c, int l, const float *b, float *x) {
   const int g = nb(n);
   const bool last = (l == (int)A->lv.size() - 1);
   {
-    int done = 0, rc = cycle_tail<float>(c, l, &done);
+    int done = 0, rc = cycle_tail_f(c, l, &done);
     if (rc || done) return rc;
   }
   if (last && L.cinv) {
