@@ -965,7 +965,9 @@ __global__ void __launch_bounds__(NT) k_gj(int n, double *M, int *piv_out) {
 // column p and the two rows to swap through shared memory, three barriers, and 2 n^2 FP64
 // operations on one SM (512 cycles at n = 128).  The augmented matrix in global memory took
 // 0.50 ms at 76 rows and 0.84 ms at 128, six barriers and a read and a write of 2 n^2 values
-// from L2 per pivot; here 0.083 ms at 60 rows against 0.279.
+// from L2 per pivot; in registers 0.066 ms at 60 rows and 0.35 at 128 with a branch around
+// each row, 0.055 and 0.26 with all rows updated alike (a row whose factor is zero keeps its
+// bits by selection) and the two rows that change places mended after.
 constexpr int kGjReg = 128;
 template <int NB>
 __global__ void __launch_bounds__(512) k_gj_reg(int n, const int *__restrict__ rowptr, const int *__restrict__ col,
@@ -1015,17 +1017,17 @@ __global__ void __launch_bounds__(512) k_gj_reg(int n, const int *__restrict__ r
     // one warp finds the pivot: largest magnitude (its bits, which order as the values do; a
     // NaN does not count), ties to the lowest row
     if (tr == 0) {
-      unsigned hi = 0, lo = 0;
+      unsigned long long key = 0;   // the top bit is set where there is a candidate
       int row = n;
 #pragma unroll
       for (int i = 0; i < NB; ++i) {
         const int r = tc + 32 * i;
-        if (r >= p && r < n) {
-          const double v = fabs(sc[r]);
-          const unsigned h = (unsigned)__double2hiint(v) | 0x80000000u, l = (unsigned)__double2loint(v);
-          if (v == v && (h > hi || (h == hi && l > lo))) { hi = h; lo = l; row = r; }
-        }
+        const unsigned long long v = (unsigned long long)__double_as_longlong(fabs(sc[r]));
+        const unsigned long long u = r >= p && r < n && v <= 0x7ff0000000000000ull ? v | 0x8000000000000000ull : 0ull;
+        row = u > key ? r : row;
+        key = u > key ? u : key;
       }
+      const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
       const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
       const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
       row = (int)__reduce_min_sync(0xffffffffu, hi == mh && lo == ml ? (unsigned)row : (unsigned)n);
@@ -1040,10 +1042,10 @@ __global__ void __launch_bounds__(512) k_gj_reg(int n, const int *__restrict__ r
     }
     __syncthreads();
     const int piv = s_piv;
+    if (tr == (p & 15) || tr == (piv & 15)) {   // the same in all lanes of the warp
 #pragma unroll
-    for (int i = 0; i < NR; ++i) {
-      const int r = tr + 16 * i;
-      if (r == p || r == piv) {
+      for (int i = 0; i < NR; ++i) {
+        const int r = tr + 16 * i;
 #pragma unroll
         for (int j = 0; j < NB; ++j) {
           if (r == p) sr[tc + 32 * j] = m[i][j];
@@ -1058,24 +1060,28 @@ __global__ void __launch_bounds__(512) k_gj_reg(int n, const int *__restrict__ r
     double prow[NB];
 #pragma unroll
     for (int j = 0; j < NB; ++j) prow[j] = __dmul_rn(j == pb && mine ? 1.0 : sp[tc + 32 * j], pinv);
+    // all rows alike, without branches between them; the two rows that change places after
 #pragma unroll
     for (int i = 0; i < NR; ++i) {
-      const int r = tr + 16 * i;   // the same in all lanes of the warp
-      if (r == p) {
-#pragma unroll
-        for (int j = 0; j < NB; ++j) m[i][j] = prow[j];
-        continue;
-      }
-      double f = sc[r];
-      if (r == piv) {
-        f = sc[p];
-#pragma unroll
-        for (int j = 0; j < NB; ++j) m[i][j] = sr[tc + 32 * j];
-      }
+      const double f = sc[tr + 16 * i];
       if (mine) m[i][pb] = 0.0;
-      if (f != 0.0) {
 #pragma unroll
-        for (int j = 0; j < NB; ++j) m[i][j] = __dsub_rn(m[i][j], __dmul_rn(f, prow[j]));
+      for (int j = 0; j < NB; ++j) {
+        const double v = __dsub_rn(m[i][j], __dmul_rn(f, prow[j]));
+        m[i][j] = f != 0.0 ? v : m[i][j];
+      }
+    }
+    if (tr == (p & 15) || tr == (piv & 15)) {   // the same in all lanes of the warp
+      const double f = sc[p];
+#pragma unroll
+      for (int i = 0; i < NR; ++i) {
+        const int r = tr + 16 * i;
+#pragma unroll
+        for (int j = 0; j < NB; ++j) {
+          const double o = j == pb && mine ? 0.0 : sr[tc + 32 * j];
+          if (r == p) m[i][j] = prow[j];
+          else if (r == piv) m[i][j] = f != 0.0 ? __dsub_rn(o, __dmul_rn(f, prow[j])) : o;
+        }
       }
     }
   }
