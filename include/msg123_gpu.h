@@ -312,7 +312,7 @@ MSG_API int msg_gpu_convlog(msg_ctx_t *ctx, msg_convrec_t *out, int32_t cap);
  * Result in ms per launch. */
 MSG_API int msg_gpu_kernel_time(msg_ctx_t *ctx, int32_t which, int32_t reps, double *ms_per_launch);
 
-/* AMG hierarchy of the last setup (structural tests): level 0 is the Jacobian in CSR
+/* AMG hierarchy of the last setup (structural tests): level 0 is the current Jacobian in CSR
  * form; level l > 0 holds its operator (off-diagonals CSR, 0-based columns, diagonal
  * apart as in array_var(l)%{dmat,lumat}), the prolongation P from it to level l-1 and
  * the aggregate of every level l-1 row (-1: none).  No counterpart returns these in

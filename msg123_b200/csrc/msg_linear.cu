@@ -242,8 +242,8 @@ __global__ void k_bicg_p(int n, const double *pin, double *p, const double *r, c
 
 // Sums of NV values over groups of 256 consecutive elements, one partial per group (the order
 // of block_sum): a block takes kGr groups, so a thread has that many loads in flight and one
-// barrier serves them all.  One group per block, with two barriers per value, left k_dot2 at
-// a third of the copy rate.
+// barrier serves them all.  One group per block, with two barriers per value, left the
+// two-dot pass at a third of the copy rate.
 constexpr int kGr = 4;
 static int ngroups(int n) { return (n + 255) / 256; }
 static int gblk(int n) { return (ngroups(n) + kGr - 1) / kGr; }
@@ -720,8 +720,8 @@ int scale(msg_ctx *c, double *y, double a, int n) {
 // the two that it waits for, so they progress however many of them are resident; a wait
 // that lasts 1 s is given up and reported, and the sweep ends with wrong values.
 //
-// 96 x 81 x 40 cells: factor 1390 -> 134 us, solve 2000 -> 226 us against a grid-wide barrier
-// per plane of cells (4.6 to 6.5 us each); 20 x 20 x 50: 165 -> 40 and 195 -> 83 us against
+// 96 x 81 x 40 cells: factor 1390 -> 134 us, solve 2000 -> 214 us against a grid-wide barrier
+// per plane of cells (4.6 to 6.5 us each); 20 x 20 x 50: 165 -> 40 and 195 -> 76 us against
 // one block for the grid, whose scattered loads took 1.1 to 1.9 us per plane.  A step is now
 // about 250 ns (the division 66 of them), a hop from tile to tile about 1 us; looking at a
 // slot more than one step ahead (kWAhead) only lengthens the lag between tiles (267 us per
