@@ -2323,7 +2323,6 @@ static bool tail_takes(const AmgState *A, int l) {
 static int tail_setup(msg_ctx *c) {
   AmgState *A = S(c);
   int l = 1, rc;
-  A->tail_level = -1;
   while (l < (int)A->lv.size() && !tail_takes(A, l)) ++l;
   if (c->prm.precision != 1 || l >= (int)A->lv.size()) return MSG_OK;
   TailArgsF &a = A->tail;
@@ -2394,6 +2393,7 @@ int amg_setup(msg_ctx *c) {
   cudaStream_t s = c->stream;
   for (size_t l = 1; l < A->lv.size(); ++l) free_level(A, A->lv[l], s);
   A->lv.clear();
+  A->tail_level = -1;
   // reset the arena; enlarge it first when the previous build did not fit
   if (A->arena_spill) {
     const size_t need = A->arena_cap + A->arena_spill;   // what did not fit beside a full arena
