@@ -312,6 +312,13 @@ MSG_API int msg_gpu_convlog(msg_ctx_t *ctx, msg_convrec_t *out, int32_t cap);
  * Result in ms per launch. */
 MSG_API int msg_gpu_kernel_time(msg_ctx_t *ctx, int32_t which, int32_t reps, double *ms_per_launch);
 
+/* Test hooks: failures made on the host, so that what follows them is tested without a fault on
+ * the GPU.  value 0 switches a hook off.
+ * MSG_HOOK_SWEEP_LAUNCH: the value-th DILU sweep from now asks for more shared memory than a
+ * block can have, so that the runtime refuses its launch. */
+enum { MSG_HOOK_SWEEP_LAUNCH = 0, MSG_HOOK_COUNT };
+MSG_API int msg_gpu_test_hook(msg_ctx_t *ctx, int32_t hook, int32_t value);
+
 /* AMG hierarchy of the last setup (structural tests): level 0 is the current Jacobian in CSR
  * form; level l > 0 holds its operator (off-diagonals CSR, 0-based columns, diagonal
  * apart as in array_var(l)%{dmat,lumat}), the prolongation P from it to level l-1 and

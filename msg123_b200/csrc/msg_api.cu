@@ -1187,6 +1187,12 @@ int msg_gpu_set_tuning(msg_ctx_t *c, int32_t blk_cell, int32_t blk_smooth) {
   return MSG_OK;
 }
 
+int msg_gpu_test_hook(msg_ctx_t *c, int32_t hook, int32_t value) {
+  if (!c || hook < 0 || hook >= MSG_HOOK_COUNT || value < 0) { set_error("test_hook: bad arguments"); return MSG_ERR_ARG; }
+  c->hook[hook] = value;
+  return MSG_OK;
+}
+
 // Ensemble driver: worker threads take members from a shared queue and advance each
 // for nsteps accepted steps on the member's own stream, so members of uneven size and
 // uneven Newton counts keep the GPU busy together.

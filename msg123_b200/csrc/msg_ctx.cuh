@@ -82,7 +82,7 @@ struct msg_ctx {
   unsigned box_token;
   // ---- DILU sweeps (msg_linear.cu): tile order, ticket counter, hand-over slots between tiles
   int *wave_order;
-  unsigned *wave_ticket, wave_sweeps;            // ticket and error word; sweeps launched so far
+  unsigned *wave_ticket;                         // ticket and error word
   void *wave_slots;
   int wave_tiles;
   int *wave_err;                                 // pinned: a wait between tiles ran out
@@ -114,9 +114,14 @@ struct msg_ctx {
   // ---- launch shapes chosen by the autotuner (kernels without reductions only) ---------------
   int blk_cell;      // block size of the van Genuchten / storage pass (k_cell)
   int blk_smooth;    // block size of the level-1 Jacobi / residual passes of the V-cycle
+  // ---- tests (msg_gpu_test_hook) -------------------------------------------------------------
+  int hook[MSG_HOOK_COUNT];
 };
 
 namespace msg {
+
+// Counts a hook down; true in the call that it is due in.
+inline bool hook_due(msg_ctx *c, int hook) { return c->hook[hook] > 0 && --c->hook[hook] == 0; }
 
 // ---- msg_physics.cu ---------------------------------------------------------------------------
 int build_connectivity(msg_ctx *c, const msg_grid_t *g);

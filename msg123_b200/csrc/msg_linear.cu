@@ -717,7 +717,8 @@ int scale(msg_ctx *c, double *y, double a, int n) {
 // value in global memory: an empty slot holds a signalling NaN, which no arithmetic result
 // is, so the value is its own flag and needs no fence; the reader empties it again for the
 // next sweep.  Blocks take their tiles from a counter in an order in which a tile follows
-// the two that it waits for, so they progress however many of them are resident; a wait
+// the two that it waits for, so they progress however many of them are resident (the last
+// block sets the counter back, so nothing on the host has to follow it); a wait
 // that lasts 1 s is given up and reported, and the sweep ends with wrong values.
 //
 // 96 x 81 x 40 cells: factor 1390 -> 134 us, solve 2000 -> 214 us against a grid-wide barrier
@@ -737,8 +738,7 @@ struct SweepArgs {
   Geo3 g;
   int tx;                        // tiles in x
   const int *order;              // tile (x + tx * y) of each ticket
-  unsigned *ticket;
-  unsigned base;                 // ticket of this sweep's first tile
+  unsigned *ticket;              // 0 between sweeps
   unsigned long long *west, *north;   // slots: west[(tile * nz + z) * kWY + ly], north[.. * kWX + lx]
   int *err, *err_host;           // a wait was given up: device word, pinned word
   const double *dmat, *lu;
@@ -798,7 +798,7 @@ __global__ void __launch_bounds__(kWThreads) k_sweep(SweepArgs a) {
   __shared__ double ex[2][kWY + 1][kWPitch];     // step parity; row and column 0: the tiles before
   __shared__ int s_tile;
   const int t = threadIdx.x, wp = t >> 5, ln = t & 31;
-  if (t == 0) s_tile = a.order[atomicAdd(a.ticket, 1u) - a.base];
+  if (t == 0) s_tile = a.order[atomicInc(a.ticket, gridDim.x - 1)];   // back at 0 with the last block
   __syncthreads();
   const int tile = s_tile, bx = tile % a.tx, by = tile / a.tx;
   const int nx = a.g.nx, ny = a.g.ny, nz = a.g.nz, nxy = a.g.nxy;
@@ -960,7 +960,6 @@ int build_wavefront(msg_ctx *c) {
   c->wave_err = reinterpret_cast<int *>(c->hpin + kRedBlocks * 8 + 8);
   *c->wave_err = 0;
   c->wave_tiles = nt;
-  c->wave_sweeps = 0;
   std::vector<unsigned long long> empty(nslot, kWEmpty);
   MSG_CUDA(cudaMemcpyAsync(c->wave_slots, empty.data(), nslot * 8, cudaMemcpyHostToDevice, c->stream));
   MSG_CUDA(cudaMemcpyAsync(c->wave_order, order.data(), (size_t)nt * 4, cudaMemcpyHostToDevice, c->stream));
@@ -985,10 +984,10 @@ static int launch_sweep(msg_ctx *c, const double *b, double *x) {
   if (rc) return rc;
   unsigned long long *slots = (unsigned long long *)c->wave_slots;
   SweepArgs a{geo3(c), (c->nx + kWX - 1) / kWX, c->wave_order, c->wave_ticket,
-              c->wave_sweeps * (unsigned)c->wave_tiles, slots, slots + (size_t)c->wave_tiles * c->nz * kWY,
+              slots, slots + (size_t)c->wave_tiles * c->nz * kWY,
               (int *)c->wave_ticket + 1, c->wave_err, c->dmat, c->lu, c->dilu_d, b, x};
-  k_sweep<MODE><<<c->wave_tiles, kWThreads, Sweep<MODE>::smem, c->stream>>>(a);
-  c->wave_sweeps++;
+  const bool refuse = hook_due(c, MSG_HOOK_SWEEP_LAUNCH);   // more shared memory than a block can have
+  k_sweep<MODE><<<c->wave_tiles, kWThreads, Sweep<MODE>::smem + (refuse ? 1 << 20 : 0), c->stream>>>(a);
   MSG_CHECK_LAUNCH();
   return MSG_OK;
 }

@@ -63,6 +63,7 @@ def load_library():
     L.msg_gpu_set_timing.argtypes = [vp, C.c_int32]
     L.msg_gpu_kernel_time.argtypes = [vp, C.c_int32, C.c_int32, abi.PD]
     L.msg_gpu_set_tuning.argtypes = [vp, C.c_int32, C.c_int32]
+    L.msg_gpu_test_hook.argtypes = [vp, C.c_int32, C.c_int32]
     L.msg_gpu_amg_nlevel.argtypes = [vp]
     L.msg_gpu_amg_level_sizes.argtypes = [vp, C.c_int32, abi.PI, abi.PI, abi.PI]
     L.msg_gpu_amg_level.argtypes = [vp, C.c_int32, abi.PI, abi.PI, abi.PD, abi.PD, abi.PI, abi.PI, abi.PD, abi.PI]
@@ -374,6 +375,10 @@ class GpuSolver:
                                        dptr(d["lumat"]), *args), "amg level")
             levels.append(d)
         return levels
+
+    def test_hook(self, hook, value):
+        """Test hook (abi.HOOK_*): a failure made on the host; value 0 switches it off."""
+        _check(load_library().msg_gpu_test_hook(self.h, int(hook), int(value)), "test_hook")
 
     def set_timing(self, on=True):
         _check(load_library().msg_gpu_set_timing(self.h, int(bool(on))), "set_timing")

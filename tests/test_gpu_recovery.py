@@ -1,0 +1,38 @@
+"""A call that fails on the host's side or gives up a bounded wait leaves a context that works:
+the next call gives the bits of the oracle."""
+import numpy as np
+import pytest
+
+from msg123_b200 import abi
+from msg123_b200.config import make_config
+from oracle.oracle import Oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _system(shape, **kw):
+    """Problem, system at a perturbed head, and the oracle that holds it."""
+    p = make_config("hetero", shape=shape, seed=4, **kw)
+    o = Oracle(p)
+    o.init_state()
+    o.set_state(head_new=p.head0 + 0.01 * np.random.default_rng(7).standard_normal(p.ncalc))
+    sys = o.make_matvec()
+    o.set_system(*sys)
+    return p, o, sys
+
+
+@pytest.mark.parametrize("sweep", [1, 2, 3])
+def test_refused_sweep_launch(sweep):
+    """A DILU sweep (factor, forward, backward) whose launch is refused: the following sweeps
+    take their tiles from the start of the order again."""
+    from msg123_b200.solver import GpuSolver, MsgError
+    p, o, sys = _system((40, 20, 5), precon_type=0)
+    v = np.random.default_rng(1).standard_normal(p.ncalc)
+    with GpuSolver(p) as g:
+        g.set_system(*sys)
+        g.test_hook(abi.HOOK_SWEEP_LAUNCH, sweep)
+        with pytest.raises(MsgError, match="launch"):
+            g.precond(v)
+        for _ in range(2):
+            assert np.array_equal(g.precond(v), o.precond(v))
+    o.close()
