@@ -1176,7 +1176,7 @@ int msg_gpu_kernel_time(msg_ctx_t *c, int32_t which, int32_t reps, double *ms_pe
   MSG_CUDA(cudaEventElapsedTime(&ms, c->ev[5], c->ev[6]));
   *ms_per_launch = (double)ms / reps;
   if (which == 5) return learned_check(c);
-  return MSG_OK;
+  return wave_check(c);
 }
 
 int msg_gpu_set_tuning(msg_ctx_t *c, int32_t blk_cell, int32_t blk_smooth) {

@@ -718,8 +718,10 @@ int scale(msg_ctx *c, double *y, double a, int n) {
 // is, so the value is its own flag and needs no fence; the reader empties it again for the
 // next sweep.  Blocks take their tiles from a counter in an order in which a tile follows
 // the two that it waits for, so they progress however many of them are resident (the last
-// block sets the counter back, so nothing on the host has to follow it); a wait
-// that lasts 1 s is given up and reported, and the sweep ends with wrong values.
+// block sets the counter back, so nothing on the host has to follow it).  A wait is given up
+// after kWLooks looks at its slot (about 2 s; looks, not time, so that a GPU that other
+// processes share, or a debugger stops, does not end it) and reported: the sweep ends with wrong
+// values, the call with an error, and the slots are emptied for the next one.
 //
 // 96 x 81 x 40 cells: factor 1390 -> 134 us, solve 2000 -> 214 us against a grid-wide barrier
 // per plane of cells (4.6 to 6.5 us each); 20 x 20 x 50: 165 -> 40 and 195 -> 76 us against
@@ -733,6 +735,7 @@ constexpr int kWX = 16, kWY = 8, kWCols = kWX * kWY, kWThreads = 2 * kWCols + 32
 // to 7 + 3 steps after it
 constexpr int kWRing = 16, kWFetch = 6, kWAhead = 1, kWPitch = 24;
 constexpr unsigned long long kWEmpty = 0x7ff4a5a5a5a5a5a5ull;   // a signalling NaN
+constexpr unsigned kWLooks = 1u << 22;
 
 struct SweepArgs {
   Geo3 g;
@@ -741,6 +744,8 @@ struct SweepArgs {
   unsigned *ticket;              // 0 between sweeps
   unsigned long long *west, *north;   // slots: west[(tile * nz + z) * kWY + ly], north[.. * kWX + lx]
   int *err, *err_host;           // a wait was given up: device word, pinned word
+  unsigned looks;                // of a wait
+  int withhold;                  // test hook: the tile that hands nothing over (-1: none)
   const double *dmat, *lu;
   double *dd;                    // DILU diagonal (out for factor, in for solve)
   const double *b;
@@ -759,17 +764,12 @@ __device__ __forceinline__ void st_slot(unsigned long long *p, unsigned long lon
 // slot is left empty.
 __device__ __forceinline__ double take_slot(const SweepArgs &a, unsigned long long *p, unsigned long long v, bool &dead) {
   if (v == kWEmpty && !dead) {
-    unsigned long long t0 = 0, t1;
-    for (int it = 0; (v = ld_slot(p)) == kWEmpty; ++it) {
-      if ((it & 1023) == 1023) {
-        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
-        if (!t0) t0 = t1;
-        if (t1 - t0 > 1000000000ull || *(volatile int *)a.err) {
-          *(volatile int *)a.err = 1;
-          *(volatile int *)a.err_host = 1;
-          dead = true;
-          break;
-        }
+    for (unsigned it = 1; (v = ld_slot(p)) == kWEmpty; ++it) {
+      if ((it & 1023) == 0 && (it >= a.looks || *(volatile int *)a.err)) {
+        *(volatile int *)a.err = 1;
+        *(volatile int *)a.err_host = 1;
+        dead = true;
+        break;
       }
     }
   }
@@ -813,10 +813,10 @@ __global__ void __launch_bounds__(kWThreads) k_sweep(SweepArgs a) {
     // ---- the chain: a warp owns 8 x 4 columns
     const int lx = 8 * (wp % (kWX / 8)) + (ln & 7), ly = 4 * (wp / (kWX / 8)) + (ln >> 3);
     const int gx = bx * kWX + lx, gy = by * kWY + ly;
-    const bool col = gx < nx && gy < ny, hx = gx > 0, hy = gy > 0;
+    const bool col = gx < nx && gy < ny, hx = gx > 0, hy = gy > 0, give = col && tile != a.withhold;
     const int layers = col ? nz : 0;
-    unsigned long long *wout = lx == kWX - 1 && gx + 1 < nx && col ? a.west + ((size_t)(tile + 1) * nz) * kWY + ly : nullptr;
-    unsigned long long *nout = ly == kWY - 1 && gy + 1 < ny && col ? a.north + ((size_t)(tile + a.tx) * nz) * kWX + lx : nullptr;
+    unsigned long long *wout = lx == kWX - 1 && gx + 1 < nx && give ? a.west + ((size_t)(tile + 1) * nz) * kWY + ly : nullptr;
+    unsigned long long *nout = ly == kWY - 1 && gy + 1 < ny && give ? a.north + ((size_t)(tile + a.tx) * nz) * kWX + lx : nullptr;
     const bool edge = wout || nout;
     size_t i = col ? first(gx, gy) : 0;
     int z = -lx - ly;
@@ -943,7 +943,21 @@ __global__ void __launch_bounds__(kWThreads) k_sweep(SweepArgs a) {
   }
 }
 
-// Tile order, slots (all empty), ticket counter and error words of the sweeps.
+__global__ void k_slots_empty(size_t n, unsigned long long *p) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) p[i] = kWEmpty;
+}
+
+// All slots empty, ticket counter and error words zero; no sweep may be under way.
+static int wave_reset(msg_ctx *c) {
+  k_slots_empty<<<kRedBlocks, 256, 0, c->stream>>>((size_t)c->wave_tiles * c->nz * (kWX + kWY), (unsigned long long *)c->wave_slots);
+  MSG_CHECK_LAUNCH();
+  MSG_CUDA(cudaMemsetAsync(c->wave_ticket, 0, 8, c->stream));
+  MSG_CUDA(cudaStreamSynchronize(c->stream));
+  *(volatile int *)c->wave_err = 0;
+  return MSG_OK;
+}
+
+// Tile order, slots, ticket counter and error words of the sweeps.
 int build_wavefront(msg_ctx *c) {
   const int tx = (c->nx + kWX - 1) / kWX, ty = (c->ny + kWY - 1) / kWY, nt = tx * ty;
   std::vector<int> order;
@@ -960,22 +974,20 @@ int build_wavefront(msg_ctx *c) {
   c->wave_err = reinterpret_cast<int *>(c->hpin + kRedBlocks * 8 + 8);
   *c->wave_err = 0;
   c->wave_tiles = nt;
-  std::vector<unsigned long long> empty(nslot, kWEmpty);
-  MSG_CUDA(cudaMemcpyAsync(c->wave_slots, empty.data(), nslot * 8, cudaMemcpyHostToDevice, c->stream));
   MSG_CUDA(cudaMemcpyAsync(c->wave_order, order.data(), (size_t)nt * 4, cudaMemcpyHostToDevice, c->stream));
-  MSG_CUDA(cudaMemsetAsync(c->wave_ticket, 0, 8, c->stream));
-  MSG_CUDA(cudaStreamSynchronize(c->stream));
-  return MSG_OK;
+  return wave_reset(c);   // and waits for the copy
 }
 
 // A sweep that gave up a wait has said so in wave_err (host memory); looked at after every
-// host wait on the stream.  The slots are then in an unknown state, so no sweep runs again.
+// host wait on the stream and before every sweep.  The call that finds it fails; the sweeps
+// still queued end at once (they see the device word), and the next call starts clean.
 int wave_check(msg_ctx *c) {
-  if (c->wave_err && *(volatile int *)c->wave_err) {
-    set_error("DILU sweep: a wait between tiles ran out");
-    return MSG_ERR_CUDA;
-  }
-  return MSG_OK;
+  if (!c->wave_err || !*(volatile int *)c->wave_err) return MSG_OK;
+  MSG_CUDA(cudaStreamSynchronize(c->stream));
+  int rc = wave_reset(c);
+  if (rc) return rc;
+  set_error("DILU sweep: a wait between tiles ran out");
+  return MSG_ERR_CUDA;
 }
 
 template <int MODE>
@@ -985,7 +997,12 @@ static int launch_sweep(msg_ctx *c, const double *b, double *x) {
   unsigned long long *slots = (unsigned long long *)c->wave_slots;
   SweepArgs a{geo3(c), (c->nx + kWX - 1) / kWX, c->wave_order, c->wave_ticket,
               slots, slots + (size_t)c->wave_tiles * c->nz * kWY,
-              (int *)c->wave_ticket + 1, c->wave_err, c->dmat, c->lu, c->dilu_d, b, x};
+              (int *)c->wave_ticket + 1, c->wave_err, kWLooks, -1, c->dmat, c->lu, c->dilu_d, b, x};
+  if (c->hook[MSG_HOOK_SWEEP_WITHHOLD] > 0) {
+    a.withhold = c->hook[MSG_HOOK_SWEEP_WITHHOLD] - 1;
+    a.looks = 1u << 12;
+    c->hook[MSG_HOOK_SWEEP_WITHHOLD] = 0;
+  }
   const bool refuse = hook_due(c, MSG_HOOK_SWEEP_LAUNCH);   // more shared memory than a block can have
   k_sweep<MODE><<<c->wave_tiles, kWThreads, Sweep<MODE>::smem + (refuse ? 1 << 20 : 0), c->stream>>>(a);
   MSG_CHECK_LAUNCH();

@@ -36,3 +36,27 @@ def test_refused_sweep_launch(sweep):
         for _ in range(2):
             assert np.array_equal(g.precond(v), o.precond(v))
     o.close()
+
+
+@pytest.mark.parametrize("shape,tile", [((40, 20, 5), 1), ((40, 20, 5), 5), ((33, 25, 2), 4)], ids=str)
+def test_wait_between_tiles_runs_out(shape, tile):
+    """A tile that hands nothing over: the call reports the wait that ran out, through the
+    preconditioner and through the solver (whose host waits look at another word), and the same
+    context goes on with right values."""
+    from msg123_b200.solver import GpuSolver, MsgError
+    p, o, sys = _system(shape, precon_type=0)
+    v = np.random.default_rng(1).standard_normal(p.ncalc)
+    with GpuSolver(p) as g:
+        g.set_system(*sys)
+        good = g.solve_linalg(float(sys[2] @ sys[2]), 1e-8, np.zeros(p.ncalc))
+        for _ in range(2):
+            g.test_hook(abi.HOOK_SWEEP_WITHHOLD, tile)
+            with pytest.raises(MsgError, match="wait between tiles"):
+                g.precond(v)
+            assert np.array_equal(g.precond(v), o.precond(v))
+        g.test_hook(abi.HOOK_SWEEP_WITHHOLD, tile)
+        with pytest.raises(MsgError, match="wait between tiles"):
+            g.solve_linalg(float(sys[2] @ sys[2]), 1e-8, np.zeros(p.ncalc))
+        again = g.solve_linalg(float(sys[2] @ sys[2]), 1e-8, np.zeros(p.ncalc))
+        assert all(np.array_equal(a, b) for a, b in zip(good, again))
+    o.close()
