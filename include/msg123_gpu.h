@@ -317,8 +317,10 @@ MSG_API int msg_gpu_kernel_time(msg_ctx_t *ctx, int32_t which, int32_t reps, dou
  * MSG_HOOK_SWEEP_LAUNCH: the value-th DILU sweep from now asks for more shared memory than a
  * block can have, so that the runtime refuses its launch.
  * MSG_HOOK_SWEEP_WITHHOLD: in the next DILU sweep the value-th tile (of 16 x 8 columns, x first)
- * hands nothing over, and the tiles that wait for it give up soon. */
-enum { MSG_HOOK_SWEEP_LAUNCH = 0, MSG_HOOK_SWEEP_WITHHOLD = 1, MSG_HOOK_COUNT };
+ * hands nothing over, and the tiles that wait for it give up soon.
+ * MSG_HOOK_AMG_ALLOC: hierarchy builds take their memory from the pool, and the value-th
+ * allocation from now asks for more than any device has. */
+enum { MSG_HOOK_SWEEP_LAUNCH = 0, MSG_HOOK_SWEEP_WITHHOLD = 1, MSG_HOOK_AMG_ALLOC = 2, MSG_HOOK_COUNT };
 MSG_API int msg_gpu_test_hook(msg_ctx_t *ctx, int32_t hook, int32_t value);
 
 /* AMG hierarchy of the last setup (structural tests): level 0 is the current Jacobian in CSR

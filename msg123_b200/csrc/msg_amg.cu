@@ -1967,44 +1967,58 @@ __global__ void k_col0(int nnz, const int *offrow1, int *col0) {
 // ---------------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------------
-// Allocation of one hierarchy build: from the arena, else (arena full) from the pool.
+// Allocation of one hierarchy build: from the arena, else (arena full, or a test wants it) from
+// the pool.
+static bool in_arena(const msg_ctx *c, size_t bytes) {
+  const AmgState *A = S(const_cast<msg_ctx *>(c));
+  return A->arena && !c->hook[MSG_HOOK_AMG_ALLOC] && A->arena_used + A->arena_tmp + bytes <= A->arena_cap;
+}
+static int from_pool(msg_ctx *c, void **p, size_t bytes) {
+  const bool armed = c->hook[MSG_HOOK_AMG_ALLOC] > 0, refuse = hook_due(c, MSG_HOOK_AMG_ALLOC);   // more than any device has
+  MSG_CUDA(cudaMallocAsync(p, refuse ? (size_t)1 << 60 : bytes, c->stream));
+  if (!armed) S(c)->arena_spill += bytes;
+  return MSG_OK;
+}
 template <typename T>
 static int halloc(msg_ctx *c, T **p, size_t n) {
   AmgState *A = S(c);
   const size_t bytes = ((n ? n : 1) * sizeof(T) + 255) & ~(size_t)255;
-  if (A->arena && A->arena_used + A->arena_tmp + bytes <= A->arena_cap) {
+  if (in_arena(c, bytes)) {
     *p = reinterpret_cast<T *>(A->arena + A->arena_used);
     A->arena_used += bytes;
     return MSG_OK;
   }
-  A->arena_spill += bytes;
-  MSG_CUDA(cudaMallocAsync((void **)p, bytes, c->stream));
-  return MSG_OK;
+  void *q = nullptr;
+  int rc = from_pool(c, &q, bytes);
+  if (!rc) *p = reinterpret_cast<T *>(q);
+  return rc;
 }
 
 // Temporaries of one level's building, given back together (stream order: the next level's
 // kernels may take the memory over).
 struct Temps {
+  static constexpr int kMax = 32;         // a level takes up to 27
   msg_ctx *c;
-  std::vector<void *> pool;
+  void *pool[kMax];
+  int n = 0;
   explicit Temps(msg_ctx *ctx) : c(ctx) {}
   ~Temps() {
     S(c)->arena_tmp = 0;
-    for (void *q : pool) cudaFreeAsync(q, c->stream);
+    for (int k = 0; k < n; ++k) cudaFreeAsync(pool[k], c->stream);
   }
   template <typename T>
-  int get(T **p, size_t n) {
+  int get(T **p, size_t count) {
     AmgState *A = S(c);
-    const size_t bytes = ((n ? n : 1) * sizeof(T) + 255) & ~(size_t)255;
-    if (A->arena && A->arena_used + A->arena_tmp + bytes <= A->arena_cap) {
+    const size_t bytes = ((count ? count : 1) * sizeof(T) + 255) & ~(size_t)255;
+    if (in_arena(c, bytes)) {
       A->arena_tmp += bytes;
       *p = reinterpret_cast<T *>(A->arena + A->arena_cap - A->arena_tmp);
       return MSG_OK;
     }
-    A->arena_spill += bytes;
-    MSG_CUDA(cudaMallocAsync((void **)p, bytes, c->stream));
-    pool.push_back(*p);
-    return MSG_OK;
+    if (n == kMax) { set_error("AMG build: more than %d temporaries", kMax); return MSG_ERR_STATE; }
+    int rc = from_pool(c, &pool[n], bytes);
+    if (!rc) *p = reinterpret_cast<T *>(pool[n++]);
+    return rc;
   }
 };
 
@@ -2022,6 +2036,17 @@ static void free_level(AmgState *A, AmgLevel &L, cudaStream_t s) {
   for (void *q : p) hfree(A, q, s);
   L = AmgLevel();
 }
+
+// A level on its way: given back unless it gets its place in the hierarchy.
+struct NewLevel : AmgLevel {
+  msg_ctx *c;
+  explicit NewLevel(msg_ctx *ctx) : c(ctx) {}
+  ~NewLevel() { free_level(S(c), *this, c->stream); }
+  void keep() {
+    S(c)->lv.push_back(*this);
+    static_cast<AmgLevel &>(*this) = AmgLevel();
+  }
+};
 
 template <typename T>
 static int dalloc(msg_ctx *c, T **p, size_t n) {
@@ -2112,7 +2137,7 @@ static int coarsen(msg_ctx *c, AmgState *A, int lv, int *made) {
   if ((rc = scan_exclusive(c, cnt, aggid, n, got))) return rc;
   const int nc = got[0];
   if (nc == 0 || nc >= n) return MSG_OK;
-  AmgLevel C;
+  NewLevel C(c);
   C.n = nc;
   if ((rc = halloc(c, &C.agg, n))) return rc;
   if (dia) {
@@ -2140,7 +2165,7 @@ static int coarsen(msg_ctx *c, AmgState *A, int lv, int *made) {
   MSG_CHECK_LAUNCH();
   if ((rc = halloc(c, &C.pptr, n + 1))) return rc;
   if ((rc = scan_exclusive(c, cnt, C.pptr, n, got, ovf_p))) return rc;
-  if (got[1]) { free_level(A, C, s); return MSG_OK; }   // a row beyond kPRowMax
+  if (got[1]) return MSG_OK;              // a row beyond kPRowMax
   const int pnnz = got[0];
   C.pnnz = pnnz;
   if ((rc = halloc(c, &C.pcol, pnnz)) || (rc = halloc(c, &C.pval, pnnz))) return rc;
@@ -2183,7 +2208,7 @@ static int coarsen(msg_ctx *c, AmgState *A, int lv, int *made) {
   Spg ra{C.rptr, C.rcol, C.rval, nullptr, ap.start, ap.len, ap.ccol, ap.cval, 1, nullptr, nullptr, nullptr, nullptr, C.diag};
   if ((rc = spgemm_rows(c, tmp, nc, ra, cnt, ovf))) return rc;
   if ((rc = scan_exclusive(c, ra.len, C.rowptr, nc, got, ovf))) return rc;
-  if (got[1]) { free_level(A, C, s); return MSG_OK; }   // a row beyond kHashMax
+  if (got[1]) return MSG_OK;              // a row beyond kHashMax
   C.nnz = got[0];
   if ((rc = halloc(c, &C.col, C.nnz)) || (rc = halloc(c, &C.val, C.nnz))) return rc;
   if (c->prm.precision == 1) {
@@ -2199,7 +2224,7 @@ static int coarsen(msg_ctx *c, AmgState *A, int lv, int *made) {
   k_spg_pack<<<(8 * (long long)nc + 255) / 256, 256, 0, s>>>(nc, ra.start, C.rowptr, ra.ccol, ra.cval, C.diag, C.col,
                                                             C.val, C.val_h, C.diag_f);
   MSG_CHECK_LAUNCH();
-  A->lv.push_back(C);
+  C.keep();
   *made = 1;
   return MSG_OK;
 }
@@ -2213,8 +2238,8 @@ static int dense_inverse(msg_ctx *c, AmgLevel &L) {
     if ((rc = halloc(c, &L.cinv, (size_t)n * n))) return rc;
     return launch_gj_reg(n, L.rowptr, L.col, L.val, L.diag, nullptr, L.cinv, s);
   }
-  if ((rc = halloc(c, &M, (size_t)n * 2 * n))) return rc;
-  if ((rc = halloc(c, &piv, 1))) return rc;
+  Temps tmp(c);
+  if ((rc = tmp.get(&M, (size_t)n * 2 * n)) || (rc = tmp.get(&piv, 1))) return rc;
   if ((rc = halloc(c, &L.cinv, (size_t)n * n))) return rc;
   k_dense_fill<<<n, 256, 0, s>>>(n, L.rowptr, L.col, L.val, L.diag, M);
   MSG_CHECK_LAUNCH();
@@ -2233,8 +2258,6 @@ static int dense_inverse(msg_ctx *c, AmgLevel &L) {
   }
   k_dense_extract<<<n, 256, 0, s>>>(n, M, L.cinv);
   MSG_CHECK_LAUNCH();
-  hfree(S(c), M, s);
-  hfree(S(c), piv, s);
   return MSG_OK;
 }
 
@@ -2386,14 +2409,18 @@ static int tail_setup(msg_ctx *c) {
   return MSG_OK;
 }
 
-int amg_setup(msg_ctx *c) {
-  int rc;
-  if ((rc = amg_state(c))) return rc;
+static void drop_levels(msg_ctx *c) {
   AmgState *A = S(c);
-  cudaStream_t s = c->stream;
-  for (size_t l = 1; l < A->lv.size(); ++l) free_level(A, A->lv[l], s);
+  for (size_t l = 1; l < A->lv.size(); ++l) free_level(A, A->lv[l], c->stream);
   A->lv.clear();
   A->tail_level = -1;
+  c->amg_nlevel = 0;
+}
+
+static int build_levels(msg_ctx *c) {
+  int rc;
+  AmgState *A = S(c);
+  cudaStream_t s = c->stream;
   // reset the arena; enlarge it first when the previous build did not fit
   if (A->arena_spill) {
     const size_t need = A->arena_cap + A->arena_spill;   // what did not fit beside a full arena
@@ -2421,9 +2448,18 @@ int amg_setup(msg_ctx *c) {
   if (A->lv.size() > 1 && A->lv.back().n <= std::max(c->prm.amg_coarse_max, 1)) {
     if ((rc = dense_inverse(c, A->lv.back()))) return rc;
   }
-  if ((rc = tail_setup(c))) return rc;
-  c->amg_nlevel = (int)A->lv.size();
-  return MSG_OK;
+  return tail_setup(c);
+}
+
+// A build that fails leaves no hierarchy: amg_apply refuses to run and the next assembly builds
+// again, whatever amg_lag says.
+int amg_setup(msg_ctx *c) {
+  int rc;
+  if ((rc = amg_state(c))) return rc;
+  drop_levels(c);
+  if ((rc = build_levels(c))) drop_levels(c);
+  else c->amg_nlevel = (int)S(c)->lv.size();
+  return rc;
 }
 
 static int cycle_tail(msg_ctx *c, int l, int *done) {

@@ -18,10 +18,13 @@ namespace msg {
 void set_error(const char *fmt, ...);
 const char *get_error();
 
+// A failure that the context survives (no memory) is taken from the runtime's record too, where
+// the next launch check would find it again.
 #define MSG_CUDA(call)                                                                  \
   do {                                                                                  \
     cudaError_t e_ = (call);                                                            \
     if (e_ != cudaSuccess) {                                                            \
+      cudaGetLastError();                                                               \
       ::msg::set_error("%s:%d %s: %s", __FILE__, __LINE__, #call, cudaGetErrorString(e_)); \
       return MSG_ERR_CUDA;                                                              \
     }                                                                                   \

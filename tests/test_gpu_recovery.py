@@ -60,3 +60,63 @@ def test_wait_between_tiles_runs_out(shape, tile):
         again = g.solve_linalg(float(sys[2] @ sys[2]), 1e-8, np.zeros(p.ncalc))
         assert all(np.array_equal(a, b) for a, b in zip(good, again))
     o.close()
+
+
+def _pool_bytes():
+    """Bytes handed out by the device's default memory pool (cudaMemPoolAttrUsedMemCurrent)."""
+    import ctypes as C
+    from msg123_b200.solver import load_library
+    load_library()
+    rt, pool, used = C.CDLL("libcudart.so.12"), C.c_void_p(), C.c_uint64()
+    assert rt.cudaDeviceSynchronize() == 0
+    assert rt.cudaDeviceGetDefaultMemPool(C.byref(pool), 0) == 0
+    assert rt.cudaMemPoolGetAttribute(pool, 7, C.byref(used)) == 0
+    return used.value
+
+
+@pytest.mark.parametrize("precision,coarse", [(0, 16), (1, 16), (0, 200)])
+def test_failed_hierarchy_build(precision, coarse):
+    """No memory at any of a build's allocations: set_system fails, the preconditioner refuses to
+    run on what there is, nothing stays allocated, and the next call of a run that would keep its
+    hierarchy for several steps (amg_lag) builds one."""
+    from msg123_b200.solver import GpuSolver, MsgError
+    kw = dict(precon_type=1, ref_quirks=0, amg_coarse_max=coarse, amg_lag=8)
+    p, o, sys = _system((33, 27, 19))
+    v = np.random.default_rng(1).standard_normal(p.ncalc)
+    with GpuSolver(p, precision=precision, **kw) as ref:
+        ref.set_system(*sys)
+        want = ref.precond(v)
+    if precision == 0:
+        oa = Oracle(p, **kw)
+        oa.set_system(*sys)
+        assert np.array_equal(want, oa.precond(v))
+        oa.close()
+    before = _pool_bytes()
+    with GpuSolver(p, precision=precision, **kw) as g:
+        g.init_state()
+        g.set_system(*sys)
+        empty = None
+        for k in range(1, 400):
+            g.test_hook(abi.HOOK_AMG_ALLOC, k)
+            try:
+                g.set_system(*sys)
+            except MsgError as e:
+                assert "memory" in str(e)
+            else:
+                break                       # more than a build's allocations
+            with pytest.raises(MsgError, match="not built"):
+                g.precond(v)
+            empty = empty or _pool_bytes()
+            assert _pool_bytes() == empty, k
+        assert k > 60
+        g.test_hook(abi.HOOK_AMG_ALLOC, 0)
+        g.set_system(*sys)
+        assert np.array_equal(g.precond(v), want)
+        # a step after a build that failed: the hierarchy is built again, lag or not
+        g.test_hook(abi.HOOK_AMG_ALLOC, 30)
+        with pytest.raises(MsgError):
+            g.set_system(*sys)
+        g.calc_numsol()
+        assert g.amg_levels()[1]["n"] > 1
+    assert _pool_bytes() == before
+    o.close()
