@@ -312,6 +312,10 @@ MSG_API int msg_gpu_convlog(msg_ctx_t *ctx, msg_convrec_t *out, int32_t cap);
  * Result in ms per launch. */
 MSG_API int msg_gpu_kernel_time(msg_ctx_t *ctx, int32_t which, int32_t reps, double *ms_per_launch);
 
+/* The exclusive scan of the hierarchy build and of the connectivity, on n <= ncalc host values of
+ * at least 0 (structural tests): out [n + 1] in 32 bits, *total the sum in 64. */
+MSG_API int msg_gpu_scan(msg_ctx_t *ctx, int32_t n, const int32_t *in, int32_t *out, int64_t *total);
+
 /* Test hooks: failures made on the host, so that what follows them is tested without a fault on
  * the GPU.  value 0 switches a hook off.
  * MSG_HOOK_SWEEP_LAUNCH: the value-th DILU sweep from now asks for more shared memory than a
@@ -319,8 +323,11 @@ MSG_API int msg_gpu_kernel_time(msg_ctx_t *ctx, int32_t which, int32_t reps, dou
  * MSG_HOOK_SWEEP_WITHHOLD: in the next DILU sweep the value-th tile (of 16 x 8 columns, x first)
  * hands nothing over, and the tiles that wait for it give up soon.
  * MSG_HOOK_AMG_ALLOC: hierarchy builds take their memory from the pool, and the value-th
- * allocation from now asks for more than any device has. */
-enum { MSG_HOOK_SWEEP_LAUNCH = 0, MSG_HOOK_SWEEP_WITHHOLD = 1, MSG_HOOK_AMG_ALLOC = 2, MSG_HOOK_COUNT };
+ * allocation from now asks for more than any device has.
+ * MSG_HOOK_AMG_PRODUCTS: hierarchy builds find the rows' lengths first where a product of two
+ * operators has more than value products (as where 32-bit offsets or the memory end). */
+enum { MSG_HOOK_SWEEP_LAUNCH = 0, MSG_HOOK_SWEEP_WITHHOLD = 1, MSG_HOOK_AMG_ALLOC = 2, MSG_HOOK_AMG_PRODUCTS = 3,
+       MSG_HOOK_COUNT };
 MSG_API int msg_gpu_test_hook(msg_ctx_t *ctx, int32_t hook, int32_t value);
 
 /* AMG hierarchy of the last setup (structural tests): level 0 is the current Jacobian in CSR

@@ -18,6 +18,7 @@
 #include <cuda_bf16.h>
 #include <vector>
 #include <algorithm>
+#include <climits>
 #include <type_traits>
 
 namespace cg = cooperative_groups;
@@ -600,7 +601,9 @@ __global__ void k_r_rank(int nnz, const int *__restrict__ rptr, const int *__res
 //
 // A row's number of products is known from the row lengths alone, so its result goes to a
 // place of that size (`start`, a scan of the product counts) and its length beside it; no
-// pass counts distinct columns first.  A*P is read back through start and length as it
+// pass counts distinct columns first.  Only where the products are more than 32-bit offsets
+// or the memory hold (with every neighbour strong there are 28 per fine cell on 3 columns) does a
+// first pass over the rows find the lengths, and the places are exact.  A*P is read back through start and length as it
 // stands; the Galerkin operator, which stays, is then copied together, ascending columns,
 // diagonal apart (1.0 if absent).  More than kHashMax distinct columns set *overflow, and the
 // caller stops coarsening at that level.
@@ -613,8 +616,8 @@ struct Spg {
   const int *bs, *bl, *bc;       // B: row starts, lengths (null: bs[j + 1] - bs[j]), columns
   const double *bv;
   int split;                     // C's diagonal goes to cdiag and rows are sorted
-  const int *start;              // place of each row of C
-  int *len, *ccol;
+  const int *cnt, *start;        // products and place of each row of C
+  int *len, *ccol;               // ccol null: lengths only
   double *cval, *cdiag;
   __device__ __forceinline__ int blen(int j) const { return bl ? bl[j] : bs[j + 1] - bs[j]; }
 };
@@ -663,7 +666,7 @@ __global__ void __launch_bounds__(32 * SpgShape<T>::warps) k_spg_row(Spg s, int 
   const int nr = rows ? *nrows : n;
   for (int rid = blockIdx.x * W + w; rid < nr; rid += gridDim.x * W) {
     const int row = rows ? rows[rid] : rid, o = s.start[row];
-    if (T == kTabShort && s.start[row + 1] - o > kShort) {
+    if (T == kTabShort && s.cnt[row] > kShort) {
       if (lane == 0) next[atomicAdd(nnext, 1)] = row;
       continue;
     }
@@ -770,7 +773,7 @@ __global__ void __launch_bounds__(32 * SpgShape<T>::warps) k_spg_row(Spg s, int 
     if (lane < 4) K[u + lane] = 0x7fffffff;   // the rank loop reads four at a time
     __syncwarp();
     // rank sort by column
-    for (int t = lane; t < u; t += 32) {
+    for (int t = lane; t < (s.ccol ? u : 0); t += 32) {
       const int key = K[t];
       int rank = t;
       if (s.split) {
@@ -791,7 +794,8 @@ __global__ void __launch_bounds__(32 * SpgShape<T>::warps) k_spg_row(Spg s, int 
 // A*P on level 1: a thread per cell walks its bands (diagonal first) and the prolongation
 // rows behind them (0 to 3 entries, most one or none) and keeps the columns it has met in
 // shared memory (8 to 10 where there are any; as an unrolled search through registers this
-// took twice as long); the rare row of more than kTU columns works in its place in memory.
+// took twice as long); the rare row of more than kTU columns works in its place in memory, or,
+// where only the length is wanted (COUNT), looks back through the products before.
 constexpr int kTU = 12, kApT = 128;
 __global__ void k_ap_bound_dia(Bands g, const int *__restrict__ pptr, int *cnt) {
   const int ix = blockIdx.x * 32 + threadIdx.x, iy = blockIdx.y * 8 + threadIdx.y, iz = blockIdx.z;
@@ -807,6 +811,7 @@ __global__ void k_ap_bound_dia(Bands g, const int *__restrict__ pptr, int *cnt) 
     }
   cnt[i] = m;
 }
+template <bool COUNT>
 __global__ void __launch_bounds__(kApT) k_ap_dia(Bands g, const int *__restrict__ pptr, const int *__restrict__ pcol,
                                                  const double *__restrict__ pval, const int *__restrict__ start,
                                                  int *len, int *ccol, double *cval) {
@@ -834,29 +839,41 @@ __global__ void __launch_bounds__(kApT) k_ap_dia(Bands g, const int *__restrict_
     fc[e] = q0[e] < q1[e] ? pcol[q0[e]] : -1;
     fv[e] = q0[e] < q1[e] ? __dmul_rn(e == 0 ? g.d[i] : g.lu[(e - 1) * N + i], pval[q0[e]]) : 0.0;
   }
-  const int o = start[i];
+  const int o = COUNT ? 0 : start[i];
   int u = 0;
-  auto add = [&](int cc, double p) {
+  // entry q of prolongation row e
+  auto add = [&](int cc, double p, int e, int q) {
     const int m = min(u, kTU);
     for (int t = 0; t < m; ++t)
       if (uc[t][tt] == cc) { uv[t][tt] = __dadd_rn(uv[t][tt], p); return; }
-    for (int t = kTU; t < u; ++t)
-      if (ccol[o + t] == cc) { cval[o + t] = __dadd_rn(cval[o + t], p); return; }
+    if constexpr (COUNT) {
+      if (u >= kTU) {
+#pragma unroll
+        for (int f = 0; f < 7; ++f)
+          if (f <= e)
+            for (int k = q0[f], end = f == e ? q : q1[f]; k < end; ++k)
+              if (pcol[k] == cc) return;
+      }
+    } else {
+      for (int t = kTU; t < u; ++t)
+        if (ccol[o + t] == cc) { cval[o + t] = __dadd_rn(cval[o + t], p); return; }
+    }
     if (u < kTU) { uc[u][tt] = cc; uv[u][tt] = p; }
-    else { ccol[o + u] = cc; cval[o + u] = p; }
+    else if (!COUNT) { ccol[o + u] = cc; cval[o + u] = p; }
     ++u;
   };
 #pragma unroll
   for (int e = 0; e < 7; ++e) {
     if (fc[e] < 0) continue;
-    add(fc[e], fv[e]);
+    add(fc[e], fv[e], e, q0[e]);
     if (q0[e] + 1 < q1[e]) {
       const double coef = e == 0 ? g.d[i] : g.lu[(e - 1) * N + i];
-      for (int q = q0[e] + 1; q < q1[e]; ++q) add(pcol[q], __dmul_rn(coef, pval[q]));
+      for (int q = q0[e] + 1; q < q1[e]; ++q) add(pcol[q], __dmul_rn(coef, pval[q]), e, q);
     }
   }
   len[i] = u;
-  for (int t = 0; t < min(u, kTU); ++t) { ccol[o + t] = uc[t][tt]; cval[o + t] = uv[t][tt]; }
+  if constexpr (!COUNT)
+    for (int t = 0; t < min(u, kTU); ++t) { ccol[o + t] = uc[t][tt]; cval[o + t] = uv[t][tt]; }
 }
 
 // The Galerkin rows copied together, eight lanes per row, and their FP32 / BF16 images.
@@ -2020,6 +2037,14 @@ struct Temps {
     if (!rc) *p = reinterpret_cast<T *>(pool[n++]);
     return rc;
   }
+  // columns and values of n entries, together or not at all
+  int entries(int **col, double **val, size_t count) {
+    char *b = nullptr;
+    const size_t v = (count * 8 + 255) & ~(size_t)255;
+    int rc = get(&b, v + count * 4);
+    if (!rc) { *val = reinterpret_cast<double *>(b); *col = reinterpret_cast<int *>(b + v); }
+    return rc;
+  }
 };
 
 // Release a pointer from halloc: arena memory is reclaimed at the next reset.
@@ -2054,28 +2079,43 @@ static int dalloc(msg_ctx *c, T **p, size_t n) {
   return MSG_OK;
 }
 
-// C = A*B into rows of the places `start` (their scan, product counts by `bound`); long rows
-// through the hash kernels.  *ovf: device word set when a row has too many columns.
+// Places and memory of C's rows: of the products' size (their counts in g.cnt), or, when that is
+// too much, of the size that `lengths` finds (into g.len).
+template <typename F>
+static int spgemm_places(msg_ctx *c, Temps &tmp, int n, Spg &g, F lengths) {
+  int rc, got[1], *start = nullptr;
+  long long total = 0;
+  if ((rc = tmp.get(&start, n + 1)) || (rc = tmp.get(&g.len, n))) return rc;
+  g.start = start;
+  if ((rc = scan_exclusive(c, g.cnt, start, n, got, nullptr, nullptr, &total))) return rc;
+  const long long most = c->hook[MSG_HOOK_AMG_PRODUCTS] > 0 ? c->hook[MSG_HOOK_AMG_PRODUCTS] : INT_MAX;
+  if (total <= most && !tmp.entries(&g.ccol, &g.cval, total)) return MSG_OK;
+  if ((rc = lengths()) || (rc = scan_exclusive(c, g.len, start, n, got))) return rc;
+  return tmp.entries(&g.ccol, &g.cval, got[0]);
+}
+
+// C = A*B; long rows through the larger tables.  *ovf: device word set when a row has too many
+// columns.
 static int spgemm_rows(msg_ctx *c, Temps &tmp, int n, Spg &g, int *cnt, int *ovf) {
   cudaStream_t s = c->stream;
-  int rc, total = 0, *start = nullptr, *longrows = nullptr, *biggest = nullptr, *nl = nullptr;
+  int rc, *longrows = nullptr, *biggest = nullptr, *nl = nullptr;
   k_spg_bound<<<(8 * (long long)n + 255) / 256, 256, 0, s>>>(n, g, cnt);
   MSG_CHECK_LAUNCH();
-  if ((rc = tmp.get(&start, n + 1)) || (rc = tmp.get(&longrows, n)) || (rc = tmp.get(&biggest, n)) ||
-      (rc = tmp.get(&nl, 2)) || (rc = tmp.get(&g.len, n)))
-    return rc;
-  MSG_CUDA(cudaMemsetAsync(nl, 0, 8, s));
-  if ((rc = scan_exclusive(c, cnt, start, n, &total))) return rc;
-  if ((rc = tmp.get(&g.ccol, total)) || (rc = tmp.get(&g.cval, total))) return rc;
-  g.start = start;
-  k_spg_row<kTabShort><<<(n + 3) / 4, 128, 0, s>>>(g, n, nullptr, nullptr, longrows, nl, nullptr);
-  MSG_CHECK_LAUNCH();
-  // the counts of the long rows stay on the device: grids that fill the chip walk them
-  k_spg_row<kTabMid><<<std::min((n + 3) / 4, 12 * kNumSM), 128, 0, s>>>(g, n, nl, longrows, biggest, nl + 1, nullptr);
-  MSG_CHECK_LAUNCH();
-  k_spg_row<kTabMax><<<std::min((n + 2) / 3, 4 * kNumSM), 96, 0, s>>>(g, n, nl + 1, biggest, nullptr, nullptr, ovf);
-  MSG_CHECK_LAUNCH();
-  return MSG_OK;
+  g.cnt = cnt;
+  if ((rc = tmp.get(&longrows, n)) || (rc = tmp.get(&biggest, n)) || (rc = tmp.get(&nl, 2))) return rc;
+  auto rows = [&]() -> int {
+    MSG_CUDA(cudaMemsetAsync(nl, 0, 8, s));
+    k_spg_row<kTabShort><<<(n + 3) / 4, 128, 0, s>>>(g, n, nullptr, nullptr, longrows, nl, nullptr);
+    MSG_CHECK_LAUNCH();
+    // the counts of the long rows stay on the device: grids that fill the chip walk them
+    k_spg_row<kTabMid><<<std::min((n + 3) / 4, 12 * kNumSM), 128, 0, s>>>(g, n, nl, longrows, biggest, nl + 1, nullptr);
+    MSG_CHECK_LAUNCH();
+    k_spg_row<kTabMax><<<std::min((n + 2) / 3, 4 * kNumSM), 96, 0, s>>>(g, n, nl + 1, biggest, nullptr, nullptr, ovf);
+    MSG_CHECK_LAUNCH();
+    return MSG_OK;
+  };
+  if ((rc = spgemm_places(c, tmp, n, g, rows))) return rc;
+  return rows();
 }
 
 // Build level lv+1 from level lv; returns 1 when a coarser level was made, 0 otherwise.
@@ -2189,23 +2229,25 @@ static int coarsen(msg_ctx *c, AmgState *A, int lv, int *made) {
   k_r_rank<<<nb(pnnz), kThreads, 0, s>>>(pnnz, C.rptr, trow, tcol, tval, C.rcol, C.rval, C.rval_f);
   MSG_CHECK_LAUNCH();
   // AP = A*P (diagonal first)
-  Spg ap{F.rowptr, F.col, F.val, F.diag, C.pptr, nullptr, C.pcol, C.pval, 0, nullptr, nullptr, nullptr, nullptr, nullptr};
+  Spg ap{F.rowptr, F.col, F.val, F.diag, C.pptr, nullptr, C.pcol, C.pval, 0};
   if (dia) {
-    int *start = nullptr;
     k_ap_bound_dia<<<tg, tb, 0, s>>>(g, C.pptr, cnt);
     MSG_CHECK_LAUNCH();
-    if ((rc = tmp.get(&start, n + 1)) || (rc = tmp.get(&ap.len, n))) return rc;
-    if ((rc = scan_exclusive(c, cnt, start, n, got))) return rc;
-    if ((rc = tmp.get(&ap.ccol, got[0])) || (rc = tmp.get(&ap.cval, got[0]))) return rc;
-    ap.start = start;
-    k_ap_dia<<<dim3(tg.x, (c->ny + kApT / 32 - 1) / (kApT / 32), tg.z), dim3(32, kApT / 32), 0, s>>>(g, C.pptr, C.pcol, C.pval, start, ap.len, ap.ccol, ap.cval);
-    MSG_CHECK_LAUNCH();
+    ap.cnt = cnt;
+    auto rows = [&](auto count) -> int {
+      k_ap_dia<decltype(count)::value><<<dim3(tg.x, (c->ny + kApT / 32 - 1) / (kApT / 32), tg.z), dim3(32, kApT / 32), 0, s>>>(
+          g, C.pptr, C.pcol, C.pval, ap.start, ap.len, ap.ccol, ap.cval);
+      MSG_CHECK_LAUNCH();
+      return MSG_OK;
+    };
+    if ((rc = spgemm_places(c, tmp, n, ap, [&] { return rows(std::true_type()); })) || (rc = rows(std::false_type()))) return rc;
   } else if ((rc = spgemm_rows(c, tmp, n, ap, cnt, ovf))) {
     return rc;
   }
   // A_c = R * AP, diagonal split off
   if ((rc = halloc(c, &C.diag, nc)) || (rc = halloc(c, &C.rowptr, nc + 1))) return rc;
-  Spg ra{C.rptr, C.rcol, C.rval, nullptr, ap.start, ap.len, ap.ccol, ap.cval, 1, nullptr, nullptr, nullptr, nullptr, C.diag};
+  Spg ra{C.rptr, C.rcol, C.rval, nullptr, ap.start, ap.len, ap.ccol, ap.cval, 1};
+  ra.cdiag = C.diag;
   if ((rc = spgemm_rows(c, tmp, nc, ra, cnt, ovf))) return rc;
   if ((rc = scan_exclusive(c, ra.len, C.rowptr, nc, got, ovf))) return rc;
   if (got[1]) return MSG_OK;              // a row beyond kHashMax

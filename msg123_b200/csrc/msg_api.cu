@@ -1187,6 +1187,21 @@ int msg_gpu_set_tuning(msg_ctx_t *c, int32_t blk_cell, int32_t blk_smooth) {
   return MSG_OK;
 }
 
+int msg_gpu_scan(msg_ctx_t *c, int32_t n, const int32_t *in, int32_t *out, int64_t *total) {
+  if (!c || n < 1 || n > c->N || !in || !out || !total) { set_error("scan: bad arguments"); return MSG_ERR_ARG; }
+  int *d = nullptr, got[1];
+  long long wide = 0;
+  ALLOC(d, ((size_t)2 * n + 1) * 4);
+  cudaError_t e = cudaMemcpyAsync(d, in, (size_t)n * 4, cudaMemcpyHostToDevice, c->stream);
+  int rc = e == cudaSuccess ? scan_exclusive(c, d, d + n, n, got, nullptr, nullptr, &wide) : MSG_OK;
+  if (!rc && e == cudaSuccess) e = cudaMemcpyAsync(out, d + n, ((size_t)n + 1) * 4, cudaMemcpyDeviceToHost, c->stream);
+  if (!rc && e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  cudaFree(d);
+  MSG_CUDA(e);
+  *total = wide;
+  return rc;
+}
+
 int msg_gpu_test_hook(msg_ctx_t *c, int32_t hook, int32_t value) {
   if (!c || hook < 0 || hook >= MSG_HOOK_COUNT || value < 0) { set_error("test_hook: bad arguments"); return MSG_ERR_ARG; }
   c->hook[hook] = value;

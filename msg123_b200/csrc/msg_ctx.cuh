@@ -18,6 +18,7 @@ struct DevScalars {
 // Words that a kernel hands to the host: pinned memory, complete when token is the awaited one.
 struct HostBox {
   int v[4];
+  long long total;
   unsigned token;
 };
 
@@ -77,7 +78,8 @@ struct msg_ctx {
   unsigned *res_word, res_token;                 // pinned word behind published results, and its value
   int one_half;                                  // the last solve from x = 0 ended at its first residual norm
   // ---- scans (msg_linear.cu): chunk sums, and the box their totals reach the host in -------
-  int *scan_sums, scan_cap;
+  unsigned *scan_sums;
+  int scan_cap;
   msg::HostBox *box;
   unsigned box_token;
   // ---- DILU sweeps (msg_linear.cu): tile order, ticket counter, hand-over slots between tiles
@@ -220,6 +222,6 @@ int apply_prec(msg_ctx *c, const double *r, double *z);
 // ---- scan (msg_linear.cu) ---------------------------------------------------------------------------
 int scan_reserve(msg_ctx *c, int n);
 int scan_exclusive(msg_ctx *c, const int *in, int *out, int n, int *got, const int *w1 = nullptr,
-                   const int *w2 = nullptr);
+                   const int *w2 = nullptr, long long *wide = nullptr);
 
 }  // namespace msg

@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <atomic>
 #include <vector>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <thread>
@@ -33,27 +34,28 @@ __device__ __forceinline__ void ijk(const Geo3 &g, int i, int &ix, int &iy, int 
 // ---------------------------------------------------------------------------------
 // Exclusive scan of int32 in two passes over chunks of kScanE elements: the chunks' sums,
 // then every block adds up the sums before its own chunk and scans the chunk (int sums are
-// the same in any order).  The last block writes the total behind the output and into the
-// context's box.  A serial pass over the chunk sums by one thread, and a third pass to add
+// the same in any order).  The last block writes the total behind the output and, in 64 bits,
+// into the context's box: a sum that 32 bits do not hold is known as such.  A serial pass over the chunk sums by one thread, and a third pass to add
 // them, took 7 us of the 22 us of a scan of 4.2M elements.
 // ---------------------------------------------------------------------------------
 constexpr int kScanT = 256, kScanU = 16, kScanE = kScanT * kScanU;
 
-__device__ __forceinline__ int scan_block_sum(int v, int *sh) {   // valid in every thread
+template <typename T>
+__device__ __forceinline__ T scan_block_sum(T v, T *sh) {   // valid in every thread
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
   __syncthreads();
-  int r = 0;
+  T r = 0;
 #pragma unroll
   for (int w = 0; w < kScanT / 32; ++w) r += sh[w];
   __syncthreads();
   return r;
 }
 
-__global__ void __launch_bounds__(kScanT) k_scan_sum(const int *__restrict__ in, int n, int *bsum) {
-  __shared__ int sh[kScanT / 32];
+__global__ void __launch_bounds__(kScanT) k_scan_sum(const int *__restrict__ in, int n, unsigned *bsum) {
+  __shared__ unsigned sh[kScanT / 32];
   const int base = blockIdx.x * kScanE;
-  int v = 0;
+  unsigned v = 0;                                        // a chunk's sum is below 2^32
 #pragma unroll
   for (int u = 0; u < kScanU; ++u) {
     const int i = base + u * kScanT + threadIdx.x;
@@ -64,40 +66,41 @@ __global__ void __launch_bounds__(kScanT) k_scan_sum(const int *__restrict__ in,
 }
 
 __global__ void __launch_bounds__(kScanT) k_scan_apply(const int *__restrict__ in, int *out, int n,
-                                                       const int *__restrict__ bsum, const int *w1, const int *w2,
+                                                       const unsigned *__restrict__ bsum, const int *w1, const int *w2,
                                                        HostBox *box, unsigned token) {
-  __shared__ int sh[kScanT / 32];
+  __shared__ unsigned sh[kScanT / 32];
+  __shared__ unsigned long long sh64[kScanT / 32];
   __shared__ int e[kScanE + kScanE / 32];                // one pad word per 32
   const int t = threadIdx.x, base = blockIdx.x * kScanE;
-  int v = 0;
+  unsigned long long v = 0;
   for (int k = t; k < (int)blockIdx.x; k += kScanT) v += bsum[k];
-  const int before = scan_block_sum(v, sh);
+  const unsigned long long before = scan_block_sum(v, sh64);
 #pragma unroll
   for (int u = 0; u < kScanU; ++u) {
     const int k = u * kScanT + t, i = base + k;
     e[k + (k >> 5)] = i < n ? in[i] : 0;
   }
   __syncthreads();
-  int x[kScanU], sum = 0;
+  unsigned x[kScanU], sum = 0;
 #pragma unroll
   for (int u = 0; u < kScanU; ++u) {
     const int k = t * kScanU + u;
     x[u] = sum;
     sum += e[k + (k >> 5)];
   }
-  int inc = sum;
+  unsigned inc = sum;
   for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, inc, o);
+    const unsigned y = __shfl_up_sync(0xffffffffu, inc, o);
     if ((t & 31) >= o) inc += y;
   }
   if ((t & 31) == 31) sh[t >> 5] = inc;
   __syncthreads();
-  int off = before + inc - sum;
+  unsigned off = inc - sum;                              // in the chunk
   for (int w = 0; w < (t >> 5); ++w) off += sh[w];
 #pragma unroll
   for (int u = 0; u < kScanU; ++u) {
     const int k = t * kScanU + u;
-    e[k + (k >> 5)] = off + x[u];
+    e[k + (k >> 5)] = (int)((unsigned)before + off + x[u]);
   }
   __syncthreads();
 #pragma unroll
@@ -106,10 +109,10 @@ __global__ void __launch_bounds__(kScanT) k_scan_apply(const int *__restrict__ i
     if (i < n) out[i] = e[k + (k >> 5)];
   }
   if (blockIdx.x == gridDim.x - 1 && t == kScanT - 1) {
-    const int total = off + sum;
-    out[n] = total;
+    const unsigned long long total = before + (off + sum);
+    out[n] = (int)total;
     if (box) {
-      box->v[0] = total;
+      box->total = (long long)total;
       box->v[1] = w1 ? *w1 : 0;
       box->v[2] = w2 ? *w2 : 0;
       __threadfence_system();
@@ -139,8 +142,9 @@ static int token_wait(msg_ctx *c, const unsigned *at, unsigned token) {
 }
 
 // out[0 .. n]: exclusive scan of in[0 .. n) and, at n, the total.  got, when given, receives
-// the total and the device words w1, w2 (waits for them).
-int scan_exclusive(msg_ctx *c, const int *in, int *out, int n, int *got, const int *w1, const int *w2) {
+// the total and the device words w1, w2 (waits for them).  A total beyond 32 bits is an error
+// unless the caller takes it in `wide`; out is then of no use.
+int scan_exclusive(msg_ctx *c, const int *in, int *out, int n, int *got, const int *w1, const int *w2, long long *wide) {
   const int nb = std::max(1, (n + kScanE - 1) / kScanE);
   if (nb > c->scan_cap) { set_error("scan: %d elements", n); return MSG_ERR_STATE; }
   if (nb > 1) {
@@ -153,7 +157,13 @@ int scan_exclusive(msg_ctx *c, const int *in, int *out, int n, int *got, const i
   if (got) {
     int rc = token_wait(c, &c->box->token, c->box_token);
     if (rc) return rc;
-    got[0] = c->box->v[0];
+    const long long total = c->box->total;
+    if (wide) *wide = total;
+    else if (total > INT_MAX) {
+      set_error("%lld entries do not fit in 32-bit offsets", total);
+      return MSG_ERR_SIZE;
+    }
+    got[0] = (int)total;
     if (w1) got[1] = c->box->v[1];
     if (w2) got[2] = c->box->v[2];
   }

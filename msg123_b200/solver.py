@@ -376,6 +376,15 @@ class GpuSolver:
             levels.append(d)
         return levels
 
+    def scan(self, counts):
+        """Exclusive scan of at most ncalc counts on the GPU: (32-bit sums [n + 1], 64-bit total)."""
+        L = load_library()
+        L.msg_gpu_scan.argtypes = [C.c_void_p, C.c_int32, abi.PI, abi.PI, C.POINTER(C.c_int64)]
+        a = np.ascontiguousarray(counts, dtype=np.int32)
+        out, total = np.empty(a.size + 1, np.int32), C.c_int64()
+        _check(L.msg_gpu_scan(self.h, a.size, iptr(a), iptr(out), C.byref(total)), "scan")
+        return out, total.value
+
     def test_hook(self, hook, value):
         """Test hook (abi.HOOK_*): a failure made on the host; value 0 switches it off."""
         _check(load_library().msg_gpu_test_hook(self.h, int(hook), int(value)), "test_hook")
