@@ -110,6 +110,7 @@ static int nb(int n) { return (n + kThreads - 1) / kThreads; }
 struct Bands {   // level 1
   int nx, ny, nz, nxy, N;
   const double *d, *lu;
+  int y0 = 0, z0 = 0;   // first row and layer of a launch over tiles (level1_tiles)
 };
 __device__ __forceinline__ int band_off(const Bands &g, int d) {
   return d == 0 ? -g.nxy : d == 1 ? -g.nx : d == 2 ? -1 : d == 3 ? 1 : d == 4 ? g.nx : g.nxy;
@@ -126,7 +127,7 @@ __device__ __forceinline__ bool strong_entry(double di, double dj, double lu, do
 }
 // 3D grid of 32 x 8 tiles: mask byte and starting state of each cell.
 __global__ void k_strength_dia(Bands g, double th2, unsigned char *msk, unsigned char *st) {
-  const int ix = blockIdx.x * 32 + threadIdx.x, iy = blockIdx.y * 8 + threadIdx.y, iz = blockIdx.z;
+  const int ix = blockIdx.x * 32 + threadIdx.x, iy = g.y0 + blockIdx.y * 8 + threadIdx.y, iz = g.z0 + blockIdx.z;
   if (ix >= g.nx || iy >= g.ny) return;
   const size_t N = g.N;
   const int i = ix + g.nx * (iy + g.ny * iz);
@@ -798,7 +799,7 @@ __global__ void __launch_bounds__(32 * SpgShape<T>::warps) k_spg_row(Spg s, int 
 // where only the length is wanted (COUNT), looks back through the products before.
 constexpr int kTU = 12, kApT = 128;
 __global__ void k_ap_bound_dia(Bands g, const int *__restrict__ pptr, int *cnt) {
-  const int ix = blockIdx.x * 32 + threadIdx.x, iy = blockIdx.y * 8 + threadIdx.y, iz = blockIdx.z;
+  const int ix = blockIdx.x * 32 + threadIdx.x, iy = g.y0 + blockIdx.y * 8 + threadIdx.y, iz = g.z0 + blockIdx.z;
   if (ix >= g.nx || iy >= g.ny) return;
   const int i = ix + g.nx * (iy + g.ny * iz);
   const bool has[6] = {iz > 0, iy > 0, ix > 0, ix < g.nx - 1, iy < g.ny - 1, iz < g.nz - 1};
@@ -817,7 +818,7 @@ __global__ void __launch_bounds__(kApT) k_ap_dia(Bands g, const int *__restrict_
                                                  int *len, int *ccol, double *cval) {
   __shared__ int uc[kTU][kApT];
   __shared__ double uv[kTU][kApT];
-  const int ix = blockIdx.x * 32 + threadIdx.x, iy = blockIdx.y * (kApT / 32) + threadIdx.y, iz = blockIdx.z;
+  const int ix = blockIdx.x * 32 + threadIdx.x, iy = g.y0 + blockIdx.y * (kApT / 32) + threadIdx.y, iz = g.z0 + blockIdx.z;
   if (ix >= g.nx || iy >= g.ny) return;
   const int tt = threadIdx.y * 32 + threadIdx.x;
   const size_t N = g.N;
@@ -2118,6 +2119,23 @@ static int spgemm_rows(msg_ctx *c, Temps &tmp, int n, Spg &g, int *cnt, int *ovf
   return rows();
 }
 
+// A pass over level 1 in blocks of 32 x `rows` cells of a layer; more launches where the rows or
+// the layers are more than a grid has blocks in y or z.
+template <typename F>
+static int level1_tiles(const Bands &g, int rows, F launch) {
+  constexpr int kMaxYZ = 65535;
+  const int by = (g.ny + rows - 1) / rows;
+  for (int z = 0; z < g.nz; z += kMaxYZ)
+    for (int y = 0; y < by; y += kMaxYZ) {
+      Bands part = g;
+      part.y0 = y * rows;
+      part.z0 = z;
+      launch(dim3((g.nx + 31) / 32, std::min(by - y, kMaxYZ), std::min(g.nz - z, kMaxYZ)), dim3(32, rows), part);
+      MSG_CHECK_LAUNCH();
+    }
+  return MSG_OK;
+}
+
 // Build level lv+1 from level lv; returns 1 when a coarser level was made, 0 otherwise.
 static int coarsen(msg_ctx *c, AmgState *A, int lv, int *made) {
   *made = 0;
@@ -2128,7 +2146,6 @@ static int coarsen(msg_ctx *c, AmgState *A, int lv, int *made) {
   cudaStream_t s = c->stream;
   Temps tmp(c);
   const Bands g{c->nx, c->ny, c->nz, c->nxy, c->N, c->dmat, c->lu};
-  const dim3 tb(32, 8), tg((c->nx + 31) / 32, (c->ny + 7) / 8, c->nz);   // level-1 stencil passes
   const double th = (double)c->prm.amg_theta, th2 = th * th, om = (double)c->prm.jac_omega;
   unsigned char *msk = nullptr, *st = nullptr, *w1b = nullptr;
   int *scol = nullptr, *cnt = nullptr, *aggid = nullptr, *agg2 = nullptr, *words = nullptr;
@@ -2143,8 +2160,7 @@ static int coarsen(msg_ctx *c, AmgState *A, int lv, int *made) {
   // strength and aggregates
   if (dia) {
     if ((rc = tmp.get(&msk, n + 3)) || (rc = tmp.get(&w1b, n + 3))) return rc;
-    k_strength_dia<<<tg, tb, 0, s>>>(g, th2, msk, st);
-    MSG_CHECK_LAUNCH();
+    if ((rc = level1_tiles(g, 8, [&](dim3 tg, dim3 tb, const Bands &part) { k_strength_dia<<<tg, tb, 0, s>>>(part, th2, msk, st); }))) return rc;
   } else {
     if ((rc = tmp.get(&scol, F.nnz)) || (rc = tmp.get(&w1, n)) || (rc = tmp.get(&tdm, n)) || (rc = tmp.get(&prow, n)))
       return rc;
@@ -2231,14 +2247,12 @@ static int coarsen(msg_ctx *c, AmgState *A, int lv, int *made) {
   // AP = A*P (diagonal first)
   Spg ap{F.rowptr, F.col, F.val, F.diag, C.pptr, nullptr, C.pcol, C.pval, 0};
   if (dia) {
-    k_ap_bound_dia<<<tg, tb, 0, s>>>(g, C.pptr, cnt);
-    MSG_CHECK_LAUNCH();
+    if ((rc = level1_tiles(g, 8, [&](dim3 tg, dim3 tb, const Bands &part) { k_ap_bound_dia<<<tg, tb, 0, s>>>(part, C.pptr, cnt); }))) return rc;
     ap.cnt = cnt;
     auto rows = [&](auto count) -> int {
-      k_ap_dia<decltype(count)::value><<<dim3(tg.x, (c->ny + kApT / 32 - 1) / (kApT / 32), tg.z), dim3(32, kApT / 32), 0, s>>>(
-          g, C.pptr, C.pcol, C.pval, ap.start, ap.len, ap.ccol, ap.cval);
-      MSG_CHECK_LAUNCH();
-      return MSG_OK;
+      return level1_tiles(g, kApT / 32, [&](dim3 tg, dim3 tb, const Bands &part) {
+        k_ap_dia<decltype(count)::value><<<tg, tb, 0, s>>>(part, C.pptr, C.pcol, C.pval, ap.start, ap.len, ap.ccol, ap.cval);
+      });
     };
     if ((rc = spgemm_places(c, tmp, n, ap, [&] { return rows(std::true_type()); })) || (rc = rows(std::false_type()))) return rc;
   } else if ((rc = spgemm_rows(c, tmp, n, ap, cnt, ovf))) {
