@@ -144,13 +144,14 @@ __device__ __forceinline__ float gelu_d(float x) {
 // about three times its 200 MB at the copy rate.
 constexpr int kConvSmem = kHCells * 32 + kWl * 2;
 template <int MODE>
-__global__ void __launch_bounds__(32 * kTY) k_conv(Grid3 g, const __nv_bfloat16 *__restrict__ in,
+__global__ void __launch_bounds__(32 * kTY) k_conv(Grid3 g, int tx, int ty, const __nv_bfloat16 *__restrict__ in,
                                                    const __nv_bfloat16 *__restrict__ W, const float *__restrict__ bias,
                                                    float *z_out, __nv_bfloat16 *a_out, float *out,
                                                    const float *__restrict__ zprev, __nv_bfloat16 *dz_out) {
   extern __shared__ __align__(128) unsigned char smem_tile[];
   const unsigned act = (unsigned)__cvta_generic_to_shared(smem_tile), wts = act + kHCells * 32;
-  const int x0 = blockIdx.x * kTX, y0 = blockIdx.y * kTY, z0 = blockIdx.z * kTZ;
+  const int row = blockIdx.x / tx;       // tiles in one dimension: any shape of grid
+  const int x0 = (blockIdx.x - row * tx) * kTX, y0 = row % ty * kTY, z0 = row / ty * kTZ;
   load_tile<true>(g, in, x0, y0, z0, act);
   for (int e = threadIdx.x; e < kWl / 8; e += blockDim.x) cp16z(tile_addr(wts, e >> 1, e & 1), W + 8 * e, true);
   asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
@@ -459,22 +460,26 @@ static int cnn_reserve(Net &n, int N) {
   return MSG_OK;
 }
 
-static dim3 tiles(const Grid3 &g) {
-  return dim3((g.nx + kTX - 1) / kTX, (g.ny + kTY - 1) / kTY, (g.nz + kTZ - 1) / kTZ);
+struct Tiles {
+  int x, y, n;
+};
+static Tiles tiles(const Grid3 &g) {
+  const int x = (g.nx + kTX - 1) / kTX, y = (g.ny + kTY - 1) / kTY;
+  return Tiles{x, y, x * y * ((g.nz + kTZ - 1) / kTZ)};
 }
 
 static int cnn_forward(Net &n, const Grid3 &g, const __nv_bfloat16 *x) {
   cudaStream_t s = n.stream;
-  const dim3 blocks = tiles(g);
+  const Tiles t = tiles(g);
   const __nv_bfloat16 *in = x;
   for (int l = 0; l < kLayers - 1; ++l) {
-    k_conv<0><<<blocks, 32 * kTY, kConvSmem, s>>>(g, in, n.w16 + (size_t)l * kWl, n.w32 + (size_t)l * kPl + kWl, n.z[l],
-                                     n.a[l + 1], nullptr, nullptr, nullptr);
+    k_conv<0><<<t.n, 32 * kTY, kConvSmem, s>>>(g, t.x, t.y, in, n.w16 + (size_t)l * kWl, n.w32 + (size_t)l * kPl + kWl,
+                                               n.z[l], n.a[l + 1], nullptr, nullptr, nullptr);
     MSG_CHECK_LAUNCH();
     in = n.a[l + 1];
   }
-  k_conv<1><<<blocks, 32 * kTY, kConvSmem, s>>>(g, in, n.w16 + (size_t)3 * kWl, n.w32 + (size_t)3 * kPl + kWl, nullptr, nullptr,
-                                   n.z[3], nullptr, nullptr);
+  k_conv<1><<<t.n, 32 * kTY, kConvSmem, s>>>(g, t.x, t.y, in, n.w16 + (size_t)3 * kWl, n.w32 + (size_t)3 * kPl + kWl,
+                                             nullptr, nullptr, n.z[3], nullptr, nullptr);
   MSG_CHECK_LAUNCH();
   return MSG_OK;
 }
@@ -482,21 +487,21 @@ static int cnn_forward(Net &n, const Grid3 &g, const __nv_bfloat16 *x) {
 // backward from dz (channel 0 = dL/dout) at the output; grad filled
 static int cnn_backward(Net &n, const Grid3 &g, const __nv_bfloat16 *x) {
   cudaStream_t s = n.stream;
-  const dim3 blocks = tiles(g);
-  const int ntiles = (int)(blocks.x * blocks.y * blocks.z), wb = std::min(ntiles, kWgBlocks);
+  const Tiles t = tiles(g);
+  const int wb = std::min(t.n, kWgBlocks);
   __nv_bfloat16 *dz = n.dz, *dzn = n.dz2;
   float *bpart = n.part + (size_t)2 * kWgBlocks * kWl;
   for (int l = kLayers - 1; l >= 0; --l) {
     const __nv_bfloat16 *in = (l == 0) ? x : n.a[l];
-    k_wgrad<<<wb, kWgThreads, kWgSmem, s>>>(g, blocks.x, blocks.y, ntiles, dz, in, n.part, bpart);
+    k_wgrad<<<wb, kWgThreads, kWgSmem, s>>>(g, t.x, t.y, t.n, dz, in, n.part, bpart);
     MSG_CHECK_LAUNCH();
     k_reduce_parts<<<(kWl + 31) / 32, 256, 0, s>>>(2 * wb, n.part, kWl, n.grad + (size_t)l * kPl);
     MSG_CHECK_LAUNCH();
     k_reduce_parts<<<1, 256, 0, s>>>(wb, bpart, kC, n.grad + (size_t)l * kPl + kWl);
     MSG_CHECK_LAUNCH();
     if (l > 0) {
-      k_conv<2><<<blocks, 32 * kTY, kConvSmem, s>>>(g, dz, n.wt16 + (size_t)l * kWl, nullptr, nullptr, nullptr, nullptr,
-                                       n.z[l - 1], dzn);
+      k_conv<2><<<t.n, 32 * kTY, kConvSmem, s>>>(g, t.x, t.y, dz, n.wt16 + (size_t)l * kWl, nullptr, nullptr, nullptr,
+                                                 nullptr, n.z[l - 1], dzn);
       MSG_CHECK_LAUNCH();
       std::swap(dz, dzn);
     }
