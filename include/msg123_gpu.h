@@ -317,7 +317,7 @@ MSG_API int msg_gpu_kernel_time(msg_ctx_t *ctx, int32_t which, int32_t reps, dou
 MSG_API int msg_gpu_scan(msg_ctx_t *ctx, int32_t n, const int32_t *in, int32_t *out, int64_t *total);
 
 /* Test hooks: failures made on the host, so that what follows them is tested without a fault on
- * the GPU.  value 0 switches a hook off.
+ * the GPU, and paths that are otherwise a matter of size.  value 0 switches a hook off.
  * MSG_HOOK_SWEEP_LAUNCH: the value-th DILU sweep from now asks for more shared memory than a
  * block can have, so that the runtime refuses its launch.
  * MSG_HOOK_SWEEP_WITHHOLD: in the next DILU sweep the value-th tile (of 16 x 8 columns, x first)
@@ -325,9 +325,11 @@ MSG_API int msg_gpu_scan(msg_ctx_t *ctx, int32_t n, const int32_t *in, int32_t *
  * MSG_HOOK_AMG_ALLOC: hierarchy builds take their memory from the pool, and the value-th
  * allocation from now asks for more than any device has.
  * MSG_HOOK_AMG_PRODUCTS: hierarchy builds find the rows' lengths first where a product of two
- * operators has more than value products (as where 32-bit offsets or the memory end). */
+ * operators has more than value products (as where 32-bit offsets or the memory end).
+ * MSG_HOOK_CYCLE_LAUNCHES: V-cycles take the small levels by a launch per pass, like the larger
+ * ones. */
 enum { MSG_HOOK_SWEEP_LAUNCH = 0, MSG_HOOK_SWEEP_WITHHOLD = 1, MSG_HOOK_AMG_ALLOC = 2, MSG_HOOK_AMG_PRODUCTS = 3,
-       MSG_HOOK_COUNT };
+       MSG_HOOK_CYCLE_LAUNCHES = 4, MSG_HOOK_COUNT };
 MSG_API int msg_gpu_test_hook(msg_ctx_t *ctx, int32_t hook, int32_t value);
 
 /* AMG hierarchy of the last setup (structural tests): level 0 is the current Jacobian in CSR

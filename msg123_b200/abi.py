@@ -15,7 +15,7 @@ MSG_ERR_ARG = -1
 MSG_ERR_CUDA = -2
 MSG_ERR_SIZE = -3
 MSG_ERR_STATE = -4
-HOOK_SWEEP_LAUNCH, HOOK_SWEEP_WITHHOLD, HOOK_AMG_ALLOC, HOOK_AMG_PRODUCTS = 0, 1, 2, 3
+HOOK_SWEEP_LAUNCH, HOOK_SWEEP_WITHHOLD, HOOK_AMG_ALLOC, HOOK_AMG_PRODUCTS, HOOK_CYCLE_LAUNCHES = range(5)
 
 STATUS_NAMES = {
     MSG_OK: "ok", MSG_NEWTON_MAXIT: "newton_maxit", MSG_NAN: "nan",

@@ -2521,7 +2521,7 @@ int amg_setup(msg_ctx *c) {
 static int cycle_tail(msg_ctx *c, int l, int *done) {
   AmgState *A = S(c);
   *done = 0;
-  if (!tail_takes(A, l)) return MSG_OK;
+  if (c->hook[MSG_HOOK_CYCLE_LAUNCHES] || !tail_takes(A, l)) return MSG_OK;
   TailArgs a;
   a.nl = (int)A->lv.size() - l;
   a.sweeps = std::max(c->prm.amg_sweeps, 0);
@@ -2536,7 +2536,7 @@ static int cycle_tail(msg_ctx *c, int l, int *done) {
 }
 static int cycle_tail_f(msg_ctx *c, int l, int *done) {
   AmgState *A = S(c);
-  *done = l == A->tail_level;
+  *done = l == A->tail_level && !c->hook[MSG_HOOK_CYCLE_LAUNCHES];
   if (!*done) return MSG_OK;
   A->tail.sweeps = std::max(c->prm.amg_sweeps, 0);
   A->tail.w = c->prm.smooth_omega;

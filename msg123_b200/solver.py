@@ -386,7 +386,7 @@ class GpuSolver:
         return out, total.value
 
     def test_hook(self, hook, value):
-        """Test hook (abi.HOOK_*): a failure made on the host; value 0 switches it off."""
+        """Test hook (abi.HOOK_*): a failure made on the host, or a path; value 0 switches it off."""
         _check(load_library().msg_gpu_test_hook(self.h, int(hook), int(value)), "test_hook")
 
     def set_timing(self, on=True):
