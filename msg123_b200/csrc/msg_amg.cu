@@ -2847,15 +2847,12 @@ MSG_API int msg_gpu_amg_level(msg_ctx_t *c, int32_t lv, int32_t *offind, int32_t
   if (offrow) MSG_CUDA(cudaMemcpy(offrow, L.col, (size_t)L.nnz * 4, cudaMemcpyDeviceToHost));
   if (dmat) MSG_CUDA(cudaMemcpy(dmat, L.diag, (size_t)L.n * 8, cudaMemcpyDeviceToHost));
   if (lumat && lv == 0) {   // the Jacobian's bands in CSR order
-    double *v = nullptr;
-    MSG_CUDA(cudaMalloc(&v, (size_t)L.nnz * 8));
-    int rc = launch_dia_to_csr(c, v);
-    if (!rc) {
-      MSG_CUDA(cudaStreamSynchronize(c->stream));
-      MSG_CUDA(cudaMemcpy(lumat, v, (size_t)L.nnz * 8, cudaMemcpyDeviceToHost));
-    }
-    cudaFree(v);
+    const CsrParts parts = csr_parts(c);
+    int rc = launch_dia_to_csr(c, parts);
     if (rc) return rc;
+    MSG_CUDA(cudaStreamSynchronize(c->stream));
+    for (int k = 0; k < parts.n; ++k)
+      MSG_CUDA(cudaMemcpy(lumat + parts.first[k], parts.v[k], (size_t)(parts.first[k + 1] - parts.first[k]) * 8, cudaMemcpyDeviceToHost));
   } else if (lumat) {
     MSG_CUDA(cudaMemcpy(lumat, L.val, (size_t)L.nnz * 8, cudaMemcpyDeviceToHost));
   }

@@ -60,13 +60,15 @@ __global__ void k_to_f32(size_t n, const double *a, float *b) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     b[i] = (float)a[i];
 }
-__global__ void k_csr_to_dia(int nx, int ny, int nz, const int *offind, const double *lumat, double *lu) {
+__global__ void k_csr_to_dia(int nx, int ny, int nz, const int *offind, CsrParts parts, double *lu) {
   int N = nx * ny * nz, nxy = nx * ny;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   int iz = i / nxy, rem = i - iz * nxy, iy = rem / nx, ix = rem - iy * nx;
   const bool has[6] = {iz > 0, iy > 0, ix > 0, ix < nx - 1, iy < ny - 1, iz < nz - 1};
-  int k = offind[i];
+  const int part = i / parts.per;
+  const double *lumat = parts.v[part];
+  int k = offind[i] - parts.first[part];
   for (int d = 0; d < 6; ++d) lu[(size_t)d * N + i] = has[d] ? lumat[k++] : 0.0;
 }
 
@@ -821,12 +823,6 @@ int msg_gpu_calc_func(msg_ctx_t *c, const double *infx, double *funcv) {
   return MSG_OK;
 }
 
-// Device scratch for off-diagonals in CSR order, made by the first call that passes them.
-static int csr_scratch(msg_ctx *c) {
-  if (!c->csr_tmp) ALLOC(c->csr_tmp, (size_t)std::max(c->nnz, 1) * 8);
-  return MSG_OK;
-}
-
 int msg_gpu_make_matvec(msg_ctx_t *c, double *dmat, double *lumat, double *rhs) {
   if (!c) return MSG_ERR_ARG;
   c->amg_force = 1;   // a direct call always rebuilds the hierarchy
@@ -834,12 +830,16 @@ int msg_gpu_make_matvec(msg_ctx_t *c, double *dmat, double *lumat, double *rhs) 
   int rc = make_matvec(c, &l2, false);
   if (rc) return rc;
   size_t N = c->N;
+  CopyOut jobs[CsrParts::kMax + 2] = {{dmat, c->dmat, N * 8}, {rhs, c->rhs, N * 8}};
+  int n = 2;
   if (lumat) {
-    if ((rc = csr_scratch(c)) || (rc = launch_dia_to_csr(c, c->csr_tmp))) return rc;
+    const CsrParts parts = csr_parts(c);
+    if ((rc = launch_dia_to_csr(c, parts))) return rc;
+    for (int k = 0; k < parts.n; ++k)
+      jobs[n++] = CopyOut{lumat + parts.first[k], parts.v[k], (size_t)(parts.first[k + 1] - parts.first[k]) * 8};
   }
   MSG_CUDA(cudaStreamSynchronize(c->stream));
-  const CopyOut jobs[3] = {{lumat, c->csr_tmp, (size_t)c->nnz * 8}, {dmat, c->dmat, N * 8}, {rhs, c->rhs, N * 8}};
-  return copy_out(jobs, 3);
+  return copy_out(jobs, n);
 }
 
 int msg_gpu_set_system(msg_ctx_t *c, const double *dmat, const double *lumat, const double *rhs) {
@@ -847,10 +847,11 @@ int msg_gpu_set_system(msg_ctx_t *c, const double *dmat, const double *lumat, co
   size_t N = c->N;
   UPLOAD(c->dmat, dmat, N * 8);
   UPLOAD(c->rhs, rhs, N * 8);
-  int rc = csr_scratch(c);
-  if (rc) return rc;
-  UPLOAD(c->csr_tmp, lumat, (size_t)c->nnz * 8);
-  k_csr_to_dia<<<nblk(c->N), kThreads, 0, c->stream>>>(c->nx, c->ny, c->nz, c->offind, c->csr_tmp, c->lu);
+  int rc;
+  const CsrParts parts = csr_parts(c);
+  for (int k = 0; k < parts.n; ++k)
+    UPLOAD(parts.v[k], lumat + parts.first[k], (size_t)(parts.first[k + 1] - parts.first[k]) * 8);
+  k_csr_to_dia<<<nblk(c->N), kThreads, 0, c->stream>>>(c->nx, c->ny, c->nz, c->offind, parts, c->lu);
   MSG_CHECK_LAUNCH();
   if (c->dmat_f) {
     k_to_f32<<<kRedBlocks, kThreads, 0, c->stream>>>(N, c->dmat, c->dmat_f);
@@ -1266,7 +1267,7 @@ static void free_ctx(msg_ctx *c) {
                 c->left_off, c->right_off, c->hydf_conn, c->abyd_conn, c->head_new, c->head_old, c->head_pre,
                 c->head_change, c->srat_new, c->srat_old, c->surf_head, c->surf_old, c->new_f, c->kr, c->kr_per,
                 c->alp, c->sto, c->stod, c->tmpv, c->dmat, c->lu, c->rhs, c->rhs_alt, c->head_old2, c->slope_rhs, c->dilu_d, c->r, c->rs,
-                c->p, c->v, c->t, c->z, c->part, c->scan_sums, c->csr_tmp, c->fin_scratch, c->fin_cnt, c->wave_order, c->wave_ticket, c->wave_slots, c->dmat_f, c->lu_f, c->dres};
+                c->p, c->v, c->t, c->z, c->part, c->scan_sums, c->fin_scratch, c->fin_cnt, c->wave_order, c->wave_ticket, c->wave_slots, c->dmat_f, c->lu_f, c->dres};
   for (auto q : dp) if (q) cudaFree(q);
   if (c->hpin) cudaFreeHost(c->hpin);
   for (int k = 0; k < 8; ++k) if (c->ev[k]) cudaEventDestroy(c->ev[k]);

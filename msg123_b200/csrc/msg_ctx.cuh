@@ -55,7 +55,6 @@ struct msg_ctx {
   // ---- reference CSR built on the GPU (export / tests) -------------------------------
   int *offind, *offrow, *conn_dir, *left_off, *right_off;
   double *hydf_conn, *abyd_conn;
-  double *csr_tmp;                               // [nnz] off-diagonals on their way in or out (lazily)
   // ---- state -------------------------------------------------------------------------
   double *head_new, *head_old, *head_pre, *head_change, *srat_new, *srat_old, *head_old2;
   double *surf_head, *surf_old, *new_f;
@@ -142,7 +141,15 @@ int launch_calc_func(msg_ctx *c, double *h, double *F, bool norm, int slot = 0, 
 // ||F||^2 into dres[slot], as above; rhs_out null: c->rhs
 int launch_make_matvec(msg_ctx *c, bool reuse = false, double *rhs_out = nullptr, int slot = 0, int count = 0);
 // Export the DIA Jacobian into the reference CSR order.
-int launch_dia_to_csr(msg_ctx *c, double *lumat_dev);
+// Off-diagonals in CSR order on their way in or out: in pieces in the vectors of a solve, which
+// holds none between calls.  Cell i's are in v[i / per], whose first entry is first[i / per].
+struct CsrParts {
+  static constexpr int kMax = 7;
+  double *v[kMax];
+  int first[kMax + 1], per, n;
+};
+CsrParts csr_parts(const msg_ctx *c);
+int launch_dia_to_csr(msg_ctx *c, const CsrParts &parts);
 int launch_mass(msg_ctx *c, double out9[9]);
 int launch_velocity(msg_ctx *c, double *const out[9]);   // six faces, then x, y, z
 int launch_cell_mass(msg_ctx *c, double *sto, double *con, double *sea, double *wel, double *rec, double *sur,
