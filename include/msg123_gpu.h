@@ -378,6 +378,8 @@ MSG_API int msg_gpu_cnn_set_weights(msg_cnn_t *cnn, const float *w);
 /* append a training sample from a context right after an accepted step */
 MSG_API int msg_gpu_cnn_collect(msg_cnn_t *cnn, msg_ctx_t *ctx);
 MSG_API int msg_gpu_cnn_nsamples(msg_cnn_t *cnn);
+/* cells of stored sample `sample` (a negative status: no such sample) */
+MSG_API int msg_gpu_cnn_sample_cells(msg_cnn_t *cnn, int32_t sample);
 /* bound the sample store to cap samples (0: unbounded): once full, each collected step
    replaces a uniformly drawn stored sample with probability cap / (steps collected), so the
    store stays a uniform sample of every step seen (reservoir sampling; seed seeds the draws) */

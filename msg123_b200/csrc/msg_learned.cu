@@ -778,6 +778,11 @@ MSG_API int msg_gpu_cnn_add_sample(msg_cnn_t *h, int32_t nx, int32_t ny, int32_t
   return MSG_OK;
 }
 
+// Cells of stored sample `sample` (MSG_ERR_ARG: no such sample).
+MSG_API int msg_gpu_cnn_sample_cells(msg_cnn_t *h, int32_t sample) {
+  return h && sample >= 0 && sample < (int)h->net.data.size() ? h->net.data[sample].g.N : MSG_ERR_ARG;
+}
+
 // Loss (mean squared error) and optionally the gradient (host, kNParam floats) on one sample.
 MSG_API int msg_gpu_cnn_loss_grad(msg_cnn_t *h, int32_t sample, double *loss, float *grad, float *out) {
   if (!h || sample < 0 || sample >= (int)h->net.data.size()) return MSG_ERR_ARG;

@@ -35,6 +35,7 @@ def _lib():
         L.msg_gpu_cnn_seen.argtypes = [vp]
         L.msg_gpu_cnn_seen.restype = C.c_longlong
         L.msg_gpu_cnn_add_sample.argtypes = [vp, C.c_int32, C.c_int32, C.c_int32, abi.PF, abi.PF]
+        L.msg_gpu_cnn_sample_cells.argtypes = [vp, C.c_int32]
         L.msg_gpu_cnn_loss_grad.argtypes = [vp, C.c_int32, abi.PD, abi.PF, abi.PF]
         L.msg_gpu_cnn_infer.argtypes = [vp, C.c_int32, abi.PF]
         L.msg_gpu_cnn_infer_withhold.argtypes = [vp, C.c_int32, C.c_int32, abi.PF]
@@ -98,17 +99,23 @@ class Cnn:
         y = np.ascontiguousarray(y, dtype=np.float32)
         _check(_lib().msg_gpu_cnn_add_sample(self.h, nx, ny, nz, abi.fptr(x), abi.fptr(y)), "cnn_add_sample")
 
+    def _output(self, sample, n):
+        """Array for a sample's output: zero behind its cells, the rest is written by the call."""
+        o = np.empty(n, np.float32)
+        o[max(_lib().msg_gpu_cnn_sample_cells(self.h, int(sample)), 0):] = 0.0
+        return o
+
     def loss_grad(self, sample=0, want_grad=True, want_out=False, n=None):
         loss = C.c_double()
         g = np.zeros(self.nparam, np.float32) if want_grad else None
-        o = np.empty(n, np.float32) if want_out else None
+        o = self._output(sample, n) if want_out else None
         _check(_lib().msg_gpu_cnn_loss_grad(self.h, int(sample), C.byref(loss), abi.fptr(g), abi.fptr(o)),
                "cnn_loss_grad")
         return loss.value, g, o
 
     def infer(self, sample, n):
         """Output of the tensor-core (tcgen05) inference path on stored sample `sample`."""
-        o = np.empty(n, np.float32)
+        o = self._output(sample, n)
         _check(_lib().msg_gpu_cnn_infer(self.h, int(sample), abi.fptr(o)), "cnn_infer")
         return o
 
