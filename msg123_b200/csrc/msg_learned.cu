@@ -21,6 +21,7 @@
 #include <cuda_bf16.h>
 #include <vector>
 #include <mutex>
+#include <new>
 #include <cmath>
 #include <algorithm>
 
@@ -620,11 +621,7 @@ using namespace msg;
 
 extern "C" {
 
-MSG_API int msg_gpu_cnn_create(int32_t seed, msg_cnn_t **out) {
-  if (!out) return MSG_ERR_ARG;
-  msg_cnn *h = new msg_cnn();
-  Net &n = h->net;
-  stage_ref();
+static int cnn_init(Net &n, int32_t seed) {
   MSG_CUDA(cudaStreamCreateWithFlags(&n.stream, cudaStreamNonBlocking));
   MSG_CUDA(cudaMalloc(&n.w32, kNParam * 4));
   MSG_CUDA(cudaMalloc(&n.m, kNParam * 4));
@@ -659,20 +656,30 @@ MSG_API int msg_gpu_cnn_create(int32_t seed, msg_cnn_t **out) {
   int rc = cnn_pack(n);
   if (rc) return rc;
   MSG_CUDA(cudaStreamSynchronize(n.stream));
-  *out = h;
   return MSG_OK;
+}
+
+MSG_API int msg_gpu_cnn_create(int32_t seed, msg_cnn_t **out) {
+  if (!out) return MSG_ERR_ARG;
+  msg_cnn *h = new (std::nothrow) msg_cnn();
+  if (!h) { set_error("out of host memory"); return MSG_ERR_ARG; }
+  stage_ref();
+  int rc = cnn_init(h->net, seed);
+  if (rc) msg_gpu_cnn_destroy(h);
+  else *out = h;
+  return rc;
 }
 
 MSG_API void msg_gpu_cnn_destroy(msg_cnn_t *h) {
   if (!h) return;
   Net &n = h->net;
-  cudaStreamSynchronize(n.stream);
+  if (n.stream) cudaStreamSynchronize(n.stream);
   void *p[] = {n.w32, n.w16, n.wt16, n.wtc, n.m, n.v, n.grad, n.part, n.dz, n.dz2, n.loss_part};
   conv_plan_free(n.plan);
   for (void *q : p) if (q) cudaFree(q);
   for (int l = 0; l < kLayers; ++l) { if (n.a[l]) cudaFree(n.a[l]); if (n.z[l]) cudaFree(n.z[l]); }
   for (auto &smp : n.data) { cudaFree(smp.x); cudaFree(smp.y); }
-  cudaStreamDestroy(n.stream);
+  if (n.stream) cudaStreamDestroy(n.stream);
   stage_unref();
   delete h;
 }
