@@ -15,10 +15,10 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstring>
+#include <exception>
 #include <memory>
 #include <mutex>
 #include <new>
-#include <system_error>
 #include <thread>
 
 namespace msg {
@@ -117,7 +117,7 @@ struct Stage {
     const int want = std::max(1, std::min<int>(kMaxThreads, (int)std::thread::hardware_concurrency() - 1));
     try {
       for (; nthreads < want; ++nthreads) thread[nthreads] = std::thread(&Stage::serve, this, nthreads);
-    } catch (const std::system_error &) {   // as many as the system gives
+    } catch (const std::exception &) {   // as many as the system gives (no thread, no memory)
     }
     return true;
   }
