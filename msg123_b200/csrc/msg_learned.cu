@@ -440,22 +440,26 @@ __global__ void __launch_bounds__(256) k_sumsq_diff(int n, const double *a, cons
 // ---------------------------------------------------------------------------------
 static int cnn_reserve(Net &n, int N) {
   if (n.cap >= N) return MSG_OK;
+  n.cap = 0;                              // until all of them are there
+  auto drop = [](auto *&p) {
+    if (p) cudaFree(p);
+    p = nullptr;
+  };
+  for (int l = 0; l < kLayers; ++l) { drop(n.a[l]); drop(n.z[l]); }
+  drop(n.dz);
+  drop(n.dz2);
   for (int l = 0; l < kLayers; ++l) {
-    if (n.a[l]) cudaFree(n.a[l]);
-    if (n.z[l]) cudaFree(n.z[l]);
     MSG_CUDA(cudaMalloc(&n.a[l], (size_t)N * kC * 2));
     MSG_CUDA(cudaMalloc(&n.z[l], (size_t)N * kC * 4));
   }
-  if (n.dz) cudaFree(n.dz);
-  if (n.dz2) cudaFree(n.dz2);
   MSG_CUDA(cudaMalloc(&n.dz, (size_t)N * kC * 2));
   MSG_CUDA(cudaMalloc(&n.dz2, (size_t)N * kC * 2));
   if (!n.part) {
-    MSG_CUDA(cudaMalloc(&n.part, ((size_t)2 * kWgBlocks * kWl + kWgBlocks * kC) * 4));
     MSG_CUDA(cudaFuncSetAttribute(k_conv<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSmem));
     MSG_CUDA(cudaFuncSetAttribute(k_conv<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSmem));
     MSG_CUDA(cudaFuncSetAttribute(k_conv<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSmem));
     MSG_CUDA(cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem));
+    MSG_CUDA(cudaMalloc(&n.part, ((size_t)2 * kWgBlocks * kWl + kWgBlocks * kC) * 4));
   }
   n.cap = N;
   return MSG_OK;
