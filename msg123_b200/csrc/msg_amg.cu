@@ -39,7 +39,7 @@ struct AmgLevel {
   double *cinv = nullptr;                 // dense inverse (coarsest level only)
   double *x = nullptr, *b = nullptr, *r = nullptr, *x2 = nullptr;
   // mixed precision images
-  float *diag_f = nullptr, *val_f = nullptr, *pval_f = nullptr, *rval_f = nullptr;
+  float *diag_f = nullptr, *pval_f = nullptr, *rval_f = nullptr;
   __nv_bfloat16 *val_h = nullptr;
   float *xf = nullptr, *bf = nullptr, *rf = nullptr, *x2f = nullptr;
   void *pack = nullptr;                   // rows of this and the following levels for k_cycle_tail_f
@@ -2058,7 +2058,7 @@ static void hfree(AmgState *A, void *q, cudaStream_t s) {
 
 static void free_level(AmgState *A, AmgLevel &L, cudaStream_t s) {
   void *p[] = {L.rowptr, L.col, L.diag, L.val, L.pptr, L.pcol, L.pval, L.rptr, L.rcol, L.rval, L.agg, L.cinv,
-               L.x, L.b, L.r, L.x2, L.diag_f, L.val_f, L.pval_f, L.rval_f, L.val_h, L.xf, L.bf, L.rf, L.x2f, L.pack};
+               L.x, L.b, L.r, L.x2, L.diag_f, L.pval_f, L.rval_f, L.val_h, L.xf, L.bf, L.rf, L.x2f, L.pack};
   for (void *q : p) hfree(A, q, s);
   L = AmgLevel();
 }
@@ -2183,8 +2183,10 @@ static int coarsen(msg_ctx *c, AmgState *A, int lv, int *made) {
         cudaLaunchConfig_t cf = {};
         cf.gridDim = dim3(kMisCluster); cf.blockDim = dim3(kMisBlock); cf.stream = s; cf.attrs = &at; cf.numAttrs = 1;
         MSG_CUDA(cudaLaunchKernelExC(&cf, (const void *)k_mis_csr<true>, args));
-      } else
-      MSG_CUDA(cudaLaunchCooperativeKernel((void *)k_mis_csr<false>, (int)std::min((4 * (long long)n + kMisBlock - 1) / kMisBlock, (long long)A->mis_csr), kMisBlock, args, 0, s));
+      } else {
+        const int g = (int)std::min((4 * (long long)n + kMisBlock - 1) / kMisBlock, (long long)A->mis_csr);
+        MSG_CUDA(cudaLaunchCooperativeKernel((void *)k_mis_csr<false>, g, kMisBlock, args, 0, s));
+      }
     }
     __atomic_fetch_add(&g_launches, 1LL, __ATOMIC_RELAXED);
   }

@@ -69,11 +69,4 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
   return r;   // valid in thread 0
 }
 
-// Sum a partials array of fixed length in index order (one thread).
-__device__ __forceinline__ double sum_partials(const double *p, int n) {
-  double s = 0.0;
-  for (int i = 0; i < n; ++i) s = __dadd_rn(s, p[i]);
-  return s;
-}
-
 }  // namespace msg

@@ -9,12 +9,6 @@ namespace msg {
 
 struct AmgLevel;   // msg_amg.cu
 
-// Scalars of the Krylov / Newton recurrences kept in device memory.
-struct DevScalars {
-  double sk, sk0, sk2, alpha, beta, omega, ts, tt, rnorm, bnorm, errtol;
-  int conv, in_iter, done, pad;
-};
-
 // Words that a kernel hands to the host: pinned memory, complete when token is the awaited one.
 struct HostBox {
   int v[4];
@@ -66,8 +60,6 @@ struct msg_ctx {
   float *dmat_f, *lu_f;                          // FP32 images (precision = 1)
   // ---- Krylov work ----------------------------------------------------------------------
   double *dilu_d, *r, *rs, *p, *v, *t, *z;
-  msg::DevScalars *sc;                           // device scalars
-  msg::DevScalars *sc_host;                      // pinned mirror
   double *part;                                  // reduction partials [npart]
   size_t npart;
   double *hpin;                                  // pinned host scalars

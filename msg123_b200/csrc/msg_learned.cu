@@ -62,8 +62,6 @@ struct Net {
   float *z[kLayers] = {nullptr, nullptr, nullptr, nullptr};           // pre-activations (z[3]: output)
   __nv_bfloat16 *dz = nullptr;         // gradient of the current layer's pre-activation [N][16]
   __nv_bfloat16 *dz2 = nullptr;
-  float *loss_part = nullptr;
-  double *hpin = nullptr;
   cudaStream_t stream = nullptr;
   std::vector<Sample> data;
   // bounded sample store: with store_cap > 0, a sample collected when the store is full
@@ -678,7 +676,7 @@ MSG_API void msg_gpu_cnn_destroy(msg_cnn_t *h) {
   if (!h) return;
   Net &n = h->net;
   if (n.stream) cudaStreamSynchronize(n.stream);
-  void *p[] = {n.w32, n.w16, n.wt16, n.wtc, n.m, n.v, n.grad, n.part, n.dz, n.dz2, n.loss_part};
+  void *p[] = {n.w32, n.w16, n.wt16, n.wtc, n.m, n.v, n.grad, n.part, n.dz, n.dz2};
   conv_plan_free(n.plan);
   for (void *q : p) if (q) cudaFree(q);
   for (int l = 0; l < kLayers; ++l) { if (n.a[l]) cudaFree(n.a[l]); if (n.z[l]) cudaFree(n.z[l]); }
