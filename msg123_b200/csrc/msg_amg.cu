@@ -2849,12 +2849,10 @@ MSG_API int msg_gpu_amg_level(msg_ctx_t *c, int32_t lv, int32_t *offind, int32_t
   if (offrow) MSG_CUDA(cudaMemcpy(offrow, L.col, (size_t)L.nnz * 4, cudaMemcpyDeviceToHost));
   if (dmat) MSG_CUDA(cudaMemcpy(dmat, L.diag, (size_t)L.n * 8, cudaMemcpyDeviceToHost));
   if (lumat && lv == 0) {   // the Jacobian's bands in CSR order
-    const CsrParts parts = csr_parts(c);
-    int rc = launch_dia_to_csr(c, parts);
+    int rc = launch_dia_to_csr(c, csr_scratch(c));
     if (rc) return rc;
     MSG_CUDA(cudaStreamSynchronize(c->stream));
-    for (int k = 0; k < parts.n; ++k)
-      MSG_CUDA(cudaMemcpy(lumat + parts.first[k], parts.v[k], (size_t)(parts.first[k + 1] - parts.first[k]) * 8, cudaMemcpyDeviceToHost));
+    MSG_CUDA(cudaMemcpy(lumat, csr_scratch(c), (size_t)L.nnz * 8, cudaMemcpyDeviceToHost));
   } else if (lumat) {
     MSG_CUDA(cudaMemcpy(lumat, L.val, (size_t)L.nnz * 8, cudaMemcpyDeviceToHost));
   }

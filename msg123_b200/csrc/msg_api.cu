@@ -60,15 +60,13 @@ __global__ void k_to_f32(size_t n, const double *a, float *b) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     b[i] = (float)a[i];
 }
-__global__ void k_csr_to_dia(int nx, int ny, int nz, const int *offind, CsrParts parts, double *lu) {
+__global__ void k_csr_to_dia(int nx, int ny, int nz, const int *offind, const double *lumat, double *lu) {
   int N = nx * ny * nz, nxy = nx * ny;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   int iz = i / nxy, rem = i - iz * nxy, iy = rem / nx, ix = rem - iy * nx;
   const bool has[6] = {iz > 0, iy > 0, ix > 0, ix < nx - 1, iy < ny - 1, iz < nz - 1};
-  const int part = i / parts.per;
-  const double *lumat = parts.v[part];
-  int k = offind[i] - parts.first[part];
+  int k = offind[i];
   for (int d = 0; d < 6; ++d) lu[(size_t)d * N + i] = has[d] ? lumat[k++] : 0.0;
 }
 
@@ -651,9 +649,16 @@ static int create_impl(msg_ctx *c, const msg_grid_t *g, const msg_params_t *p) {
   for (auto q : sz) { ALLOC(*q, S * 8); MSG_CUDA(cudaMemsetAsync(*q, 0, S * 8, c->stream)); }
   ALLOC(c->offind, (N + 1) * 4);
   double **vn[] = {&c->head_new, &c->head_old, &c->head_old2, &c->head_pre, &c->head_change, &c->srat_new, &c->srat_old,
-                   &c->new_f, &c->kr, &c->kr_per, &c->alp, &c->sto, &c->stod, &c->tmpv, &c->dmat, &c->rhs,
-                   &c->slope_rhs, &c->rhs_alt, &c->dilu_d, &c->r, &c->rs, &c->p, &c->v, &c->t, &c->z};
+                   &c->new_f, &c->kr, &c->kr_per, &c->alp, &c->sto, &c->stod, &c->dmat, &c->rhs,
+                   &c->slope_rhs, &c->rhs_alt, &c->dilu_d};
   for (auto q : vn) { ALLOC(*q, N * 8); MSG_CUDA(cudaMemsetAsync(*q, 0, N * 8, c->stream)); }
+  {   // seven in one block, each on a boundary of 256 bytes: at least the 6 N entries of csr_scratch
+    const size_t pitch = (N + 31) & ~(size_t)31;
+    double **kv[7] = {&c->r, &c->rs, &c->p, &c->v, &c->t, &c->z, &c->tmpv};
+    ALLOC(c->r, 7 * pitch * 8);
+    MSG_CUDA(cudaMemsetAsync(c->r, 0, 7 * pitch * 8, c->stream));
+    for (int k = 1; k < 7; ++k) *kv[k] = c->r + k * pitch;
+  }
   ALLOC(c->lu, 6 * N * 8);
   if (p->precision == 1) {
     ALLOC(c->dmat_f, N * 4);
@@ -830,16 +835,10 @@ int msg_gpu_make_matvec(msg_ctx_t *c, double *dmat, double *lumat, double *rhs) 
   int rc = make_matvec(c, &l2, false);
   if (rc) return rc;
   size_t N = c->N;
-  CopyOut jobs[CsrParts::kMax + 2] = {{dmat, c->dmat, N * 8}, {rhs, c->rhs, N * 8}};
-  int n = 2;
-  if (lumat) {
-    const CsrParts parts = csr_parts(c);
-    if ((rc = launch_dia_to_csr(c, parts))) return rc;
-    for (int k = 0; k < parts.n; ++k)
-      jobs[n++] = CopyOut{lumat + parts.first[k], parts.v[k], (size_t)(parts.first[k + 1] - parts.first[k]) * 8};
-  }
+  if (lumat && (rc = launch_dia_to_csr(c, csr_scratch(c)))) return rc;
   MSG_CUDA(cudaStreamSynchronize(c->stream));
-  return copy_out(jobs, n);
+  const CopyOut jobs[3] = {{lumat, csr_scratch(c), (size_t)c->nnz * 8}, {dmat, c->dmat, N * 8}, {rhs, c->rhs, N * 8}};
+  return copy_out(jobs, 3);
 }
 
 int msg_gpu_set_system(msg_ctx_t *c, const double *dmat, const double *lumat, const double *rhs) {
@@ -848,10 +847,8 @@ int msg_gpu_set_system(msg_ctx_t *c, const double *dmat, const double *lumat, co
   UPLOAD(c->dmat, dmat, N * 8);
   UPLOAD(c->rhs, rhs, N * 8);
   int rc;
-  const CsrParts parts = csr_parts(c);
-  for (int k = 0; k < parts.n; ++k)
-    UPLOAD(parts.v[k], lumat + parts.first[k], (size_t)(parts.first[k + 1] - parts.first[k]) * 8);
-  k_csr_to_dia<<<nblk(c->N), kThreads, 0, c->stream>>>(c->nx, c->ny, c->nz, c->offind, parts, c->lu);
+  UPLOAD(csr_scratch(c), lumat, (size_t)c->nnz * 8);
+  k_csr_to_dia<<<nblk(c->N), kThreads, 0, c->stream>>>(c->nx, c->ny, c->nz, c->offind, csr_scratch(c), c->lu);
   MSG_CHECK_LAUNCH();
   if (c->dmat_f) {
     k_to_f32<<<kRedBlocks, kThreads, 0, c->stream>>>(N, c->dmat, c->dmat_f);
@@ -1266,8 +1263,8 @@ static void free_ctx(msg_ctx *c) {
                 c->rech_base, c->sea_hydf, c->sea_abyd, c->read_seal, c->drain, c->offind, c->offrow, c->conn_dir,
                 c->left_off, c->right_off, c->hydf_conn, c->abyd_conn, c->head_new, c->head_old, c->head_pre,
                 c->head_change, c->srat_new, c->srat_old, c->surf_head, c->surf_old, c->new_f, c->kr, c->kr_per,
-                c->alp, c->sto, c->stod, c->tmpv, c->dmat, c->lu, c->rhs, c->rhs_alt, c->head_old2, c->slope_rhs, c->dilu_d, c->r, c->rs,
-                c->p, c->v, c->t, c->z, c->part, c->scan_sums, c->fin_scratch, c->fin_cnt, c->wave_order, c->wave_ticket, c->wave_slots, c->dmat_f, c->lu_f, c->dres};
+                c->alp, c->sto, c->stod, c->dmat, c->lu, c->rhs, c->rhs_alt, c->head_old2, c->slope_rhs, c->dilu_d, c->r,
+                c->part, c->scan_sums, c->fin_scratch, c->fin_cnt, c->wave_order, c->wave_ticket, c->wave_slots, c->dmat_f, c->lu_f, c->dres};
   for (auto q : dp) if (q) cudaFree(q);
   if (c->hpin) cudaFreeHost(c->hpin);
   for (int k = 0; k < 8; ++k) if (c->ev[k]) cudaEventDestroy(c->ev[k]);

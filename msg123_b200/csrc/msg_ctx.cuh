@@ -53,13 +53,14 @@ struct msg_ctx {
   double *head_new, *head_old, *head_pre, *head_change, *srat_new, *srat_old, *head_old2;
   double *surf_head, *surf_old, *new_f;
   double *kr, *kr_per, *alp, *sto, *stod;        // per-cell vG results / storage terms
-  double *tmpv;                                  // [N] spare vector (J.v, line search)
+  double *tmpv;                                  // [N] spare vector (J.v, line search), behind z
   // ---- level-1 system, DIA: lu[d*N + i] = J(i, nb_d(i)) --------------------------------
   double *dmat, *lu, *rhs, *slope_rhs;
   double *rhs_alt;                               // rhs assembled ahead by the line search (asm_ahead)
   float *dmat_f, *lu_f;                          // FP32 images (precision = 1)
   // ---- Krylov work ----------------------------------------------------------------------
-  double *dilu_d, *r, *rs, *p, *v, *t, *z;
+  double *dilu_d;
+  double *r, *rs, *p, *v, *t, *z;                // in one block with tmpv (csr_scratch)
   double *part;                                  // reduction partials [npart]
   size_t npart;
   double *hpin;                                  // pinned host scalars
@@ -133,15 +134,10 @@ int launch_calc_func(msg_ctx *c, double *h, double *F, bool norm, int slot = 0, 
 // ||F||^2 into dres[slot], as above; rhs_out null: c->rhs
 int launch_make_matvec(msg_ctx *c, bool reuse = false, double *rhs_out = nullptr, int slot = 0, int count = 0);
 // Export the DIA Jacobian into the reference CSR order.
-// Off-diagonals in CSR order on their way in or out: in pieces in the vectors of a solve, which
-// holds none between calls.  Cell i's are in v[i / per], whose first entry is first[i / per].
-struct CsrParts {
-  static constexpr int kMax = 7;
-  double *v[kMax];
-  int first[kMax + 1], per, n;
-};
-CsrParts csr_parts(const msg_ctx *c);
-int launch_dia_to_csr(msg_ctx *c, const CsrParts &parts);
+int launch_dia_to_csr(msg_ctx *c, double *lumat_dev);
+// Room for the off-diagonals in CSR order on their way in or out: the vectors of a solve, which
+// holds none between calls, lie one behind the other.
+inline double *csr_scratch(const msg_ctx *c) { return c->r; }
 int launch_mass(msg_ctx *c, double out9[9]);
 int launch_velocity(msg_ctx *c, double *const out[9]);   // six faces, then x, y, z
 int launch_cell_mass(msg_ctx *c, double *sto, double *con, double *sea, double *wel, double *rec, double *sur,

@@ -473,15 +473,13 @@ __global__ void __launch_bounds__(256, 5) k_flux_asm(FluxArgs a) {
 }
 
 // DIA -> reference CSR order export of lumat.
-__global__ void k_dia_to_csr(Geo g, const int *offind, const double *lu, CsrParts parts) {
+__global__ void k_dia_to_csr(Geo g, const int *offind, const double *lu, double *lumat) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= g.N) return;
   int ix, iy, iz;
   cell_ijk(g, i, ix, iy, iz);
   const bool has[6] = {iz > 0, iy > 0, ix > 0, ix < g.nx - 1, iy < g.ny - 1, iz < g.nz - 1};
-  const int part = i / parts.per;
-  double *lumat = parts.v[part];
-  int k = offind[i] - parts.first[part];
+  int k = offind[i];
   for (int d = 0; d < 6; ++d)
     if (has[d]) lumat[k++] = lu[(size_t)d * g.N + i];
 }
@@ -815,30 +813,8 @@ int launch_make_matvec(msg_ctx *c, bool reuse, double *rhs_out, int slot, int co
   return end_fin(c, a.fin, count);
 }
 
-// Entries of the CSR rows before cell i: along each axis a cell has two neighbours but for the ends.
-static int csr_before(const msg_ctx *c, int i) {
-  auto one = [](int j, int n) { return (j > 0) + (j < n - 1); };              // of a cell
-  auto all = [](int k, int n) { return k == 0 ? 0 : k - 1 + std::min(k, n - 1); };   // of k cells
-  const int iz = i / c->nxy, rem = i - iz * c->nxy, iy = rem / c->nx, ix = rem - iy * c->nx;
-  return iz * (c->ny * all(c->nx, c->nx) + c->nx * all(c->ny, c->ny)) + c->nxy * all(iz, c->nz) +
-         iy * (all(c->nx, c->nx) + c->nx * one(iz, c->nz)) + c->nx * all(iy, c->ny) +
-         all(ix, c->nx) + ix * (one(iy, c->ny) + one(iz, c->nz));
-}
-
-// A piece is N / 6 cells, so that its entries fit in a vector of N values and seven vectors hold
-// all; a small grid's go into the partials, one piece.
-CsrParts csr_parts(const msg_ctx *c) {
-  CsrParts p{{c->r, c->rs, c->p, c->v, c->t, c->z, c->tmpv}};
-  p.per = c->N / 6;
-  if (c->nnz <= kRedBlocks * 8) { p.v[0] = c->part; p.per = c->N; }
-  p.n = (c->N + p.per - 1) / p.per;
-  for (int k = 0; k < p.n; ++k) p.first[k] = csr_before(c, k * p.per);
-  p.first[p.n] = c->nnz;
-  return p;
-}
-
-int launch_dia_to_csr(msg_ctx *c, const CsrParts &parts) {
-  k_dia_to_csr<<<nblk(c->N), kThreads, 0, c->stream>>>(geo(c), c->offind, c->lu, parts);
+int launch_dia_to_csr(msg_ctx *c, double *lumat_dev) {
+  k_dia_to_csr<<<nblk(c->N), kThreads, 0, c->stream>>>(geo(c), c->offind, c->lu, lumat_dev);
   MSG_CHECK_LAUNCH();
   return MSG_OK;
 }

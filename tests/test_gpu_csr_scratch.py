@@ -1,6 +1,6 @@
-"""The Jacobian in CSR order through the vectors of a solve, in pieces: out as the oracle's bits and
-in again (the preconditioner of the system set equals the assembled one's), on grids of one cell
-to several pieces, and no device memory kept by either call."""
+"""The Jacobian in CSR order through the vectors of a solve: out as the oracle's bits and in again
+(the preconditioner of the system set equals the assembled one's), on grids of a few cells and
+of lengths between the vectors' boundaries, and no device memory kept by either call."""
 import ctypes as C
 
 import numpy as np
@@ -20,7 +20,7 @@ def _free_bytes():
 
 @pytest.mark.parametrize("shape", [(1, 1, 2), (1, 7, 1), (9, 1, 1), (3, 4, 5), (29, 29, 1), (10, 10, 9), (1, 60, 41), (37, 23, 11),
                                    (2, 3, 997)], ids=str)
-def test_csr_pieces(shape):
+def test_csr_through_solve_vectors(shape):
     from msg123_b200.solver import GpuSolver
     p = make_config("hetero", shape=shape, seed=6, precon_type=0)
     rng = np.random.default_rng(3)
