@@ -10,8 +10,8 @@
 // depend on thread scheduling.  Every summation order is fixed (see the Galerkin
 // kernel), which makes the whole hierarchy bit-identical to the CPU oracle's.
 //
-// Level 1 is the context's structured Jacobian (DIA for the V-cycle, its CSR image
-// for the setup); levels >= 2 are CSR with the diagonal held apart, as in the
+// Level 1 is the context's structured Jacobian, read as bands by the V-cycle and the
+// setup (its CSR image is made for the export only); levels >= 2 are CSR with the diagonal held apart, as in the
 // reference's array_var(level)%{dmat,lumat}.
 #include "msg_ctx.cuh"
 #include <cooperative_groups.h>
@@ -646,7 +646,8 @@ __global__ void __launch_bounds__(256) k_spg_bound(int n, Spg s, int *cnt) {
 // appends the others to `next`; the larger tables walk a list of rows and pass on to `next`
 // those whose columns fill more than three quarters of the table; the largest reports them.
 // (A list per row in which each product looks for its column took 1.5 times as long on rows
-// of 40 to 60 products and 6 times on rows of 500.)
+// of 40 to 60 products and 6 times on rows of 500.)  The short table's kernel spills 4 bytes at
+// its 40 registers.
 constexpr int kTabShort = 128, kTabMid = 256, kTabMax = 1024;
 template <int T>
 struct SpgShape {
@@ -1559,7 +1560,8 @@ __global__ void k_f2d(int n, const float *a, double *b) {
 // first level of at most kTailRows rows and back up, its barrier (a fraction of a
 // microsecond) between the passes that are launches of 4 us each otherwise.  Every row is
 // computed as by the kernels of the larger levels, in the same order.  (A persistent grid
-// over the whole chip, whose barrier costs as much as a launch, had not paid.)
+// over the whole chip, whose barrier costs as much as a launch, had not paid.)  Of the FP64
+// launch's 1024 threads the registers are 32, and the compiler spills 60 bytes.
 // ---------------------------------------------------------------------------------
 // A dense coarsest level beyond kTailDense rows wants the whole chip's bandwidth.
 constexpr int kTailRows = 8192, kTailDense = 512, kTailThreads = 1024, kTailThreadsF = 512;

@@ -457,7 +457,7 @@ __device__ __forceinline__ void flux_body(const FluxArgs &a, double *sh) {
 // L2), so by the loads that a multiprocessor has in flight: registers against blocks.  The
 // residual pass takes all six faces at once on five blocks of 256 threads (48 registers), the
 // assembly three at a time on five (six at a time on three blocks 2% slower, two at a time 2%,
-// three on four blocks 4%; one at a time, on four, 8%).  At 25.2M cells, with the pass over the
+// three on four blocks 4%; one at a time, on four, 8%); its 48 registers spill 8 bytes.  At 25.2M cells, with the pass over the
 // cells before them: residual 970 -> 842 us, assembly 1803 -> 1670 us.
 template <bool FUSE>
 __global__ void __launch_bounds__(256, 5) k_flux_res(FluxArgs a) {
