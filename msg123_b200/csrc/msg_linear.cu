@@ -729,7 +729,7 @@ int scale(msg_ctx *c, double *y, double a, int n) {
 // next sweep.  Blocks take their tiles from a counter in an order in which a tile follows
 // the two that it waits for, so they progress however many of them are resident (the last
 // block sets the counter back, so nothing on the host has to follow it).  A wait is given up
-// after kWLooks looks at its slot (about 2 s; looks, not time, so that a GPU that other
+// after kWLooks looks at its slot (about 1.5 s; looks, not time, so that a GPU that other
 // processes share, or a debugger stops, does not end it) and reported: the sweep ends with wrong
 // values, the call with an error, and the slots are emptied for the next one.
 //
